@@ -17,27 +17,26 @@
 //
 // Nonlinear weights: with s_k = eps + beta_k and t_k = s_k^2 the JS weights
 // alpha_k = d_k / t_k normalise to omega_k = d_k*prod_{j!=k} t_j / D with
-// D = sum_k d_k*prod_{j!=k} t_j, so one division per reconstruction suffices:
-//   v = (w0*n0 + w1*n1 + w2*n2) / (6*D),  w0 = d0*t1*t2, w1 = d1*t0*t2, w2 = d2*t0*t1,
-// where n_k = 6*q_k are the candidate stencils' numerators, written as
-// 6*u_j plus differences so that v = u_j + (sum w_k e_k) / (6*D).  The indicators
-// beta_k and the products t_i t_j belong to the cell, not to the face: a
-// cell's left-biased state (at its upper face) and right-biased state (at its
-// lower face) share them.
+// D = sum_k d_k*prod_{j!=k} t_j, so one division per reconstruction suffices.
+// The indicators beta_k and the products t_i t_j belong to the cell, not to
+// the face: a cell's left-biased state (at its upper face) and right-biased
+// state (at its lower face) share them, and neighbouring cells share the
+// differences they are made of (weno5_run).
 //
-// Range.  A jump J in the data gives s ~ 3 J^2 and t_i t_j ~ 20 J^8, which
-// leaves the FP32 range above J ~ 4e4 (a pressure jump of one bar in SI
-// units).  So in FP32 t_k is formed from s_k * 2^-e, with e the mean of the
-// binary exponents of the largest and the middle s_k (rounded down).  Scaling
-// by a power of two is exact and cancels in every ratio below.  With it the
-// dominant product t_max t_mid lies in [1, 64) and every FP32 denominator in
-// [0.6, 384]; the only products that can underflow are those of negligible
-// weights.  FP64 needs no scaling: its denominators lie in [6e-25, ~70 J^8].
+// Range.  The sums are formed as 4 s_k.  A jump J in the data gives 4 s ~ 13
+// J^2 and products of two squares ~ 5e3 J^8, which leaves the FP32 range
+// above J ~ 2e4 (a pressure jump of a fifth of a bar in SI units).  So in FP32
+// t_k is formed from s_k * 2^-e, with e the mean of the binary exponents of
+// the largest and the middle s_k (rounded down).  Scaling by a power of two is
+// exact and cancels in every ratio below.  With it the dominant product
+// t_max t_mid lies in [1, 64) and every FP32 denominator in [1, 640]; the only
+// products that can underflow are those of negligible weights.  FP64 needs no
+// scaling: its denominators lie in [2e-21, ~2e4 J^8].
 // Since the factor is an exact power of two, the scaled and unscaled forms
 // give the same values wherever the unscaled one stays in range; a tile whose
-// primitives are all within kUnscaledMax in magnitude (then t_i t_j < 1.3e30
-// and the numerators < 2e34, eps keeps them above 1e-24) skips the scaling
-// (`scaled` false).
+// primitives are all within kUnscaledMax in magnitude (then the products stay
+// below 4e32 and the numerators below 4e36, and eps keeps the products above
+// 2e-22) skips the scaling.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -49,14 +48,10 @@ namespace euler {
 constexpr float kUnscaledMax = 1000.0f;
 
 template <typename T> struct K {
-    static constexpr T c1312 = T(13.0 / 12.0);
-    static constexpr T quarter = T(0.25);
-    static constexpr T eps = T(1e-6);
-    static constexpr T d0 = T(0.1);
-    static constexpr T d1 = T(0.6);
-    static constexpr T d2 = T(0.3);
+    static constexpr T c133 = T(13.0 / 3.0);
+    static constexpr T eps4 = T(4e-6);
+    static constexpr T third = T(1.0 / 3.0);
     static constexpr T half = T(0.5);
-    static constexpr T six = T(6);
 };
 
 __device__ __forceinline__ double dfma(double a, double b, double c) { return fma(a, b, c); }
@@ -100,7 +95,7 @@ __device__ __forceinline__ float rsqrt_pos(float x) { return rsqrtf(x); }
 // and the middle of the three (E_max + E_mid = E0 + E1 + E2 - E_min).  The
 // exponents come from the bit patterns (integer instructions only).  A NaN
 // or infinite s gives NaN states, and so do two sums above 2^127 (~1.7e38,
-// jumps ~1e19: the factor leaves the normal range there).
+// jumps ~5e18: the factor leaves the normal range there).
 __device__ __forceinline__ float weno5_scale(float s0, float s1, float s2)
 {
     const int e0 = __float_as_int(s0) >> 23, e1 = __float_as_int(s1) >> 23, e2 = __float_as_int(s2) >> 23;
@@ -108,119 +103,43 @@ __device__ __forceinline__ float weno5_scale(float s0, float s1, float s2)
     return __int_as_float(int(unsigned(254 - ((e0 + e1 + e2 - emin) >> 1)) << 23));
 }
 
-// Differences of the 5-point stencil u0..u4 = v[j-2..j+2] of cell j: the
-// smoothness indicators and both reconstructions are written in them, and a
-// state is the cell value u2 plus a correction, so that smooth data loses no
-// digits to the cancellation inside the candidate stencils.
-template <typename T> struct Diff5 {
-    T d01, d12, d23, d34;
-};
-template <typename T> __device__ __forceinline__ Diff5<T> weno5_diff(T u0, T u1, T u2, T u3, T u4)
-{
-    return {u1 - u0, u2 - u1, u3 - u2, u4 - u3};
-}
-
-// Smoothness of cell j: with s_k = eps + beta_k and t_k = s_k^2 for the
-// stencils S0 = {j-2, j-1, j}, S1 = {j-1, j, j+1}, S2 = {j, j+1, j+2}, the
-// products p12 = t1 t2, p02 = t0 t2, p01 = t0 t1.  beta_k = 13/12 a_k^2 +
-// 1/4 b_k^2 with a0 = d12 - d01, a1 = d23 - d12, a2 = d34 - d23 and
-// b0/2 = a0/2 + d12, b1/2 = (d12 + d23)/2 (up to sign), b2/2 = a2/2 - d23.
-// They serve both states of the cell (left-biased at j+1/2, right-biased at
-// j-1/2), so a cell's indicators are computed once for its two faces.
-template <typename T>
-__device__ __forceinline__ void weno5_beta(const Diff5<T> &d, T &p12, T &p02, T &p01, bool scaled = true)
-{
-    using C = K<T>;
-    const T a0 = d.d12 - d.d01, a1 = d.d23 - d.d12, a2 = d.d34 - d.d23;
-    const T h0 = dfma(C::half, a0, d.d12);
-    const T h1 = C::half * (d.d12 + d.d23);
-    const T h2 = dfma(C::half, a2, -d.d23);
-    const T s0 = dfma(C::c1312 * a0, a0, dfma(h0, h0, C::eps));
-    const T s1 = dfma(C::c1312 * a1, a1, dfma(h1, h1, C::eps));
-    const T s2 = dfma(C::c1312 * a2, a2, dfma(h2, h2, C::eps));
-    T q0 = s0, q1 = s1, q2 = s2;
-    if constexpr (sizeof(T) == 4) { // FP32: exact power-of-two rescaling
-        if (scaled) {
-            const T sc = weno5_scale(s0, s1, s2);
-            q0 = s0 * sc;
-            q1 = s1 * sc;
-            q2 = s2 * sc;
-        }
-    }
-    const T t0 = q0 * q0, t1 = q1 * q1, t2 = q2 * q2;
-    p12 = t1 * t2;
-    p02 = t0 * t2;
-    p01 = t0 * t1;
-}
-
-// Left-biased state of cell j at j+1/2 (linear weights 1/10, 6/10, 3/10 on
-// S0, S1, S2): value = u2 + num / den.  The candidates' numerators 6 q_k are
-// 6 u2 + e_k with e0 = 5 d12 - 2 d01, e1 = d12 + 2 d23, e2 = 4 d23 - d34.
-// w1 = 0.6 p02 is the middle weight of both states of the cell.
-template <typename T>
-__device__ __forceinline__ void weno5_left(const Diff5<T> &d, T p12, T w1, T p01, T &num, T &den)
-{
-    using C = K<T>;
-    const T w0 = C::d0 * p12, w2 = C::d2 * p01;
-    const T e0 = dfma(T(-2), d.d01, T(5) * d.d12);
-    const T e1 = dfma(T(2), d.d23, d.d12);
-    const T e2 = dfma(T(4), d.d23, -d.d34);
-    num = dfma(w0, e0, dfma(w1, e1, w2 * e2));
-    den = C::six * ((w0 + w1) + w2);
-}
-
-// Right-biased state of cell j at j-1/2 (linear weights 3/10, 6/10, 1/10):
-// value = u2 + num / den with candidates 6 u2 + f_k, f0 = d01 - 4 d12,
-// f1 = -2 d12 - d23, f2 = 2 d34 - 5 d23.
-template <typename T>
-__device__ __forceinline__ void weno5_right(const Diff5<T> &d, T p12, T w1, T p01, T &num, T &den)
-{
-    using C = K<T>;
-    const T r0 = C::d2 * p12, r2 = C::d0 * p01;
-    const T f0 = dfma(T(-4), d.d12, d.d01);
-    const T f1 = dfma(T(-2), d.d12, -d.d23);
-    const T f2 = dfma(T(2), d.d34, T(-5) * d.d23);
-    num = dfma(r0, f0, dfma(w1, f1, r2 * f2));
-    den = C::six * ((r0 + w1) + r2);
-}
-
-// A reconstructed state u2 + num / den (den > 0: a sum of positive weights).
-template <typename T> __device__ __forceinline__ T weno5_value(T u2, T num, T den)
-{
-    return dfma(num, rcp_pos(den), u2);
-}
-
 // ---------------------------------------------------------------------------
-// FP32, two variables per instruction.  Blackwell executes FP32 add, multiply
-// and fused multiply-add on a pair of values per thread (PTX add/mul/fma
-// .rn.f32x2, CUDA's __fadd2_rn / __fmul2_rn / __ffma2_rn); the WENO5 formulas
-// above are evaluated for two primitive variables at once, lane x holding
-// one variable and lane y the other.  Same operations as the scalar forms,
-// one packed instruction per pair.  (The Rusanov flux stays scalar: packing
-// its left and right states measured slower, 11.9 against 12.5
-// Gcell-updates/s at 1024^3, from the moves that regroup the lanes.)
+// Reconstruction of a run of three faces.  The value type V is double, float,
+// or float2: Blackwell executes FP32 add, multiply and fused multiply-add on a
+// pair of values per thread (PTX add/mul/fma .rn.f32x2, CUDA's __fadd2_rn /
+// __fmul2_rn / __ffma2_rn), so the FP32 kernel reconstructs two primitive
+// variables per instruction, lane x holding one and lane y the other.  (The
+// Rusanov flux stays scalar: packing its left and right states measured
+// slower, 11.9 against 12.5 Gcell-updates/s at 1024^3, from the moves that
+// regroup the lanes.)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.0f), a); }
-
-struct Diff5x2 {
-    float2 d01, d12, d23, d34;
-};
-__device__ __forceinline__ Diff5x2 weno5_diff2(float2 u0, float2 u1, float2 u2, float2 u3, float2 u4)
+template <typename V> struct Scalar { using type = V; };
+template <> struct Scalar<float2> { using type = float; };
+template <typename V> __device__ __forceinline__ V vset(typename Scalar<V>::type a) { return a; }
+template <> __device__ __forceinline__ float2 vset<float2>(float a) { return make_float2(a, a); }
+template <typename V> __device__ __forceinline__ V vadd(V a, V b) { return a + b; }
+template <> __device__ __forceinline__ float2 vadd<float2>(float2 a, float2 b) { return __fadd2_rn(a, b); }
+template <typename V> __device__ __forceinline__ V vmul(V a, V b) { return a * b; }
+template <> __device__ __forceinline__ float2 vmul<float2>(float2 a, float2 b) { return __fmul2_rn(a, b); }
+template <typename V> __device__ __forceinline__ V vfma(V a, V b, V c) { return dfma(a, b, c); }
+template <> __device__ __forceinline__ float2 vfma<float2>(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+template <typename V> __device__ __forceinline__ V vsub(V a, V b) { return a - b; }
+template <> __device__ __forceinline__ float2 vsub<float2>(float2 a, float2 b)
 {
-    return {sub2(u1, u0), sub2(u2, u1), sub2(u3, u2), sub2(u4, u3)};
+    return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);
 }
+template <typename V> __device__ __forceinline__ V vrcp(V a) { return rcp_pos(a); }
+template <> __device__ __forceinline__ float2 vrcp<float2>(float2 a) { return make_float2(rcp_pos(a.x), rcp_pos(a.y)); }
 
+__device__ __forceinline__ double range_scale(double, double, double) { return 1.0; } // FP64 is not rescaled
+__device__ __forceinline__ float range_scale(float s0, float s1, float s2) { return weno5_scale(s0, s1, s2); }
 // weno5_scale for both lanes of a pair at once, from the top 7 bits of each
 // biased exponent (byte 3 of a positive float, E >> 1) packed as two 16-bit
 // halves: m = (E_max >> 1) + (E_mid >> 1) differs from (E_max + E_mid) / 2
 // by at most 1, so the dominant product t_max t_mid lies in [1/4, 256) and
 // the range note's bounds widen by a factor 4 at most.  The halves never
 // carry into each other (each stays below 2^9).
-__device__ __forceinline__ float2 weno5_scale2(float2 s0, float2 s1, float2 s2)
+__device__ __forceinline__ float2 range_scale(float2 s0, float2 s1, float2 s2)
 {
     // bytes [x.b3, 0, y.b3, 0]: selector nibbles 3, 7 pick byte 3 of each
     // word, 0xB / 0xF replicate its sign bit (0 for s > 0)
@@ -232,59 +151,79 @@ __device__ __forceinline__ float2 weno5_scale2(float2 s0, float2 s1, float2 s2)
     return make_float2(__uint_as_float(b << 23), __uint_as_float((b >> 16) << 23));
 }
 
-// weno5_beta for a pair (rescaling factors from weno5_scale2).  h2 enters
-// squared only, so its sign is dropped: h2' = d23 - a2/2.
-__device__ __forceinline__ void weno5_beta2(const Diff5x2 &d, float2 &p12, float2 &p02, float2 &p01,
-                                            bool scaled = true)
+// States at three consecutive faces of a line from its 8 cells around them,
+// u[0..7]; face i lies between cells u[i+2] and u[i+3].  wl[i]: the
+// left-biased state (of cell u[i+2]), wr[i]: the right-biased one (of cell
+// u[i+3]).
+//
+// Everything is written in differences along the line, each formed once and
+// shared by the cells that use it: first differences d, second differences
+// a_k = d_k - d_(k-1), third differences b.  With a0, a1, a2 the second
+// differences at cells j-1, j, j+1, d12 = u_j - u_(j-1), d23 = u_(j+1) - u_j
+// the smoothness sums are
+//   4 s0 = 13/3 a0^2 + (a0 + 2 d12)^2 + 4 eps,   4 s1 = 13/3 a1^2 + (d12 + d23)^2 + 4 eps,
+//   4 s2 = 13/3 a2^2 + (a2 - 2 d23)^2 + 4 eps
+// (the factor 4 cancels in the weights), so the term q = 13/3 a^2 + 4 eps of
+// a second difference serves the three cells around it.  The candidates
+// differ from the middle one by third differences only,
+//   6 q0 - 6 q1 = -2 b01,  6 q2 - 6 q1 = -b12,  b01 = a1 - a0, b12 = a2 - a1,
+// so with p12 = t1 t2 and so on, A = p12 b01 and B = p01 b12:
+//   left  = u_j + [ d12/2 + a1/3 - (A/3 + B/2) / (S + 2 p01) ],
+//   right = u_j + [-d23/2 + a1/3 + (A/2 + B/3) / (S + 2 p12) ],
+//   S = p12 + 6 p02 + p01.
+// The bracket is summed before u_j is added, so a state carries one rounding
+// at the cell value's magnitude.  Per variable and run 152 operations in
+// FP64 (reciprocals included), against 205 with each cell's differences,
+// indicators and candidates formed on their own; with the fluxes' fused sums
+// (rusanov) a step of 512^3 cells went from 54.1 to 46.6 ms in FP64, of 384^3
+// cells from 13.4 to 12.4 ms in FP32.
+template <typename V>
+__device__ __forceinline__ void weno5_run(const V (&u)[8], V (&wl)[3], V (&wr)[3], bool scaled)
 {
-    using C = K<float>;
-    const float2 a0 = sub2(d.d12, d.d01), a1 = sub2(d.d23, d.d12), a2 = sub2(d.d34, d.d23);
-    const float2 h0 = fma2(f2(C::half), a0, d.d12);
-    const float2 h1 = mul2(f2(C::half), add2(d.d12, d.d23));
-    const float2 h2 = fma2(f2(-C::half), a2, d.d23);
-    const float2 s0 = fma2(mul2(f2(C::c1312), a0), a0, fma2(h0, h0, f2(C::eps)));
-    const float2 s1 = fma2(mul2(f2(C::c1312), a1), a1, fma2(h1, h1, f2(C::eps)));
-    const float2 s2 = fma2(mul2(f2(C::c1312), a2), a2, fma2(h2, h2, f2(C::eps)));
-    float2 q0 = s0, q1 = s1, q2 = s2;
-    if (scaled) {
-        const float2 sc = weno5_scale2(s0, s1, s2);
-        q0 = mul2(s0, sc);
-        q1 = mul2(s1, sc);
-        q2 = mul2(s2, sc);
+    using T = typename Scalar<V>::type;
+    using C = K<T>;
+    V d[7], a[6], q[6], b[5];
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+        d[k] = vsub(u[k + 1], u[k]);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        a[k] = vsub(d[k + 1], d[k]);
+        q[k] = vfma(vmul(vset<V>(C::c133), a[k]), a[k], vset<V>(C::eps4));
     }
-    const float2 t0 = mul2(q0, q0), t1 = mul2(q1, q1), t2 = mul2(q2, q2);
-    p12 = mul2(t1, t2);
-    p02 = mul2(t0, t2);
-    p01 = mul2(t0, t1);
-}
-
-__device__ __forceinline__ void weno5_left2(const Diff5x2 &d, float2 p12, float2 w1, float2 p01, float2 &num,
-                                            float2 &den)
-{
-    using C = K<float>;
-    const float2 w0 = mul2(f2(C::d0), p12), w2 = mul2(f2(C::d2), p01);
-    const float2 e0 = fma2(f2(-2.0f), d.d01, mul2(f2(5.0f), d.d12));
-    const float2 e1 = fma2(f2(2.0f), d.d23, d.d12);
-    const float2 e2 = sub2(mul2(f2(4.0f), d.d23), d.d34);
-    num = fma2(w0, e0, fma2(w1, e1, mul2(w2, e2)));
-    den = mul2(f2(C::six), add2(add2(w0, w1), w2));
-}
-
-__device__ __forceinline__ void weno5_right2(const Diff5x2 &d, float2 p12, float2 w1, float2 p01, float2 &num,
-                                             float2 &den)
-{
-    using C = K<float>;
-    const float2 r0 = mul2(f2(C::d2), p12), r2 = mul2(f2(C::d0), p01);
-    const float2 f0 = fma2(f2(-4.0f), d.d12, d.d01);
-    const float2 f1 = sub2(mul2(f2(-2.0f), d.d12), d.d23);
-    const float2 g2 = fma2(f2(2.0f), d.d34, mul2(f2(-5.0f), d.d23));
-    num = fma2(r0, f0, fma2(w1, f1, mul2(r2, g2)));
-    den = mul2(f2(C::six), add2(add2(r0, w1), r2));
-}
-
-__device__ __forceinline__ float2 weno5_value2(float2 u2, float2 num, float2 den)
-{
-    return fma2(num, make_float2(rcp_pos(den.x), rcp_pos(den.y)), u2);
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+        b[k] = vsub(a[k + 1], a[k]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { // cell u[j + 2]
+        const V h0 = vfma(vset<V>(T(2)), d[j + 1], a[j]);
+        const V h1 = vadd(d[j + 1], d[j + 2]);
+        const V h2 = vfma(vset<V>(T(-2)), d[j + 2], a[j + 2]);
+        V s0 = vfma(h0, h0, q[j]), s1 = vfma(h1, h1, q[j + 1]), s2 = vfma(h2, h2, q[j + 2]);
+        if constexpr (sizeof(T) == 4) { // FP32: exact power-of-two rescaling
+            if (scaled) {
+                const V sc = range_scale(s0, s1, s2);
+                s0 = vmul(s0, sc);
+                s1 = vmul(s1, sc);
+                s2 = vmul(s2, sc);
+            }
+        }
+        const V t0 = vmul(s0, s0), t1 = vmul(s1, s1), t2 = vmul(s2, s2);
+        const V p12 = vmul(t1, t2), p02 = vmul(t0, t2), p01 = vmul(t0, t1);
+        const V A = vmul(p12, b[j]), B = vmul(p01, b[j + 1]);
+        const V S = vfma(vset<V>(T(6)), p02, vadd(p12, p01));
+        const V m = vmul(vset<V>(C::third), a[j + 1]);
+        if (j < 3) {
+            const V den = vfma(vset<V>(T(2)), p01, S);
+            const V num = vfma(vset<V>(-C::third), A, vmul(vset<V>(-C::half), B));
+            wl[j] = vadd(u[j + 2], vfma(num, vrcp(den), vfma(vset<V>(C::half), d[j + 1], m)));
+        }
+        if (j > 0) {
+            const V den = vfma(vset<V>(T(2)), p12, S);
+            const V num = vfma(vset<V>(C::third), B, vmul(vset<V>(C::half), A));
+            wr[j - 1] = vadd(u[j + 2], vfma(num, vrcp(den), vfma(vset<V>(-C::half), d[j + 2], m)));
+        }
+    }
 }
 
 // Twice the Rusanov flux through a face with normal direction `d` (0,1,2)
@@ -307,27 +246,22 @@ __device__ __forceinline__ void rusanov(const T (&WL)[5], const T (&WR)[5], int 
     const T cl = gpl * rsqrt_pos(gpl * rl);
     const T cr = gpr * rsqrt_pos(gpr * rr);
     const T a = dmax(dabs(unl) + cl, dabs(unr) + cr);
-    // mass
+    // per variable (fL + fR) - a (UR - UL), products of one side fused onto
+    // those of the other
     const T fl0 = rl * unl, fr0 = rr * unr;
     F[0] = dfma(-a, rr - rl, fl0 + fr0);
     // momentum: flux = mass flux * velocity (+ p along the normal)
 #pragma unroll
     for (int k = 1; k <= 3; ++k) {
-        const T ml = rl * WL[k], mr = rr * WR[k];
-        T fl = fl0 * WL[k], fr = fr0 * WR[k];
-        if (k - 1 == d) {
-            fl = fl + pl;
-            fr = fr + pr;
-        }
-        F[k] = dfma(-a, mr - ml, fl + fr);
+        const T f = dfma(fl0, WL[k], k - 1 == d ? pl : T(0)) + dfma(fr0, WR[k], k - 1 == d ? pr : T(0));
+        F[k] = dfma(-a, dfma(rr, WR[k], -(rl * WL[k])), f);
     }
     // energy
     const T kel = dfma(WL[1], WL[1], dfma(WL[2], WL[2], WL[3] * WL[3]));
     const T ker = dfma(WR[1], WR[1], dfma(WR[2], WR[2], WR[3] * WR[3]));
     const T El = dfma(C::half * rl, kel, pl * igm1);
     const T Er = dfma(C::half * rr, ker, pr * igm1);
-    const T fl4 = (El + pl) * unl, fr4 = (Er + pr) * unr;
-    F[4] = dfma(-a, Er - El, fl4 + fr4);
+    F[4] = dfma(-a, Er - El, dfma(El + pl, unl, (Er + pr) * unr));
 }
 
 // Conservative -> primitive (rho, u, v, w, p).

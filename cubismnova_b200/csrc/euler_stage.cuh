@@ -212,120 +212,57 @@ __device__ __forceinline__ void halo_cell(int D, int i, int &x, int &y, int &z, 
     }
 }
 
-// WENO5 states along a line of a sweep: a cell's smoothness indicators serve
-// its right-biased state (lower face) and its left-biased state (upper face);
-// the left state waits in a carry for the next face.  id[0..4]: shared
-// entries of the cells a-2 .. a+2 around cell a.
-template <typename T>
-__device__ __forceinline__ T cell_left(const T *Wc, const int (&id)[5], bool scaled = true)
-{
-    const T u2 = Wc[id[2]];
-    const Diff5<T> df = weno5_diff(Wc[id[0]], Wc[id[1]], u2, Wc[id[3]], Wc[id[4]]);
-    T p12, p02, p01, nl, dl;
-    weno5_beta(df, p12, p02, p01, scaled);
-    weno5_left(df, p12, K<T>::d1 * p02, p01, nl, dl);
-    return weno5_value(u2, nl, dl);
-}
-// face a: WL = carried left state of cell a-1, WR = right state of cell a;
-// with `more` the carry becomes cell a's left state
-template <typename T>
-__device__ __forceinline__ void cell_face(const T *Wc, const int (&id)[5], bool more, T &carry, T &wl, T &wr,
-                                          bool scaled = true)
-{
-    const T u2 = Wc[id[2]];
-    const Diff5<T> df = weno5_diff(Wc[id[0]], Wc[id[1]], u2, Wc[id[3]], Wc[id[4]]);
-    T p12, p02, p01, nr, dr;
-    weno5_beta(df, p12, p02, p01, scaled);
-    const T w1 = K<T>::d1 * p02;
-    weno5_right(df, p12, w1, p01, nr, dr);
-    wr = weno5_value(u2, nr, dr);
-    wl = carry;
-    if (more) {
-        T nl, dl;
-        weno5_left(df, p12, w1, p01, nl, dl);
-        carry = weno5_value(u2, nl, dl);
-    }
-}
-__device__ __forceinline__ float2 pair_left(const float2 *P, const int (&id)[5], bool scaled)
-{
-    const float2 u2 = P[id[2]];
-    const Diff5x2 df = weno5_diff2(P[id[0]], P[id[1]], u2, P[id[3]], P[id[4]]);
-    float2 p12, p02, p01, nl, dl;
-    weno5_beta2(df, p12, p02, p01, scaled);
-    weno5_left2(df, p12, mul2(f2(K<float>::d1), p02), p01, nl, dl);
-    return weno5_value2(u2, nl, dl);
-}
-__device__ __forceinline__ void pair_face(const float2 *P, const int (&id)[5], bool more, float2 &carry, float2 &wl,
-                                          float2 &wr, bool scaled)
-{
-    const float2 u2 = P[id[2]];
-    const Diff5x2 df = weno5_diff2(P[id[0]], P[id[1]], u2, P[id[3]], P[id[4]]);
-    float2 p12, p02, p01, nr, dr;
-    weno5_beta2(df, p12, p02, p01, scaled);
-    const float2 w1 = mul2(f2(K<float>::d1), p02);
-    weno5_right2(df, p12, w1, p01, nr, dr);
-    wr = weno5_value2(u2, nr, dr);
-    wl = carry;
-    if (more) {
-        float2 nl, dl;
-        weno5_left2(df, p12, w1, p01, nl, dl);
-        carry = weno5_value2(u2, nl, dl);
-    }
-}
-
-// Carried left states of the five variables: FP64 one by one, FP32 as the
-// pairs (0,1), (2,3) and variable 4.
-struct CarryD {
-    double v[5];
-};
-struct CarryF {
-    float2 p01, p23;
-    float v4;
-};
-__device__ __forceinline__ void line_left(const double *W, const int (&id)[5], CarryD &cl, bool)
+// Left- and right-biased states of the run's three faces, all five variables;
+// at[0..7]: shared entries of the run's 8 cells.  FP32 takes the variables
+// (0, 1) and (2, 3) as pairs and variable 4 alone.
+template <typename V>
+__device__ __forceinline__ void load_run(const V *P, const int (&at)[8], V (&u)[8])
 {
 #pragma unroll
-    for (int c = 0; c < 5; ++c)
-        cl.v[c] = cell_left(W + c * Stg<double>::SV, id);
+    for (int k = 0; k < 8; ++k)
+        u[k] = P[at[k]];
 }
-__device__ __forceinline__ void line_face(const double *W, const int (&id)[5], bool more, CarryD &cl,
-                                          double (&WL)[5], double (&WR)[5], bool)
+__device__ __forceinline__ void run_states(const double *W, const int (&at)[8], double (&WL)[3][5],
+                                           double (&WR)[3][5], bool scaled)
 {
 #pragma unroll
-    for (int c = 0; c < 5; ++c)
-        cell_face(W + c * Stg<double>::SV, id, more, cl.v[c], WL[c], WR[c]);
+    for (int c = 0; c < 5; ++c) {
+        double u[8], l[3], r[3];
+        load_run(W + c * Stg<double>::SV, at, u);
+        weno5_run(u, l, r, scaled);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            WL[i][c] = l[i];
+            WR[i][c] = r[i];
+        }
+    }
 }
-__device__ __forceinline__ void line_left(const float *W, const int (&id)[5], CarryF &cl, bool scaled)
+__device__ __forceinline__ void run_states(const float *W, const int (&at)[8], float (&WL)[3][5], float (&WR)[3][5],
+                                           bool scaled)
 {
     constexpr int SV = Stg<float>::SV;
-    cl.p01 = pair_left(reinterpret_cast<const float2 *>(W), id, scaled);
-    cl.p23 = pair_left(reinterpret_cast<const float2 *>(W + 2 * SV), id, scaled);
-    cl.v4 = cell_left(W + 4 * SV, id, scaled);
+#pragma unroll
+    for (int c = 0; c < 4; c += 2) {
+        float2 u[8], l[3], r[3];
+        load_run(reinterpret_cast<const float2 *>(W + c * SV), at, u);
+        weno5_run(u, l, r, scaled);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            WL[i][c] = l[i].x;
+            WL[i][c + 1] = l[i].y;
+            WR[i][c] = r[i].x;
+            WR[i][c + 1] = r[i].y;
+        }
+    }
+    float u[8], l[3], r[3];
+    load_run(W + 4 * SV, at, u);
+    weno5_run(u, l, r, scaled);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        WL[i][4] = l[i];
+        WR[i][4] = r[i];
+    }
 }
-__device__ __forceinline__ void line_face(const float *W, const int (&id)[5], bool more, CarryF &cl,
-                                          float (&WL)[5], float (&WR)[5], bool scaled)
-{
-    constexpr int SV = Stg<float>::SV;
-    float2 l01, r01, l23, r23;
-    pair_face(reinterpret_cast<const float2 *>(W), id, more, cl.p01, l01, r01, scaled);
-    pair_face(reinterpret_cast<const float2 *>(W + 2 * SV), id, more, cl.p23, l23, r23, scaled);
-    cell_face(W + 4 * SV, id, more, cl.v4, WL[4], WR[4], scaled);
-    WL[0] = l01.x;
-    WL[1] = l01.y;
-    WL[2] = l23.x;
-    WL[3] = l23.y;
-    WR[0] = r01.x;
-    WR[1] = r01.y;
-    WR[2] = r23.x;
-    WR[3] = r23.y;
-}
-template <typename T> struct CarryOf;
-template <> struct CarryOf<double> {
-    using type = CarryD;
-};
-template <> struct CarryOf<float> {
-    using type = CarryF;
-};
 
 // Face fluxes of direction D for the whole tile, differenced into the
 // per-cell accumulators R (shared memory, the core's padded layout).  Each of
@@ -352,34 +289,18 @@ __device__ __forceinline__ void sweep(int D, const T *__restrict__ W, T *__restr
     auto sidx = [&](int a) {
         return (unsigned)a < (unsigned)TB ? cbase + a * cs : hbase + (a < 0 ? a + G : a - TB + G) * cs;
     };
-    // left-biased state of cell f0-1, the lower cell of the run's first face
-    typename CarryOf<T>::type carry;
-    // shared entries of the stencil cells a-2 .. a+2.  FP32 shifts the window
-    // by one cell per face (one new entry); FP64 recomputes it (its registers
-    // are the scarcer resource)
-    int id[5];
+    int at[8]; // shared entries of the run's cells f0-3 .. f0+4
 #pragma unroll
-    for (int k = 0; k < 5; ++k)
-        id[k] = sidx(f0 - 3 + k);
-    line_left(W, id, carry, scaled);
+    for (int k = 0; k < 8; ++k)
+        at[k] = sidx(f0 - 3 + k);
+    T WL[3][5], WR[3][5];
+    run_states(W, at, WL, WR, scaled);
     T Fq[5]; // flux of the previous face of the run
-#pragma unroll 1
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const int a = f0 + i; // face a: cells a-1 (left state carried in VL) and a
-        if constexpr (sizeof(T) == 4) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                id[k] = id[k + 1];
-            id[4] = sidx(a + 2);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 5; ++k)
-                id[k] = sidx(a - 2 + k);
-        }
-        T WL[5], WR[5];
-        line_face(W, id, i < 2, carry, WL, WR, scaled);
+        const int a = f0 + i; // face a: cells a-1 and a
         T Fl[5];
-        rusanov<T>(WL, WR, D, gamma, igm1, Fl);
+        rusanov<T>(WL[i], WR[i], D, gamma, igm1, Fl);
         if (i == 0) {
             if (run > 0) {
 #pragma unroll
