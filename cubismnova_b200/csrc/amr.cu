@@ -16,9 +16,6 @@ namespace amr {
 // Euler tiles of AMR blocks: tile index -> (block, tile of 8^3 cells); a
 // work item (a CTA's unit of work) is a run of consecutive tiles of the list
 struct Src {
-    // a level-interface ghost cell resolves its geometry once for all five
-    // components (halo5)
-    static constexpr bool kHalo5 = true;
     Geom A;
     const int2 *work;  // tiles: (block, tile index in the block)
     const int2 *items; // work items: (first tile, tile count)
@@ -36,11 +33,10 @@ struct Src {
         t.ih[0] = t.ih[1] = t.ih[2] = (T)B.ih;
         t.bx = t.by = t.bz = 0;
     }
-    template <typename T> __device__ __forceinline__ void prepare(const euler::TileInfo<T> &, int *) const {}
     // a ghost from a block on the same level is a plain copy of its cell;
-    // level-interface ghosts (prolongation, restriction) take halo()
+    // level-interface ghosts (prolongation, restriction) take halo5()
     template <typename T>
-    __device__ __forceinline__ bool plain_offset(const euler::TileInfo<T> &t, int gx, int gy, int gz, const int *,
+    __device__ __forceinline__ bool plain_offset(const euler::TileInfo<T> &t, int gx, int gy, int gz,
                                                  int64_t &off) const
     {
         return same_level_offset(A, t.block, gx, gy, gz, off);
@@ -48,7 +44,7 @@ struct Src {
     // all five components of a level-interface ghost: the geometry once
     template <typename T>
     __device__ __forceinline__ void halo5(const T *const (&U)[5], const euler::TileInfo<T> &t, int gx, int gy, int gz,
-                                          const int *, T (&v)[5]) const
+                                          T (&v)[5]) const
     {
         const Ghost g = resolve(A, t.block, gx, gy, gz);
 #pragma unroll 1
@@ -57,9 +53,8 @@ struct Src {
 };
 
 // ONE: one CTA per work item of a single tile (the schedule of one CTA per
-// item with 1x1x1 work tiles): no loop around the tile, which leaves the
-// compiler the registers the loops' state takes (FP64: 52 instead of 308
-// bytes of spill stores per thread).  Otherwise persistent: each CTA walks
+// item with 1x1x1 work tiles): no loop around the tile.  Otherwise
+// persistent: each CTA walks
 // the work items with a grid stride, the tiles of an item in order.
 template <typename T, bool ONE>
 __global__ void __launch_bounds__(euler::NT, 3) stage_kernel(euler::StageParams<T> p, Src src, int nitems)
@@ -68,16 +63,15 @@ __global__ void __launch_bounds__(euler::NT, 3) stage_kernel(euler::StageParams<
     T *W = reinterpret_cast<T *>(smem_raw);
     T *A = W + 5 * euler::Stg<T>::SV;
     __shared__ double red[euler::NT / 32][5];
-    __shared__ int snb[28];
     __shared__ euler::TileInfo<T> ts;
     if constexpr (ONE) {
         const int tile = src.items[blockIdx.x].x;
-        euler::stage_tile<T>(p, src, tile, tile, W, A, red, snb, &ts);
+        euler::stage_tile<T>(p, src, tile, W, A, red, &ts);
     } else {
         for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
             const int2 it = src.items[item];
             for (int k = 0; k < it.y; ++k)
-                euler::stage_tile<T>(p, src, it.x + k, it.x + k, W, A, red, snb, &ts);
+                euler::stage_tile<T>(p, src, it.x + k, W, A, red, &ts);
         }
     }
 }
@@ -215,11 +209,14 @@ static cn_status launch_amr_stage(cn_amr *Us, cn_amr *Un, cn_amr *out, int stage
         p.Un[c] = Un ? reinterpret_cast<const T *>(Un->d_data) + (size_t)c * Un->comp_stride : nullptr;
         p.out[c] = reinterpret_cast<T *>(out->d_data) + (size_t)c * out->comp_stride;
     }
-    p.dt = (T)dt;
+    p.dt = stage == 0 ? T(1) : (T)dt;
     p.gamma = (T)gamma;
     p.gm1 = (T)(gamma - 1.0);
     p.igm1 = (T)(1.0 / (gamma - 1.0));
-    p.stage = stage;
+    p.cn = stage < 2 ? T(0) : (stage == 2 ? T(0.75) : T(1.0 / 3.0));
+    p.cs = stage < 2 ? T(1) : (stage == 2 ? T(0.25) : T(2.0 / 3.0));
+    p.use_u = stage >= 1;
+    p.use_un = stage >= 2;
     p.partials = nullptr;
     Src src;
     src.A = geom(Us);

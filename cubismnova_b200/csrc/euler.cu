@@ -3,31 +3,32 @@
 //
 // One CTA owns an 8x8x8 tile of one block.  It stages the tile's cells of all
 // five conserved variables into shared memory as primitives (rho, u, v, w, p)
-// and, before the sweep of each direction, that direction's two 3-cell halo
-// slabs (together the lab of a stencil (-3,4) non-tensorial,
-// Block/FieldLab.h:180-224): halo cells inside the block are plain loads,
-// cells outside are resolved by cn::lab_value (periodic neighbour, skip rule
-// and BC chain of each component's BC vector).  Per direction every face flux
-// of the tile is computed exactly once (runs of three faces per thread, each
-// cell's WENO5 smoothness indicators shared by its two faces, Rusanov) and
-// differenced into per-cell accumulators in shared memory.  The epilogue
+// with the tile's six 3-cell side slabs (together the lab of a stencil (-3,4)
+// non-tensorial, Block/FieldLab.h:180-224).  Per direction every face flux of
+// the tile is computed exactly once (runs of three faces per thread, Rusanov)
+// and differenced into per-cell accumulators in shared memory.  The epilogue
 // applies the SSP-RK3 (Shu & Osher 1988) convex combination and optionally
 // accumulates FP64 conservation sums per CTA (reduced in a fixed order by a
 // second kernel, so the sums are deterministic).
 //
-// The tile's cells of all five components arrive in shared memory by one TMA
-// copy (a 5-D tensor map over the state, cuTensorMapEncodeTiled) while the
-// threads stage the halo slabs; they are then converted to primitives.
+// Staging is by TMA: one warp finds the tile and starts the copies of its
+// cells and of the sides that are plain copies of cells of one block (tensor
+// maps over the state, cuTensorMapEncodeTiled); sides behind faces with BCs
+// are filled by the rule of the face.  FP64 brings the y and z sides while the
+// sweep before them runs; FP32 brings everything at once.  Bound by the FP64
+// pipe's latency (64 % active) and the FP32 issue slots (71 %); one RK3 step
+// of 512^3 cells takes 37.3 ms in FP64 (46.6 with halo cells loaded one by
+// one by the threads), of 384^3 cells 9.0 ms in FP32 (12.4).
 //
-// Shared memory per CTA: 5 x 1024 primitives (the tile plus one direction's
-// halo slabs, restaged before each sweep; FP32 keeps all three directions'
-// slabs) + 5 x 704 accumulators and exchanged face fluxes (the TMA landing
-// area of the tile's conservative cells before the sweeps).
+// Shared memory per CTA: 5 x 1280 primitives (FP32: 5 x 1664; the tile and its
+// halo slots) + 5 x 512 accumulators (the landing area of the tile's
+// conservative cells before the sweeps).
 #include "cn_internal.h"
 #include "cn_tma.cuh"
 #include "euler_math.cuh"
 #include "euler_stage.cuh"
 
+#include <algorithm>
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cstring>
@@ -37,8 +38,8 @@ namespace cn {
 namespace euler {
 
 // Dynamic shared memory, from its first 128-byte aligned address: W
-// [5][Stg<T>::SV], then A [5][NACC] from a 128-byte aligned offset (the TMA
-// destination of the tile's cells); 128 bytes of slack for the alignment.
+// [5][Stg<T>::SV], then A [5][NACC] from a 128-byte aligned offset; 128 bytes
+// of slack for the alignment.
 template <typename T> constexpr size_t acc_offset()
 {
     return (5 * Stg<T>::SV * sizeof(T) + 127) / 128 * 128;
@@ -50,21 +51,15 @@ template <typename T> constexpr size_t stage_smem()
 
 template <typename T>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 3)
-    stage_kernel(StageParams<T> p, CartSrc src, const __grid_constant__ CUtensorMap core)
+    stage_kernel(const __grid_constant__ StageParams<T> p, const __grid_constant__ CartSrc src,
+                 const __grid_constant__ TileMaps maps)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-    T *W = reinterpret_cast<T *>(base);                    // [5][Stg<T>::SV]
-    T *A = reinterpret_cast<T *>(base + acc_offset<T>()); // [5][NACC]
-    __shared__ double red[NT / 32][5];
-    __shared__ int snb[29];
-    __shared__ TileInfo<T> ts;
-    __shared__ __align__(8) uint64_t core_bar;
-    if (threadIdx.x == 0) {
-        mbar_init(&core_bar, 1);
-        fence_mbar_init();
-    }
-    stage_tile<T, CartSrc, true>(p, src, blockIdx.x, blockIdx.x, W, A, red, snb, &ts, &core, &core_bar);
+    T *W = reinterpret_cast<T *>(base);
+    T *A = reinterpret_cast<T *>(base + acc_offset<T>());
+    __shared__ __align__(8) unsigned char sh[sizeof(TileShared<T>)];
+    stage_tile_tma<T>(p, src, maps, W, A, *reinterpret_cast<TileShared<T> *>(sh));
 }
 
 // Fixed-order reduction of per-CTA partials: out[c] = sum_i partials[i][c].
@@ -140,18 +135,18 @@ static bool same_shape(const cn_grid *a, const cn_grid *b)
            a->n[2] == b->n[2] && a->dtype == b->dtype && a->block_stride == b->block_stride;
 }
 
-// Tensor map of the five components cs..cs+4 of grid g as the 5-D array
-// [comp][block][z][y][x] (innermost first: x, y, z, block, comp), box
-// 8 x 8 x 8 x 1 x 5: one TMA copy brings a tile's cells of all components.
-// Strides are byte multiples of 16 (block storage is padded to 32 bytes).
-static cn_status core_map(const cn_grid *g, int cs, size_t es, CUtensorMap *m)
+// Tensor maps of the five components cs..cs+4 of grid g as the 5-D array
+// [comp][block][z][y][x] (innermost first: x, y, z, block, comp), the sides'
+// boxes of nc components.  Strides are byte multiples of 16 (block storage is padded to
+// 32 bytes).
+static cn_status tile_maps(const cn_grid *g, int cs, size_t es, cuuint32_t nc, TileMaps *m)
 {
     void *base = static_cast<char *>(g->d_data) + (size_t)cs * g->comp_stride * es;
     const cuuint64_t dims[5] = {(cuuint64_t)g->n[0], (cuuint64_t)g->n[1], (cuuint64_t)g->n[2],
                                 (cuuint64_t)g->nblocks, 5};
     const cuuint64_t strides[4] = {(cuuint64_t)g->n[0] * es, (cuuint64_t)g->n[0] * g->n[1] * es,
                                    (cuuint64_t)g->block_stride * es, (cuuint64_t)g->comp_stride * es};
-    const cuuint32_t box[5] = {TB, TB, TB, 1, 5};
+    const cuuint32_t boxes[4][5] = {{TB, TB, TB, 1, 5}, {4, TB, TB, 1, nc}, {TB, G, TB, 1, nc}, {TB, TB, G, 1, nc}};
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     for (int i = 0; i < 4; ++i)
         if (strides[i] % 16) return fail(CN_ERR_UNSUPPORTED, "Euler stage: grid strides are not 16-byte multiples");
@@ -167,11 +162,14 @@ static cn_status core_map(const cn_grid *g, int cs, size_t es, CUtensorMap *m)
             encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     });
     if (!encode) return fail(CN_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    const CUresult r = encode(
-        m, es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, base, dims, strides, box,
-        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(CN_ERR_CUDA, "cuTensorMapEncodeTiled failed for the Euler tile map");
+    CUtensorMap *const out[4] = {&m->core, &m->hx, &m->hy, &m->hz};
+    for (int k = 0; k < 4; ++k) {
+        const CUresult r = encode(
+            out[k], es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, base, dims,
+            strides, boxes[k], estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(CN_ERR_CUDA, "cuTensorMapEncodeTiled failed for the Euler tile maps");
+    }
     return CN_OK;
 }
 
@@ -196,22 +194,32 @@ static cn_status launch_stage(cn_grid *bcsrc, cn_grid *Us, int cs, cn_grid *Un, 
         src.bc[c] = bc_view(bcsrc, cs + c);
     }
     for (int d = 0; d < 3; ++d) src.ih[d] = 1.0 / Us->h[d];
-    p.dt = (T)dt;
+    p.dt = stage == 0 ? T(1) : (T)dt;
+    p.cn = stage < 2 ? T(0) : (stage == 2 ? T(0.75) : T(1.0 / 3.0));
+    p.cs = stage < 2 ? T(1) : (stage == 2 ? T(0.25) : T(2.0 / 3.0));
+    p.use_u = stage >= 1;
+    p.use_un = stage >= 2;
     p.gamma = (T)gamma;
     p.gm1 = (T)(gamma - 1.0);
     p.igm1 = (T)(1.0 / (gamma - 1.0));
-    p.stage = stage;
     p.partials = partials;
     p.err = Us->d_err;
-    CUtensorMap core;
-    r = core_map(Us, cs, sizeof(T), &core);
+    TileMaps maps;
+    r = tile_maps(Us, cs, sizeof(T), Land<T>::NC, &maps);
     if (r != CN_OK) return r;
     const size_t smem = stage_smem<T>();
     static DeviceOnce attr_once; // per device (the first call on a device is an eager one)
     r = smem_opt_in(attr_once, stage_kernel<T>, smem);
     if (r != CN_OK) return r;
-    const int64_t ctas = (int64_t)Us->nblocks * (Us->n[0] / TB) * (Us->n[1] / TB) * (Us->n[2] / TB);
-    stage_kernel<T><<<(unsigned)ctas, NT, smem, st>>>(p, src, core);
+    const int tx = Us->n[0] / TB, ty = Us->n[1] / TB, tz = Us->n[2] / TB;
+    src.tiles = FastDiv((uint32_t)(tx * ty * tz));
+    src.tx = FastDiv((uint32_t)tx);
+    src.ty = FastDiv((uint32_t)ty);
+    src.nbx = FastDiv((uint32_t)Us->nb[0]);
+    src.nby = FastDiv((uint32_t)Us->nb[1]);
+    const int64_t ntiles = (int64_t)Us->nblocks * tx * ty * tz;
+    if (ntiles >= ((int64_t)1 << 30)) return fail(CN_ERR_UNSUPPORTED, "Euler stage: at most 2^30 - 1 tiles of 8^3 cells");
+    stage_kernel<T><<<(unsigned)ntiles, NT, smem, st>>>(p, src, maps);
     CN_CUDA_TRY(cudaGetLastError());
     return CN_OK;
 }

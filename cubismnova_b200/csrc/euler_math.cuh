@@ -131,7 +131,6 @@ template <> __device__ __forceinline__ float2 vsub<float2>(float2 a, float2 b)
 template <typename V> __device__ __forceinline__ V vrcp(V a) { return rcp_pos(a); }
 template <> __device__ __forceinline__ float2 vrcp<float2>(float2 a) { return make_float2(rcp_pos(a.x), rcp_pos(a.y)); }
 
-__device__ __forceinline__ double range_scale(double, double, double) { return 1.0; } // FP64 is not rescaled
 __device__ __forceinline__ float range_scale(float s0, float s1, float s2) { return weno5_scale(s0, s1, s2); }
 // weno5_scale for both lanes of a pair at once, from the top 7 bits of each
 // biased exponent (byte 3 of a positive float, E >> 1) packed as two 16-bit
@@ -177,8 +176,8 @@ __device__ __forceinline__ float2 range_scale(float2 s0, float2 s1, float2 s2)
 // indicators and candidates formed on their own; with the fluxes' fused sums
 // (rusanov) a step of 512^3 cells went from 54.1 to 46.6 ms in FP64, of 384^3
 // cells from 13.4 to 12.4 ms in FP32.
-template <typename V>
-__device__ __forceinline__ void weno5_run(const V (&u)[8], V (&wl)[3], V (&wr)[3], bool scaled)
+template <bool SCALED, typename V>
+__device__ __forceinline__ void weno5_run(const V (&u)[8], V (&wl)[3], V (&wr)[3])
 {
     using T = typename Scalar<V>::type;
     using C = K<T>;
@@ -200,13 +199,11 @@ __device__ __forceinline__ void weno5_run(const V (&u)[8], V (&wl)[3], V (&wr)[3
         const V h1 = vadd(d[j + 1], d[j + 2]);
         const V h2 = vfma(vset<V>(T(-2)), d[j + 2], a[j + 2]);
         V s0 = vfma(h0, h0, q[j]), s1 = vfma(h1, h1, q[j + 1]), s2 = vfma(h2, h2, q[j + 2]);
-        if constexpr (sizeof(T) == 4) { // FP32: exact power-of-two rescaling
-            if (scaled) {
-                const V sc = range_scale(s0, s1, s2);
-                s0 = vmul(s0, sc);
-                s1 = vmul(s1, sc);
-                s2 = vmul(s2, sc);
-            }
+        if constexpr (SCALED) { // FP32: exact power-of-two rescaling
+            const V sc = range_scale(s0, s1, s2);
+            s0 = vmul(s0, sc);
+            s1 = vmul(s1, sc);
+            s2 = vmul(s2, sc);
         }
         const V t0 = vmul(s0, s0), t1 = vmul(s1, s1), t2 = vmul(s2, s2);
         const V p12 = vmul(t1, t2), p02 = vmul(t0, t2), p01 = vmul(t0, t1);

@@ -157,3 +157,39 @@ def test_full_size_periodic_conservation_and_shift(cn):
         assert abs(sums[c] - before[c] * vol) <= 1e-12 * abs(before[c] * vol)
     del U, R
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("nb,n,seed", [((2, 1, 3), (8, 24, 16), 1), ((1, 2, 2), (16, 8, 8), 2),
+                                       ((3, 2, 1), (8, 8, 8), 3), ((2, 2, 2), (24, 16, 8), 4)])
+def test_mixed_bc_vectors_match_oracle(cn, oracle_lib, dtype, nb, n, seed):
+    """Every block's own BC vectors, per component: sides that are periodic
+    copies beside sides with Dirichlet, Absorbing or Symmetry, several BCs on
+    one face (the last one decides), Base between them, BCs on faces inside
+    the domain, blocks of one tile along a direction (both sides outside)."""
+    import torch
+    U = _state(cn, nb, n, dtype, seed=seed, bcs=False)
+    rng = np.random.default_rng(seed)
+    kinds = {1: cn.BC.Dirichlet, 2: cn.BC.Absorbing, 3: cn.BC.Symmetry}
+    far = cn.workloads.far_field()
+    bcl = [dict() for _ in range(5)]
+    for b in range(int(np.prod(nb))):
+        for d in range(3):
+            for s in range(2):
+                r = rng.random()
+                comps = range(5) if r < 0.4 else ([int(rng.integers(5))] if r < 0.6 else [])
+                for c in comps:
+                    chain = [int(rng.choice([0, 1, 2, 3]))] if rng.random() < 0.4 else []
+                    for kind in chain + [int(rng.choice([1, 2, 3]))]:
+                        v = float(far[c] * (1 + 0.1 * rng.random())) if kind == 1 else (
+                            (-1.0 if c == 1 + d else 1.0) if kind == 3 else 0.0)
+                        bc = cn.BC.Base(d, s) if kind == 0 else (
+                            kinds[kind](d, s) if kind == 2 else kinds[kind](d, s, v))
+                        U.field(b, c).getBC().push_back(bc)
+                        bcl[c].setdefault(b, []).append((d, s, kind, v))
+    host = _host(U)
+    R = cn.euler.like(U)
+    cn.euler.rk3_stage(U, U, None, R, 1, 1e-3)
+    torch.cuda.synchronize()
+    want = oracle_lib.euler_stage(host, None, nb, n, bcl, 1, 1e-3, GAMMA, U.getCellSize())
+    assert_close(_host(R), want, TOL_F64 if dtype == np.float64 else TOL_F32_STATE, f"mixed BCs {nb} {n}")
