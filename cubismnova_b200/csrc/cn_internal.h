@@ -333,6 +333,40 @@ __device__ __forceinline__ bool lab_value(const T *__restrict__ comp, const LabG
     return lab_resolve<T, GROW>(L, bc, bc.mode[block], block, bx, by, bz, q0, q1, q2, apply_bc, sink);
 }
 
+// What lies behind a face of a block for one component: a value, or `value`
+// times a cell of the block (its edge cell, or the mirrored one) or of the
+// periodic neighbour.
+enum { kRuleCopy = 0, kRuleValue = 1, kRuleEdge = 2, kRuleMirror = 3 };
+template <typename T> struct FaceRule {
+    int kind;
+    T value;
+};
+// The rule of face (d, s) of `block`: cn::lab_resolve for the cells of a
+// non-tensorial lab that leave the block along d only.  The last BC on that
+// face decides; Absorbing and Symmetry lead to a cell inside the block, where
+// no BC applies; without a BC it is the neighbour's cell, or undefined (read
+// as 0) if the neighbour is skipped.
+template <typename T>
+__device__ __forceinline__ FaceRule<T> face_rule(const LabGeom &L, const BcView &bc, int block, int d, int s)
+{
+    const unsigned mode = bc.mode[block];
+    if (mode & kHasBc) {
+        const int k0 = bc.off[block];
+        for (int k = bc.off[block + 1] - 1; k >= k0; --k) {
+            const int32_t m = bc.ent[k].meta;
+            if (bc_kind(m) == CN_BC_BASE || bc_dir(m) != d || bc_side(m) != s ||
+                !pick3(d, L.valid_bc[0], L.valid_bc[1], L.valid_bc[2]))
+                continue;
+            const T v = static_cast<T>(bc.ent[k].value);
+            if (bc_kind(m) == CN_BC_DIRICHLET) return {kRuleValue, v};
+            if (bc_kind(m) == CN_BC_ABSORBING) return {kRuleEdge, T(1)};
+            return {kRuleMirror, v};
+        }
+    }
+    if (((mode >> (2 * d)) & 3u) == (s ? 2u : 1u)) return {kRuleValue, T(0)};
+    return {kRuleCopy, T(1)};
+}
+
 // Lab value through the full BC chain (out of line: only blocks with BCs or
 // skip flags take it, so its code exists once per kernel; kernels calling it
 // pass L and bc from __grid_constant__ parameters or device memory).

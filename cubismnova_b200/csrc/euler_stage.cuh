@@ -90,15 +90,6 @@ struct TileMaps {
     CUtensorMap core, hx, hy, hz;
 };
 
-// What lies behind a face of a block for one component: a value, or `value`
-// times a cell of the block (its edge cell or the mirrored one) or of the
-// neighbour.
-enum { kRuleCopy = 0, kRuleValue = 1, kRuleEdge = 2, kRuleMirror = 3 };
-template <typename T> struct FaceRule {
-    int kind;
-    T value;
-};
-
 // Uniform Cartesian grid: tiles in block order, halo cells through the
 // FieldLab lab resolution (cn::lab_value) with each component's BC vector.
 struct CartSrc {
@@ -150,30 +141,6 @@ struct CartSrc {
         const int b = d == 0 ? t.bx : (d == 1 ? t.by : t.bz), m = L.nb[d];
         const int q = s ? (b + 1 < m ? b + 1 : 0) : (b > 0 ? b - 1 : m - 1);
         return t.block + (q - b) * (d == 0 ? 1 : (d == 1 ? L.nb[0] : L.nb[0] * L.nb[1]));
-    }
-    // What the lab puts behind side (d, s) of block t.block for component c
-    // (cn::lab_resolve for cells that leave the block along d only, of a
-    // non-tensorial lab): the last BC on that face decides; Absorbing and
-    // Symmetry lead to a cell inside the block, where no BC applies; without
-    // a BC it is the neighbour's cell, or undefined (read as 0) if the
-    // neighbour is skipped.
-    template <typename T> __device__ __forceinline__ FaceRule<T> face_rule(const TileInfo<T> &t, int c, int d, int s) const
-    {
-        const BcView &b = bc[c];
-        const unsigned mode = b.mode[t.block];
-        if (mode & kHasBc) {
-            const int k0 = b.off[t.block];
-            for (int k = b.off[t.block + 1] - 1; k >= k0; --k) {
-                const int32_t m = b.ent[k].meta;
-                if (bc_kind(m) == CN_BC_BASE || bc_dir(m) != d || bc_side(m) != s || !L.valid_bc[d]) continue;
-                const T v = static_cast<T>(b.ent[k].value);
-                if (bc_kind(m) == CN_BC_DIRICHLET) return {kRuleValue, v};
-                if (bc_kind(m) == CN_BC_ABSORBING) return {kRuleEdge, T(1)};
-                return {kRuleMirror, v};
-            }
-        }
-        if (((mode >> (2 * d)) & 3u) == (s ? 2u : 1u)) return {kRuleValue, T(0)};
-        return {kRuleCopy, T(1)};
     }
 };
 
@@ -788,7 +755,7 @@ __device__ __forceinline__ void stage_tile_tma(const StageParams<T> &p, const Ca
     if (sh.slow) {
         if (threadIdx.x < 30) {
             const int k = threadIdx.x / 5, c = threadIdx.x % 5;
-            if ((sh.slow >> k) & 1u) sh.rules[k][c] = src.template face_rule<T>(t, c, k >> 1, k & 1);
+            if ((sh.slow >> k) & 1u) sh.rules[k][c] = face_rule<T>(src.L, src.bc[c], t.block, k >> 1, k & 1);
         }
         __syncthreads();
 #pragma unroll 1

@@ -1,24 +1,33 @@
 // fd.cu -- K1: lab fill fused with the 2nd-order finite-difference stencils
 // (7-point Laplacian, central gradient, divergence) and the ddx kernel ABI.
 //
-// Design (one CTA per z-slab tile of one block, N0 x N1 x TZ cells):
-//   * the tile's inner cells are one contiguous range of the block (x-fastest
-//     block storage), so a single 1-D TMA bulk copy (cp.async.bulk, mbarrier
-//     completion, bounded wait) stages them into shared memory;
-//   * while that copy is in flight the threads gather the six one-cell faces
-//     of the tile with cn::lab_value (periodic neighbours, BC chain), i.e. the
-//     lab of a stencil (-1,2) non-tensorial (Block/FieldLab.h:180-224);
-//   * each thread then evaluates the stencil from shared memory and writes
-//     coalesced rows of the output blocks.
+// Design.  A thread owns V cells of a row (16 bytes where rows allow it) over a
+// run of TZ planes and marches up it: the z neighbours stay in registers, the
+// x and y neighbours are cached loads, across a face of the block at a
+// constant offset in the neighbour block.  Threads run over all columns of all
+// blocks, x fastest, so that blocks of any extent fill the warps.  Cells beside
+// faces that carry a BC or a skipped neighbour are left to a few CTAs of the
+// same launch that resolve them one by one (Absorbing and Symmetry lead to the
+// own cell at ghost width 1, Dirichlet and undefined cells to a constant):
+// together the lab of a stencil (-1,2) non-tensorial (Block/FieldLab.h:180-224).
+//
+// Bound by DRAM at large sizes and by latency and the launch at small ones.
+// Against tiles staged in shared memory (one bulk copy per z slab, faces cell
+// by cell), B200: Laplacian + gradient FP64 128^3 22.3 -> 18.5 us, 512^3 1003
+// -> 891 us (94 % of the copy bandwidth); divergence FP64 512^3 2161 -> 695
+// us, FP32 on 30 x 33 x 27 blocks with walls (25.7 M cells) 406 -> 81 us;
+// Laplacian FP32 512^3 793 -> 199 us.  BC code inlined into the march cost the
+// registers of a third of the warps (84 -> 107 us on the ragged case).
+//
 // Arithmetic uses __d*_rn / __f*_rn intrinsics so nothing is contracted into
 // an FMA: results are bit-identical to the reference loops compiled without
 // contraction (Kernel/Laplacian/Laplacian.cpp:123-130,
 // Kernel/Divergence/nova/nova.cpp:113-126, ISPC .../ddxGold.cpp:9-33).
 #include <algorithm>
+#include <cstring>
 
 #include "cn_fastdiv.h"
 #include "cn_internal.h"
-#include "cn_tma.cuh"
 
 namespace cn {
 
@@ -34,54 +43,30 @@ template <> struct Arith<float> {
     static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 };
 
+// Largest block the operators take: a plane of it with the planes and rows
+// around it, each array padded to 4 elements, within 100 KB.
+constexpr size_t kMaxPlaneBytes = 100 * 1024 - 128;
+static size_t plane_bytes(int n0, int n1, size_t es, int nc)
+{
+    auto pad4 = [](size_t n) { return (n + 3) & ~(size_t)3; };
+    return (3 * pad4((size_t)n0 * n1) + 2 * (pad4(n0) + pad4(n1))) * es * nc;
+}
+
 enum FdOp { kLap = 0, kGrad = 1, kLapGrad = 2, kDiv = 3 };
 
 template <typename T> struct FdParams {
-    const T *in[3];  // input component bases (kDiv: 3 components)
+    const T *in[3];  // component read along x, y, z (kDiv: 3 components, else the same)
     BcView bc[3];
     LabGeom L;
     T *lap;          // kLap / kLapGrad / kDiv output component base
     T *grad;         // kGrad / kLapGrad: first of 3 components
     int64_t out_cstride;
     T ih[3], ih2[3];
-    int TZ;
-    int use_bulk;
-    int *err;
-    FastDiv dv0, dv1, dv01, dvh; // N0, N1, N0 * N1, N0 / 2: cell index -> (x, y, z) without divisions
+    int TZ, block0, total;       // planes per thread, first block and threads of this launch
+    FastDiv per_block, plane, n0; // threads per block, N0 * N1, N0
+    FastDiv nb0, nb1, f0, f1;     // blocks along x, y; N0, N1
+    int faces, faces_per_cta, face_ctas; // faces of this launch's blocks, CTAs that look at them
 };
-
-// Shared-memory tile of one component: inner cells + the six faces.
-template <typename T> struct Tile {
-    T *in, *xlo, *xhi, *ylo, *yhi, *zlo, *zhi;
-};
-
-// Every array of a tile starts on a multiple of 4 elements, so each one (and
-// the next component's tile) is 16-byte aligned for the bulk copy and the
-// two-element vector loads.
-__host__ __device__ __forceinline__ size_t pad4(size_t n) { return (n + 3) & ~(size_t)3; }
-
-__host__ __device__ __forceinline__ size_t tile_elems(int N0, int N1, int TZ)
-{
-    return pad4((size_t)N0 * N1 * TZ) + 2 * (pad4((size_t)N1 * TZ) + pad4((size_t)N0 * TZ) + pad4((size_t)N0 * N1));
-}
-
-template <typename T>
-__device__ __forceinline__ Tile<T> carve(T *base, int N0, int N1, int TZ)
-{
-    Tile<T> t;
-    t.in = base;
-    t.xlo = t.in + pad4((size_t)N0 * N1 * TZ);
-    t.xhi = t.xlo + pad4((size_t)N1 * TZ);
-    t.ylo = t.xhi + pad4((size_t)N1 * TZ);
-    t.yhi = t.ylo + pad4((size_t)N0 * TZ);
-    t.zlo = t.yhi + pad4((size_t)N0 * TZ);
-    t.zhi = t.zlo + pad4((size_t)N0 * N1);
-    return t;
-}
-
-template <typename T> struct Vec2;
-template <> struct Vec2<double> { using type = double2; };
-template <> struct Vec2<float> { using type = float2; };
 
 // Outputs of one cell from its six neighbours (kDiv: x neighbours of the
 // first component, y of the second, z of the third; c0 unused).
@@ -111,214 +96,233 @@ __device__ __forceinline__ void cell_eval(const FdParams<T> &p, T c0, T xp, T xm
     }
 }
 
-// Stages one lab cell of a tile face into shared memory.  Cells inside the
-// block, and every cell of a block without BCs or skip flags (lab mode byte
-// 0: the periodic neighbour from the table snb, index (r0+1) + 3 (r1+1) +
-// 9 (r2+1)), are asynchronous copies (cp.async), so all of a thread's face
-// loads are in flight at once alongside the bulk copy of the interior; the
-// others are resolved with cn::lab_value.  Undefined lab cells (never read by
-// these stencils unless the BC set-up leaves a face undefined) are zero.
-template <typename T>
-__device__ __forceinline__ void face_cell(const T *comp, const LabGeom &L, const BcView &bc, bool plain,
-                                          const int *snb, int block, int bx, int by, int bz, int x, int y, int z,
-                                          T *dst)
+// V consecutive cells of a row, loaded and stored as one (V * sizeof(T) <= 16
+// bytes, aligned: row lengths are multiples of V then).
+template <typename T, int V> struct alignas(sizeof(T) * V) Pack {
+    T v[V];
+};
+template <typename T, int V> __device__ __forceinline__ Pack<T, V> load(const T *p)
 {
-    const int r0 = x < 0 ? -1 : (x >= L.n[0] ? 1 : 0), r1 = y < 0 ? -1 : (y >= L.n[1] ? 1 : 0),
-              r2 = z < 0 ? -1 : (z >= L.n[2] ? 1 : 0);
-    if (plain || (r0 | r1 | r2) == 0) {
-        const int sb = snb[(r0 + 1) + 3 * (r1 + 1) + 9 * (r2 + 1)];
-        const T *src = comp + (int64_t)sb * L.bstride + (x - r0 * L.n[0]) +
-                       (int64_t)L.n[0] * ((y - r1 * L.n[1]) + (int64_t)L.n[1] * (z - r2 * L.n[2]));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src),
-                     "n"((int)sizeof(T))
-                     : "memory");
-        return;
+    Pack<T, V> r;
+    if constexpr (sizeof(T) * V == 16) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
+        memcpy(&r, &q, 16);
+    } else if constexpr (sizeof(T) * V == 8) {
+        const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
+        memcpy(&r, &q, 8);
+    } else {
+        r.v[0] = __ldg(p);
     }
-    T v;
-    if (!lab_value<T>(comp, L, bc, block, bx, by, bz, x, y, z, true, v))
-        v = T(0);
-    *dst = v;
+    return r;
+}
+template <typename T, int V> __device__ __forceinline__ void store(T *p, const Pack<T, V> &r)
+{
+    *reinterpret_cast<Pack<T, V> *>(p) = r;
 }
 
-__device__ __forceinline__ void fd_cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// A neighbour of a column's cells: cell o's neighbour is in[o + off], times
+// `value` behind a face with Absorbing or Symmetry (kind 2; off leads to the
+// own cell), or `value` itself (kind 1).
+template <typename T> struct Side {
+    int64_t off;
+    T value;
+    int kind;
+};
 
-// Gathers the faces selected by mask (bit 0: x, 1: y, 2: z) of the tile that
-// starts at z0; the caller waits for the copies (fd_cp_async_wait_all) and
-// synchronises the CTA before reading them.
-template <typename T>
-__device__ __forceinline__ void gather_faces(const T *comp, const LabGeom &L, const BcView &bc,
-                                             int block, int bx, int by, int bz, int z0, int TZ,
-                                             const Tile<T> &t, unsigned mask, const int *snb,
-                                             const FastDiv &dv0, const FastDiv &dv1)
+template <typename T> __device__ __noinline__ FaceRule<T> rule_of(const LabGeom &L, const BcView &bc, int block, int d, int s)
 {
-    const int N0 = L.n[0], N1 = L.n[1];
-    const int nth = blockDim.x;
-    const bool plain = __ldg(bc.mode + block) == 0;
-    if (mask & 1u) {
-        const int m = N1 * TZ;
-        for (int i = threadIdx.x; i < 2 * m; i += nth) {
-            const int side = i >= m, r = side ? i - m : i;
-            const int z = dv1.div(r), y = r - z * N1;
-            face_cell<T>(comp, L, bc, plain, snb, block, bx, by, bz, side ? N0 : -1, y, z0 + z,
-                         (side ? t.xhi : t.xlo) + r);
-        }
-    }
-    if (mask & 2u) {
-        const int m = N0 * TZ;
-        for (int i = threadIdx.x; i < 2 * m; i += nth) {
-            const int side = i >= m, r = side ? i - m : i;
-            const int z = dv0.div(r), x = r - z * N0;
-            face_cell<T>(comp, L, bc, plain, snb, block, bx, by, bz, x, side ? N1 : -1, z0 + z,
-                         (side ? t.yhi : t.ylo) + r);
-        }
-    }
-    if (mask & 4u) {
-        const int m = N0 * N1;
-        for (int i = threadIdx.x; i < 2 * m; i += nth) {
-            const int side = i >= m, r = side ? i - m : i;
-            const int y = dv0.div(r), x = r - y * N0;
-            face_cell<T>(comp, L, bc, plain, snb, block, bx, by, bz, x, y, side ? z0 + TZ : z0 - 1,
-                         (side ? t.zhi : t.zlo) + r);
-        }
-    }
+    return face_rule<T>(L, bc, block, d, s);
 }
 
-template <typename T, int OP>
-__global__ void __launch_bounds__(256, 8) fd_kernel(FdParams<T> p)
+// side s of direction d (stride st) of a cell at coordinate q
+template <typename T>
+__device__ __forceinline__ Side<T> side_of(const LabGeom &L, const BcView &bc, int block, int b, int d, int s, int q,
+                                           int64_t st)
 {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw);
-    T *base = reinterpret_cast<T *>(smem_raw + 128);
-    const LabGeom &L = p.L;
-    const int N0 = L.n[0], N1 = L.n[1], N2 = L.n[2];
-    const int TZ = p.TZ;
-    const int tiles_per_block = N2 / TZ;
-    const int block = blockIdx.x / tiles_per_block;
-    const int z0 = (blockIdx.x - block * tiles_per_block) * TZ;
-    constexpr int NC = (OP == kDiv) ? 3 : 1;
-    const size_t te = tile_elems(N0, N1, TZ);
-    Tile<T> tl[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-        tl[c] = carve<T>(base + c * te, N0, N1, TZ);
-    const uint32_t in_bytes = (uint32_t)((size_t)N0 * N1 * TZ * sizeof(T));
-    const int64_t in_off = (int64_t)block * L.bstride + (int64_t)z0 * N0 * N1;
-    // the interior's bulk copy goes out first; the barrier below publishes
-    // the mbarrier's initialisation to the other threads
-    if (p.use_bulk && threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-        mbar_arrive_expect_tx(bar, in_bytes * NC);
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-            bulk_g2s(tl[c].in, p.in[c] + in_off, in_bytes, bar);
+    Side<T> r = {s ? st : -st, T(1), 0};
+    const int n = L.n[d];
+    if (s ? q + 1 < n : q > 0) return r;
+    if ((__ldg(bc.faces + block) >> (2 * d + s)) & 1) {
+        const FaceRule<T> f = rule_of<T>(L, bc, block, d, s);
+        if (f.kind != kRuleCopy) return {0, f.value, f.kind == kRuleValue ? 1 : 2};
     }
-    const int bx = block % L.nb[0];
-    const int by = (block / L.nb[0]) % L.nb[1];
-    const int bz = block / (L.nb[0] * L.nb[1]);
-    __shared__ int snb[27]; // periodic neighbour blocks
-    if (threadIdx.x < 27) {
-        const int t = threadIdx.x;
-        int nx = bx + t % 3 - 1, ny = by + (t / 3) % 3 - 1, nz = bz + t / 9 - 1;
-        nx = nx < 0 ? nx + L.nb[0] : (nx >= L.nb[0] ? nx - L.nb[0] : nx);
-        ny = ny < 0 ? ny + L.nb[1] : (ny >= L.nb[1] ? ny - L.nb[1] : ny);
-        nz = nz < 0 ? nz + L.nb[2] : (nz >= L.nb[2] ? nz - L.nb[2] : nz);
-        snb[t] = nx + L.nb[0] * (ny + L.nb[1] * nz);
-    }
-    if (!p.use_bulk) {
-        const int m = N0 * N1 * TZ;
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-            for (int i = threadIdx.x; i < m; i += blockDim.x)
-                tl[c].in[i] = p.in[c][in_off + i];
-    }
-    __syncthreads(); // snb, mbarrier initialised
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        const unsigned mask = (OP == kDiv) ? (1u << c) : 7u;
-        gather_faces<T>(p.in[c], L, p.bc[c], block, bx, by, bz, z0, TZ, tl[c], mask, snb, p.dv0, p.dv1);
-    }
-    fd_cp_async_wait_all();
-    if (p.use_bulk) {
-        if (!mbar_wait_bounded_sleep(bar, 0)) {
-            atomicExch(p.err, kDevErrTimeout);
-        }
-    }
-    __syncthreads();
+    const int m = L.nb[d], nbr = s ? (b + 1 < m ? b + 1 : 0) : (b > 0 ? b - 1 : m - 1);
+    const int bs = d == 0 ? 1 : (d == 1 ? L.nb[0] : L.nb[0] * L.nb[1]);
+    r.off += (int64_t)(nbr - b) * bs * L.bstride + (s ? -n : n) * st;
+    return r;
+}
 
-    // x-even blocks: two neighbouring cells of a row per thread, with
-    // two-element shared loads and global stores
-    if ((N0 & 1) == 0) {
-        using V = typename Vec2<T>::type;
-        const int h0 = N0 >> 1;
-        const int mp = h0 * N1 * TZ;
-        const Tile<T> &a = tl[0], &b = tl[NC > 1 ? 1 : 0], &c = tl[NC > 2 ? 2 : 0];
-        for (int j = threadIdx.x; j < mp; j += blockDim.x) {
-            const int row = p.dvh.div(j), x = 2 * (j - row * h0); // row = y + N1 z
-            const int z = p.dv1.div(row), y = row - z * N1;
-            const int i = x + N0 * row;
-            const int64_t o = in_off + i;
-            const V ac = *reinterpret_cast<const V *>(a.in + i);
-            const T xm = x > 0 ? a.in[i - 1] : a.xlo[row];
-            const T xp = x + 2 < N0 ? a.in[i + 2] : a.xhi[row];
-            const V yp = *reinterpret_cast<const V *>(y + 1 < N1 ? b.in + i + N0 : b.yhi + x + N0 * z);
-            const V ym = *reinterpret_cast<const V *>(y > 0 ? b.in + i - N0 : b.ylo + x + N0 * z);
-            const V zp = *reinterpret_cast<const V *>(z + 1 < TZ ? c.in + i + N0 * N1 : c.zhi + x + N0 * y);
-            const V zm = *reinterpret_cast<const V *>(z > 0 ? c.in + i - N0 * N1 : c.zlo + x + N0 * y);
-            T l0 = T(0), l1 = T(0), g00 = T(0), g01 = T(0), g02 = T(0), g10 = T(0), g11 = T(0), g12 = T(0);
-            cell_eval<T, OP>(p, ac.x, ac.y, xm, yp.x, ym.x, zp.x, zm.x, l0, g00, g01, g02);
-            cell_eval<T, OP>(p, ac.y, xp, ac.x, yp.y, ym.y, zp.y, zm.y, l1, g10, g11, g12);
-            if (OP == kLap || OP == kLapGrad || OP == kDiv)
-                *reinterpret_cast<V *>(p.lap + o) = V{l0, l1};
-            if (OP == kGrad || OP == kLapGrad) {
-                *reinterpret_cast<V *>(p.grad + o) = V{g00, g10};
-                *reinterpret_cast<V *>(p.grad + o + p.out_cstride) = V{g01, g11};
-                *reinterpret_cast<V *>(p.grad + o + 2 * p.out_cstride) = V{g02, g12};
+// One thread's run of planes from cell o, all neighbours plain cells: U planes
+// at a time, their loads before their stores.  zm, zp: offsets of the lower
+// neighbour of the first plane and of the upper one of the last.
+template <typename T, int OP, int V, int U>
+__device__ __forceinline__ void march(const FdParams<T> &p, int64_t o, int64_t s2, int planes, int64_t xm, int64_t xp,
+                                      int64_t ym, int64_t yp, int64_t zm, int64_t zp)
+{
+    using P = Pack<T, V>;
+    const T *px = p.in[0] + o, *py = p.in[1] + o, *pz = p.in[2] + o;
+    T *lap = p.lap + o, *grad = p.grad + o;
+    P a = load<T, V>(pz + zm), b = load<T, V>(pz); // planes z - 1 and z
+    for (int z = 0; z < planes; z += U) {
+        P vz[U], vym[U], vyp[U], vx[U];
+        Pack<T, 1> vxm[U], vxp[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            if (U == 1 || z + k < planes) {
+                vz[k] = load<T, V>(pz + (z + k + 1 == planes ? zp : s2));
+                vym[k] = load<T, V>(py + ym);
+                vyp[k] = load<T, V>(py + yp);
+                if (OP == kDiv && V > 1) vx[k] = load<T, V>(px);
+                vxm[k] = load<T, 1>(px + xm);
+                vxp[k] = load<T, 1>(px + (V - 1) + xp);
+                px += s2;
+                py += s2;
+                pz += s2;
             }
         }
-        return;
-    }
-    const int m = N0 * N1 * TZ;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        const int z = p.dv01.div(i), r = i - z * (N0 * N1);
-        const int y = p.dv0.div(r), x = r - y * N0;
-        const int64_t o = in_off + i;
-        const Tile<T> &a = tl[0], &b = tl[NC > 1 ? 1 : 0], &c = tl[NC > 2 ? 2 : 0];
-        const T c0 = a.in[i];
-        const T xp = x + 1 < N0 ? a.in[i + 1] : a.xhi[y + N1 * z];
-        const T xm = x > 0 ? a.in[i - 1] : a.xlo[y + N1 * z];
-        const T yp = y + 1 < N1 ? b.in[i + N0] : b.yhi[x + N0 * z];
-        const T ym = y > 0 ? b.in[i - N0] : b.ylo[x + N0 * z];
-        const T zp = z + 1 < TZ ? c.in[i + N0 * N1] : c.zhi[x + N0 * y];
-        const T zm = z > 0 ? c.in[i - N0 * N1] : c.zlo[x + N0 * y];
-        T l = T(0), g0 = T(0), g1 = T(0), g2 = T(0);
-        cell_eval<T, OP>(p, c0, xp, xm, yp, ym, zp, zm, l, g0, g1, g2);
-        if (OP == kLap || OP == kLapGrad || OP == kDiv) p.lap[o] = l;
-        if (OP == kGrad || OP == kLapGrad) {
-            p.grad[o] = g0;
-            p.grad[o + p.out_cstride] = g1;
-            p.grad[o + 2 * p.out_cstride] = g2;
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            if (U == 1 || z + k < planes) {
+                P l, g0, g1, g2;
+                const P &c = OP == kDiv ? vx[k] : b;
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    const T m = i > 0 ? c.v[i > 0 ? i - 1 : 0] : vxm[k].v[0];
+                    const T q = i + 1 < V ? c.v[i + 1 < V ? i + 1 : 0] : vxp[k].v[0];
+                    cell_eval<T, OP>(p, b.v[i], q, m, vyp[k].v[i], vym[k].v[i], vz[k].v[i], a.v[i], l.v[i], g0.v[i],
+                                     g1.v[i], g2.v[i]);
+                }
+                if (OP == kLap || OP == kLapGrad || OP == kDiv) {
+                    store<T, V>(lap, l);
+                    lap += s2;
+                }
+                if (OP == kGrad || OP == kLapGrad) {
+                    store<T, V>(grad, g0);
+                    store<T, V>(grad + p.out_cstride, g1);
+                    store<T, V>(grad + 2 * p.out_cstride, g2);
+                    grad += s2;
+                }
+                a = b;
+                b = vz[k];
+            }
         }
     }
 }
 
-static size_t fd_smem_bytes(int N0, int N1, int TZ, size_t es, int nc)
+// One cell with BCs on any side.
+template <typename T, int OP>
+__device__ __forceinline__ void bc_cell(const FdParams<T> &p, int block, int b0, int b1, int b2, int x, int y, int z)
 {
-    return 128 + tile_elems(N0, N1, TZ) * es * nc;
+    const LabGeom &L = p.L;
+    const int64_t s1 = L.n[0], s2 = (int64_t)L.n[0] * L.n[1];
+    const int64_t o = (int64_t)block * L.bstride + x + s1 * y + s2 * z;
+    Side<T> e[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        e[k] = side_of<T>(L, p.bc[k >> 1], block, pick3(k >> 1, b0, b1, b2), k >> 1, k & 1, pick3(k >> 1, x, y, z),
+                          k < 2 ? 1 : (k < 4 ? s1 : s2));
+    T v[6]; // lower and upper neighbour along x, y, z
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        v[k] = __ldg(p.in[k >> 1] + o + e[k].off);
+    const T c = __ldg(p.in[0] + o);
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        v[k] = e[k].kind == 1 ? e[k].value : (e[k].kind == 2 ? Arith<T>::mul(e[k].value, v[k]) : v[k]);
+    T l, g0, g1, g2;
+    cell_eval<T, OP>(p, c, v[1], v[0], v[3], v[2], v[5], v[4], l, g0, g1, g2);
+    if (OP == kLap || OP == kLapGrad || OP == kDiv) p.lap[o] = l;
+    if (OP == kGrad || OP == kLapGrad) {
+        p.grad[o] = g0;
+        p.grad[o + p.out_cstride] = g1;
+        p.grad[o + 2 * p.out_cstride] = g2;
+    }
 }
 
-// z-slab height: the largest divisor of N2 whose tile fits the budget and
-// holds at most 2048 cells (more, smaller CTAs balance the SMs and overlap
-// the staging of one tile with the stencil of another); at least 1.
-static int pick_tz(int N0, int N1, int N2, size_t es, int nc, size_t budget)
+// The cells beside block faces that carry a BC or a skipped neighbour, which
+// the marching threads leave out: a CTA looks at some of the nblocks * 6 faces
+// and walks the cells of those (x faces: the V cells of the columns there).
+// Out of line, so that its registers stay its own.
+constexpr int kFacesPerCta = 8; // at most
+template <typename T, int OP, int V> __device__ __noinline__ void bc_faces(const FdParams<T> &p)
 {
-    for (int tz = N2; tz >= 1; --tz) {
-        if (N2 % tz) continue;
-        if (fd_smem_bytes(N0, N1, tz, es, nc) > budget) continue;
-        if (tz > 1 && (size_t)N0 * N1 * tz > 2048) continue;
-        return tz;
+    const LabGeom &L = p.L;
+    const int lane = threadIdx.x & 31, first = blockIdx.x * p.faces_per_cta;
+    bool set = false;
+    if (lane < p.faces_per_cta && first + lane < p.faces) {
+        const int f = (first + lane) % 6;
+        const BcView &bc = f < 2 ? p.bc[0] : (f < 4 ? p.bc[1] : p.bc[2]);
+        set = (__ldg(bc.faces + p.block0 + (first + lane) / 6) >> f) & 1;
     }
-    return 0;
+    for (unsigned m = __ballot_sync(0xffffffffu, set); m; m &= m - 1) {
+        const int item = first + __ffs(m) - 1, f = item % 6, d = f >> 1, block = p.block0 + item / 6;
+        const int b12 = p.nb0.div(block), b0 = block - b12 * (int)p.nb0.d, b2 = p.nb1.div(b12), b1 = b12 - b2 * (int)p.nb1.d;
+        const int n = d == 0 ? V * L.n[1] * L.n[2] : L.n[0] * pick3(d, 0, L.n[2], L.n[1]);
+        for (int i = threadIdx.x; i < n; i += 256) {
+            int x, y, z;
+            if (d == 0) {
+                const int q = i / V;
+                z = p.f1.div(q);
+                y = q - z * L.n[1];
+                x = i - q * V + (f & 1 ? L.n[0] - V : 0);
+            } else {
+                const int q = p.f0.div(i);
+                x = i - q * L.n[0];
+                y = d == 1 ? (f & 1 ? L.n[1] - 1 : 0) : q;
+                z = d == 2 ? (f & 1 ? L.n[2] - 1 : 0) : q;
+            }
+            bc_cell<T, OP>(p, block, b0, b1, b2, x, y, z);
+        }
+    }
+}
+
+// offset to a neighbour across a side without BCs: side s of direction d
+// (stride st) at coordinate q of block coordinate b
+__device__ __forceinline__ int64_t side_offset(const LabGeom &L, int b, int d, int s, int q, int64_t st)
+{
+    const int n = L.n[d];
+    if (s ? q + 1 < n : q > 0) return s ? st : -st;
+    const int m = L.nb[d], nbr = s ? (b + 1 < m ? b + 1 : 0) : (b > 0 ? b - 1 : m - 1);
+    const int bs = d == 0 ? 1 : (d == 1 ? L.nb[0] : L.nb[0] * L.nb[1]);
+    return (s ? st : -st) + (int64_t)(nbr - b) * bs * L.bstride + (s ? -n : n) * st;
+}
+
+template <typename T, int OP, int V, int U>
+__global__ void __launch_bounds__(256) fd_kernel(const __grid_constant__ FdParams<T> p)
+{
+    if ((int)blockIdx.x < p.face_ctas) {
+        bc_faces<T, OP, V>(p);
+        return;
+    }
+    const int t = ((int)blockIdx.x - p.face_ctas) * 256 + threadIdx.x;
+    if (t >= p.total) return;
+    const LabGeom &L = p.L;
+    const int bl = p.per_block.div(t), r = t - bl * (int)p.per_block.d;
+    const int zc = p.plane.div(r), c = r - zc * (int)p.plane.d;
+    const int y = p.n0.div(c), x = V * (c - y * (int)p.n0.d);
+    const int block = p.block0 + bl;
+    int z0 = zc * p.TZ, z1 = min(z0 + p.TZ, L.n[2]);
+    // faces of the block that this run touches; those with BCs are bc_faces'
+    const unsigned fx = (x == 0 ? 1u : 0u) | (x + V == L.n[0] ? 2u : 0u), fy = (y == 0 ? 4u : 0u) | (y + 1 == L.n[1] ? 8u : 0u),
+                   fz = (z0 == 0 ? 16u : 0u) | (z1 == L.n[2] ? 32u : 0u);
+    bool skip0 = false, skip1 = false;
+    if (fx && (__ldg(p.bc[0].faces + block) & fx)) return;
+    if (fy && (__ldg(p.bc[1].faces + block) & fy)) return;
+    if (fz) {
+        const unsigned f = __ldg(p.bc[2].faces + block) & fz;
+        skip0 = f & 16u;
+        skip1 = f & 32u;
+    }
+    const int b12 = p.nb0.div(block), b0 = block - b12 * (int)p.nb0.d;
+    const int b2 = p.nb1.div(b12), b1 = b12 - b2 * (int)p.nb1.d;
+    const int64_t s1 = L.n[0], s2 = (int64_t)L.n[0] * L.n[1];
+    z0 += skip0;
+    z1 -= skip1;
+    if (z0 >= z1) return;
+    march<T, OP, V, U>(p, (int64_t)block * L.bstride + x + s1 * y + s2 * z0, s2, z1 - z0, side_offset(L, b0, 0, 0, x, 1),
+                       side_offset(L, b0, 0, 1, x + V - 1, 1), side_offset(L, b1, 1, 0, y, s1),
+                       side_offset(L, b1, 1, 1, y, s1), side_offset(L, b2, 2, 0, z0, s2),
+                       side_offset(L, b2, 2, 1, z1 - 1, s2));
 }
 
 static cn_status check_out(const cn_grid *in, const cn_grid *out, int out_comp, int ncomp_out)
@@ -329,6 +333,43 @@ static cn_status check_out(const cn_grid *in, const cn_grid *out, int out_comp, 
         return fail(CN_ERR_SIZE_MISMATCH, "Cartesian: Can not assign two grids of unequal size.");
     if (out_comp < 0 || out_comp + ncomp_out > out->ncomp)
         return fail(CN_ERR_INVALID_ARGUMENT, "output component out of range");
+    return CN_OK;
+}
+
+// Threads that fill the GPU (148 SMs, four CTAs): blocks with fewer columns in
+// all are cut into shorter runs of planes (twice as many threads measured the
+// same within 2 %).
+constexpr int64_t kFillThreads = 148 * 1024;
+
+template <typename T, int OP, int V> static cn_status launch_march(const cn_grid *u, FdParams<T> &p, cudaStream_t st)
+{
+    // planes whose loads are in flight together (FP64 divergence: its three
+    // fields' loads fill the registers with one, 695 against 837 us on 512^3)
+    constexpr int U = OP == kDiv && sizeof(T) == 8 ? 1 : 2;
+    const int N2 = u->n[2], cols = u->n[0] / V * u->n[1]; // columns of a block
+    const int64_t all = (int64_t)u->nblocks * cols;
+    int nzc = (int)std::min<int64_t>((N2 + U - 1) / U, std::max<int64_t>(1, (kFillThreads + all - 1) / all));
+    p.TZ = ((N2 + nzc - 1) / nzc + U - 1) / U * U;
+    nzc = (N2 + p.TZ - 1) / p.TZ;
+    const int per_block = cols * nzc;
+    p.per_block = FastDiv((uint32_t)per_block);
+    p.plane = FastDiv((uint32_t)cols);
+    p.n0 = FastDiv((uint32_t)(u->n[0] / V));
+    p.nb0 = FastDiv((uint32_t)u->nb[0]);
+    p.nb1 = FastDiv((uint32_t)u->nb[1]);
+    p.f0 = FastDiv((uint32_t)u->n[0]);
+    p.f1 = FastDiv((uint32_t)u->n[1]);
+    // one launch; beyond 2^30 threads, several over block ranges
+    const int most = (1 << 30) / per_block;
+    for (p.block0 = 0; p.block0 < u->nblocks; p.block0 += most) {
+        p.total = std::min(most, u->nblocks - p.block0) * per_block;
+        p.faces = p.total / per_block * 6;
+        // few blocks: a CTA each, so that their cells are resolved side by side
+        p.faces_per_cta = std::min(kFacesPerCta, p.faces / (148 * 2) + 1);
+        p.face_ctas = (p.faces + p.faces_per_cta - 1) / p.faces_per_cta;
+        fd_kernel<T, OP, V, U><<<(unsigned)(p.face_ctas + (p.total + 255) / 256), 256, 0, st>>>(p);
+        CN_CUDA_TRY(cudaGetLastError());
+    }
     return CN_OK;
 }
 
@@ -343,10 +384,10 @@ static cn_status launch_fd(cn_grid *u, int comp, cn_grid *o1, int c1, cn_grid *o
     if (stt != CN_OK) return stt;
     FdParams<T> p = {};
     p.L = make_geom(u, &s);
-    const int NC = OP == kDiv ? 3 : 1;
-    for (int c = 0; c < NC; ++c) {
-        p.in[c] = reinterpret_cast<const T *>(u->d_data) + (size_t)(comp + c) * u->comp_stride;
-        p.bc[c] = bc_view(u, comp + c);
+    for (int c = 0; c < 3; ++c) {
+        const int k = comp + (OP == kDiv ? c : 0);
+        p.in[c] = reinterpret_cast<const T *>(u->d_data) + (size_t)k * u->comp_stride;
+        p.bc[c] = bc_view(u, k);
     }
     if (o1) p.lap = reinterpret_cast<T *>(o1->d_data) + (size_t)c1 * o1->comp_stride;
     if (o2) {
@@ -357,28 +398,13 @@ static cn_status launch_fd(cn_grid *u, int comp, cn_grid *o1, int c1, cn_grid *o
         p.ih[d] = (T)(1. / u->h[d]);
         p.ih2[d] = (T)(1. / (u->h[d] * u->h[d]));
     }
-    const int N0 = u->n[0], N1 = u->n[1], N2 = u->n[2];
-    const int tz = pick_tz(N0, N1, N2, sizeof(T), NC, 100 * 1024);
-    if (tz == 0) return fail(CN_ERR_UNSUPPORTED, "block too large for the fused stencil tile");
-    p.TZ = tz;
-    p.dv0 = FastDiv((uint32_t)N0);
-    p.dv1 = FastDiv((uint32_t)N1);
-    p.dv01 = FastDiv((uint32_t)(N0 * N1));
-    p.dvh = FastDiv((uint32_t)(N0 / 2 > 0 ? N0 / 2 : 1));
-    const size_t tile_bytes = (size_t)N0 * N1 * tz * sizeof(T);
-    p.use_bulk = (tile_bytes % 16 == 0) && ((u->block_stride * sizeof(T)) % 16 == 0);
-    p.err = u->d_err;
-    const size_t smem = fd_smem_bytes(N0, N1, tz, sizeof(T), NC);
-    CN_CUDA_TRY(cudaFuncSetAttribute(fd_kernel<T, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-    // eight 256-thread CTAs per SM fit the registers (32 per thread): ask for
-    // the shared-memory carve-out that lets their tiles fit as well
-    CN_CUDA_TRY(cudaFuncSetAttribute(fd_kernel<T, OP>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared));
-    const int64_t ctas = (int64_t)u->nblocks * (N2 / tz);
-    fd_kernel<T, OP><<<(unsigned)ctas, 256, smem, st>>>(p);
-    CN_CUDA_TRY(cudaGetLastError());
-    return CN_OK;
+    const int N0 = u->n[0], N1 = u->n[1];
+    if (plane_bytes(N0, N1, sizeof(T), OP == kDiv ? 3 : 1) > kMaxPlaneBytes)
+        return fail(CN_ERR_UNSUPPORTED, "block too large for the fused stencil tile");
+    // cells per thread along x: 16 bytes where rows are multiples of them
+    if (sizeof(T) == 4 && N0 % 4 == 0) return launch_march<T, OP, 16 / sizeof(T)>(u, p, st);
+    if (N0 % 2 == 0) return launch_march<T, OP, 2>(u, p, st);
+    return launch_march<T, OP, 1>(u, p, st);
 }
 
 template <int OP>

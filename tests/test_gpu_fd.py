@@ -209,3 +209,62 @@ def test_fp32_lap_grad_div_periodic_vs_numpy(cn, oracle_lib, n):
     for d in range(3):
         assert np.array_equal(_glob(grad.download(d), nb, n, stride), want_g[d])
     assert np.array_equal(_glob(div.download(0), nb, n, stride), want_div)
+
+
+def _random_bcs(O, rng, nb):
+    """BC lists of one component: on about half of the block faces one to
+    three BCs (Base and repeats among them), faces inside the domain too."""
+    out = {}
+    for b in range(int(np.prod(nb))):
+        lst = [(int(d), int(s), int(k), float(v)) for d in range(3) for s in range(2) if rng.random() < 0.5
+               for k, v in zip(rng.integers(0, 4, size=rng.integers(1, 4)), (0.5, -1.0, 0.25))]
+        if lst:
+            out[b] = [lst[i] for i in rng.permutation(len(lst))]
+    return out
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("nb,n", [((2, 1, 3), (8, 5, 3)), ((1, 3, 2), (6, 4, 9)), ((3, 2, 1), (7, 1, 2)),
+                                  ((2, 2, 2), (12, 3, 33)), ((1, 1, 1), (4, 2, 1)), ((1, 2, 1), (1, 33, 40))])
+def test_random_bc_vectors_vs_oracle_labs(cn, oracle_lib, dtype, nb, n):
+    """Every component's own random BC vectors; rows of 4, 2 and 1 cells per
+    thread, runs of one plane and longer, blocks of one cell along a
+    direction.  The stencils, rounded operation by operation in numpy on the
+    oracle's labs, give the same bits."""
+    import torch
+    O = oracle_lib
+    rng = np.random.default_rng(sum(n))
+    nbk, stride = int(np.prod(nb)), O.block_stride(n, dtype)
+    comps = [rng.standard_normal(nbk * stride).astype(dtype) for _ in range(3)]
+    bcl = [_random_bcs(O, rng, nb) for _ in range(3)]
+    g = cn.Grid.Cartesian(nb, n, ncomp=3, dtype=dtype)
+    kinds = {0: cn.BC.Base, 1: cn.BC.Dirichlet, 2: cn.BC.Absorbing, 3: cn.BC.Symmetry}
+    for c in range(3):
+        g.upload(comps[c], c)
+        for b, lst in bcl[c].items():
+            for d, s, k, v in lst:
+                g.field(b, c).getBC().push_back(kinds[k](d, s, v) if k in (1, 3) else kinds[k](d, s))
+    lap, div = (cn.Grid.Cartesian(nb, n, dtype=dtype) for _ in range(2))
+    grad = cn.Grid.Cartesian(nb, n, ncomp=3, dtype=dtype)
+    _run(cn, "lap_grad", g, (lap, grad))
+    _run(cn, "divergence", g, (div,))
+    T = dtype
+    ih = [T(1.0 / x) for x in g.getCellSize()]
+    ih2 = [T(1.0 / (x * x)) for x in g.getCellSize()]
+    got = [a.blocks_view(a.download(k)) for a, k in ((lap, 0), (grad, 0), (grad, 1), (grad, 2), (div, 0))]
+    m = slice(1, -1)
+    for b in range(nbk):
+        labs = []
+        for c in range(3):
+            lab, ok = O.lab_fill(comps[c], nb, n, (1, 1, 1), (1, 1, 1), False, bcl[c], b)
+            labs.append(np.where(ok, lab, T(0)).astype(T))
+        lo = [(m, m, slice(0, -2)), (m, slice(0, -2), m), (slice(0, -2), m, m)]
+        hi = [(m, m, slice(2, None)), (m, slice(2, None), m), (slice(2, None), m, m)]
+        u = labs[0]
+        c2 = T(2) * u[m, m, m]
+        dd = [ih2[d] * ((u[hi[d]] - c2) + u[lo[d]]) for d in range(3)]
+        dv = [(labs[d][hi[d]] - labs[d][lo[d]]) * ih[d] for d in range(3)]
+        want = [(dd[0] + dd[1]) + dd[2]] + [T(0.5) * ((u[hi[d]] - u[lo[d]]) * ih[d]) for d in range(3)]
+        want.append(T(0.5) * ((dv[0] + dv[1]) + dv[2]))
+        for what, (a, w) in enumerate(zip(got, want)):
+            assert np.array_equal(a[b], w), f"output {what}, block {b}"
