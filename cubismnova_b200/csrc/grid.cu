@@ -510,6 +510,7 @@ cn_status cn_bc_push(cn_grid *g, int comp, int block, int dir, int side, cn_bc_k
         return fail(CN_ERR_TOO_MANY_BC, "cn_bc_push: BC vector of this block field is full");
     }
     v.push_back(HostBC{dir, side, (int)kind, value});
+    ++g->bc_count;
     g->bc_dirty = true;
     return CN_OK;
 }
@@ -536,8 +537,12 @@ cn_status cn_bc_clear(cn_grid *g, int comp, int block)
         return fail(CN_ERR_INVALID_ARGUMENT, "cn_bc_clear: bad grid, component or block");
     }
     if (block < 0) {
-        for (auto &v : g->bcs[comp]) v.clear();
+        for (auto &v : g->bcs[comp]) {
+            g->bc_count -= (int64_t)v.size();
+            v.clear();
+        }
     } else {
+        g->bc_count -= (int64_t)g->bcs[comp][block].size();
         g->bcs[comp][block].clear();
     }
     g->bc_dirty = true;

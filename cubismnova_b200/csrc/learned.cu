@@ -820,6 +820,8 @@ static cn_status features(cn_mg *m, int l, const float *p, const float *f, float
                           uint16_t *packed = nullptr)
 {
     cn_grid *X = m->nn_bufs[4 * l];
+    const cn_status cs = mg_ensure_coef(m, st);
+    if (cs != CN_OK) return cs;
     FeatArgs A;
     A.L = make_geom(m->p[l], &kS1);
     A.pbc = bc_view(m->p[l], 0);

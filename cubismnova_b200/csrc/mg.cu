@@ -17,8 +17,10 @@
 // the same lab resolution as every other stencil (periodic block wrap, and the
 // grid's BCs if any); halo cells inside a block are plain cached loads.
 #include "cn_internal.h"
+#include "mg_march.cuh"
 #include "mg_tile.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -75,99 +77,69 @@ __device__ __forceinline__ int64_t dense_cell(const LabGeom &L, const TilePos &q
     return (q.x0 + x) + (int64_t)L.n[0] * ((q.y0 + y) + (int64_t)L.n[1] * (q.z0 + z));
 }
 
-// Coefficients of one level (see op7_coef) in precision TC (float for the
-// V-cycle; resid64_kernel forms the FP64 means itself with the same
-// operations): k staged per tile with its one-cell halo, then per cell the
-// operations of op7_math in TC.
-template <typename TC>
-__global__ void __launch_bounds__(kTileThreads, kTileMinCtas) coef_kernel(const __grid_constant__ KArgs a,
-                                                                          const __grid_constant__ Tile T, TC ih2,
-                                                                          TC *coef)
+// Face means of one level from the lab of k, and with D the diagonal, with the
+// operations of op7_math in T.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    faces_kernel(const __grid_constant__ LabGeom L, const __grid_constant__ BcView kbc, const float *k, int nblocks, T ih2,
+                 const __grid_constant__ Faces<T> F, T *D)
 {
-    __shared__ __align__(16) float sk[kRegionMax];
-    __shared__ int snb[27];
-    const LabGeom &L = a.G.L;
-    TilePos q = tile_pos(T);
-    region_layout<float>(q, a.G.Lk);
-    neighbour_blocks(L.nb, q.block, snb);
-    __syncthreads();
-    stage_region<float>(a.k, a.G.Lk, a.kbc, q, false, snb, sk);
-    cp_async_wait_all();
-    __syncthreads();
-    int x, y, z0, zl;
-    if (!column_run(T, x, y, z0, zl)) return;
-    const int st[3] = {1, q.rs, q.rs * q.ey};
-    const int64_t cells = (int64_t)L.n[0] * L.n[1] * L.n[2];
-    for (int z = z0; z < z0 + zl; ++z) {
-        TC *cv = coef + ((int64_t)q.block * cells + dense_cell(L, q, x, y, z)) * kCoefPerCell;
-        const int u = ridx(q, x, y, z);
-        const TC kc = (TC)sk[u];
-        TC sd[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const TC kp = harm<TC>(kc, (TC)sk[u + st[d]]);
-            const TC km = harm<TC>((TC)sk[u - st[d]], kc);
-            cv[d] = kp;
-            cv[3 + d] = km;
-            sd[d] = kp + km;
-        }
-        cv[6] = ih2 * ((sd[0] + sd[1]) + sd[2]);
-        cv[7] = TC(0);
-    }
-}
-
-// FP64 harmonic face means of the finest level, each face once: per block
-// the x faces ((n0 + 1) n1 n2, face i between cells i - 1 and i), then the y
-// and z faces, x fastest.  A cell writes its +d faces, and cells on the
-// block's lower side also their -d face, with the operations of coef_kernel:
-// harm(kc, k(+e_d)) and harm(k(-e_d), kc), which are the same bits since
-// harm is symmetric.  Boundary faces use this block's lab of k.
-__host__ __device__ inline int64_t face_count(const int n[3])
-{
-    return (int64_t)(n[0] + 1) * n[1] * n[2] + (int64_t)n[0] * (n[1] + 1) * n[2] + (int64_t)n[0] * n[1] * (n[2] + 1);
-}
-
-__device__ __forceinline__ int64_t face_index(const int n[3], int d, int x, int y, int z)
-{
-    if (d == 0) return x + (int64_t)(n[0] + 1) * (y + (int64_t)n[1] * z);
-    const int64_t fx = (int64_t)(n[0] + 1) * n[1] * n[2];
-    if (d == 1) return fx + x + (int64_t)n[0] * (y + (int64_t)(n[1] + 1) * z);
-    return fx + (int64_t)n[0] * (n[1] + 1) * n[2] + x + (int64_t)n[0] * (y + (int64_t)n[1] * z);
-}
-
-__global__ void __launch_bounds__(kTileThreads, kTileMinCtas) face64_kernel(const __grid_constant__ KArgs a,
-                                                                            const __grid_constant__ Tile T,
-                                                                            double *faces)
-{
-    __shared__ __align__(16) float sk[kRegionMax];
-    __shared__ int snb[27];
-    const LabGeom &L = a.G.Lk;
-    TilePos q = tile_pos(T);
-    region_layout<float>(q, L);
-    neighbour_blocks(L.nb, q.block, snb);
-    __syncthreads();
-    stage_region<float>(a.k, L, a.kbc, q, false, snb, sk);
-    cp_async_wait_all();
-    __syncthreads();
-    int x, y, z0, zl;
-    if (!column_run(T, x, y, z0, zl)) return;
-    const int st[3] = {1, q.rs, q.rs * q.ey};
-    double *fb = faces + (int64_t)q.block * face_count(L.n);
-    for (int z = z0; z < z0 + zl; ++z) {
-        const int u = ridx(q, x, y, z);
-        const double kc = (double)sk[u];
-        const int g[3] = {q.x0 + x, q.y0 + y, q.z0 + z};
+    const int cells = L.n[0] * L.n[1] * L.n[2];
+    const int64_t total = (int64_t)nblocks * cells;
+    for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < total; t += (int64_t)gridDim.x * 256) {
+        int b, x, y, z;
+        cell_of(t, L, b, x, y, z);
+        const T kc = (T)fetch<float>(k, L, kbc, b, x, y, z);
+        const int q[3] = {x, y, z};
+        T sd[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const int ex = d == 0, ey = d == 1, ez = d == 2;
-            fb[face_index(L.n, d, g[0] + ex, g[1] + ey, g[2] + ez)] = harm<double>(kc, (double)sk[u + st[d]]);
-            if (g[d] == 0)
-                fb[face_index(L.n, d, g[0], g[1], g[2])] = harm<double>((double)sk[u - st[d]], kc);
+            const T kp = harm<T>(kc, (T)fetch<float>(k, L, kbc, b, x + ex, y + ey, z + ez));
+            const T km = harm<T>((T)fetch<float>(k, L, kbc, b, x - ex, y - ey, z - ez), kc);
+            F.k[d][t] = km;
+            if (q[d] == L.n[d] - 1) {
+                const int64_t i = d == 0 ? y + (int64_t)L.n[1] * z : (d == 1 ? x + (int64_t)L.n[0] * z : x + (int64_t)L.n[0] * y);
+                F.u[d][(int64_t)b * (cells / L.n[d]) + i] = kp;
+            }
+            sd[d] = kp + km;
         }
+        if (D) D[t] = ih2 * ((sd[0] + sd[1]) + sd[2]);
     }
 }
 
-// weighted Jacobi sweep: pout = pin + omega (L pin - f) / D  (pin == NULL: zero guess)
+// mean across the upper face along d of dense cell t = (b, x, y, z)
+template <typename T>
+__device__ __forceinline__ T upper_mean(const Faces<T> &F, const LabGeom &L, int64_t t, int b, int x, int y, int z, int d)
+{
+    const int q = d == 0 ? x : (d == 1 ? y : z);
+    const int64_t st = d == 0 ? 1 : (d == 1 ? L.n[0] : (int64_t)L.n[0] * L.n[1]);
+    if (q + 1 < L.n[d]) return __ldg(F.k[d] + t + st);
+    const int64_t i = d == 0 ? y + (int64_t)L.n[1] * z : (d == 1 ? x + (int64_t)L.n[0] * z : x + (int64_t)L.n[0] * y);
+    return __ldg(F.u[d] + (int64_t)b * ((int64_t)L.n[0] * L.n[1] * L.n[2] / L.n[d]) + i);
+}
+
+// The tile kernels' coefficients (see op7_coef) from the face means.
+__global__ void __launch_bounds__(256)
+    coef_kernel(const __grid_constant__ LabGeom L, int nblocks, const __grid_constant__ Faces<float> F, const float *D,
+                float *coef)
+{
+    const int64_t total = (int64_t)nblocks * L.n[0] * L.n[1] * L.n[2];
+    for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < total; t += (int64_t)gridDim.x * 256) {
+        int b, x, y, z;
+        cell_of(t, L, b, x, y, z);
+        float *cv = coef + t * kCoefPerCell;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            cv[d] = upper_mean<float>(F, L, t, b, x, y, z, d);
+            cv[3 + d] = F.k[d][t];
+        }
+        cv[6] = D[t];
+        cv[7] = 0.0f;
+    }
+}
+
+// weighted Jacobi sweep: pout = pin + omega (L pin - f) / D
 __global__ void __launch_bounds__(kTileThreads, kTileMinCtas) jacobi_kernel(const __grid_constant__ KArgs a,
                                                               const __grid_constant__ Tile T, const float *pin,
                                                               const float *f, float *pout, float omega)
@@ -177,13 +149,11 @@ __global__ void __launch_bounds__(kTileThreads, kTileMinCtas) jacobi_kernel(cons
     const LabGeom &L = a.G.L;
     TilePos q = tile_pos(T);
     region_layout<float>(q, L);
-    if (pin) {
-        neighbour_blocks(L.nb, q.block, snb);
-        __syncthreads();
-        stage_region<float>(pin, L, a.G.bc, q, false, snb, sp);
-        cp_async_wait_all();
-        __syncthreads();
-    }
+    neighbour_blocks(L.nb, q.block, snb);
+    __syncthreads();
+    stage_region<float>(pin, L, a.G.bc, q, false, snb, sp);
+    cp_async_wait_all();
+    __syncthreads();
     int x, y, z0, zl;
     if (!column_run(T, x, y, z0, zl)) return;
     const int st[3] = {1, q.rs, q.rs * q.ey};
@@ -205,20 +175,16 @@ __global__ void __launch_bounds__(kTileThreads, kTileMinCtas) jacobi_kernel(cons
             nb = __ldg(cv + cvz + 1);
             nf = __ldg(f + o + oz);
         }
-        if (pin) {
-            const float cc[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
-            const float pc = sp[u];
-            float fl[3];
+        const float cc[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+        const float pc = sp[u];
+        float fl[3];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const float kp = cc[d], km = cc[3 + d];
-                fl[d] = kp * (sp[u + st[d]] - pc) - km * (pc - sp[u - st[d]]);
-            }
-            const float Lp = a.ih2 * ((fl[0] + fl[1]) + fl[2]);
-            pout[o] = pc + omega * ((Lp - fc) / cb.z);
-        } else {
-            pout[o] = 0.0f + omega * ((0.0f - fc) / cb.z);
+        for (int d = 0; d < 3; ++d) {
+            const float kp = cc[d], km = cc[3 + d];
+            fl[d] = kp * (sp[u + st[d]] - pc) - km * (pc - sp[u - st[d]]);
         }
+        const float Lp = a.ih2 * ((fl[0] + fl[1]) + fl[2]);
+        pout[o] = pc + omega * ((Lp - fc) / cb.z);
         ca = na;
         cb = nb;
         fc = nf;
@@ -351,13 +317,12 @@ __global__ void __launch_bounds__(kTileThreads, kTileMinCtas) prolong_kernel(con
 
 // FP64 residual of the outer iteration: r = f - L p64, r32 = (float) r,
 // per-CTA FP64 partial sums of r^2 and f^2.  The tile's p64 is staged with
-// its one-cell halo; the six face means of a cell come from the FP64 face
-// arrays (face64_kernel) and are applied in op7_coef's order, so L p64 is
-// bit for bit the operator of the per-cell coefficients.
+// its one-cell halo; the six FP64 face means of a cell are applied in
+// op7_coef's order.
 __global__ void __launch_bounds__(kTileThreads, 4) resid64_kernel(const __grid_constant__ KArgs a,
                                                                const __grid_constant__ Tile T, const double *p64,
                                                                const float *f, float *r32, double *partials,
-                                                               const double *faces)
+                                                               const __grid_constant__ Faces<double> F)
 {
     __shared__ __align__(16) double sp[kRegionMax];
     __shared__ double sh[2][kTileThreads / 32];
@@ -374,47 +339,19 @@ __global__ void __launch_bounds__(kTileThreads, 4) resid64_kernel(const __grid_c
     int x, y, z0, zl;
     if (column_run(T, x, y, z0, zl)) {
         const int st[3] = {1, q.rs, q.rs * q.ey};
-        const double *fb = faces + (int64_t)q.block * face_count(Lk.n);
-        // the six face indices of the column's first cell; along z they
-        // advance by each face array's plane size, and the next cell's
-        // loads go out before this cell's arithmetic
-        const int gx = q.x0 + x, gy = q.y0 + y, gz = q.z0 + z0;
-        const int64_t dz[3] = {(int64_t)(Lk.n[0] + 1) * Lk.n[1], (int64_t)Lk.n[0] * (Lk.n[1] + 1),
-                               (int64_t)Lk.n[0] * Lk.n[1]};
-        int64_t im[3], ip[3];
-        im[0] = face_index(Lk.n, 0, gx, gy, gz);
-        ip[0] = im[0] + 1;
-        im[1] = face_index(Lk.n, 1, gx, gy, gz);
-        ip[1] = im[1] + Lk.n[0];
-        im[2] = face_index(Lk.n, 2, gx, gy, gz);
-        ip[2] = im[2] + dz[2];
-        int64_t o = (int64_t)q.block * Lk.bstride + dense_cell(Lk, q, x, y, z0); // FP32 fields (f, r32)
-        const int64_t oz = (int64_t)Lk.n[0] * Lk.n[1];
-        double km[3], kp[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            km[d] = __ldg(fb + im[d]);
-            kp[d] = __ldg(fb + ip[d]);
-        }
-        float fcf = __ldg(f + o);
+        const int gx = q.x0 + x, gy = q.y0 + y;
+        int64_t dc = dense_cell(Lk, q, x, y, z0);
+        const int64_t cells = (int64_t)Lk.n[0] * Lk.n[1] * Lk.n[2], oz = (int64_t)Lk.n[0] * Lk.n[1];
+        int64_t o = (int64_t)q.block * Lk.bstride + dc; // FP32 fields (f, r32)
         int u = ridx(q, x, y, z0);
-        for (int k = 0; k < zl; ++k, u += st[2], o += oz) {
-            double nkm[3], nkp[3];
-            float nf = fcf;
+        for (int k = 0; k < zl; ++k, u += st[2], o += oz, dc += oz) {
+            const int64_t t = (int64_t)q.block * cells + dc;
+            const float fcf = __ldg(f + o);
+            double km[3], kp[3];
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                nkm[d] = km[d];
-                nkp[d] = kp[d];
-            }
-            if (k + 1 < zl) {
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    im[d] += dz[d];
-                    ip[d] += dz[d];
-                    nkm[d] = __ldg(fb + im[d]);
-                    nkp[d] = __ldg(fb + ip[d]);
-                }
-                nf = __ldg(f + o + oz);
+                km[d] = __ldg(F.k[d] + t);
+                kp[d] = upper_mean<double>(F, Lk, t, q.block, gx, gy, q.z0 + z0 + k, d);
             }
             const double pc = sp[u];
             double fd[3];
@@ -427,12 +364,6 @@ __global__ void __launch_bounds__(kTileThreads, 4) resid64_kernel(const __grid_c
             if (r32) r32[o] = (float)r;
             rr += r * r;
             ff += fc * fc;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                km[d] = nkm[d];
-                kp[d] = nkp[d];
-            }
-            fcf = nf;
         }
     }
     for (int off = 16; off > 0; off >>= 1) {
@@ -710,22 +641,154 @@ unsigned grid_for(int64_t n)
 
 float *fptr(cn_grid *g) { return reinterpret_cast<float *>(g->d_data); }
 
-// weighted Jacobi sweeps on level l (p = 0 on entry if zero_guess)
-static cn_status smooth(cn_mg *m, int l, int sweeps, bool zero_guess, cudaStream_t st)
+// Threads that fill the GPU (148 SMs, eight CTAs of 256): levels with fewer
+// columns in all are cut into shorter runs of planes (half as many: 5 % more
+// per solve on 256^3; twice as many: 1 %).
+constexpr int64_t kFillThreads = 148 * 2048;
+
+// Layout of a marching launch over a level shaped like g: V cells and R rows a
+// thread, runs of planes in multiples of `unit`.
+static Layer layer_of(const cn_grid *g, int V, int R, int unit, const cn_grid *g64 = nullptr)
 {
-    KArgs a = kargs(m, l);
-    const Tile T = tile_of(m->p[l]->n);
+    Layer a;
+    for (int d = 0; d < 3; ++d) {
+        a.n[d] = g->n[d];
+        a.nb[d] = g->nb[d];
+    }
+    a.bs = (uint32_t)g->block_stride;
+    a.bs64 = g64 ? (uint32_t)g64->block_stride : 0;
+    const int cols = g->n[0] / V * (g->n[1] / R), N2 = g->n[2];
+    const int64_t all = (int64_t)g->nblocks * cols;
+    int nzc = (int)std::min<int64_t>((N2 + unit - 1) / unit, std::max<int64_t>(1, (kFillThreads + all - 1) / all));
+    a.TZ = ((N2 + nzc - 1) / nzc + unit - 1) / unit * unit;
+    nzc = (N2 + a.TZ - 1) / a.TZ;
+    a.per_block = FastDiv((uint32_t)(cols * nzc));
+    a.plane = FastDiv((uint32_t)cols);
+    a.row = FastDiv((uint32_t)(g->n[0] / V));
+    a.nb0 = FastDiv((uint32_t)g->nb[0]);
+    a.nb1 = FastDiv((uint32_t)g->nb[1]);
+    a.total = (int)(all * nzc);
+    return a;
+}
+static unsigned ctas_of(const Layer &a) { return (unsigned)((a.total + 255) / 256); }
+static int width_of(const cn_grid *g, int most)
+{
+    for (int v = most; v > 1; v /= 2)
+        if (g->n[0] % v == 0) return v;
+    return 1;
+}
+static float level_ih2(const cn_grid *g) { return (float)(1.0 / (g->h[0] * g->h[0])); }
+
+// one sweep by the marching kernel; with p64: also p64 += pout
+template <int V> static void launch_jacobi(cn_mg *m, int l, const float *src, const float *f, float *dst, cn_grid *p64, cudaStream_t st)
+{
+    const cn_grid *g = m->p[l];
+    const float ih2 = level_ih2(g), om = (float)m->omega;
+    if (p64) {
+        const Layer a = layer_of(g, V, 1, 1, p64);
+        jacobi_march<V, 2, true><<<ctas_of(a), 256, 0, st>>>(a, m->faces[l], ih2, om, src, f, dst,
+                                                             reinterpret_cast<double *>(p64->d_data));
+    } else {
+        const Layer a = layer_of(g, V, 1, 1);
+        jacobi_march<V, 2, false><<<ctas_of(a), 256, 0, st>>>(a, m->faces[l], ih2, om, src, f, dst, nullptr);
+    }
+}
+// (g: the grid whose BCs hold, m->p[l] as the smoothing starts; with p64, dst
+// is m->p[l] by now)
+static cn_status jacobi_sweep(cn_mg *m, int l, const cn_grid *g, const float *src, const float *f, float *dst, cn_grid *p64,
+                              cudaStream_t st)
+{
+    if (g->bc_count) {
+        cn_status s = mg_ensure_coef(m, st);
+        if (s != CN_OK) return s;
+        const Tile T = tile_of(g->n);
+        KArgs a = kargs(m, l);
+        a.G.bc = bc_view(g, 0);
+        jacobi_kernel<<<(unsigned)(g->nblocks * T.count), kTileThreads, 0, st>>>(a, T, src, f, dst, (float)m->omega);
+        CN_CUDA_TRY(cudaGetLastError());
+        return p64 ? cn_mg_accumulate(m, p64, st) : CN_OK;
+    }
+    switch (width_of(g, 4)) {
+    case 4: launch_jacobi<4>(m, l, src, f, dst, p64, st); break;
+    case 2: launch_jacobi<2>(m, l, src, f, dst, p64, st); break;
+    default: launch_jacobi<1>(m, l, src, f, dst, p64, st);
+    }
+    CN_CUDA_TRY(cudaGetLastError());
+    return CN_OK;
+}
+
+// weighted Jacobi sweeps on level l.  From a zero guess the first sweep needs
+// only f and D; `first_done`: the kernel that made f has already written it to
+// pt.  add: p64 += the result, by the last sweep (at least one).
+static cn_status smooth(cn_mg *m, int l, int sweeps, bool zero_guess, bool first_done, cn_grid *add, cudaStream_t st)
+{
+    const cn_grid *g = m->p[l];
     for (int s = 0; s < sweeps; ++s) {
-        const bool zg = zero_guess && s == 0;
         // ping-pong so that the result of the last sweep lands in p
         float *src = fptr(m->p[l]), *dst = fptr(m->pt[l]);
-        jacobi_kernel<<<(unsigned)(m->p[l]->nblocks * T.count), kTileThreads, 0, st>>>(
-            a, T, zg ? nullptr : src, fptr(m->f[l]), dst, (float)m->omega);
-        CN_CUDA_TRY(cudaGetLastError());
         std::swap(m->p[l], m->pt[l]);
+        if (zero_guess && s == 0) {
+            if (first_done) continue;
+            const int cells = g->n[0] * g->n[1] * g->n[2];
+            const int64_t total = (int64_t)g->nblocks * cells;
+            jacobi_first<<<grid_for(total), 256, 0, st>>>(total, FastDiv((uint32_t)cells), (uint32_t)g->block_stride,
+                                                          m->diag[l], fptr(m->f[l]), dst, (float)m->omega);
+            CN_CUDA_TRY(cudaGetLastError());
+            continue;
+        }
+        const cn_status r = jacobi_sweep(m, l, g, src, fptr(m->f[l]), dst, s == sweeps - 1 ? add : nullptr, st);
+        if (r != CN_OK) return r;
     }
     if (sweeps == 0 && zero_guess)
         CN_CUDA_TRY(cudaMemsetAsync(m->p[l]->d_data, 0, (size_t)m->p[l]->comp_stride * 4, st));
+    return CN_OK;
+}
+
+// residual of level l restricted into fc (a grid shaped like level l + 1);
+// with pc, also the coarse level's first sweep from zero
+static cn_status restrict_residual(cn_mg *m, int l, const float *p, const float *f, cn_grid *fc, float *pc, cudaStream_t st)
+{
+    const cn_grid *g = m->p[l];
+    if (g->bc_count) {
+        cn_status s = mg_ensure_coef(m, st);
+        if (s != CN_OK) return s;
+        const Tile T = tile_of(g->n);
+        resid_restrict_kernel<<<(unsigned)(g->nblocks * T.count), kTileThreads, 0, st>>>(kargs(m, l), T, p, f, make_geom(fc, &kS1),
+                                                                                         fptr(fc));
+    } else {
+        const int V = width_of(g, 4);
+        const Layer a = layer_of(g, V, 2, 2);
+        const float ih2 = level_ih2(g), om = (float)m->omega;
+        const uint32_t bsc = (uint32_t)fc->block_stride;
+        if (V == 4)
+            resid_restrict_march<4><<<ctas_of(a), 256, 0, st>>>(a, m->faces[l], ih2, om, p, f, fptr(fc), pc,
+                                                                pc ? m->diag[l + 1] : nullptr, bsc);
+        else
+            resid_restrict_march<2><<<ctas_of(a), 256, 0, st>>>(a, m->faces[l], ih2, om, p, f, fptr(fc), pc,
+                                                                pc ? m->diag[l + 1] : nullptr, bsc);
+    }
+    CN_CUDA_TRY(cudaGetLastError());
+    return CN_OK;
+}
+
+// p += prolongation of the coarse correction ec
+static cn_status prolong(const cn_grid *ec, cn_grid *p, cudaStream_t st)
+{
+    if (ec->bc_count) {
+        const LabGeom Lf = make_geom(p, &kS1), Lct = make_geom(ec, &kS1t);
+        const Tile T = tile_of(p->n);
+        prolong_kernel<<<(unsigned)(p->nblocks * T.count), kTileThreads, 0, st>>>(
+            Lf, T, fptr(p), Lct, bc_view(ec, 0), reinterpret_cast<const float *>(ec->d_data));
+    } else {
+        const int V = width_of(p, 4);
+        const Layer a = layer_of(p, V, 1, 2);
+        const float *e = reinterpret_cast<const float *>(ec->d_data);
+        if (V == 4)
+            prolong_march<4><<<ctas_of(a), 256, 0, st>>>(a, fptr(p), e, (uint32_t)ec->block_stride);
+        else
+            prolong_march<2><<<ctas_of(a), 256, 0, st>>>(a, fptr(p), e, (uint32_t)ec->block_stride);
+    }
+    CN_CUDA_TRY(cudaGetLastError());
     return CN_OK;
 }
 
@@ -751,42 +814,142 @@ static cn_status coarsest(cn_mg *m, int l, cudaStream_t st)
 }
 
 
-// pre-smoothing (post = false, from a zero guess) or post-smoothing of level
-// l: the learned smoother where its level masks select it, else Jacobi
-static cn_status smooth_any(cn_mg *m, int l, bool post, cudaStream_t st)
+// whether level l is smoothed by Jacobi in the given phase (else by the network)
+static bool jacobi_level(const cn_mg *m, int l, bool post)
 {
-    const int sweeps = post ? m->nu2 : m->nu1;
-    const unsigned mask = post ? m->nn_post_levels : m->nn_levels;
-    if (m->nn && ((mask >> l) & 1)) {
-        const int apps = post ? m->nn_post_apps : m->nn_pre_apps;
-        return nn_smooth(m, l, apps >= 0 ? apps : sweeps, !post, st);
-    }
-    return smooth(m, l, sweeps, !post, st);
+    return !(m->nn && (((post ? m->nn_post_levels : m->nn_levels) >> l) & 1));
+}
+// whether the kernel that makes level l's right-hand side also writes its
+// first pre-smoothing sweep (into pt)
+static bool first_fused(const cn_mg *m, int l)
+{
+    return l < m->nlevels - 1 && m->nu1 > 0 && jacobi_level(m, l, false);
 }
 
-cn_status vcycle(cn_mg *m, int l, cudaStream_t st)
+// First level of the V-cycle's coarse part that one launch takes (tail_kernel),
+// or nlevels: at most kTailCells cells, the coarsest level solved by its dense
+// inverse, Jacobi smoothing, no BCs.
+static int tail_level(const cn_mg *m)
 {
-    if (l == m->nlevels - 1) return coarsest(m, l, st);
-    cn_status s = smooth_any(m, l, false, st);
-    if (s != CN_OK) return s;
-    KArgs a = kargs(m, l);
-    const LabGeom Lc = make_geom(m->p[l + 1], &kS1);
-    const Tile T = tile_of(m->p[l]->n);
-    resid_restrict_kernel<<<(unsigned)(m->p[l]->nblocks * T.count), kTileThreads, 0, st>>>(
-        a, T, fptr(m->p[l]), fptr(m->f[l]), Lc, fptr(m->f[l + 1]));
+    if (!m->coarse_inv || m->nlevels < 2) return m->nlevels;
+    int l = m->nlevels - 1;
+    if (m->p[l]->bc_count) return m->nlevels;
+    while (l > 1 && m->nlevels - l < kTailLevels) {
+        const cn_grid *g = m->p[l - 1];
+        if ((int64_t)g->nblocks * g->n[0] * g->n[1] * g->n[2] > kTailCells || g->bc_count || !jacobi_level(m, l - 1, false) ||
+            !jacobi_level(m, l - 1, true))
+            break;
+        --l;
+    }
+    return l < m->nlevels - 1 ? l : m->nlevels;
+}
+
+static cn_status tail(cn_mg *m, int l0, bool first_done, cudaStream_t st)
+{
+    Tail t = {};
+    t.levels = m->nlevels - l0;
+    t.nu1 = m->nu1;
+    t.nu2 = m->nu2;
+    t.omega = (float)m->omega;
+    t.first_done = first_done;
+    t.inv = m->coarse_inv;
+    t.N = m->coarse_n;
+    for (int l = l0; l < m->nlevels; ++l) {
+        TailLevel &L = t.lev[l - l0];
+        const cn_grid *g = m->p[l];
+        const bool last = l == m->nlevels - 1;
+        L.one = layer_of(g, last ? 1 : 2, 1, 1);
+        if (!last) {
+            L.two = layer_of(g, 2, 2, 2);
+            L.pro = layer_of(g, 2, 1, 2);
+        }
+        L.F = m->faces[l];
+        L.D = m->diag[l];
+        L.p = fptr(m->p[l]);
+        L.pt = fptr(m->pt[l]);
+        L.f = fptr(m->f[l]);
+        L.ih2 = level_ih2(g);
+        if (!last && ((m->nu1 + m->nu2) & 1)) std::swap(m->p[l], m->pt[l]);
+    }
+    tail_kernel<<<kTailCtas, kTailThreads, 0, st>>>(t);
     CN_CUDA_TRY(cudaGetLastError());
-    s = vcycle(m, l + 1, st);
+    return CN_OK;
+}
+
+// One V-cycle from level l down, from a zero guess.  first_done: see smooth;
+// add (level 0): p64 += the cycle's result.
+static cn_status vcycle_from(cn_mg *m, int l, bool first_done, cn_grid *add, cudaStream_t st)
+{
+    if (l == m->nlevels - 1) {
+        cn_status s = coarsest(m, l, st);
+        return s == CN_OK && add ? cn_mg_accumulate(m, add, st) : s;
+    }
+    if (l > 0 && l == tail_level(m)) return tail(m, l, first_done, st);
+    cn_status s = jacobi_level(m, l, false)
+                      ? smooth(m, l, m->nu1, true, first_done, nullptr, st)
+                      : nn_smooth(m, l, m->nn_pre_apps >= 0 ? m->nn_pre_apps : m->nu1, true, st);
     if (s != CN_OK) return s;
-    const LabGeom Lf = make_geom(m->p[l], &kS1);
-    const LabGeom Lct = make_geom(m->p[l + 1], &kS1t);
-    prolong_kernel<<<(unsigned)(m->p[l]->nblocks * T.count), kTileThreads, 0, st>>>(
-        Lf, T, fptr(m->p[l]), Lct, bc_view(m->p[l + 1], 0), fptr(m->p[l + 1]));
-    CN_CUDA_TRY(cudaGetLastError());
+    const bool fused = first_fused(m, l + 1) && !m->p[l]->bc_count;
+    s = restrict_residual(m, l, fptr(m->p[l]), fptr(m->f[l]), m->f[l + 1], fused ? fptr(m->pt[l + 1]) : nullptr, st);
+    if (s == CN_OK) s = vcycle_from(m, l + 1, fused, nullptr, st);
+    if (s == CN_OK) s = prolong(m->p[l + 1], m->p[l], st);
+    if (s != CN_OK) return s;
     if (l == 0 && m->capture) {
         s = m->capture(m, st);
         if (s != CN_OK) return s;
     }
-    return smooth_any(m, l, true, st);
+    const bool jac = jacobi_level(m, l, true);
+    s = jac ? smooth(m, l, m->nu2, false, false, add, st)
+            : nn_smooth(m, l, m->nn_post_apps >= 0 ? m->nn_post_apps : m->nu2, false, st);
+    if (s == CN_OK && add && !(jac && m->nu2 > 0)) s = cn_mg_accumulate(m, add, st);
+    return s;
+}
+
+cn_status vcycle(cn_mg *m, int l, cudaStream_t st) { return vcycle_from(m, l, false, nullptr, st); }
+
+cn_status mg_ensure_coef(cn_mg *m, cudaStream_t st)
+{
+    for (int l = (int)m->coef.size(); l < m->nlevels; ++l) {
+        const cn_grid *g = m->p[l];
+        const int64_t cells = (int64_t)g->nblocks * g->n[0] * g->n[1] * g->n[2];
+        float *c = nullptr;
+        if (cudaMalloc(&c, sizeof(float) * kCoefPerCell * cells) != cudaSuccess)
+            return fail(CN_ERR_OUT_OF_MEMORY, "multigrid: coefficients");
+        m->coef.push_back(c);
+        coef_kernel<<<grid_for(cells), 256, 0, st>>>(make_geom(g, &kS1), g->nblocks, m->faces[l], m->diag[l], c);
+        CN_CUDA_TRY(cudaGetLastError());
+    }
+    return CN_OK;
+}
+
+// Allocates and fills the face means of a level (and its diagonal).
+template <typename T> static cn_status make_faces(cn_mg *m, int l, Faces<T> &F, T ih2, T **diag)
+{
+    const cn_grid *g = m->p[l];
+    const int64_t n0 = g->n[0], n1 = g->n[1], n2 = g->n[2], cells = (int64_t)g->nblocks * n0 * n1 * n2;
+    const int64_t face[3] = {n1 * n2, n0 * n2, n0 * n1};
+    auto pad = [](int64_t n) { return (n + 31) / 32 * 32; };
+    int64_t total = (diag ? 4 : 3) * pad(cells);
+    for (int d = 0; d < 3; ++d) total += pad(g->nblocks * face[d]);
+    T *mem = nullptr;
+    if (cudaMalloc(&mem, sizeof(T) * total) != cudaSuccess) return fail(CN_ERR_OUT_OF_MEMORY, "cn_mg_create: face means");
+    m->owned.push_back(mem);
+    for (int d = 0; d < 3; ++d) {
+        F.k[d] = mem;
+        mem += pad(cells);
+    }
+    if (diag) {
+        *diag = mem;
+        mem += pad(cells);
+    }
+    for (int d = 0; d < 3; ++d) {
+        F.u[d] = mem;
+        mem += pad(g->nblocks * face[d]);
+    }
+    faces_kernel<T><<<grid_for(cells), 256>>>(make_geom(g, &kS1), bc_view(m->k[l], 0), fptr(m->k[l]), g->nblocks, ih2, F,
+                                              diag ? *diag : nullptr);
+    CN_CUDA_TRY(cudaGetLastError());
+    return CN_OK;
 }
 
 // Inverse of the regularised coarsest operator (see coarsest_dense_kernel),
@@ -865,6 +1028,58 @@ static cn_status coarse_inverse(cn_mg *m)
     return CN_OK;
 }
 
+// whether the FP64 residual of p64 takes the marching kernel
+static bool marches64(const cn_mg *m, const cn_grid *p64)
+{
+    return !p64->bc_count && p64->n[1] == m->p[0]->n[1] && p64->n[2] == m->p[0]->n[2];
+}
+
+// The FP64 residual of cn_mg_residual; with p0 (only where marches64), also
+// the first Jacobi sweep on it from zero.
+static cn_status residual(cn_mg *m, const cn_grid *p64, const cn_grid *f, cn_grid *r32, float *p0, double *rr, double *ff,
+                          cudaStream_t st)
+{
+    if (!m || !p64 || !f) return fail(CN_ERR_INVALID_ARGUMENT, "NULL argument");
+    if (p64->dtype != CN_FLOAT64 || f->dtype != CN_FLOAT32 || p64->nblocks != m->p[0]->nblocks ||
+        p64->n[0] != m->p[0]->n[0] || f->comp_stride != m->p[0]->comp_stride)
+        return fail(CN_ERR_SIZE_MISMATCH, "Cartesian: Can not assign two grids of unequal size.");
+    cn_status s = sync_bc(const_cast<cn_grid *>(p64), st);
+    if (s != CN_OK) return s;
+    const double *p = reinterpret_cast<const double *>(p64->d_data);
+    const float *fin = reinterpret_cast<const float *>(f->d_data);
+    float *out = r32 ? fptr(r32) : nullptr;
+    if (!marches64(m, p64)) {
+        KArgs a = kargs(m, 0);
+        a.G.L.bstride = p64->block_stride;
+        a.G.bc = bc_view(p64, 0);
+        const Tile T = tile_of(p64->n);
+        const int ctas = m->p[0]->nblocks * tile_of(m->p[0]->n).count;
+        resid64_kernel<<<ctas, kTileThreads, 0, st>>>(a, T, p, fin, out, m->partials, m->faces64);
+        CN_CUDA_TRY(cudaGetLastError());
+        sum_pairs_kernel<<<1, 256, 0, st>>>(m->partials, ctas, m->sums);
+        CN_CUDA_TRY(cudaGetLastError());
+    } else {
+        const cn_grid *g = m->p[0];
+        const double ih2 = 1.0 / (g->h[0] * g->h[0]);
+        const float om = (float)m->omega;
+        if (width_of(g, 2) == 2) {
+            const Layer a = layer_of(g, 2, 1, 1, p64);
+            resid64_march<2, 1><<<ctas_of(a), 256, 0, st>>>(a, m->faces64, ih2, om, p, fin, out, p0, m->diag[0], m->partials,
+                                                            m->done, m->sums);
+        } else {
+            const Layer a = layer_of(g, 1, 1, 1, p64);
+            resid64_march<1, 1><<<ctas_of(a), 256, 0, st>>>(a, m->faces64, ih2, om, p, fin, out, p0, m->diag[0], m->partials,
+                                                            m->done, m->sums);
+        }
+        CN_CUDA_TRY(cudaGetLastError());
+    }
+    CN_CUDA_TRY(cudaStreamSynchronize(st));
+    const volatile double *h = m->sums;
+    if (rr) *rr = h[0];
+    if (ff) *ff = h[1];
+    return CN_OK;
+}
+
 extern "C" {
 
 cn_status cn_mg_create(cn_grid *k, int nu1, int nu2, double omega, int max_levels, cn_mg **out)
@@ -918,11 +1133,13 @@ cn_status cn_mg_create(cn_grid *k, int nu1, int nu2, double omega, int max_level
         for (int d = 0; d < 3; ++d) cells[d] /= 2;
     }
     if (s == CN_OK) s = cn_grid_create(k->nb, k->n, 1, CN_FLOAT32, b0, e0, &m->r32);
-    m->nparts = k->nblocks * tile_of(k->n).count;
-    if (s == CN_OK && cudaMalloc(&m->partials, sizeof(double) * 2 * m->nparts) != cudaSuccess)
-        s = fail(CN_ERR_OUT_OF_MEMORY, "cn_mg_create: partials");
-    if (s == CN_OK && cudaMalloc(&m->sums, sizeof(double) * 2) != cudaSuccess)
-        s = fail(CN_ERR_OUT_OF_MEMORY, "cn_mg_create: sums");
+    if (s == CN_OK) {
+        m->nparts = std::max(k->nblocks * tile_of(k->n).count, (int)ctas_of(layer_of(k, width_of(k, 2), 1, 1)));
+        if (cudaMalloc(&m->partials, sizeof(double) * 2 * m->nparts) != cudaSuccess ||
+            cudaMalloc(&m->done, sizeof(unsigned)) != cudaSuccess || cudaMemset(m->done, 0, sizeof(unsigned)) != cudaSuccess ||
+            cudaHostAlloc(&m->sums, sizeof(double) * 2, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
+            s = fail(CN_ERR_OUT_OF_MEMORY, "cn_mg_create: sums");
+    }
     if (s == CN_OK && cudaMalloc(&m->iters, sizeof(int)) != cudaSuccess)
         s = fail(CN_ERR_OUT_OF_MEMORY, "cn_mg_create: iters");
     // coarse coefficients
@@ -937,32 +1154,12 @@ cn_status cn_mg_create(cn_grid *k, int nu1, int nu2, double omega, int max_level
     }
     if (s == CN_OK) s = sync_bc(m->p[0], nullptr);
     if (s == CN_OK) s = sync_bc(k, nullptr);
-    // operator coefficients of every level (k is fixed from here on): 8 FP32
-    // values per cell for the V-cycle, FP64 face means of the finest level for
-    // the outer residual
-    for (int l = 0; l < levels && s == CN_OK; ++l) {
-        const int64_t cells = (int64_t)k->nblocks * m->p[l]->n[0] * m->p[l]->n[1] * m->p[l]->n[2];
-        float *c = nullptr;
-        if (cudaMalloc(&c, sizeof(float) * kCoefPerCell * cells) != cudaSuccess) {
-            s = fail(CN_ERR_OUT_OF_MEMORY, "cn_mg_create: coefficients");
-            break;
-        }
-        m->coef.push_back(c);
-        const KArgs a = kargs(m, l);
-        const Tile T = tile_of(m->p[l]->n);
-        coef_kernel<float><<<(unsigned)(m->p[l]->nblocks * T.count), kTileThreads>>>(a, T, a.ih2, c);
-        if (cudaGetLastError() != cudaSuccess) s = fail(CN_ERR_CUDA, "coef_kernel launch");
-    }
-    if (s == CN_OK) {
-        if (cudaMalloc(&m->face64, sizeof(double) * face_count(k->n) * k->nblocks) != cudaSuccess) {
-            s = fail(CN_ERR_OUT_OF_MEMORY, "cn_mg_create: face means");
-        } else {
-            const KArgs a = kargs(m, 0);
-            const Tile T = tile_of(k->n);
-            face64_kernel<<<(unsigned)(k->nblocks * T.count), kTileThreads>>>(a, T, m->face64);
-            if (cudaGetLastError() != cudaSuccess) s = fail(CN_ERR_CUDA, "face64_kernel launch");
-        }
-    }
+    // the operator of every level (k is fixed from here on)
+    m->faces.resize(levels);
+    m->diag.resize(levels, nullptr);
+    for (int l = 0; l < levels && s == CN_OK; ++l)
+        s = make_faces<float>(m, l, m->faces[l], level_ih2(m->p[l]), &m->diag[l]);
+    if (s == CN_OK) s = make_faces<double>(m, 0, m->faces64, 0.0, nullptr);
     if (s == CN_OK && cudaDeviceSynchronize() != cudaSuccess) s = fail(CN_ERR_CUDA, "cn_mg_create");
     if (s == CN_OK && coarse_cells <= kCoarseDenseMax) s = coarse_inverse(m);
     if (s != CN_OK) {
@@ -984,7 +1181,7 @@ cn_status cn_mg_destroy(cn_mg *m)
         if (l > 0) cn_grid_destroy(m->k[l]);
     }
     cn_grid_destroy(m->r32);
-    if (m->face64) cudaFree(m->face64);
+    for (void *q : m->owned) cudaFree(q);
     for (float *c : m->coef)
         if (c) cudaFree(c);
     if (m->coarse_inv) cudaFree(m->coarse_inv);
@@ -992,7 +1189,8 @@ cn_status cn_mg_destroy(cn_mg *m)
     for (void *a : m->nn_act)
         if (a) cudaFree(a);
     if (m->partials) cudaFree(m->partials);
-    if (m->sums) cudaFree(m->sums);
+    if (m->done) cudaFree(m->done);
+    if (m->sums) cudaFreeHost(m->sums);
     if (m->iters) cudaFree(m->iters);
     delete m;
     return CN_OK;
@@ -1032,28 +1230,7 @@ cn_status cn_mg_vcycle(cn_mg *m, const cn_grid *rhs, cn_grid *e, void *stream)
 cn_status cn_mg_residual(cn_mg *m, const cn_grid *p64, const cn_grid *f, cn_grid *r32, double *rr,
                          double *ff, void *stream)
 {
-    if (!m || !p64 || !f) return fail(CN_ERR_INVALID_ARGUMENT, "NULL argument");
-    if (p64->dtype != CN_FLOAT64 || f->dtype != CN_FLOAT32 || p64->nblocks != m->p[0]->nblocks ||
-        p64->n[0] != m->p[0]->n[0] || f->comp_stride != m->p[0]->comp_stride)
-        return fail(CN_ERR_SIZE_MISMATCH, "Cartesian: Can not assign two grids of unequal size.");
-    cudaStream_t st = as_stream(stream);
-    cn_status s = sync_bc(const_cast<cn_grid *>(p64), st);
-    if (s != CN_OK) return s;
-    KArgs a = kargs(m, 0);
-    a.G.L.bstride = p64->block_stride;
-    a.G.bc = bc_view(p64, 0);
-    resid64_kernel<<<m->nparts, kTileThreads, 0, st>>>(
-        a, tile_of(p64->n), reinterpret_cast<const double *>(p64->d_data), reinterpret_cast<const float *>(f->d_data),
-        r32 ? fptr(r32) : nullptr, m->partials, m->face64);
-    CN_CUDA_TRY(cudaGetLastError());
-    sum_pairs_kernel<<<1, 256, 0, st>>>(m->partials, m->nparts, m->sums);
-    CN_CUDA_TRY(cudaGetLastError());
-    double h[2];
-    CN_CUDA_TRY(cudaMemcpyAsync(h, m->sums, sizeof(h), cudaMemcpyDeviceToHost, st));
-    CN_CUDA_TRY(cudaStreamSynchronize(st));
-    if (rr) *rr = h[0];
-    if (ff) *ff = h[1];
-    return CN_OK;
+    return residual(m, p64, f, r32, nullptr, rr, ff, as_stream(stream));
 }
 
 // Solve L p = f to ||f - L p|| <= rtol ||f||: p (FP64) is zeroed, then
@@ -1065,17 +1242,19 @@ cn_status cn_mg_solve(cn_mg *m, const cn_grid *f, cn_grid *p64, double rtol, int
     cudaStream_t st = as_stream(stream);
     CN_CUDA_TRY(cudaMemsetAsync(p64->d_data, 0, (size_t)p64->comp_stride * 8, st));
     double rr = 0, ff = 0;
-    cn_status s = cn_mg_residual(m, p64, f, m->f[0], &rr, &ff, stream);
+    // the residual also writes the cycle's first sweep where that is Jacobi's
+    const bool fused = first_fused(m, 0) && marches64(m, p64);
+    float *p0 = fused ? fptr(m->pt[0]) : nullptr;
+    cn_status s = residual(m, p64, f, m->f[0], p0, &rr, &ff, st);
     if (s != CN_OK) return s;
     const double fn = std::sqrt(ff);
     double rel = fn > 0 ? std::sqrt(rr) / fn : 0.0;
     int c = 0;
     while (c < max_cycles && rel > rtol) {
-        s = vcycle(m, 0, st);
+        s = vcycle_from(m, 0, fused, p64, st);
         if (s != CN_OK) return s;
-        s = cn_mg_accumulate(m, p64, stream);
-        if (s != CN_OK) return s;
-        s = cn_mg_residual(m, p64, f, m->f[0], &rr, nullptr, stream);
+        p0 = fused ? fptr(m->pt[0]) : nullptr;
+        s = residual(m, p64, f, m->f[0], p0, &rr, nullptr, st);
         if (s != CN_OK) return s;
         rel = std::sqrt(rr) / fn;
         ++c;
@@ -1109,25 +1288,15 @@ cn_status cn_mg_accumulate(cn_mg *m, cn_grid *p64, void *stream)
 cn_status cn_mg_jacobi(cn_mg *m, const cn_grid *pin, const cn_grid *f, cn_grid *pout, void *stream)
 {
     if (!m || !pin || !f || !pout) return fail(CN_ERR_INVALID_ARGUMENT, "NULL argument");
-    KArgs a = kargs(m, 0);
-    const Tile T = tile_of(pin->n);
-    jacobi_kernel<<<(unsigned)(pin->nblocks * T.count), kTileThreads, 0, as_stream(stream)>>>(
-        a, T, reinterpret_cast<const float *>(pin->d_data), reinterpret_cast<const float *>(f->d_data),
-        fptr(pout), (float)m->omega);
-    CN_CUDA_TRY(cudaGetLastError());
-    return CN_OK;
+    return jacobi_sweep(m, 0, m->p[0], reinterpret_cast<const float *>(pin->d_data), reinterpret_cast<const float *>(f->d_data),
+                        fptr(pout), nullptr, as_stream(stream));
 }
 
 cn_status cn_mg_restrict_residual(cn_mg *m, const cn_grid *p, const cn_grid *f, cn_grid *fc, void *stream)
 {
     if (!m || !p || !f || !fc || m->nlevels < 2) return fail(CN_ERR_INVALID_ARGUMENT, "bad argument");
-    KArgs a = kargs(m, 0);
-    const LabGeom Lc = make_geom(fc, &kS1);
-    const Tile T = tile_of(p->n);
-    resid_restrict_kernel<<<(unsigned)(p->nblocks * T.count), kTileThreads, 0, as_stream(stream)>>>(
-        a, T, reinterpret_cast<const float *>(p->d_data), reinterpret_cast<const float *>(f->d_data), Lc, fptr(fc));
-    CN_CUDA_TRY(cudaGetLastError());
-    return CN_OK;
+    return restrict_residual(m, 0, reinterpret_cast<const float *>(p->d_data), reinterpret_cast<const float *>(f->d_data), fc,
+                             nullptr, as_stream(stream));
 }
 
 cn_status cn_mg_prolong(cn_mg *m, const cn_grid *ec, cn_grid *p, void *stream)
@@ -1135,12 +1304,7 @@ cn_status cn_mg_prolong(cn_mg *m, const cn_grid *ec, cn_grid *p, void *stream)
     if (!m || !ec || !p) return fail(CN_ERR_INVALID_ARGUMENT, "bad argument");
     cn_status s = sync_bc(const_cast<cn_grid *>(ec), as_stream(stream));
     if (s != CN_OK) return s;
-    const LabGeom Lf = make_geom(p, &kS1), Lct = make_geom(ec, &kS1t);
-    const Tile T = tile_of(p->n);
-    prolong_kernel<<<(unsigned)(p->nblocks * T.count), kTileThreads, 0, as_stream(stream)>>>(
-        Lf, T, fptr(p), Lct, bc_view(ec, 0), reinterpret_cast<const float *>(ec->d_data));
-    CN_CUDA_TRY(cudaGetLastError());
-    return CN_OK;
+    return prolong(ec, p, as_stream(stream));
 }
 
 // Coarse coefficient grid of level l (read-only view for tests).

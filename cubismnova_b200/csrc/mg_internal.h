@@ -7,16 +7,34 @@
 
 struct cn_nn;
 
+namespace cn {
+namespace mg {
+// Harmonic face means of a level, one per face: across the lower face along d
+// of every cell (dense [block][cell]) and across each block's upper boundary
+// faces along d ([block][n1 n2], [n0 n2], [n0 n1]).
+template <typename T> struct Faces {
+    T *k[3] = {nullptr, nullptr, nullptr};
+    T *u[3] = {nullptr, nullptr, nullptr};
+};
+} // namespace mg
+} // namespace cn
+
 struct cn_mg {
     int nlevels;
     int nu1, nu2;
     double omega;
     std::vector<cn_grid *> p, pt, f, k; // per level (FP32); k[0] is the caller's grid
-    std::vector<float *> coef;          // per level: 8 FP32 per cell (k+ faces x,y,z, k- faces x,y,z, D, 0)
-    double *face64 = nullptr;           // finest level: FP64 harmonic face means, per block x, y, z faces
+    std::vector<cn::mg::Faces<float>> faces; // per level
+    std::vector<float *> diag;          // per level: D of every cell, dense
+    cn::mg::Faces<double> faces64;      // finest level, FP64
+    std::vector<void *> owned;          // device allocations of the above
+    // per level: 8 FP32 per cell (k+ faces x,y,z, k- faces x,y,z, D, 0), made
+    // from the faces when a tile kernel first needs them (mg_ensure_coef)
+    std::vector<float *> coef;
     cn_grid *r32 = nullptr;             // finest FP32 residual
     double *partials = nullptr;
-    double *sums = nullptr;
+    unsigned *done = nullptr; // CTAs of a residual that have finished
+    double *sums = nullptr;   // sums of r^2 and f^2: pinned host memory the kernel writes
     int *iters = nullptr;
     int nparts = 0;
     int coarse_iters_max = 0;
@@ -47,6 +65,8 @@ extern const cn_stencil kS1, kS1t;
 unsigned grid_for(int64_t n);
 float *fptr(cn_grid *g);
 cn_status vcycle(cn_mg *m, int l, cudaStream_t st);
+// the tile kernels' per-cell coefficients (m->coef) of every level
+cn_status mg_ensure_coef(cn_mg *m, cudaStream_t st);
 // learned smoothing: `apps` applications of the network on level l
 extern "C" cn_status cn_mg_accumulate(cn_mg *m, cn_grid *p64, void *stream);
 extern "C" cn_status cn_mg_residual(cn_mg *m, const cn_grid *p64, const cn_grid *f, cn_grid *r32, double *rr,

@@ -167,3 +167,42 @@ def test_solve_matches_oracle_solve(cn, oracle_lib, nb, n):
     ref = p64.blocks_view(want)
     got, ref = got - got.mean(), ref - ref.mean()
     assert np.max(np.abs(got - ref)) <= 1e-5 * np.ptp(ref)
+
+
+@pytest.mark.parametrize("nb,n,nu", [((4, 4, 4), (16, 16, 16), (2, 2)), ((2, 2, 2), (12, 12, 12), (2, 1)),
+                                     ((3, 2, 2), (8, 8, 8), (1, 2)), ((1, 1, 1), (32, 32, 32), (2, 0)),
+                                     ((2, 1, 1), (8, 8, 8), (0, 2)), ((2, 2, 2), (2, 4, 8), (1, 1)),
+                                     ((3, 3, 3), (5, 5, 5), (2, 2))])
+def test_march_and_tail_match_tile_kernels(cn, nb, n, nu):
+    """A Base BC (the periodic no-op) on every level's solution sends each
+    operator through the tile kernels and its own launch; without BCs the
+    marching kernels (rows of 4, 2 and 1 cells per thread) and the one-launch
+    coarse part run.  Same operations in the same order: the same bits."""
+    import torch
+    k, f = _setup(cn, nb, n)
+    out = []
+    for plain in (True, False):
+        m = cn.mg.Multigrid(k, nu1=nu[0], nu2=nu[1], omega=0.8)
+        if not plain:
+            for l in range(m.nlevels):
+                g = m.level(l, "p")
+                for b in range(g.size()):
+                    g.field(b, 0).getBC().push_back(cn.BC.Base(0, 0))
+                g.sync_bcs()
+        e = cn.Grid.Cartesian(nb, n, end=_end(nb, n), dtype=np.float32)
+        m.vcycle(f, e)
+        p64 = cn.Grid.Cartesian(nb, n, end=_end(nb, n), dtype=np.float64)
+        cycles, rel = m.solve(f, p64, rtol=1e-3, max_cycles=4)
+        r32 = cn.Grid.Cartesian(nb, n, end=_end(nb, n), dtype=np.float32)
+        if not plain:
+            for b in range(p64.size()):
+                p64.field(b, 0).getBC().push_back(cn.BC.Base(1, 0))
+        rr, ff = m.residual(p64, f, r32)
+        torch.cuda.synchronize()
+        out.append((e.blocks_view(e.download()).copy(), p64.blocks_view(p64.download()).copy(),
+                    r32.blocks_view(r32.download()).copy(), cycles, rr, ff))
+    a, b = out
+    assert a[3] == b[3]
+    for x, y in zip(a[:3], b[:3]):
+        assert np.array_equal(x, y)
+    assert abs(a[4] - b[4]) <= 1e-12 * b[4] and abs(a[5] - b[5]) <= 1e-12 * b[5]
