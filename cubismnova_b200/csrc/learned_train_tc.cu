@@ -446,53 +446,135 @@ static bool brick_geo(int So, BrickGeo &g)
 }
 
 // ---------------------------------------------------- CUDA-core layers
-// layer 1 forward: x [B][2][S^3] FP32 -> h1 [B][(S-2)^3][16] BF16, ReLU
+// The first and last layers and their gradients: FP32 arithmetic on pairs of
+// channels (two multiply-adds per instruction), bound by instruction issue.
+// Every kernel tiles its cells so that an operand unpacked from BF16, or a
+// tap's weights read from shared memory, serves several cells or taps; B200,
+// batch of 32 patches of 32^3 cells, against one cell and tap at a time:
+// l1_fwd_cl 170 -> 90 us, l3_fwd_cl 118 -> 62, l3_bwd_data_cl 113 -> 64,
+// l3_wgrad_cl 194 -> 73, l1_wgrad_cl 294 -> 170.
+__device__ __forceinline__ float2 fma2(float a, float2 b, float2 c) { return __ffma2_rn(make_float2(a, a), b, c); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+// 16 channels of a cell as pairs
+struct Raw16 { // as they are in memory
+    uint4 a, b;
+};
+__device__ __forceinline__ Raw16 load_raw(const uint16_t *p)
+{
+    const uint4 *s = reinterpret_cast<const uint4 *>(p);
+    return {__ldg(s), __ldg(s + 1)};
+}
+__device__ __forceinline__ void unpack_raw(const Raw16 &r, float2 (&v)[8])
+{
+    const uint32_t w[8] = {r.a.x, r.a.y, r.a.z, r.a.w, r.b.x, r.b.y, r.b.z, r.b.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        v[j] = make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xFFFF0000u));
+}
+__device__ __forceinline__ void unpack16(const uint16_t *p, float2 (&v)[8]) { unpack_raw(load_raw(p), v); }
+// 16 weights of a tap from shared memory, as pairs
+__device__ __forceinline__ void weights16(const float *w, float2 (&v)[8])
+{
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 q = *reinterpret_cast<const float4 *>(w + 4 * j);
+        v[2 * j] = make_float2(q.x, q.y);
+        v[2 * j + 1] = make_float2(q.z, q.w);
+    }
+}
+__device__ __forceinline__ void store16(uint16_t *p, const uint32_t (&h)[8])
+{
+    uint4 *dst = reinterpret_cast<uint4 *>(p);
+    dst[0] = make_uint4(h[0], h[1], h[2], h[3]);
+    dst[1] = make_uint4(h[4], h[5], h[6], h[7]);
+}
+
+// layer 1 forward: x [B][2][S^3] FP32 -> h1 [B][(S-2)^3][16] BF16, ReLU.  A
+// thread computes 4 cells of a row: per (dy, dz) it holds the row's 6 inputs of
+// both channels and takes the three taps in order (the same order of
+// summation as cell by cell).
 __global__ void __launch_bounds__(128) l1_fwd_cl(const float *__restrict__ x, const float *__restrict__ W1,
                                                   uint16_t *__restrict__ h1, int B, int S)
 {
     __shared__ __align__(16) float sw[27 * 2 * 16];
     for (int i = threadIdx.x; i < 27 * 32; i += blockDim.x) sw[i] = W1[i];
     __syncthreads();
-    const int So = S - 2;
-    const int64_t per = (int64_t)So * So * So, s3 = (int64_t)S * S * S, total = per * B;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-        const CubeIdx ci = cube_idx((uint32_t)q, (uint32_t)So, (uint32_t)per);
-        const int b = ci.b, xx = ci.x, yy = ci.y, zz = ci.z;
-        const float *x0 = x + (int64_t)b * 2 * s3, *x1 = x0 + s3;
-        float acc[16];
+    const int So = S - 2, quads = (So + 3) / 4;
+    const int64_t per = (int64_t)So * So * So, s3 = (int64_t)S * S * S;
+    const uint32_t rows = (uint32_t)(B * So * So), total = rows * (uint32_t)quads;
+    const bool vec = S % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0; // rows of x are 16-byte aligned
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        const uint32_t row = t / (uint32_t)quads, xx = 4 * (t - row * quads), zb = row / (uint32_t)So, yy = row - zb * So,
+                       b = zb / (uint32_t)So, zz = zb - b * So;
+        const float *x0 = x + (int64_t)b * 2 * s3 + xx + (int64_t)S * (yy + (int64_t)S * zz);
+        float2 acc[4][8];
 #pragma unroll
-        for (int o = 0; o < 16; ++o) acc[o] = 0.f;
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int o = 0; o < 8; ++o) acc[c][o] = make_float2(0.f, 0.f);
 #pragma unroll 1
-        for (int t = 0; t < 27; ++t) {
-            const int64_t e = (xx + t % 3) + (int64_t)S * ((yy + (t / 3) % 3) + (int64_t)S * (zz + t / 9));
-            const float v0 = __ldg(x0 + e), v1 = __ldg(x1 + e);
-            const float *w = sw + t * 32;
+        for (int r = 0; r < 9; ++r) {
+            const float *p = x0 + (int64_t)S * (r % 3 + (int64_t)S * (r / 3));
+            float v[2][6];
 #pragma unroll
-            for (int o = 0; o < 16; ++o) acc[o] = fmaf(v0, w[o], fmaf(v1, w[16 + o], acc[o]));
+            for (int i = 0; i < 2; ++i) {
+                const float *q = p + i * s3;
+                if (vec) {
+                    // positions 4 and 5 belong to no valid cell at a row's end
+                    const float4 a = __ldg(reinterpret_cast<const float4 *>(q));
+                    const float2 e = __ldg(reinterpret_cast<const float2 *>((int)xx + 5 < S ? q + 4 : q));
+                    v[i][0] = a.x;
+                    v[i][1] = a.y;
+                    v[i][2] = a.z;
+                    v[i][3] = a.w;
+                    v[i][4] = e.x;
+                    v[i][5] = e.y;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) v[i][k] = (int)xx + k < S ? __ldg(q + k) : 0.f;
+                }
+            }
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                float2 w0[8], w1[8];
+                weights16(sw + (3 * r + dx) * 32, w0);
+                weights16(sw + (3 * r + dx) * 32 + 16, w1);
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int o = 0; o < 8; ++o) acc[c][o] = fma2(v[0][c + dx], w0[o], fma2(v[1][c + dx], w1[o], acc[c][o]));
+            }
         }
-        uint32_t h[8];
+        uint16_t *dst = h1 + ((int64_t)b * per + xx + (int64_t)So * (yy + (int64_t)So * zz)) * 16;
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            h[j] = (uint32_t)bf16_bits(fmaxf(acc[2 * j], 0.f)) | ((uint32_t)bf16_bits(fmaxf(acc[2 * j + 1], 0.f)) << 16);
-        uint4 *dst = reinterpret_cast<uint4 *>(h1 + q * 16);
-        dst[0] = make_uint4(h[0], h[1], h[2], h[3]);
-        dst[1] = make_uint4(h[4], h[5], h[6], h[7]);
+        for (int c = 0; c < 4; ++c) {
+            if ((int)xx + c >= So) break;
+            uint32_t h[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                h[j] = (uint32_t)bf16_bits(fmaxf(acc[c][j].x, 0.f)) | ((uint32_t)bf16_bits(fmaxf(acc[c][j].y, 0.f)) << 16);
+            store16(dst + 16 * c, h);
+        }
     }
 }
 
-__device__ __forceinline__ void unpack16(const uint16_t *p, float (&v)[16])
+// A thread's run of ZT cells along z of a cube of side So (lanes along x):
+// item t -> patch b, (x, y), first z.
+constexpr int ZT = 4;
+struct ZRun {
+    int b, x, y, z;
+};
+__device__ __forceinline__ ZRun z_run(uint32_t t, uint32_t So)
 {
-    const uint4 *s = reinterpret_cast<const uint4 *>(p);
-    const uint4 a = __ldg(s), b = __ldg(s + 1);
-    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        v[2 * j] = __uint_as_float(w[j] << 16);
-        v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
-    }
+    const uint32_t nz = (So + ZT - 1) / ZT, xy = t / So, q = xy / So, b = q / nz;
+    return {(int)b, (int)(t - xy * So), (int)(xy - q * So), (int)((q - b * nz) * ZT)};
 }
+__host__ __device__ inline uint32_t z_runs(int B, int So) { return (uint32_t)B * So * So * ((So + ZT - 1) / ZT); }
 
-// layer 3 forward: h2 [B][S^3][16] BF16 -> y [B][(S-2)^3] FP32
+// layer 3 forward: h2 [B][S^3][16] BF16 -> y [B][(S-2)^3] FP32.  ZT cells along
+// z per thread: per (dx, dy) the column's ZT + 2 inputs are unpacked once and a
+// tap's weights serve all cells.
 __global__ void __launch_bounds__(128) l3_fwd_cl(const uint16_t *__restrict__ h2, const float *__restrict__ W3,
                                                   float *__restrict__ y, int B, int S)
 {
@@ -500,25 +582,40 @@ __global__ void __launch_bounds__(128) l3_fwd_cl(const uint16_t *__restrict__ h2
     for (int i = threadIdx.x; i < 27 * 16; i += blockDim.x) sw[i] = W3[i];
     __syncthreads();
     const int So = S - 2;
-    const int64_t per = (int64_t)So * So * So, s3 = (int64_t)S * S * S, total = per * B;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-        const CubeIdx ci = cube_idx((uint32_t)q, (uint32_t)So, (uint32_t)per);
-        const int b = ci.b, xx = ci.x, yy = ci.y, zz = ci.z;
-        float acc = 0.f;
-#pragma unroll 1
-        for (int t = 0; t < 27; ++t) {
-            const int64_t e = (xx + t % 3) + (int64_t)S * ((yy + (t / 3) % 3) + (int64_t)S * (zz + t / 9));
-            float v[16];
-            unpack16(h2 + ((int64_t)b * s3 + e) * 16, v);
+    const int64_t s2 = (int64_t)S * S, s3 = s2 * S;
+    const uint32_t total = z_runs(B, So);
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        const ZRun q = z_run(t, (uint32_t)So);
+        const uint16_t *src = h2 + (q.b * s3 + q.x + (int64_t)S * q.y + s2 * q.z) * 16;
+        float2 acc[ZT];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) acc = fmaf(v[i], sw[t * 16 + i], acc);
+        for (int c = 0; c < ZT; ++c) acc[c] = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int r = 0; r < 9; ++r) {
+            const uint16_t *p = src + (r % 3 + (int64_t)S * (r / 3)) * 16;
+            float2 v[ZT + 2][8];
+#pragma unroll
+            for (int k = 0; k < ZT + 2; ++k)
+                unpack16(p + (q.z + k < S ? k : 0) * s2 * 16, v[k]);
+#pragma unroll
+            for (int dz = 0; dz < 3; ++dz) {
+                float2 w[8];
+                weights16(sw + (r + 9 * dz) * 16, w);
+#pragma unroll
+                for (int c = 0; c < ZT; ++c)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[c] = fma2(v[c + dz][i], w[i], acc[c]);
+            }
         }
-        y[q] = acc;
+        float *dst = y + ((int64_t)q.b * So * So * So + q.x + (int64_t)So * (q.y + (int64_t)So * q.z));
+#pragma unroll
+        for (int c = 0; c < ZT; ++c)
+            if (q.z + c < So) dst[(int64_t)c * So * So] = acc[c].x + acc[c].y;
     }
 }
 
 // layer 3 backward-data: gh2[c][ci] = (h2[c][ci] > 0) sum_e gc[c - 2 + e] W3[26 - e][ci]
-// for c in S^3 (gc on (S-2)^3, zero outside)
+// for c in S^3 (gc on (S-2)^3, zero outside); ZT cells along z per thread
 __global__ void __launch_bounds__(128) l3_bwd_data_cl(const float *__restrict__ gc, const float *__restrict__ W3,
                                                        const uint16_t *__restrict__ h2, uint16_t *__restrict__ gh2,
                                                        int B, int S)
@@ -527,126 +624,203 @@ __global__ void __launch_bounds__(128) l3_bwd_data_cl(const float *__restrict__ 
     for (int i = threadIdx.x; i < 27 * 16; i += blockDim.x) sw[i] = W3[i];
     __syncthreads();
     const int So = S - 2;
-    const int64_t per = (int64_t)S * S * S, pero = (int64_t)So * So * So, total = per * B;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-        const CubeIdx ci = cube_idx((uint32_t)q, (uint32_t)S, (uint32_t)per);
-        const int b = ci.b, xx = ci.x, yy = ci.y, zz = ci.z;
-        float acc[16];
+    const int64_t o2 = (int64_t)So * So, s2 = (int64_t)S * S;
+    const uint32_t total = z_runs(B, S);
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        const ZRun q = z_run(t, (uint32_t)S);
+        float2 acc[ZT][8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+        for (int c = 0; c < ZT; ++c)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[c][i] = make_float2(0.f, 0.f);
 #pragma unroll 1
-        for (int e = 0; e < 27; ++e) {
-            const int ox = xx - 2 + e % 3, oy = yy - 2 + (e / 3) % 3, oz = zz - 2 + e / 9;
-            if ((unsigned)ox >= (unsigned)So || (unsigned)oy >= (unsigned)So || (unsigned)oz >= (unsigned)So) continue;
-            const float g = __ldg(gc + (int64_t)b * pero + ox + (int64_t)So * (oy + (int64_t)So * oz));
-            const float *w = sw + (26 - e) * 16;
+        for (int r = 0; r < 9; ++r) {
+            const int ox = q.x - 2 + r % 3, oy = q.y - 2 + r / 3;
+            if ((unsigned)ox >= (unsigned)So || (unsigned)oy >= (unsigned)So) continue;
+            const float *p = gc + q.b * (o2 * So) + ox + (int64_t)So * oy;
+            float g[ZT + 2]; // gc at z - 2 .. z + ZT - 1
 #pragma unroll
-            for (int i = 0; i < 16; ++i) acc[i] = fmaf(g, w[i], acc[i]);
+            for (int k = 0; k < ZT + 2; ++k) {
+                const int oz = q.z - 2 + k;
+                g[k] = (unsigned)oz < (unsigned)So ? __ldg(p + oz * o2) : 0.f;
+            }
+#pragma unroll
+            for (int ez = 0; ez < 3; ++ez) {
+                float2 w[8];
+                weights16(sw + (26 - r - 9 * ez) * 16, w);
+#pragma unroll
+                for (int c = 0; c < ZT; ++c)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[c][i] = fma2(g[c + ez], w[i], acc[c][i]);
+            }
         }
-        float m[16];
-        unpack16(h2 + q * 16, m);
-        uint32_t h[8];
+        const int64_t e = (q.b * (s2 * S) + q.x + (int64_t)S * q.y + s2 * q.z) * 16;
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            h[j] = (uint32_t)bf16_bits(m[2 * j] > 0.f ? acc[2 * j] : 0.f) |
-                   ((uint32_t)bf16_bits(m[2 * j + 1] > 0.f ? acc[2 * j + 1] : 0.f) << 16);
-        uint4 *dst = reinterpret_cast<uint4 *>(gh2 + q * 16);
-        dst[0] = make_uint4(h[0], h[1], h[2], h[3]);
-        dst[1] = make_uint4(h[4], h[5], h[6], h[7]);
+        for (int c = 0; c < ZT; ++c) {
+            if (q.z + c >= S) break;
+            float2 m[8];
+            unpack16(h2 + e + c * s2 * 16, m);
+            uint32_t h[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                h[j] = (uint32_t)bf16_bits(m[j].x > 0.f ? acc[c][j].x : 0.f) |
+                       ((uint32_t)bf16_bits(m[j].y > 0.f ? acc[c][j].y : 0.f) << 16);
+            store16(gh2 + e + c * s2 * 16, h);
+        }
     }
 }
 
-// warp sum of v[0..N) into lane 0
-template <int N> __device__ __forceinline__ void warp_sum(float (&v)[N])
+// Warp sums of v[0..16): the lanes halve the values they carry at each step
+// (16 shuffles, not 80), and lane l ends with the sum of value l / 2.
+__device__ __forceinline__ float warp_sum16(float (&v)[16])
 {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int i = 0; i < N; ++i)
+    for (int n = 8; n > 0; n >>= 1) {
+        const bool up = lane & (2 * n);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+        for (int i = 0; i < n; ++i) {
+            const float keep = up ? v[n + i] : v[i], send = up ? v[i] : v[n + i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * n);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-// The weight gradients of the first and last layers: blocks of 27 warps,
-// warp w = tap w.  A block walks whole planes (patch b, z) of the output
-// cells; the lanes of all 27 warps take the same cells of the plane (index
-// y So + x, advanced without divisions), so the per-cell operand (gc or
-// gh1) is read from DRAM once and the 27 taps' shifted reads hit L1.
-// Per-warp sums, then atomics.
-constexpr int WG_THREADS = 27 * 32;
+// The weight gradients of the first and last layers: blocks of 9 warps, warp w
+// = taps (dx, dy) = (w % 3, w / 3) with all three dz.  The lanes of all 9 warps
+// take the same 32 columns (patch b, x, y) of output cells and walk up runs of
+// them, with the BF16 operand unpacked once per cell (the next plane's in
+// flight) and the other one in a window of three planes.  The shifted reads of
+// the 9 warps hit L1.  Layer 1's two input channels are two blocks (its 96
+// accumulators in one thread left one block per SM: 318 us).  The warps' sums
+// go to FP32 atomics, 16 neighbouring words each: one word per lane and 5
+// shuffles per value made them the end of every small batch (8 patches of
+// 16^3, the whole step: 299 us, this way 252).
+constexpr int WG_THREADS = 9 * 32;
+constexpr int WG_CTAS = 3; // resident per SM
+
+struct WgItem {
+    int b, x, y, z0, z1;
+    bool ok;
+};
+// item k of `runs` runs of a column group: 32 consecutive columns of patch-major (b, y, x)
+__device__ __forceinline__ WgItem wg_item(int item, int runs, int run, int columns, int So)
+{
+    const int group = item / runs, k = item - group * runs, col = group * 32 + (threadIdx.x & 31);
+    WgItem w;
+    w.ok = col < columns;
+    const int c = w.ok ? col : 0, yb = c / So;
+    w.x = c - yb * So;
+    w.b = yb / So;
+    w.y = yb - w.b * So;
+    w.z0 = k * run;
+    w.z1 = min(So, w.z0 + run);
+    return w;
+}
+// the block's sums of the three dz taps' 16 values into dst[tap stride][16]
+__device__ __forceinline__ void wg_add(float2 (&acc)[3][8], float *dst, int tap_stride)
+{
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        float a[16];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            a[2 * i] = acc[d][i].x;
+            a[2 * i + 1] = acc[d][i].y;
+        }
+        const float sum = warp_sum16(a);
+        if ((threadIdx.x & 1) == 0) atomicAdd(dst + 9 * d * tap_stride + ((threadIdx.x & 31) >> 1), sum);
+    }
+}
 
 // layer 3: gW3[t][ci] += sum_q h2[q + d(t)][ci] gc[q], q in (S-2)^3, h2 side S
-__global__ void __launch_bounds__(WG_THREADS) l3_wgrad_cl(const uint16_t *__restrict__ h2,
-                                                           const float *__restrict__ gc, float *__restrict__ gW3,
-                                                           int B, int S)
+__global__ void __launch_bounds__(WG_THREADS, WG_CTAS)
+    l3_wgrad_cl(const uint16_t *__restrict__ h2, const float *__restrict__ gc, float *__restrict__ gW3, int B, int S,
+                int run)
 {
-    const int t = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int dx = t % 3, dy = (t / 3) % 3, dz = t / 9;
-    const int So = S - 2, plane = So * So;
-    const int64_t s3 = (int64_t)S * S * S;
-    float acc[16];
+    const int w = threadIdx.x >> 5, dx = w % 3, dy = w / 3;
+    const int So = S - 2, columns = B * So * So, runs = (So + run - 1) / run, items = (columns + 31) / 32 * runs;
+    const int64_t s2 = (int64_t)S * S, s3 = s2 * S, o2 = (int64_t)So * So;
+    float2 acc[3][8];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-    for (int pz = blockIdx.x; pz < B * So; pz += gridDim.x) {
-        const int b = pz / So, zz = pz - b * So;
-        const float *gp = gc + (int64_t)pz * plane;
-        const uint16_t *hp = h2 + ((int64_t)b * s3 + dx + (int64_t)S * (dy + (int64_t)S * (zz + dz))) * 16;
-        int xx = lane, yy = 0;
-        for (int idx = lane; idx < plane; idx += 32) {
-            while (xx >= So) {
-                xx -= So;
-                ++yy;
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[d][i] = make_float2(0.f, 0.f);
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        const WgItem q = wg_item(item, runs, run, columns, So);
+        const uint16_t *hp = h2 + (q.b * s3 + q.x + dx + (int64_t)S * (q.y + dy) + s2 * q.z0) * 16;
+        const float *gp = gc + q.b * (o2 * So) + q.x + (int64_t)So * q.y;
+        float g1 = 0.f, g2 = 0.f; // gc one and two planes below
+        Raw16 next = load_raw(hp);
+        float gn = q.ok ? __ldg(gp + q.z0 * o2) : 0.f;
+        for (int z = q.z0; z < q.z1 + 2; ++z) {
+            const Raw16 cur = next;
+            const float g0 = gn;
+            if (z + 1 < q.z1 + 2) {
+                hp += s2 * 16;
+                next = load_raw(hp);
+                gn = q.ok && z + 1 < q.z1 ? __ldg(gp + (z + 1) * o2) : 0.f;
             }
-            const float g = __ldg(gp + idx);
-            float v[16];
-            unpack16(hp + (xx + (int64_t)S * yy) * 16, v);
+            float2 v[8];
+            unpack_raw(cur, v); // plane z of h2: dz 0 of cell z, 1 of z - 1, 2 of z - 2
 #pragma unroll
-            for (int i = 0; i < 16; ++i) acc[i] = fmaf(v[i], g, acc[i]);
-            xx += 32;
+            for (int i = 0; i < 8; ++i) {
+                acc[0][i] = fma2(g0, v[i], acc[0][i]);
+                acc[1][i] = fma2(g1, v[i], acc[1][i]);
+                acc[2][i] = fma2(g2, v[i], acc[2][i]);
+            }
+            g2 = g1;
+            g1 = g0;
         }
     }
-    warp_sum(acc);
-    if (lane == 0)
-#pragma unroll
-        for (int i = 0; i < 16; ++i) atomicAdd(gW3 + t * 16 + i, acc[i]);
+    wg_add(acc, gW3 + w * 16, 16);
 }
 
-// layer 1: gW1[t][i][o] += sum_q x[i][q + d(t)] gh1[q][o], q in (S-2)^3, x side S
-__global__ void __launch_bounds__(WG_THREADS) l1_wgrad_cl(const float *__restrict__ x,
-                                                           const uint16_t *__restrict__ gh1, float *__restrict__ gW1,
-                                                           int B, int S)
+// layer 1, input channel blockIdx.y: gW1[t][i][o] += sum_q x[i][q + d(t)] gh1[q][o],
+// q in (S-2)^3, x side S
+__global__ void __launch_bounds__(WG_THREADS, WG_CTAS)
+    l1_wgrad_cl(const float *__restrict__ x, const uint16_t *__restrict__ gh1, float *__restrict__ gW1, int B, int S,
+                int run)
 {
-    const int t = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int dx = t % 3, dy = (t / 3) % 3, dz = t / 9;
-    const int So = S - 2, plane = So * So;
-    const int64_t s3 = (int64_t)S * S * S;
-    float acc[32];
+    const int w = threadIdx.x >> 5, dx = w % 3, dy = w / 3, i = blockIdx.y;
+    const int So = S - 2, columns = B * So * So, runs = (So + run - 1) / run, items = (columns + 31) / 32 * runs;
+    const int64_t s2 = (int64_t)S * S, s3 = s2 * S, o2 = (int64_t)So * So;
+    float2 acc[3][8];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-    for (int pz = blockIdx.x; pz < B * So; pz += gridDim.x) {
-        const int b = pz / So, zz = pz - b * So;
-        const uint16_t *gp = gh1 + (int64_t)pz * plane * 16;
-        const float *xp = x + (int64_t)b * 2 * s3 + dx + (int64_t)S * (dy + (int64_t)S * (zz + dz));
-        int xx = lane, yy = 0;
-        for (int idx = lane; idx < plane; idx += 32) {
-            while (xx >= So) {
-                xx -= So;
-                ++yy;
-            }
-            const int64_t e = xx + (int64_t)S * yy;
-            const float v0 = __ldg(xp + e), v1 = __ldg(xp + e + s3);
-            float g[16];
-            unpack16(gp + (int64_t)idx * 16, g);
+    for (int d = 0; d < 3; ++d)
 #pragma unroll
-            for (int o = 0; o < 16; ++o) {
-                acc[o] = fmaf(v0, g[o], acc[o]);
-                acc[16 + o] = fmaf(v1, g[o], acc[16 + o]);
+        for (int o = 0; o < 8; ++o) acc[d][o] = make_float2(0.f, 0.f);
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        const WgItem q = wg_item(item, runs, run, columns, So);
+        const float *xp = x + (2 * q.b + i) * s3 + q.x + dx + (int64_t)S * (q.y + dy) + s2 * q.z0;
+        const uint16_t *gp = gh1 + (q.b * (o2 * So) + q.x + (int64_t)So * q.y + o2 * q.z0) * 16;
+        // x at planes z .. z + 2 (0 for lanes without a column), the next one in flight
+        float v0 = q.ok ? __ldg(xp) : 0.f, v1 = q.ok ? __ldg(xp + s2) : 0.f, vn = q.ok ? __ldg(xp + 2 * s2) : 0.f;
+        xp += 2 * s2;
+        Raw16 next = load_raw(gp);
+        for (int z = q.z0; z < q.z1; ++z) {
+            const Raw16 cur = next;
+            const float v2 = vn;
+            if (z + 1 < q.z1) {
+                gp += o2 * 16;
+                xp += s2;
+                next = load_raw(gp);
+                vn = q.ok ? __ldg(xp) : 0.f;
             }
-            xx += 32;
+            float2 g[8];
+            unpack_raw(cur, g);
+#pragma unroll
+            for (int o = 0; o < 8; ++o) {
+                acc[0][o] = fma2(v0, g[o], acc[0][o]);
+                acc[1][o] = fma2(v1, g[o], acc[1][o]);
+                acc[2][o] = fma2(v2, g[o], acc[2][o]);
+            }
+            v0 = v1;
+            v1 = v2;
         }
     }
-    warp_sum(acc);
-    if (lane == 0)
-#pragma unroll
-        for (int i = 0; i < 32; ++i) atomicAdd(gW1 + t * 32 + i, acc[i]);
+    wg_add(acc, gW1 + w * 32 + 16 * i, 32);
 }
 
 static unsigned grid_of(int64_t n, int threads, int64_t cap)
@@ -654,6 +828,19 @@ static unsigned grid_of(int64_t n, int threads, int64_t cap)
     int64_t b = (n + threads - 1) / threads;
     if (b > cap) b = cap;
     return (unsigned)(b < 1 ? 1 : b);
+}
+
+// Run length and CTAs of a first/last-layer weight gradient over output cubes
+// of side So: whole columns where there is a group of 32 for every CTA, else
+// runs short enough for that, of 4 cells at least (a run re-reads two planes).
+static unsigned wg_launch(int B, int So, int ctas, int &run)
+{
+    const int64_t groups = ((int64_t)B * So * So + 31) / 32;
+    const int64_t runs = (ctas + groups - 1) / groups;
+    run = (int)((So + runs - 1) / runs);
+    if (run < 4) run = 4;
+    const int64_t items = groups * ((So + run - 1) / run);
+    return (unsigned)(items < ctas ? items : ctas);
 }
 
 static DeviceOnce wgrad_once, brick_once[2];
@@ -705,7 +892,7 @@ cn_status train_forward_tc(const TrainBufs &T, const float *x, const float *W, i
     // packed B tiles of the hidden layer: forward, backward-data
     if ((s = pack_weights(W2, 16, 16, T.wfwd, st)) != CN_OK) return s;
     pack_bwd_kernel<<<27, 256, 0, st>>>(W2, T.wbwd);
-    l1_fwd_cl<<<grid_of((int64_t)B * S1 * S1 * S1, 128, 148 * 64), 128, 0, st>>>(x, W1, T.h1, B, S);
+    l1_fwd_cl<<<grid_of((int64_t)B * S1 * S1 * ((S1 + 3) / 4), 128, 148 * 64), 128, 0, st>>>(x, W1, T.h1, B, S);
     CN_CUDA_TRY(cudaGetLastError());
     Args a = {};
     a.src = T.h1;
@@ -718,7 +905,7 @@ cn_status train_forward_tc(const TrainBufs &T, const float *x, const float *W, i
     a.total = (int64_t)B * S2 * S2 * S2;
     a.err = T.err;
     if ((s = launch_conv<FWD>(a, B, st)) != CN_OK) return s;
-    l3_fwd_cl<<<grid_of((int64_t)B * S3 * S3 * S3, 128, 148 * 64), 128, 0, st>>>(T.h2, W3, T.y, B, S2);
+    l3_fwd_cl<<<grid_of(z_runs(B, S3), 128, 148 * 64), 128, 0, st>>>(T.h2, W3, T.y, B, S2);
     CN_CUDA_TRY(cudaGetLastError());
     return CN_OK;
 }
@@ -735,8 +922,10 @@ cn_status train_backward_tc(const TrainBufs &T, const float *x, const float *W, 
     int dev = 0, sms = 148;
     CN_CUDA_TRY(cudaGetDevice(&dev));
     CN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    l3_wgrad_cl<<<grid_of((int64_t)B * S3, 1, sms), WG_THREADS, 0, st>>>(T.h2, T.gc, gW3, B, S2);
-    l3_bwd_data_cl<<<grid_of((int64_t)B * S2 * S2 * S2, 128, 148 * 64), 128, 0, st>>>(T.gc, W3, T.h2, T.gh2, B, S2);
+    int run = 0;
+    unsigned ctas = wg_launch(B, S3, WG_CTAS * sms, run);
+    l3_wgrad_cl<<<ctas, WG_THREADS, 0, st>>>(T.h2, T.gc, gW3, B, S2, run);
+    l3_bwd_data_cl<<<grid_of(z_runs(B, S2), 128, 148 * 64), 128, 0, st>>>(T.gc, W3, T.h2, T.gh2, B, S2);
     CN_CUDA_TRY(cudaGetLastError());
     Args w = {};
     w.src = T.h1;
@@ -759,7 +948,8 @@ cn_status train_backward_tc(const TrainBufs &T, const float *x, const float *W, 
     d.total = (int64_t)B * S1 * S1 * S1;
     d.err = T.err;
     if ((s = launch_conv<BWD>(d, B, st)) != CN_OK) return s;
-    l1_wgrad_cl<<<grid_of((int64_t)B * S1, 1, sms), WG_THREADS, 0, st>>>(x, T.gh1, gW1, B, S);
+    ctas = wg_launch(B, S1, WG_CTAS * sms / 2, run);
+    l1_wgrad_cl<<<dim3(ctas, 2), WG_THREADS, 0, st>>>(x, T.gh1, gW1, B, S, run);
     CN_CUDA_TRY(cudaGetLastError());
     return CN_OK;
 }

@@ -85,6 +85,28 @@ def test_tensor_core_training_matches_bf16_oracle(cn, B, P):
         assert e < TOL_TC_GRAD, errs
 
 
+@pytest.mark.parametrize("B,P,offset", [(1, 1, 0), (5, 3, 0), (3, 7, 0), (2, 8, 1)])
+def test_tensor_core_training_edges(cn, B, P, offset):
+    """The first and last layers where their tiles end: cubes shorter than a
+    run of cells along x or z, column groups with idle lanes, and inputs whose
+    rows are not on 16-byte boundaries.  The tolerances of the other sizes."""
+    import torch
+    from oracle import nn_oracle as N
+    x, k, r = _batch(B, P, 31 + P)
+    nn = cn.learned.LearnedSmoother(seed=5, omega=0.8, init_scale=0.05)
+    nn.set_training("tensor")
+    W1, W2, W3 = [w.astype(np.float64) for w in nn.weights()]
+    tx, tk, tr = (torch.tensor(a, dtype=torch.float32, device="cuda") for a in (x, k, r))
+    buf = torch.zeros(offset + tx.numel(), dtype=torch.float32, device="cuda")
+    buf[offset:] = tx.reshape(-1)
+    loss, grads = nn.loss_grad(buf[offset:].view(B, 2, -1), tk.reshape(B, -1), tr.reshape(B, -1), P, 16.0)
+    x32, k32, r32 = (a.astype(np.float32).astype(np.float64) for a in (x, k, r))
+    want, *bw = N.loss_and_grad(x32, k32, r32, W1, W2, W3, 0.8, 16.0, bf16_path=True)
+    assert abs(loss - want) <= TOL_TC_LOSS * abs(want)
+    for g, w in zip(grads, bw):
+        assert _rel(g, w) < TOL_TC_GRAD
+
+
 def test_tensor_core_training_step_matches_fp32(cn):
     """One Adam step from the same weights with either training path moves
     the weights the same way (BF16 gradients point where the FP32 ones do)."""
