@@ -108,6 +108,25 @@ def test_fp32_vs_fp64_error(cn):
         assert linf < 1e-6 and l1 < 5e-7, (c, l1, linf)
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("nb,n", [((1, 1, 1), (8, 8, 8)), ((2, 1, 3), (24, 8, 8)), ((1, 2, 1), (40, 16, 24))])
+def test_max_speed_sees_every_cell(cn, dtype, nb, n):
+    """The wave-speed maximum over blocks of half, one and a half, and 15
+    passes of a CTA, with the largest value in a block's first, middle and
+    last cell in turn.  The device may contract and divide differently by a
+    few units in the last place: 16 of the data type."""
+    U = _state(cn, nb, n, dtype, bcs=False)
+    cells, blocks = int(np.prod(n)), int(np.prod(nb))
+    for blk, cell in ((0, 0), (blocks - 1, cells // 2), (blocks // 2, cells - 1)):
+        U.tensor(1)[blk, cell] += 3.0
+        U.tensor(4)[blk, cell] += 9.0
+        r, m0, m1, m2, E = (np.asarray(U.tensor(c)[:, :cells].cpu(), dtype=np.float64) for c in range(5))
+        p = (GAMMA - 1) * (E - 0.5 * (m0 ** 2 + m1 ** 2 + m2 ** 2) / r)
+        c = np.sqrt(GAMMA * p / r)
+        want = [np.max(np.abs(m / r) + c) for m in (m0, m1, m2)]
+        np.testing.assert_allclose(cn.euler.max_speed(U), want, rtol=16 * np.finfo(dtype).eps)
+
+
 def test_uniform_state_full_size_is_steady(cn):
     """512^3 cells (16^3 blocks of 32^3), C2 BCs: a uniform far-field state has
     an exactly zero RHS (every face sees the same six cells)."""
