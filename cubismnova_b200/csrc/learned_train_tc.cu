@@ -19,22 +19,11 @@
 // shifted (K-major, M = 128 cells, K = 16 channels, N = 16), 27 MMAs per
 // 128-row tile.
 //   weight grad    gW[t][ci][co] = sum_q h1[q + d][ci] gout[q][co]
-// needs M = (tap, channel), which no shifted descriptor gives (the tap
-// offsets are not evenly spaced): wgrad_tc_kernel gathers, for a chunk of
-// 128 consecutive output cells (linear over batch and cube), per tap t and
-// channel half h a plane of 128 rows x 16 bytes (row r = channels
-// 8h..8h+7 of source cell (cell r) + d(t), zero outside the cube; one
-// 16-byte cp.async each), reads them MN-major (8 taps = 16 planes per
-// M = 128 tile, planes one SBO apart; K = cells, 16 rows per MMA) against
-// the chunk's gout rows (MN-major B, N = 16): 4 tiles x 8 MMAs per chunk,
-// accumulated over all chunks of a CTA in tensor memory, added to gW with
-// atomics at the end.  Rows of taps >= 27 in the last tile read whatever
-// the buffer holds; those accumulator rows are never read.  Taps are
-// gathered in 4 groups of 8 into two 32 KB buffers, one group ahead of the
-// MMAs (issued by one thread, committed to the buffer's mbarrier); lanes 2i
-// and 2i+1 copy the two channel halves of one row.  Persistent CTAs, two
-// per SM.  Every wait in both kernels is bounded (an error word is set and
-// the CTA stops issuing).
+// runs on bricks too, with the cells as K (wgrad_tc_kernel): both operands
+// MN-major, A = (dz, channel) of the source region against the brick's gout
+// rows, one accumulator per (dx, dy), added to gW with atomics once per CTA.
+// Every wait in both kernels is bounded (an error word is set and the CTA
+// stops issuing).
 #include "cn_internal.h"
 #include "cn_tc.cuh"
 #include "cn_tma.cuh"
@@ -42,25 +31,15 @@
 
 #include <cuda_bf16.h>
 
-#include <type_traits>
+#include <algorithm>
 
 namespace cn {
 namespace nntr {
 
-constexpr int ROWS = 128;                        // cells per chunk
-constexpr int GT = 8;                            // taps per gather group
-constexpr int NG = 4;                            // groups per chunk (taps 0-7, 8-15, 16-23, 24-26)
-constexpr uint32_t PL = ROWS * 16;               // bytes of one plane
-constexpr uint32_t GBUF = 2 * GT * PL;           // one group buffer: 16 planes, 32 KB
-constexpr int NT = 2 * ROWS;                     // two threads per row (channel halves)
 constexpr uint32_t WBYTES = 27 * 512;            // packed weights of one layer
-constexpr uint32_t GOUT_BYTES = 2 * PL;          // gout rows of a chunk (2 planes)
-constexpr size_t OFF_G = 2 * (size_t)GBUF;       // two gout buffers
-constexpr size_t OFF_BAR = OFF_G + 2 * GOUT_BYTES;
-constexpr size_t SMEM = OFF_BAR + 4 * 8 + 16;
 constexpr uint32_t IDESC_K = tc::idesc_bf16_f32(128, 16);
-// both operands MN-major (bits 15 and 16)
-constexpr uint32_t IDESC_MN = tc::idesc_bf16_f32(128, 16) | (1u << 15) | (1u << 16);
+// M = 64, both operands MN-major (bits 15 and 16)
+constexpr uint32_t IDESC_MN = tc::idesc_bf16_f32(64, 16) | (1u << 15) | (1u << 16);
 
 enum { FWD = 0, BWD = 1 };
 
@@ -73,28 +52,10 @@ struct Args {
     float *gw;            // weight gradient: [27][16][16] FP32, accumulated
     int Sin, Sout, shift;
     int relu;
-    int64_t total;        // B * Sout^3
-    int64_t chunks;       // ceil(total / ROWS)
     int *err;
 };
 
 __device__ __forceinline__ uint16_t bf16_bits(float v) { return __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
-
-// cell index q of a batch of cubes of side n (n3 = n^3; indices below 2^31,
-// checked on the host) -> patch b and (x, y, z); 32-bit divisions
-struct CubeIdx {
-    int b, x, y, z;
-};
-__device__ __forceinline__ CubeIdx cube_idx(uint32_t q, uint32_t n, uint32_t n3)
-{
-    CubeIdx c;
-    const uint32_t b = q / n3, rem = q - b * n3, zy = rem / n, z = zy / n;
-    c.b = (int)b;
-    c.x = (int)(rem - zy * n);
-    c.z = (int)z;
-    c.y = (int)(zy - z * n);
-    return c;
-}
 
 // 16-byte asynchronous copy; src_bytes 0 writes zeros (nothing is read)
 __device__ __forceinline__ void cp16(void *dst, const void *src, uint32_t src_bytes)
@@ -103,143 +64,139 @@ __device__ __forceinline__ void cp16(void *dst, const void *src, uint32_t src_by
                  : "memory");
 }
 
-template <int V> using ic = std::integral_constant<int, V>;
+// ------------------------------------------------------ weight gradient
+// gW[t][ci][co] = sum over cells q of h1[q + d(t)][ci] gout[q][co]: K = cells.
+// A CTA takes bricks of BX x BY x BZ output cells and stages, per z plane and
+// channel half, the rows (16 bytes: 8 channels of a cell) of the source region
+// (row x + RX y, RX = BX + 2) and of gout in the same numbering, zero in rows
+// that are no cell of the brick.  MN-major, a plane of rows is 8 rows of A^T,
+// and the planes (z, half) are evenly spaced: 8 of them from plane z on are the
+// M = 64 of the three dz taps (the last 16 rows, a plane too far, are dropped),
+// and the taps (dx, dy) are start addresses dx + RX dy rows on.  9 MMAs per
+// 16 cells (K) into 9 accumulators of 16 columns, kept over all bricks of the
+// CTA.  Against a gather of every tap's rows (27 copies of 32 bytes a cell) a
+// cell is staged about 1.5 times; B200, 32 patches of 32^3: 384 -> 155 us, of
+// which the MMAs alone 122 (37 cycles each, M = 64 N = 16) and the staging alone
+// 66: two CTAs per SM, one staging while the other's MMAs run.
+constexpr int WGT_NT = 256;
+constexpr int WGT_SMEM = 110 * 1024; // two CTAs per SM
+constexpr uint32_t WGT_COLS = 256;   // 9 x 16, a power of two
 
-__global__ void __launch_bounds__(NT, 2) wgrad_tc_kernel(const __grid_constant__ Args a)
+struct WgGeo {
+    int BX, BY, BZ;  // brick of output cells
+    int RX;          // BX + 2
+    int H, KP;       // rows per staged plane: source region, gout (a multiple of 16)
+    int bricks[3];   // per patch
+    int total;       // in all
+};
+
+__global__ void __launch_bounds__(WGT_NT, 2) wgrad_tc_kernel(const __grid_constant__ Args a,
+                                                             const __grid_constant__ WgGeo g)
 {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *Abuf = smem;                 // [2][16 planes][ROWS][16 B]
-    unsigned char *Gbuf = smem + OFF_G;         // [2][2 planes][ROWS][16 B]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + OFF_BAR);
-    uint64_t *empty = bars, *done = bars + 2;   // empty[2]: group buffer free; done: all MMAs complete
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 4);
-    int *flag = reinterpret_cast<int *>(slot + 1); // [0]: buffer waits, [1]: the final wait
-    constexpr uint32_t TCOLS = 64;                 // 4 accumulator tiles x 16 columns
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t slot;
+    __shared__ int flag;
+    const uint32_t aplane = (uint32_t)g.H * 16u, gplane = (uint32_t)g.KP * 16u;
+    unsigned char *A = smem;                              // [BZ + 3][2][H][16 B], the last z plane never written
+    unsigned char *G = smem + 2 * (g.BZ + 3) * aplane;    // [BZ][2][KP][16 B]
     const int r = threadIdx.x, warp = r >> 5;
-
     if (r == 0) {
-        mbar_init(empty, 1);
-        mbar_init(empty + 1, 1);
-        mbar_init(done, 1);
+        mbar_init(&bar, 1);
         fence_mbar_init();
     }
     if (warp == 0) {
-        tc::tmem_alloc(slot, TCOLS);
+        tc::tmem_alloc(&slot, WGT_COLS);
         tc::tmem_relinquish();
     }
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tbase = *slot;
+    const uint32_t tbase = slot;
 
-    const uint32_t so3 = (uint32_t)a.Sout * a.Sout * a.Sout;
-    const int64_t si3 = (int64_t)a.Sin * a.Sin * a.Sin, sin1 = a.Sin, sin2 = (int64_t)a.Sin * a.Sin;
-    const int nch = (int64_t)blockIdx.x < a.chunks ? (int)((a.chunks - 1 - blockIdx.x) / gridDim.x + 1) : 0;
-    const int nitems = NG * nch; // items (chunk j of this CTA, tap group g): i = NG j + g, buffer g & 1
-    // gather: thread r copies channel half hh of row rho (a warp: 16 rows =
-    // 512 contiguous source bytes where the cells are contiguous)
-    const int hh = r & 1, rho = r >> 1;
-    int64_t rL = 0, roff = 0; // the row's cell; source element of its tap (0, 0, 0)
-    uint32_t mx = 0, my = 0, mz = 0; // per axis: offsets k = 0..2 with the source inside the cube
-    auto set_row = [&](int j) {
-        rL = (blockIdx.x + (int64_t)j * gridDim.x) * ROWS + rho;
-        mx = my = mz = 0;
-        if (rL < a.total) {
-            const CubeIdx ci = cube_idx((uint32_t)rL, (uint32_t)a.Sout, so3);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                mx |= ((unsigned)(ci.x + k) < (unsigned)a.Sin ? 1u : 0u) << k;
-                my |= ((unsigned)(ci.y + k) < (unsigned)a.Sin ? 1u : 0u) << k;
-                mz |= ((unsigned)(ci.z + k) < (unsigned)a.Sin ? 1u : 0u) << k;
-            }
-            roff = (int64_t)ci.b * si3 + ci.x + sin1 * ci.y + sin2 * ci.z;
-        }
-    };
-    auto gather = [&](int j, auto G) {
-        constexpr int g = decltype(G)::value;
-        if (g == 0) {
-            set_row(j);
-            // the chunk's gradient rows (buffer j & 1 was last read by chunk j - 2's
-            // MMAs, complete before item NG j - 2's)
-            const bool v = rL < a.total;
-            cp16(Gbuf + (j & 1) * GOUT_BYTES + hh * PL + rho * 16, v ? a.gout + rL * 16 + 8 * hh : a.gout,
-                 v ? 16u : 0u);
-        }
-        unsigned char *A = Abuf + (g & 1) * GBUF;
-#pragma unroll
-        for (int tl = 0; tl < GT; ++tl) {
-            const int t = g * GT + tl;
-            if (t < 27) {
-                const int dx = t % 3, dy = (t / 3) % 3, dz = t / 9;
-                const bool in = ((mx >> dx) & (my >> dy) & (mz >> dz) & 1u) != 0;
-                const uint16_t *src = in ? a.src + (roff + dx + sin1 * dy + sin2 * dz) * 16 + 8 * hh : a.src;
-                cp16(A + (2 * tl + hh) * PL + rho * 16, src, in ? 16u : 0u);
+    const int Si = a.Sin, So = a.Sout, per = g.bricks[0] * g.bricks[1] * g.bricks[2];
+    const int64_t si2 = (int64_t)Si * Si, so2 = (int64_t)So * So;
+    bool ok = true;
+    int it = 0;
+    for (int brick = blockIdx.x; brick < g.total; brick += gridDim.x, ++it) {
+        const int b = brick / per;
+        int br = brick - b * per;
+        const int ox = (br % g.bricks[0]) * g.BX;
+        br /= g.bricks[0];
+        const int oy = (br % g.bricks[1]) * g.BY, oz = (br / g.bricks[1]) * g.BZ;
+        const int nx = min(g.BX, So - ox), ny = min(g.BY, So - oy), nz = min(g.BZ, So - oz);
+        const int ks = (g.RX * ny + 15) / 16; // K steps per z plane
+        if (it > 0) {                         // the previous brick's MMAs have read the buffers
+            if (r == 0) flag = mbar_wait_bounded(&bar, (it - 1) & 1) ? 1 : 0;
+            __syncthreads();
+            if (!flag) {
+                ok = false;
+                break;
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    // one item: gather the next (after its buffer's previous MMAs), wait
-    // for this item's copies, issue its MMAs.  False when a bounded wait ran
-    // out.
-    auto item = [&](int j, auto G) -> bool {
-        constexpr int g = decltype(G)::value;
-        const int i = NG * j + g;
-        if (i + 1 < nitems) {
-            if (i >= 1) {
-                if (r == 0)
-                    flag[0] = mbar_wait_bounded(empty + ((g + 1) & 1), (((i + 1) >> 1) - 1) & 1) ? 1 : 0;
-                __syncthreads();
-                if (!flag[0]) return false;
+        // source region: all rows the shifted K steps read, zero past the region
+        const int arows = 16 * ks + 2 + 2 * g.RX;
+        for (int t = r; t < 2 * arows; t += WGT_NT) {
+            const int u = t >> 1, hh = t & 1, y = u / g.RX, x = u - y * g.RX;
+            const bool in = x < nx + 2 && y < ny + 2;
+            const uint16_t *src = in ? a.src + (((int64_t)b * Si + oz) * si2 + (int64_t)(oy + y) * Si + ox + x) * 16 + 8 * hh
+                                     : a.src;
+            unsigned char *dst = A + hh * aplane + u * 16;
+            for (int z = 0; z < nz + 2; ++z) {
+                cp16(dst + 2 * z * aplane, src, in ? 16u : 0u);
+                if (in) src += si2 * 16;
             }
-            if constexpr (g == NG - 1) gather(j + 1, ic<0>{});
-            else gather(j, ic<g + 1>{});
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
+        for (int t = r; t < 32 * ks; t += WGT_NT) {
+            const int u = t >> 1, hh = t & 1, y = u / g.RX, x = u - y * g.RX;
+            const bool in = x < nx && y < ny;
+            const uint16_t *src = in ? a.gout + (((int64_t)b * So + oz) * so2 + (int64_t)(oy + y) * So + ox + x) * 16 + 8 * hh
+                                     : a.gout;
+            unsigned char *dst = G + hh * gplane + u * 16;
+            for (int z = 0; z < nz; ++z) {
+                cp16(dst + 2 * z * gplane, src, in ? 16u : 0u);
+                if (in) src += so2 * 16;
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         fence_proxy_async_smem(); // generic-proxy smem writes -> visible to the tensor cores
         tc::fence_before_sync();
         __syncthreads();
         if (r == 0) {
             tc::fence_after_sync();
-            const uint32_t A = smem_u32(Abuf + (g & 1) * GBUF), Gs = smem_u32(Gbuf + (j & 1) * GOUT_BYTES);
-#pragma unroll
-            for (int ks = 0; ks < ROWS / 16; ++ks) {
-                const uint64_t da = tc::smem_desc(A + 256u * ks, 128u, PL);
-                const uint64_t db = tc::smem_desc(Gs + 256u * ks, 128u, PL);
-                tc::mma_bf16(tbase + 16u * g, da, db, IDESC_MN, (j > 0 || ks > 0) ? 1u : 0u);
-            }
-            tc::mma_commit(empty + (g & 1));
-        }
-        return true;
-    };
-
-    bool ok = true;
-    if (nitems > 0) gather(0, ic<0>{});
-    for (int j = 0; j < nch && ok; ++j)
-        ok = item(j, ic<0>{}) && item(j, ic<1>{}) && item(j, ic<2>{}) && item(j, ic<3>{});
-    asm volatile("cp.async.wait_all;" ::: "memory"); // nothing in flight past this point
-    // ---- wait for every MMA of this CTA, then add the 4 accumulator tiles
-    // (row m = 16 (tap - 8 g) + ci, column co) to gW; warp w reads rows
-    // 32 (w % 4) + lane, columns 8 (w / 4) .. + 7
-    if (ok && nitems > 0) {
-        if (r == 0) {
-            tc::mma_commit(done);
-            flag[1] = mbar_wait_bounded(done, 0) ? 1 : 0;
-        }
-        __syncthreads();
-        ok = flag[1] != 0;
-        if (ok) {
-            tc::fence_after_sync();
-            const int m = 32 * (warp & 3) + (r & 31), ch = 8 * (warp >> 2);
+            // descriptors: K cores 128 bytes apart, planes H or KP rows; the
+            // address field counts rows (16 bytes)
+            const uint64_t da = tc::smem_desc(smem_u32(A), 128u, aplane), db = tc::smem_desc(smem_u32(G), 128u, gplane);
+            for (int z = 0; z < nz; ++z) {
 #pragma unroll 1
-            for (int g = 0; g < NG; ++g) {
-                float v[8];
-                tc::tmem_ld8(tbase + ((uint32_t)(32 * (warp & 3)) << 16) + 16u * g + (uint32_t)ch, v);
-                const int t = g * GT + m / 16, ci = m % 16;
-                if (t < 27) {
+                for (int k = 0; k < ks; ++k) {
+                    const uint64_t ak = da + (uint32_t)(2 * z * g.H + 16 * k), bk = db + (uint32_t)(2 * z * g.KP + 16 * k);
+                    const uint32_t acc = it + z + k > 0 ? 1u : 0u;
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) atomicAdd(a.gw + (t * 16 + ci) * 16 + ch + k, v[k]);
+                    for (int t = 0; t < 9; ++t)
+                        tc::mma_bf16(tbase + 16u * t, ak + (uint32_t)(t % 3 + g.RX * (t / 3)), bk, IDESC_MN, acc);
+                }
+            }
+            tc::mma_commit(&bar);
+        }
+    }
+    if (ok && it > 0) { // the last brick's MMAs, then gW
+        if (r == 0) flag = mbar_wait_bounded(&bar, (it - 1) & 1) ? 1 : 0;
+        __syncthreads();
+        ok = flag != 0;
+        // row 16 dz + ci of an M = 64 accumulator lies in lane 32 dz + ci; warp w
+        // reads dz = w % 4 (3: the dropped rows), columns 8 (w / 4) .. + 7
+        if (ok && (warp & 3) < 3) {
+            tc::fence_after_sync();
+            const int dz = warp & 3, ci = r & 31, co = 8 * (warp >> 2);
+#pragma unroll 1
+            for (int t = 0; t < 9; ++t) {
+                float v[8];
+                tc::tmem_ld8(tbase + ((uint32_t)(32 * dz) << 16) + 16u * t + (uint32_t)co, v);
+                if (ci < 16) { // gw rows are 64-byte aligned
+                    float4 *dst = reinterpret_cast<float4 *>(a.gw + ((t + 9 * dz) * 16 + ci) * 16 + co);
+                    atomicAdd(dst, make_float4(v[0], v[1], v[2], v[3]));
+                    atomicAdd(dst + 1, make_float4(v[4], v[5], v[6], v[7]));
                 }
             }
         }
@@ -247,7 +204,42 @@ __global__ void __launch_bounds__(NT, 2) wgrad_tc_kernel(const __grid_constant__
     if (!ok && r == 0 && a.err) atomicExch(a.err, kDevErrTimeout);
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tbase, TCOLS);
+    if (warp == 0) tc::tmem_dealloc(tbase, WGT_COLS);
+}
+
+// Brick shape of the weight gradient for B output cubes of side So: of the
+// splits that fit the shared memory of half an SM, the least of (bricks per
+// CTA) x (a brick's MMAs at 16 cycles each, its staging at 40 bytes a cycle and
+// 2500 cycles of latency) + 16 cycles of atomics per CTA.
+static WgGeo wgrad_geo(int B, int So, int ctas, size_t *smem)
+{
+    WgGeo best = {};
+    double least = 0;
+    for (int nx = (So + 63) / 64, last = nx + 2; nx <= last && nx <= So; ++nx) {
+        WgGeo g;
+        g.BX = (So + nx - 1) / nx;
+        g.RX = g.BX + 2;
+        g.bricks[0] = (So + g.BX - 1) / g.BX;
+        for (g.BZ = 1; g.BZ <= 8 && g.BZ <= So; ++g.BZ)
+            for (g.BY = 1; g.BY <= So; ++g.BY) {
+                g.KP = (g.RX * g.BY + 15) / 16 * 16;
+                g.H = (g.KP + 2 + 2 * g.RX + 7) / 8 * 8;
+                const int64_t bytes = 32LL * ((g.BZ + 3) * g.H + g.BZ * g.KP);
+                if (bytes > WGT_SMEM) break;
+                g.bricks[1] = (So + g.BY - 1) / g.BY;
+                g.bricks[2] = (So + g.BZ - 1) / g.BZ;
+                g.total = B * g.bricks[0] * g.bricks[1] * g.bricks[2];
+                            const double cost = (double)((g.total + ctas - 1) / ctas) *
+                                        (9.0 * g.BZ * g.KP + bytes / 40.0 + 2500.0) +
+                                    16.0 * (g.total < ctas ? g.total : ctas);
+                if (best.total == 0 || cost < least) {
+                    least = cost;
+                    best = g;
+                    *smem = (size_t)bytes;
+                }
+            }
+    }
+    return best;
 }
 
 // backward-data B tiles: tap e, K = the layer's output channel co, N = its
@@ -846,16 +838,13 @@ static unsigned wg_launch(int B, int So, int ctas, int &run)
 static DeviceOnce wgrad_once, brick_once[2];
 
 // weight gradient: persistent CTAs, two per SM
-static cn_status launch_wgrad(Args &a, cudaStream_t st)
+static cn_status launch_wgrad(Args &a, int B, int sms, cudaStream_t st)
 {
-    cn_status s = smem_opt_in(wgrad_once, wgrad_tc_kernel, SMEM);
+    cn_status s = smem_opt_in(wgrad_once, wgrad_tc_kernel, WGT_SMEM);
     if (s != CN_OK) return s;
-    int dev = 0, sms = 148;
-    CN_CUDA_TRY(cudaGetDevice(&dev));
-    CN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    a.chunks = (a.total + ROWS - 1) / ROWS;
-    const int64_t grid = a.chunks < 2LL * sms ? a.chunks : 2LL * sms;
-    wgrad_tc_kernel<<<(unsigned)grid, NT, SMEM, st>>>(a);
+    size_t smem = 0;
+    const WgGeo g = wgrad_geo(B, a.Sout, 2 * sms, &smem);
+    wgrad_tc_kernel<<<(unsigned)std::min(g.total, 2 * sms), WGT_NT, smem, st>>>(a, g);
     CN_CUDA_TRY(cudaGetLastError());
     return CN_OK;
 }
@@ -902,7 +891,6 @@ cn_status train_forward_tc(const TrainBufs &T, const float *x, const float *W, i
     a.Sout = S2;
     a.shift = 0;
     a.relu = 1;
-    a.total = (int64_t)B * S2 * S2 * S2;
     a.err = T.err;
     if ((s = launch_conv<FWD>(a, B, st)) != CN_OK) return s;
     l3_fwd_cl<<<grid_of(z_runs(B, S3), 128, 148 * 64), 128, 0, st>>>(T.h2, W3, T.y, B, S2);
@@ -934,9 +922,8 @@ cn_status train_backward_tc(const TrainBufs &T, const float *x, const float *W, 
     w.Sin = S1;
     w.Sout = S2;
     w.shift = 0;
-    w.total = (int64_t)B * S2 * S2 * S2;
     w.err = T.err;
-    if ((s = launch_wgrad(w, st)) != CN_OK) return s;
+    if ((s = launch_wgrad(w, B, sms, st)) != CN_OK) return s;
     Args d = {};
     d.src = T.gh2;
     d.act = T.h1;
@@ -945,7 +932,6 @@ cn_status train_backward_tc(const TrainBufs &T, const float *x, const float *W, 
     d.Sin = S2;
     d.Sout = S1;
     d.shift = -2;
-    d.total = (int64_t)B * S1 * S1 * S1;
     d.err = T.err;
     if ((s = launch_conv<BWD>(d, B, st)) != CN_OK) return s;
     ctas = wg_launch(B, S1, WG_CTAS * sms / 2, run);
