@@ -1,23 +1,22 @@
 // labfill.cu -- K0: explicit lab fill (Cartesian::loadLab into lab buffers).
 //
-// One CTA per (block, slab of lab planes along z).  The slab's lab cells
-// fall into four classes: the block's own cells, the x ghosts of the rows
-// inside the block, the y-ghost rows of the inside planes and the z-ghost
-// planes (non-tensorial labs: edges and corners stay undefined, as in the
-// reference).  The block's own planes are one contiguous run of memory,
-// brought by one bulk copy into shared memory; meanwhile the threads walk
-// the ghosts, those behind faces without a BC or a skipped neighbour in
-// closed form (the periodic neighbour's cell), eight loads in flight per
-// thread; ghost rows behind faces with BCs are resolved once per row (x
-// passes through the FieldLab resolution unchanged), other BC-chain cells
-// one by one (cn::lab_resolve: skip rule, BC chain); this one-pass form is
-// lab_fill_rows_kernel.  Tensorial labs and labs with ghost rows longer than
-// its row table (lab_fill_kernel), node and face grids
-// (lab_fill_grow_kernel) take per-class or per-cell resolution.  Stores
-// are coalesced along the lab's rows; the kernel is bound by memory
-// latency and HBM.  The stencil kernels fuse the same resolution into their
-// shared-memory staging; this kernel gives the reference's FieldLab
-// contents for user stencils and the bit-exact comparison with it.
+// One CTA per (block, slab of lab planes along z).  The slab's lab cells are
+// the block's own cells, the x ghosts, the y-ghost rows of the inside planes
+// and the z-ghost planes (non-tensorial labs: edges and corners stay
+// undefined, as in the reference).  The block's own planes are one contiguous
+// run of memory, brought by one bulk copy into shared memory; meanwhile the
+// threads walk the ghosts, those behind faces without a BC or a skipped
+// neighbour in closed form (the periodic neighbour's cell), several loads in
+// flight per thread; ghost rows are resolved once per row (x passes through
+// the FieldLab resolution unchanged), other BC-chain cells one by one
+// (cn::lab_resolve: skip rule, BC chain).  lab_fill_rows_kernel is the one-pass
+// form of labs without edges and corners, lab_fill_kernel walks row by row
+// (tensorial labs, and labs with more ghost rows than the former's table);
+// node and face grids (lab_fill_grow_kernel) take per-cell resolution.  Stores
+// are coalesced along the lab's rows.  The stencil kernels fuse the same
+// resolution into their shared-memory staging; this kernel gives the
+// reference's FieldLab contents for user stencils and the bit-exact comparison
+// with it.
 #include "cn_fastdiv.h"
 #include "cn_internal.h"
 #include "cn_tma.cuh"
@@ -27,15 +26,17 @@
 namespace cn {
 
 constexpr int KL = 4;              // cells per thread resolved before their loads
-constexpr int KL0 = 8;             // pairs of the block's own cells per thread in flight
 constexpr int KLM = 8;             // cells per thread in flight in the one-pass form
+constexpr int KLR = 3;             // rows in flight per thread of the row form
+constexpr int KLX = 3;             // x ghosts in flight per thread of the row form
 constexpr int kBulkBytes = 24576;  // largest bulk copy of a slab's block planes
 // target cells of a CTA's slab: three planes of the 38^2 lab of 32^3 blocks
 // with three ghosts.  Thinner slabs leave more of the SM's on-chip memory
 // to the L1 cache (the shared-memory carve-out follows the resident CTAs'
 // needs), which measured faster than thicker slabs
 constexpr int kCellsPerCta = 4332;
-constexpr int kRowsCtas = 4;       // resident CTAs per SM of the one-pass kernel
+constexpr int kRowsCtas = 4;       // resident CTAs per SM of the one-pass form
+constexpr int kWarpRowCtas = 6;    // of the row form
 
 // a cell's source, collected from lab_resolve
 template <typename T> struct LabSource {
@@ -123,32 +124,22 @@ __global__ void __launch_bounds__(256)
 
 // a row of class 2 or 3: the source of its first cell and its first cell's
 // offset in the lab
-template <typename T> struct RowSrc {
-    LabSource<T> s;
-    int dst;
+template <typename T> struct alignas(16) RowSrc {
+    int64_t idx; // of the first cell in the component
+    int dst;     // the first cell's offset in the lab
+    int kind;    // 0 undefined, 1 the value v, 2 + n: the cells times n signs
+    T v, s0, s1, s2;
 };
 constexpr int kRows = 96; // rows resolved per round
 
-template <typename T> struct Vec2;
-template <> struct Vec2<double> {
-    using type = double2;
-};
-template <> struct Vec2<float> {
-    using type = float2;
-};
-template <> struct Vec2<int32_t> {
-    using type = int2;
-};
-
-// Divisors of the cell-grid kernel's four cell classes (fixed per launch).
+// Divisors of the row form (fixed per launch).
 struct LabDivs {
-    FastDiv n0, n1;   // block extents along x, y
-    FastDiv gx;       // x ghosts per row: lo0 + hi0
-    FastDiv wrow, gy; // cells per ghost row (n0, or E0 if tensorial); y ghost rows: lo1 + hi1
-    FastDiv wpl;      // rows per z-ghost plane (n1, or E1 if tensorial)
+    FastDiv n0, n1; // block extents along x, y
+    FastDiv gx, gy; // ghosts per row along x: lo0 + hi0, along y: lo1 + hi1
+    FastDiv wpl;    // rows per z-ghost plane, and rows with x ghosts per plane: n1, or E1 if tensorial
 };
 
-// lab coordinates of class-1 cell u (the x ghosts of the inside rows)
+// lab coordinates of x ghost u of the inside rows
 __device__ __forceinline__ void class1_cell(const LabDivs &dv, int u, int gx, int n0, int n1, int lo0, int lo1, int zi0,
                                             int &x, int &y, int &z)
 {
@@ -159,16 +150,17 @@ __device__ __forceinline__ void class1_cell(const LabDivs &dv, int u, int gx, in
     z = zi0 + zp;
 }
 
-// Row `row` of classes 2 and 3 of a non-tensorial lab (rows [0, ny): the
-// y-ghost rows of the slab's inside planes; then the rows of its z-ghost
-// planes): the source of its first cell (x = 0 of the block) and that
+// Ghost row `row` of a slab: rows [0, ny) are the y-ghost rows of its inside
+// planes, then come the rows of its z-ghost planes (tensorial: the y-ghost rows
+// among them); the source of its first cell (x = 0 of the block) and that
 // cell's offset in the lab.  x passes through every step of the resolution
 // unchanged, so cell x of the row is the source shifted by x (or the same
 // value).
 template <typename T>
 __device__ __forceinline__ RowSrc<T> lab_row(const LabGeom &L, const BcView &bc, uint8_t mode, uint8_t faces,
                                              int block, int bx, int by, int bz, bool abc, const LabDivs &dv, int row,
-                                             int ny, int gy, int zi0, int nlo, int zhi, int z0, int E0, int E1)
+                                             int ny, int gy, bool tens, int zi0, int nlo, int zhi, int z0, int E0,
+                                             int E1)
 {
     const int n0 = L.n[0], n1 = L.n[1], n2 = L.n[2];
     int y, z; // lab coordinates of the row
@@ -177,8 +169,8 @@ __device__ __forceinline__ RowSrc<T> lab_row(const LabGeom &L, const BcView &bc,
         y = g < L.lo[1] ? g : g + n1;
         z = zi0 + zp;
     } else {
-        const int rr = row - ny, zp = dv.n1.div(rr);
-        y = rr - zp * n1 + L.lo[1];
+        const int rr = row - ny, zp = dv.wpl.div(rr);
+        y = rr - zp * (tens ? E1 : n1) + (tens ? 0 : L.lo[1]);
         z = zp < nlo ? z0 + zp : zhi + (zp - nlo);
     }
     const int q1 = y - L.lo[1], q2 = z - L.lo[2];
@@ -186,13 +178,20 @@ __device__ __forceinline__ RowSrc<T> lab_row(const LabGeom &L, const BcView &bc,
     const int crossed = (r1 ? (r1 < 0 ? 4 : 8) : 0) | (r2 ? (r2 < 0 ? 16 : 32) : 0);
     RowSrc<T> R;
     if (faces & crossed) {
-        lab_resolve<T, false>(L, bc, mode, block, bx, by, bz, 0, q1, q2, abc, R.s);
+        LabSource<T> s;
+        lab_resolve<T, false>(L, bc, mode, block, bx, by, bz, 0, q1, q2, abc, s);
+        R.idx = s.idx;
+        R.kind = s.kind == 2 ? 2 + s.nsign : s.kind;
+        R.v = s.v;
+        R.s0 = s.s0;
+        R.s1 = s.s1;
+        R.s2 = s.s2;
     } else {
         int nby = by + r1, nbz = bz + r2;
         nby = nby < 0 ? nby + L.nb[1] : (nby >= L.nb[1] ? nby - L.nb[1] : nby);
         nbz = nbz < 0 ? nbz + L.nb[2] : (nbz >= L.nb[2] ? nbz - L.nb[2] : nbz);
-        R.s.kind = 2;
-        R.s.idx = (int64_t)(bx + L.nb[0] * (nby + L.nb[1] * nbz)) * L.bstride + n0 * ((q1 - r1 * n1) + n1 * (q2 - r2 * n2));
+        R.kind = 2;
+        R.idx = (int64_t)(bx + L.nb[0] * (nby + L.nb[1] * nbz)) * L.bstride + n0 * ((q1 - r1 * n1) + n1 * (q2 - r2 * n2));
     }
     R.dst = L.lo[0] + E0 * (y + E1 * z);
     return R;
@@ -262,8 +261,7 @@ __global__ void __launch_bounds__(256, kRowsCtas)
     const int gx = L.lo[0] + L.hi[0], gy = L.lo[1] + L.hi[1];
     T *o = out + (int64_t)bl * E0 * E1 * E2;
     const int ny = nin * gy, nrows = ny + P.nghost * n1;
-    __shared__ __align__(16) unsigned char rows_raw[kRows * sizeof(RowSrc<T>)];
-    RowSrc<T> *rows = reinterpret_cast<RowSrc<T> *>(rows_raw);
+    __shared__ RowSrc<T> rows[kRows];
     // One pass over all three kinds of plain copies, KLM loads in flight
     // per thread: the block's own cells, the x ghosts behind clear faces
     // and the rows (classes 2, 3) whose source is a plain cell run.  The
@@ -285,7 +283,8 @@ __global__ void __launch_bounds__(256, kRowsCtas)
         bulk_g2s(lab_bulk, comp + bbase, bytes0, &bulk_bar);
     }
     for (int j = threadIdx.x; j < nrows; j += blockDim.x)
-        rows[j] = lab_row<T>(L, bc, mode, faces, block, bx, by, bz, abc, dv, j, ny, gy, zi0, nlo, zhi, z0, E0, E1);
+        rows[j] = lab_row<T>(L, bc, mode, faces, block, bx, by, bz, abc, dv, j, ny, gy, false, zi0, nlo, zhi, z0, E0,
+                             E1);
     __syncthreads(); // the rows, and the barrier's initialisation
     bool deferred = false;
     const int base = use_bulk ? A : 0; // the first item of the pass
@@ -316,9 +315,9 @@ __global__ void __launch_bounds__(256, kRowsCtas)
             } else if (t < tot) {
                 const int u = t - A - B, j = dv.n0.div(u), x = u - j * n0;
                 const RowSrc<T> &R = rows[j];
-                if (R.s.kind == 2 && R.s.nsign == 0) {
+                if (R.kind == 2) {
                     dst[k] = R.dst + x;
-                    idx[k] = R.s.idx + x;
+                    idx[k] = R.idx + x;
                 } else {
                     deferred = true;
                 }
@@ -369,9 +368,14 @@ __global__ void __launch_bounds__(256, kRowsCtas)
             } else {
                 const int u = t - A - B, j = dv.n0.div(u), x = u - j * n0;
                 const RowSrc<T> &R = rows[j];
-                if (R.s.kind == 2 && R.s.nsign == 0) continue;
-                src[0] = R.s;
-                src[0].idx += x;
+                if (R.kind == 2) continue;
+                src[0].kind = min(R.kind, 2);
+                src[0].nsign = R.kind - 2;
+                src[0].idx = R.idx + x;
+                src[0].v = R.v;
+                src[0].s0 = R.s0;
+                src[0].s1 = R.s1;
+                src[0].s2 = R.s2;
                 dst[0] = R.dst + x;
             }
             lab_store1<T>(comp, src[0], dst[0], o);
@@ -379,180 +383,173 @@ __global__ void __launch_bounds__(256, kRowsCtas)
     }
 }
 
-// Cell grids: the CTA's slab of lab planes as four classes of cells, each
-// walked by all threads so that a warp's cells take the same path:
-//   0  the block's own cells (planes and rows inside): plain copies;
-//   1  the x ghosts of those rows;
-//   2  the y-ghost rows of inside planes (x inside, or the whole row when
-//      tensorial);
-//   3  the z-ghost planes (x, y inside, or the whole plane when tensorial).
-// Class 1-3 cells beyond faces that carry no BC and no skipped neighbour are
-// the periodic neighbour's cells (closed form); the others take lab_resolve
-// (skips, BC chains).  Without tensorial ghosts, classes 2 and 3 are walked
-// as rows resolved once each.  Cells no class lists are the edges and corners of a
-// non-tensorial lab, which the reference leaves undefined.
-template <typename T>
-__global__ void __launch_bounds__(256, 4)
-    lab_fill_kernel(const T *__restrict__ comp, LabGeom L, BcView bc, int block_begin, int pz, LabDivs dv,
-                    int apply_bc, T *__restrict__ out)
+// Cell grids by rows: 2^wl threads (the least power of two that holds a row,
+// at most a warp) walk the cells of a row, so that a row's place and source are
+// found once for all its cells.  Tensorial labs, whose x ghosts cross other
+// faces too, and labs with more ghost rows than lab_fill_rows_kernel's table.
+// Tensorial labs are bound by instruction issue when each ghost is located by
+// itself: B200, all tensorial labs of 512^3 FP64 with three ghosts 873 -> 598
+// us, of 256^3 FP32 115 -> 81.  Labs without edges and corners are not (596 us by
+// the one-pass form, 615 by this one): their bound is the memory's latency.
+template <typename T, bool TENS>
+__global__ void __launch_bounds__(256, kWarpRowCtas)
+    lab_fill_kernel(const T *__restrict__ comp, LabGeom L, BcView bc, int block_begin, int pz, LabDivs dv, int wl,
+                         int apply_bc, int bulk, int *err, T *__restrict__ out)
 {
-    const int n0 = L.n[0], n1 = L.n[1], n2 = L.n[2];
+    const int n0 = L.n[0], n1 = L.n[1];
     const int E0 = n0 + L.lo[0] + L.hi[0];
     const int E1 = n1 + L.lo[1] + L.hi[1];
-    const int E2 = n2 + L.lo[2] + L.hi[2];
-    const int bl = blockIdx.y, z0 = blockIdx.x * pz; // block-major, as lab_fill_rows_kernel
-    const int z1 = min(z0 + pz, E2);
+    const int E2 = L.n[2] + L.lo[2] + L.hi[2];
+    // one CTA per (slab, block): x the slab, so that a block's slabs run
+    // together (CTAs start in the order of their linear index) and the ghost
+    // planes read from a block's z neighbours are read close in time to the
+    // neighbours' own CTAs, while they are in L2
+    const int bl = blockIdx.y, z0 = blockIdx.x * pz;
     const int block = block_begin + bl;
     const int bx = block % L.nb[0];
     const int by = (block / L.nb[0]) % L.nb[1];
     const int bz = block / (L.nb[0] * L.nb[1]);
     const uint8_t mode = bc.mode[block];
-    // faces of the block that carry a BC (other than Base) or a skipped
-    // neighbour: cells beyond them take the full resolution
     const uint8_t faces = bc.faces[block];
-    const bool abc = apply_bc != 0, tens = L.tensorial != 0;
-    // planes of the slab inside the block, and its z-ghost planes below / above
-    const SlabPlanes P = slab_planes(L, z0, z1);
-    const int zi0 = P.zi0, nin = P.nin, nlo = P.nlo, zhi = P.zhi, nghost = P.nghost;
-    const int wrow = tens ? E0 : n0, wpl = tens ? E1 : n1;
+    const bool abc = apply_bc != 0;
+    const SlabPlanes P = slab_planes(L, z0, min(z0 + pz, E2));
+    const int zi0 = P.zi0, nin = P.nin;
     const int gx = L.lo[0] + L.hi[0], gy = L.lo[1] + L.hi[1];
     T *o = out + (int64_t)bl * E0 * E1 * E2;
-    const int ny = nin * gy, nrows = ny + nghost * n1;
-    __shared__ __align__(16) unsigned char rows_raw[kRows * sizeof(RowSrc<T>)];
-    RowSrc<T> *rows = reinterpret_cast<RowSrc<T> *>(rows_raw);
-    // class 0: rows of the block's own cells, plain copies (KL loads in flight)
-    {
-        const T *blk = comp + (int64_t)block * L.bstride + (int64_t)n0 * n1 * (zi0 - L.lo[2]);
-        T *ob = o + L.lo[0] + E0 * (L.lo[1] + E1 * zi0);
-        const int cnt = nin * n1 * n0;
-        if ((n0 & 1) == 0) {
-            // pairs of cells along x: one 2-element load (the block's rows
-            // start on 2-element boundaries), two stores (lab rows need not)
-            using V = typename Vec2<T>::type;
-            const V *blk2 = reinterpret_cast<const V *>(blk);
-            const int cnt2 = cnt >> 1;
-            for (int p0 = threadIdx.x; p0 < cnt2; p0 += KL0 * blockDim.x) {
-                V v[KL0];
-                int d[KL0];
-#pragma unroll
-                for (int k = 0; k < KL0; ++k) {
-                    const int p = p0 + k * blockDim.x, t = 2 * p;
-                    const int r = dv.n0.div(t), zp = dv.n1.div(r);
-                    d[k] = p < cnt2 ? (t - r * n0) + E0 * ((r - zp * n1) + E1 * zp) : -1;
-                    if (p < cnt2) v[k] = blk2[p];
-                }
-#pragma unroll
-                for (int k = 0; k < KL0; ++k)
-                    if (d[k] >= 0) {
-                        ob[d[k]] = v[k].x;
-                        ob[d[k] + 1] = v[k].y;
-                    }
-            }
-        } else {
-            for (int t0 = threadIdx.x; t0 < cnt; t0 += KL * blockDim.x) {
-                T v[KL];
-                int d[KL];
-#pragma unroll
-                for (int k = 0; k < KL; ++k) {
-                    const int t = t0 + k * blockDim.x;
-                    const int r = dv.n0.div(t), zp = dv.n1.div(r);
-                    d[k] = t < cnt ? (t - r * n0) + E0 * ((r - zp * n1) + E1 * zp) : -1;
-                    v[k] = t < cnt ? blk[t] : T(0);
-                }
-#pragma unroll
-                for (int k = 0; k < KL; ++k)
-                    if (d[k] >= 0) ob[d[k]] = v[k];
-            }
-        }
+    const int own = nin * n1, ny = nin * gy, nrows = ny + P.nghost * (TENS ? E1 : n1);
+    const int lx = threadIdx.x & ((1 << wl) - 1), grp = threadIdx.x >> wl, ngrp = blockDim.x >> wl;
+    __shared__ RowSrc<T> rows[kRows];
+    // The block's own planes of the slab are one contiguous run of
+    // memory: with room in the dynamic shared memory (`bulk` bytes) one
+    // bulk copy brings them while the threads work on the ghosts.
+    extern __shared__ __align__(128) unsigned char lab_bulk[];
+    __shared__ __align__(8) uint64_t bulk_bar;
+    const T *src0 = comp + (int64_t)block * L.bstride + (int64_t)n0 * n1 * (zi0 - L.lo[2]);
+    const uint32_t bytes0 = (uint32_t)(own * n0) * (uint32_t)sizeof(T);
+    const bool use_bulk = own > 0 && bytes0 <= (uint32_t)bulk && ((uint32_t)(n0 * n1) * sizeof(T)) % 16 == 0;
+    if (use_bulk && threadIdx.x == 0) {
+        mbar_init(&bulk_bar, 1);
+        fence_mbar_init();
+        mbar_arrive_expect_tx(&bulk_bar, bytes0);
+        bulk_g2s(lab_bulk, src0, bytes0, &bulk_bar);
     }
-    // classes 1-3 cell by cell; without tensorial ghosts, classes 2 and 3 go
-    // by rows below
-#pragma unroll 1
-    for (int cls = 1; cls < (tens ? 4 : 2); ++cls) {
-        const int cnt = cls == 1 ? nin * n1 * gx : (cls == 2 ? nin * gy * wrow : nghost * wpl * wrow);
-        for (int t0 = threadIdx.x; t0 < cnt; t0 += KL * blockDim.x) {
-            LabSource<T> src[KL];
-            int dst[KL];
-#pragma unroll
-            for (int k = 0; k < KL; ++k) {
-                const int t = t0 + k * blockDim.x;
-                dst[k] = -1;
-                if (t >= cnt) continue;
-                int x, y, z; // lab coordinates
-                if (cls == 1) {
-                    const int r = dv.gx.div(t), zp = dv.n1.div(r);
-                    const int g = t - r * gx;
-                    x = g < L.lo[0] ? g : g + n0;
-                    y = r - zp * n1 + L.lo[1];
-                    z = zi0 + zp;
-                } else if (cls == 2) {
-                    const int r = dv.wrow.div(t), zp = dv.gy.div(r);
-                    const int g = r - zp * gy;
-                    x = t - r * wrow + (tens ? 0 : L.lo[0]);
-                    y = g < L.lo[1] ? g : g + n1;
-                    z = zi0 + zp;
-                } else {
-                    const int r = dv.wrow.div(t), zp = dv.wpl.div(r);
-                    x = t - r * wrow + (tens ? 0 : L.lo[0]);
-                    y = r - zp * wpl + (tens ? 0 : L.lo[1]);
-                    z = zp < nlo ? z0 + zp : zhi + (zp - nlo);
-                }
-                dst[k] = x + E0 * (y + E1 * z);
-                {
-                    const int q0 = x - L.lo[0], q1 = y - L.lo[1], q2 = z - L.lo[2];
-                    const int r0 = q0 < 0 ? -1 : (q0 >= n0 ? 1 : 0), r1 = q1 < 0 ? -1 : (q1 >= n1 ? 1 : 0),
-                              r2 = q2 < 0 ? -1 : (q2 >= n2 ? 1 : 0);
-                    const int crossed = (r0 ? (r0 < 0 ? 1 : 2) : 0) | (r1 ? (r1 < 0 ? 4 : 8) : 0) |
-                                        (r2 ? (r2 < 0 ? 16 : 32) : 0);
-                    if (faces & crossed) {
-                        lab_resolve<T, false>(L, bc, mode, block, bx, by, bz, q0, q1, q2, abc, src[k]);
-                    } else {
-                        // beyond clear faces only: no BC covers the cell, and it is the
-                        // periodic neighbour's cell (as lab_resolve gives it)
-                        int nbx = bx + r0, nby = by + r1, nbz = bz + r2;
-                        nbx = nbx < 0 ? nbx + L.nb[0] : (nbx >= L.nb[0] ? nbx - L.nb[0] : nbx);
-                        nby = nby < 0 ? nby + L.nb[1] : (nby >= L.nb[1] ? nby - L.nb[1] : nby);
-                        nbz = nbz < 0 ? nbz + L.nb[2] : (nbz >= L.nb[2] ? nbz - L.nb[2] : nbz);
-                        src[k].kind = 2;
-                        src[k].idx = (int64_t)(nbx + L.nb[0] * (nby + L.nb[1] * nbz)) * L.bstride + (q0 - r0 * n0) +
-                                     n0 * ((q1 - r1 * n1) + n1 * (q2 - r2 * n2));
-                    }
-                }
-            }
-            lab_store<T>(comp, src, dst, o);
-        }
-    }
-    if (tens) return;
-    // Classes 2 and 3 of a non-tensorial lab by rows: a y-ghost row of an
-    // inside plane, or a row of a z-ghost plane, holds the n0 cells with x
-    // inside the block, and x passes through every step of the resolution
-    // unchanged (no x BC covers them, the neighbour is the same), so the
-    // cells of a row are the row's first cell's source shifted by x (or its
-    // one value).  One thread resolves a row's first cell into shared
-    // memory; all threads then copy the rows' cells.
-#pragma unroll 1
+    // The y-ghost rows of the inside planes and the rows of the z-ghost
+    // planes: kRows at a time resolved by a thread each, then copied, KLR rows
+    // in flight per thread.
     for (int rb = 0; rb < nrows; rb += kRows) {
         const int nr = min(kRows, nrows - rb);
-        __syncthreads(); // the previous rows are copied
+        if (rb > 0) __syncthreads(); // the previous rows are copied
         for (int j = threadIdx.x; j < nr; j += blockDim.x)
-            rows[j] = lab_row<T>(L, bc, mode, faces, block, bx, by, bz, abc, dv, rb + j, ny, gy, zi0, nlo, zhi, z0, E0,
-                                 E1);
+            rows[j] = lab_row<T>(L, bc, mode, faces, block, bx, by, bz, abc, dv, rb + j, ny, gy, TENS, zi0, P.nlo, P.zhi,
+                                 z0, E0, E1);
         __syncthreads();
-        const int cells = nr * n0;
-        for (int t0 = threadIdx.x; t0 < cells; t0 += KL * blockDim.x) {
-            LabSource<T> src[KL];
-            int dst[KL];
+        for (int x = lx; x < n0; x += 1 << wl)
+            for (int j0 = grp; j0 < nr; j0 += KLR * ngrp) {
+                T v[KLR];
+                int dst[KLR], kind[KLR];
 #pragma unroll
-            for (int k = 0; k < KL; ++k) {
-                const int t = t0 + k * blockDim.x;
-                dst[k] = -1;
-                if (t >= cells) continue;
-                const int j = dv.n0.div(t), x = t - j * n0;
-                src[k] = rows[j].s;
-                src[k].idx += x;
-                dst[k] = rows[j].dst + x;
+                for (int k = 0; k < KLR; ++k) {
+                    const int j = j0 + k * ngrp;
+                    kind[k] = 0;
+                    if (j < nr) {
+                        const int4 h = *reinterpret_cast<const int4 *>(&rows[j]); // idx, dst, kind
+                        kind[k] = h.w;
+                        dst[k] = h.z + x;
+                        if (h.w == 1) v[k] = rows[j].v;
+                        else if (h.w) v[k] = comp[(((int64_t)h.y << 32) | (uint32_t)h.x) + x];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < KLR; ++k) {
+                    if (kind[k] == 0) continue;
+                    const RowSrc<T> &R = rows[j0 + k * ngrp];
+                    T q = v[k];
+                    if (kind[k] > 4) q = R.s2 * q;
+                    if (kind[k] > 3) q = R.s1 * q;
+                    if (kind[k] > 2) q = R.s0 * q;
+                    o[dst[k]] = q;
+                }
             }
-            lab_store<T>(comp, src, dst, o);
+    }
+    if (nrows == 0) __syncthreads(); // the barrier's initialisation
+    // The x ghosts of the own rows (tensorial: of all rows), KLX at a time: the
+    // periodic neighbour's cell where only clear faces lie between (as
+    // lab_resolve gives it), the others in a second pass.
+    const int xrows = TENS ? (min(z0 + pz, E2) - z0) * E1 : own, B = xrows * gx;
+    bool deferred = false;
+    auto ghost = [&](int t, int &x, int &y, int &z) { // lab coordinates of x ghost t
+        const int r = dv.gx.div(t), zp = dv.wpl.div(r), g = t - r * gx;
+        x = g < L.lo[0] ? g : g + n0;
+        y = TENS ? r - zp * E1 : r - zp * n1 + L.lo[1];
+        z = (TENS ? z0 : zi0) + zp;
+    };
+    auto beyond = [](int q, int n) { return q < 0 ? -1 : (q >= n ? 1 : 0); };
+    auto crossed = [](int r, int lo) { return r ? (r < 0 ? lo : 2 * lo) : 0; };
+    auto wrap = [](int b, int nb) { return b < 0 ? b + nb : (b >= nb ? b - nb : b); };
+    for (int t0 = threadIdx.x; t0 < B; t0 += KLX * blockDim.x) {
+        T v[KLX];
+        int dst[KLX];
+#pragma unroll
+        for (int k = 0; k < KLX; ++k) {
+            const int t = t0 + k * blockDim.x;
+            dst[k] = -1;
+            if (t >= B) continue;
+            int x, y, z;
+            ghost(t, x, y, z);
+            const int q0 = x - L.lo[0], q1 = y - L.lo[1], q2 = z - L.lo[2];
+            const int r0 = q0 < 0 ? -1 : 1, r1 = TENS ? beyond(q1, n1) : 0, r2 = TENS ? beyond(q2, L.n[2]) : 0;
+            if (faces & (crossed(r0, 1) | crossed(r1, 4) | crossed(r2, 16))) {
+                deferred = true;
+            } else {
+                const int nbx = wrap(bx + r0, L.nb[0]), nby = wrap(by + r1, L.nb[1]), nbz = wrap(bz + r2, L.nb[2]);
+                dst[k] = x + E0 * (y + E1 * z);
+                v[k] = comp[(int64_t)(nbx + L.nb[0] * (nby + L.nb[1] * nbz)) * L.bstride + (q0 - r0 * n0) +
+                            n0 * ((q1 - r1 * n1) + n1 * (q2 - r2 * L.n[2]))];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < KLX; ++k)
+            if (dst[k] >= 0) o[dst[k]] = v[k];
+    }
+    // the block's own rows
+    if (use_bulk) {
+        if (!mbar_wait_bounded_sleep(&bulk_bar, 0, 200)) {
+            // record the error; a second bounded wait keeps the copy from
+            // landing in a later CTA's shared memory
+            if (threadIdx.x == 0 && err) atomicExch(err, kDevErrTimeout);
+            mbar_wait_bounded_sleep(&bulk_bar, 0, 200);
+        } else {
+            const T *sb = reinterpret_cast<const T *>(lab_bulk);
+#pragma unroll 4
+            for (int r = grp; r < own; r += ngrp) {
+                const int zp = dv.n1.div(r), d = L.lo[0] + E0 * ((r - zp * n1 + L.lo[1]) + E1 * (zi0 + zp));
+                for (int x = lx; x < n0; x += 1 << wl) o[d + x] = sb[r * n0 + x];
+            }
+        }
+    } else {
+        for (int x = lx; x < n0; x += 1 << wl)
+            for (int r0 = grp; r0 < own; r0 += KLR * ngrp) {
+                T v[KLR];
+#pragma unroll
+                for (int k = 0; k < KLR; ++k)
+                    if (r0 + k * ngrp < own) v[k] = src0[(r0 + k * ngrp) * n0 + x];
+#pragma unroll
+                for (int k = 0; k < KLR; ++k) {
+                    const int r = r0 + k * ngrp, zp = dv.n1.div(r);
+                    if (r < own) o[L.lo[0] + E0 * ((r - zp * n1 + L.lo[1]) + E1 * (zi0 + zp)) + x] = v[k];
+                }
+            }
+    }
+    if (deferred) { // this thread's x ghosts beyond faces with BCs or skips, one by one
+        for (int t = threadIdx.x; t < B; t += blockDim.x) {
+            int x, y, z;
+            ghost(t, x, y, z);
+            const int q0 = x - L.lo[0], q1 = y - L.lo[1], q2 = z - L.lo[2];
+            if (!(faces & (crossed(beyond(q0, n0), 1) | crossed(beyond(q1, n1), 4) | crossed(beyond(q2, L.n[2]), 16))))
+                continue;
+            LabSource<T> src;
+            lab_resolve<T, false>(L, bc, mode, block, bx, by, bz, q0, q1, q2, abc, src);
+            lab_store1<T>(comp, src, x + E0 * (y + E1 * z), o);
         }
     }
 }
@@ -570,19 +567,19 @@ static cn_status launch_fill(cn_grid *g, int comp, const cn_stencil *s, int b0, 
     // planes per CTA: about kCellsPerCta cells
     int pz = (int)std::max<int64_t>(1, std::min<int64_t>(E2, kCellsPerCta / plane));
     const bool grow = L.grow[0] || L.grow[1] || L.grow[2];
-    // The one-pass kernel holds a slab's ghost rows (classes 2, 3) in a
-    // table of kRows: slabs of fewer planes until every slab's rows fit.
+    // Both forms resolve kRows ghost rows of a slab at a time: slabs of fewer
+    // planes until every slab's rows fit.  The one-pass form needs that.
     auto rows_fit = [&](int p) {
         for (int z0 = 0; z0 < E2; z0 += p) {
             const SlabPlanes P = slab_planes(L, z0, (int)std::min<int64_t>(z0 + p, E2));
-            if (P.nin * (L.lo[1] + L.hi[1]) + P.nghost * L.n[1] > kRows) return false;
+            if (P.nin * (L.lo[1] + L.hi[1]) + P.nghost * (L.tensorial ? E1 : L.n[1]) > kRows) return false;
         }
         return true;
     };
-    bool rows_form = !grow && !L.tensorial;
-    if (rows_form) {
+    bool one_pass = !grow && !L.tensorial;
+    if (one_pass) {
         while (pz > 1 && !rows_fit(pz)) --pz;
-        rows_form = rows_fit(pz);
+        one_pass = rows_fit(pz);
     }
     const int64_t slabs = (E2 + pz - 1) / pz;
     if (slabs > 65535) return fail(CN_ERR_UNSUPPORTED, "cn_lab_fill: more than 65535 lab slabs per block");
@@ -591,15 +588,18 @@ static cn_status launch_fill(cn_grid *g, int comp, const cn_stencil *s, int b0, 
     dv.n0 = FastDiv((uint32_t)L.n[0]);
     dv.n1 = FastDiv((uint32_t)L.n[1]);
     dv.gx = FastDiv((uint32_t)(L.lo[0] + L.hi[0]));
-    dv.wrow = FastDiv((uint32_t)(L.tensorial ? E0 : L.n[0]));
     dv.gy = FastDiv((uint32_t)(L.lo[1] + L.hi[1]));
     dv.wpl = FastDiv((uint32_t)(L.tensorial ? E1 : L.n[1]));
+    int wl = 2;
+    while (wl < 5 && (1 << wl) < L.n[0]) ++wl;
     // dynamic shared memory for the bulk copy of a slab's block planes
     const int64_t bulk = (int64_t)pz * L.n[0] * L.n[1] * (int64_t)sizeof(T);
-    const int nbulk = rows_form && bulk <= kBulkBytes ? (int)bulk : 0;
-    if (rows_form) {
-        static DeviceOnce once;
-        cn_status r = smem_opt_in(once, lab_fill_rows_kernel<T>, (size_t)kBulkBytes);
+    const int nbulk = !grow && bulk <= kBulkBytes ? (int)bulk : 0;
+    if (!grow) {
+        static DeviceOnce once[3];
+        cn_status r = one_pass       ? smem_opt_in(once[0], lab_fill_rows_kernel<T>, (size_t)kBulkBytes)
+                      : L.tensorial ? smem_opt_in(once[1], lab_fill_kernel<T, true>, (size_t)kBulkBytes)
+                                    : smem_opt_in(once[2], lab_fill_kernel<T, false>, (size_t)kBulkBytes);
         if (r != CN_OK) return r;
     }
     // CTAs in block-major order: the slab along x, the block along y (a
@@ -611,11 +611,13 @@ static cn_status launch_fill(cn_grid *g, int comp, const cn_stencil *s, int b0, 
             lab_fill_grow_kernel<T><<<grid, threads, 0, st>>>(src, L, bc_view(g, comp), b0 + c0, pz,
                                                               FastDiv((uint32_t)E0), FastDiv((uint32_t)plane),
                                                               apply_bc, out);
-        } else if (rows_form) {
+        } else if (one_pass) {
             lab_fill_rows_kernel<T><<<grid, threads, nbulk, st>>>(src, L, bc_view(g, comp), b0 + c0, pz, dv,
                                                                   apply_bc, nbulk, g->d_err, out);
         } else {
-            lab_fill_kernel<T><<<grid, threads, 0, st>>>(src, L, bc_view(g, comp), b0 + c0, pz, dv, apply_bc, out);
+            auto kernel = L.tensorial ? lab_fill_kernel<T, true> : lab_fill_kernel<T, false>;
+            kernel<<<grid, threads, nbulk, st>>>(src, L, bc_view(g, comp), b0 + c0, pz, dv, wl, apply_bc, nbulk,
+                                                 g->d_err, out);
         }
     }
     CN_CUDA_TRY(cudaGetLastError());

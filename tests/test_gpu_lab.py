@@ -197,3 +197,23 @@ def test_lab_fill_thinner_slabs_vs_oracle(cn, oracle_lib):
             want, wdef = O.lab_fill(comp, nb, n, lo, hi, False, bcl, b)
             LC.compare_defined(labs[b], written[b], want, wdef)
         g.close()
+
+
+@pytest.mark.parametrize("n0", [9, 31, 33, 70])
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
+def test_tensorial_row_widths_vs_oracle(cn, oracle_lib, n0, dt):
+    """Tensorial labs whose rows fill a part of a warp, all but one lane, a
+    warp and one cell, and more than two warps; slabs that end inside the
+    block and rows resolved in several rounds; bit-exact against the oracle."""
+    O = oracle_lib
+    rng = np.random.default_rng(41 + n0)
+    nb, n, lo, hi = (2, 1, 2), (n0, 37, 8), (3, 2, 1), (1, 3, 2)
+    comp = (rng.standard_normal(4 * O.block_stride(n, dt)) * 10).astype(dt)
+    bcl = {b: [(int(rng.integers(0, 3)), int(rng.integers(0, 2)), int(rng.integers(0, 4)),
+                float(rng.choice([-1, 0.5, 2]))) for _ in range(3)] for b in (1, 2)}
+    g = make_grid(cn, comp, nb, n, bcl)
+    labs, written = lab_fill_all(cn, g, lo, hi, True)
+    for b in range(4):
+        want, wdef = O.lab_fill(comp, nb, n, lo, hi, True, bcl, b)
+        LC.compare_defined(labs[b], written[b], want, wdef)
+    g.close()
