@@ -108,6 +108,37 @@ def test_from_aos_matches_oracle(cn, grid_dtype, file_dtype):
         g.close()
 
 
+@pytest.mark.parametrize("entity", [0, 1])
+@pytest.mark.parametrize("ncomp", [1, 4, 5, 9])
+def test_aos_item_edges(cn, ncomp, entity):
+    """Rows longer than an item (5 x 520 cells), items that span rows and end
+    inside one, and ranges that are whole planes of the file (cut from all
+    points) or parts of rows; both directions, bit for bit."""
+    import torch
+    rng = np.random.default_rng(60 + ncomp)
+    nb, cells = (5, 1, 3), (520, 3, 2)
+    g, comps = _grid(cn, rng, entity, ncomp, np.float64, nb, cells)
+    top = cn.IO.index_range(g)[1]
+    for sb, se in (([0, 0, 0], list(top)), ([0, 0, 1], [top[0], top[1], top[2] - 1]), ([3, 0, 0], list(top)),
+                   ([0, 1, 0], [top[0], top[1], top[2] + 1])):
+        shape = (se[2] - sb[2], se[1] - sb[1], se[0] - sb[0], ncomp)
+        init = np.full(shape, -5, dtype=np.float32)
+        out = torch.from_numpy(init.copy()).cuda()
+        cn.IO.Field2AOS(g, (sb, se), np.float32, out=out)
+        want = A.grid_to_aos(comps, nb, cells, entity, g.block_stride, sb, se, init.copy().ravel())
+        assert np.array_equal(out.cpu().numpy().ravel().view(np.uint8), want.view(np.uint8)), (sb, se)
+        buf = rng.standard_normal(shape).astype(np.float32)
+        back = A.aos_to_grid(buf.ravel(), comps, nb, cells, entity, g.block_stride, sb, se)
+        cn.IO.AOS2Field(torch.from_numpy(buf).cuda(), g, (sb, se))
+        for c in range(ncomp):
+            got = g.download(c)
+            for flat, beg, ext in A._blocks(nb, cells, entity):
+                k = slice(flat * g.block_stride, flat * g.block_stride + ext[0] * ext[1] * ext[2])
+                assert np.array_equal(got[k].view(np.uint8), back[c][k].view(np.uint8)), (sb, se, c, flat)
+        comps = back
+    g.close()
+
+
 def test_face_container_directions(cn):
     """A FaceContainer grid writes the face grid of the requested direction
     (AOSDriver<FaceContainer>, IO/FieldAOS.h:136-141)."""
