@@ -33,21 +33,28 @@ struct Src {
         t.ih[0] = t.ih[1] = t.ih[2] = (T)B.ih;
         t.bx = t.by = t.bz = 0;
     }
-    // a ghost from a block on the same level is a plain copy of its cell;
-    // level-interface ghosts (prolongation, restriction) take halo5()
-    template <typename T>
-    __device__ __forceinline__ bool plain_offset(const euler::TileInfo<T> &t, int gx, int gy, int gz,
-                                                 int64_t &off) const
+    // The source of a quarter (4 x 4 cells, 3 deep) of a tile's side.  Tiles,
+    // block origins and the lookup grid's cells are multiples of 8 level-1
+    // cells, so the quarter lies in one cell of that grid, hence in one block:
+    // it is looked up once for its cells (a lookup per cell is three dependent
+    // loads and two divisions).  B200, 3885 blocks of 8^3 to 32^3 cells (12.8 M
+    // cells), an RK3 step in FP64: 4654 -> 4522 us; 4408 with the loads of all
+    // components of a level-interface ghost in flight together.
+    // i = 8 axis + 4 (upper side) + quarter
+    using Side = SideSrc;
+    template <typename T> __device__ __forceinline__ Side side(const euler::TileInfo<T> &t, int i) const
     {
-        return same_level_offset(A, t.block, gx, gy, gz, off);
+        const int D = i >> 3, n = (i & 4) ? 8 : -1, a = 4 * (i & 1), b = 2 * (i & 2);
+        return side_source(A, t.block, t.x0 + (D == 0 ? n : a), t.y0 + (D == 1 ? n : (D == 0 ? a : b)),
+                           t.z0 + (D == 2 ? n : b));
     }
-    // all five components of a level-interface ghost: the geometry once
+    // all five components of a level-interface ghost
     template <typename T>
-    __device__ __forceinline__ void halo5(const T *const (&U)[5], const euler::TileInfo<T> &t, int gx, int gy, int gz,
+    __device__ __forceinline__ void halo5(const T *const (&U)[5], const Side &S, int gx, int gy, int gz,
                                           T (&v)[5]) const
     {
-        const Ghost g = resolve(A, t.block, gx, gy, gz);
-#pragma unroll 1
+        const Ghost g = S.ghost(gx, gy, gz);
+#pragma unroll
         for (int c = 0; c < 5; ++c) v[c] = gather<T>(U[c], g);
     }
 };
@@ -64,14 +71,15 @@ __global__ void __launch_bounds__(euler::NT, 3) stage_kernel(euler::StageParams<
     T *A = W + 5 * euler::Stg<T>::SV;
     __shared__ double red[euler::NT / 32][5];
     __shared__ euler::TileInfo<T> ts;
+    __shared__ SideSrc sides[euler::NSIDES];
     if constexpr (ONE) {
         const int tile = src.items[blockIdx.x].x;
-        euler::stage_tile<T>(p, src, tile, W, A, red, &ts);
+        euler::stage_tile<T>(p, src, tile, W, A, red, &ts, sides);
     } else {
         for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
             const int2 it = src.items[item];
             for (int k = 0; k < it.y; ++k)
-                euler::stage_tile<T>(p, src, it.x + k, W, A, red, &ts);
+                euler::stage_tile<T>(p, src, it.x + k, W, A, red, &ts, sides);
         }
     }
 }

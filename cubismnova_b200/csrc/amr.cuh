@@ -49,26 +49,13 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ int clampi(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
 
+__device__ __forceinline__ double2 pair(const double *p) { return *reinterpret_cast<const double2 *>(p); }
+__device__ __forceinline__ float2 pair(const float *p) { return *reinterpret_cast<const float2 *>(p); }
+
 template <typename T>
 __device__ __forceinline__ T cell(const T *comp, const BlockDev &B, int x, int y, int z)
 {
     return comp[B.off + x + (int64_t)B.n * (y + (int64_t)B.n * z)];
-}
-
-// Element offset (in every component) of lab cell q of block b, outside b,
-// when the block covering it is on b's level: the ghost is a plain copy of
-// that cell, as value() gives it.  False for level-interface ghosts.
-__device__ __forceinline__ bool same_level_offset(const Geom &A, int b, int qx, int qy, int qz, int64_t &off)
-{
-    const BlockDev B = A.blk[b];
-    const int cs = B.level == 0 ? 2 : 1;
-    const int X = wrap(B.ox + qx * cs, A.L[0]), Y = wrap(B.oy + qy * cs, A.L[1]), Z = wrap(B.oz + qz * cs, A.L[2]);
-    const int s = A.block_at(X, Y, Z);
-    const BlockDev S = A.blk[s];
-    if (S.level != B.level) return false;
-    const int fx = (X - S.ox) / cs, fy = (Y - S.oy) / cs, fz = (Z - S.oz) / cs;
-    off = S.off + fx + (int64_t)S.n * (fy + (int64_t)S.n * fz);
-    return true;
 }
 
 // Where lab cell q (tile coordinates of block b, possibly outside it) takes
@@ -138,12 +125,58 @@ template <typename T> __device__ __forceinline__ T gather(const T *comp, const G
         const T b1 = add_rn(mul_rn(a, a2), mul_rn(c, a3));
         return add_rn(mul_rn(a, b0), mul_rn(c, b1));
     }
-    // coarse ghost cell over a fine block: mean of its 8 children
+    // coarse ghost cell over a fine block: mean of its 8 children (pairs along
+    // x: offsets, extents and g.fx are even)
     T v[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
-        v[k] = cell<T>(comp, S, g.fx + (k & 1), g.fy + ((k >> 1) & 1), g.fz + (k >> 2));
+    for (int k = 0; k < 8; k += 2) {
+        const auto w = pair(&comp[S.off + g.fx + (int64_t)S.n * ((g.fy + ((k >> 1) & 1)) + (int64_t)S.n * (g.fz + (k >> 2)))]);
+        v[k] = w.x;
+        v[k + 1] = w.y;
+    }
     return (((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]))) * T(0.125);
+}
+
+// The source of all lab cells of block b in one cell of the lookup grid, for
+// any of them, q: the block that covers them and the shift from b's tile
+// coordinates (times b's cell size, cs) to offsets inside it.
+struct SideSrc {
+    int64_t off; // kind 0: element offset of tile coordinate (0, 0, 0) of b; else of the block
+    int n, kind; // as Ghost
+    int dx, dy, dz;
+    __device__ __forceinline__ bool plain() const { return kind == 0; }
+    __device__ __forceinline__ int64_t offset(int x, int y, int z) const // kind 0
+    {
+        return off + x + (int64_t)n * (y + (int64_t)n * z);
+    }
+    __device__ __forceinline__ Ghost ghost(int x, int y, int z) const // kinds 1 (cs = 1) and 2 (cs = 2)
+    {
+        Ghost g;
+        g.kind = kind;
+        g.S.n = n;
+        g.S.off = off;
+        g.fx = x * kind + dx;
+        g.fy = y * kind + dy;
+        g.fz = z * kind + dz;
+        return g;
+    }
+};
+__device__ __forceinline__ SideSrc side_source(const Geom &A, int b, int qx, int qy, int qz)
+{
+    const BlockDev B = A.blk[b];
+    const int cs = B.level == 0 ? 2 : 1;
+    const int X = B.ox + qx * cs, Y = B.oy + qy * cs, Z = B.oz + qz * cs;
+    const int wx = wrap(X, A.L[0]), wy = wrap(Y, A.L[1]), wz = wrap(Z, A.L[2]);
+    const BlockDev S = A.blk[A.block_at(wx, wy, wz)];
+    SideSrc r;
+    r.n = S.n;
+    r.kind = S.level == B.level ? 0 : (S.level < B.level ? 1 : 2);
+    r.dx = wx - X + B.ox - S.ox;
+    r.dy = wy - Y + B.oy - S.oy;
+    r.dz = wz - Z + B.oz - S.oz;
+    r.off = S.off;
+    if (r.kind == 0) r.off += r.dx / cs + (int64_t)S.n * (r.dy / cs + (int64_t)S.n * (r.dz / cs));
+    return r;
 }
 
 // value of lab cell q (tile coordinates of block b, possibly outside it)

@@ -21,6 +21,7 @@ constexpr int G = 3;                  // ghost width
 constexpr int NCORE = TB * TB * TB;   // tile cells: 512
 constexpr int NLINE = TB * TB;        // lines along one direction: 64
 constexpr int NHALO = 2 * G * NLINE;  // one direction's halo slabs: 384
+constexpr int NSIDES = 24;            // quarters (4 x 4 cells) of a tile's six sides
 // Shared-memory entry of core cell (x, y, z): a permutation of the dense
 // index without padding, e = (x ^ y) + 8 (y ^ z) + 64 z.  For lines along
 // any direction the 16 (FP64, FP32 pairs) or 32 (FP32) lines that one
@@ -321,12 +322,12 @@ __device__ __forceinline__ void sweep(int D, T *__restrict__ W, T *__restrict__ 
 }
 
 // Starts the copies of direction D's two 3-cell halo slabs into its slot as
-// conservative values, cell by cell: plain cells (inside the block, or a copy
-// of another block's cell) asynchronously, the others resolved by the source
-// policy, all five components at once, and stored.  The caller commits the
-// group.
+// conservative values, cell by cell: plain copies of a cell asynchronously, the
+// others resolved by the source policy, all five components at once, and
+// stored.  The caller commits the group.
 template <typename T, typename Src>
-__device__ __forceinline__ void issue_halo(int D, const StageParams<T> &p, const Src &src, const TileInfo<T> &t, T *W)
+__device__ __forceinline__ void issue_halo(int D, const StageParams<T> &p, const Src &src, const TileInfo<T> &t,
+                                           const typename Src::Side *sides, T *W)
 {
     static_assert(NHALO % NT == 0, "whole halo cells per thread");
 #pragma unroll
@@ -334,20 +335,18 @@ __device__ __forceinline__ void issue_halo(int D, const StageParams<T> &p, const
         int x, y, z, e;
         halo_cell(D, threadIdx.x + j * NT, x, y, z, e);
         e += Stg<T>::slot(D);
+        // the quarter of the side the cell lies in: the other two axes, in order
+        const int q = D == 0 ? x : (D == 1 ? y : z), a = D == 0 ? y : x, b = D == 2 ? y : z;
+        const typename Src::Side &S = sides[8 * D + 4 * (q > 0) + (a >> 2) + 2 * (b >> 2)];
         const int gx = t.x0 + x, gy = t.y0 + y, gz = t.z0 + z;
-        int64_t o = 0;
-        bool plain = (unsigned)gx < (unsigned)t.N0 && (unsigned)gy < (unsigned)t.N1 && (unsigned)gz < (unsigned)t.N2;
-        if (plain)
-            o = t.boff + gx + (int64_t)t.N0 * (gy + (int64_t)t.N1 * gz);
-        else
-            plain = src.plain_offset(t, gx, gy, gz, o);
-        if (plain) {
+        if (S.plain()) {
+            const int64_t o = S.offset(gx, gy, gz);
 #pragma unroll
             for (int c = 0; c < 5; ++c)
                 cp_async(&prim(W, c, e), p.U[c] + o);
         } else {
             T v[5];
-            src.halo5(p.U, t, gx, gy, gz, v);
+            src.halo5(p.U, S, gx, gy, gz, v);
 #pragma unroll
             for (int c = 0; c < 5; ++c)
                 prim(W, c, e) = v[c];
@@ -496,17 +495,19 @@ template <typename T> struct Epilogue {
 // The whole stage for one tile whose cells the threads copy themselves (rows
 // of 8 cells, 16-byte aligned: block offsets and extents are multiples of 8
 // cells): staging, three sweeps, epilogue.  Uses W [5][Stg<T>::SV], A [5][NACC]
-// (16-byte aligned) and red [NT/32][5] in shared memory.
+// (16-byte aligned), red [NT/32][5], ts and sides [NSIDES] in shared memory.
 template <typename T, typename Src>
 __device__ __forceinline__ void stage_tile(const StageParams<T> &p, const Src &src, int item, T *W, T *A,
-                                           double (*red)[5], TileInfo<T> *ts)
+                                           double (*red)[5], TileInfo<T> *ts, typename Src::Side *sides)
 {
-    // the tile's geometry is kept in shared memory (ts) and re-read after each
-    // barrier, so it does not occupy registers across the three sweeps
+    // the tile's geometry is kept in shared memory (ts, and the sources of the
+    // quarters of its six sides) and re-read after each barrier, so it does not
+    // occupy registers across the three sweeps
     {
         TileInfo<T> w;
         src.template tile<T>(item, w);
         if (threadIdx.x == 0) *ts = w;
+        if (threadIdx.x < NSIDES) sides[threadIdx.x] = src.side(w, threadIdx.x);
     }
     __syncthreads();
     const TileInfo<T> &t = *ts;
@@ -524,7 +525,7 @@ __device__ __forceinline__ void stage_tile(const StageParams<T> &p, const Src &s
     constexpr int first = Stg<T>::all ? 3 : 2; // directions whose slots are free now
 #pragma unroll 1
     for (int D = 0; D < first; ++D) {
-        issue_halo<T>(D, p, src, t, W);
+        issue_halo<T>(D, p, src, t, sides, W);
         cp_commit();
     }
     cp_wait<first>();
@@ -548,7 +549,7 @@ __device__ __forceinline__ void stage_tile(const StageParams<T> &p, const Src &s
             // W, this slot; every thread is done with the previous sweep
             __syncthreads();
             if (D == 1) {
-                issue_halo<T>(2, p, src, t, W);
+                issue_halo<T>(2, p, src, t, sides, W);
                 cp_commit();
             }
             sweep_dir<T, false>(D, p, t, W, A);
