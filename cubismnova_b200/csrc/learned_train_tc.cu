@@ -444,7 +444,7 @@ static bool brick_geo(int So, BrickGeo &g)
 // tap's weights read from shared memory, serves several cells or taps; B200,
 // batch of 32 patches of 32^3 cells, against one cell and tap at a time:
 // l1_fwd_cl 170 -> 90 us, l3_fwd_cl 118 -> 62, l3_bwd_data_cl 113 -> 64,
-// l3_wgrad_cl 194 -> 73, l1_wgrad_cl 294 -> 170.
+// l3_wgrad_cl 194 -> 60, l1_wgrad_cl 294 -> 152.
 __device__ __forceinline__ float2 fma2(float a, float2 b, float2 c) { return __ffma2_rn(make_float2(a, a), b, c); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
@@ -682,7 +682,7 @@ __device__ __forceinline__ float warp_sum16(float (&v)[16])
 // The weight gradients of the first and last layers: blocks of 9 warps, warp w
 // = taps (dx, dy) = (w % 3, w / 3) with all three dz.  The lanes of all 9 warps
 // take the same 32 columns (patch b, x, y) of output cells and walk up runs of
-// them, with the BF16 operand unpacked once per cell (the next plane's in
+// them, with the BF16 operand unpacked once per cell (the next planes in
 // flight) and the other one in a window of three planes.  The shifted reads of
 // the 9 warps hit L1.  Layer 1's two input channels are two blocks (its 96
 // accumulators in one thread left one block per SM: 318 us).  The warps' sums
@@ -690,7 +690,11 @@ __device__ __forceinline__ float warp_sum16(float (&v)[16])
 // shuffles per value made them the end of every small batch (8 patches of
 // 16^3, the whole step: 299 us, this way 252).
 constexpr int WG_THREADS = 9 * 32;
-constexpr int WG_CTAS = 3; // resident per SM
+// Resident per SM, planes in flight: the batch of 32 patches of 32^3 in all, us:
+// 3 and 1 1011, 2 and 2 986, 2 and 3 1112 (spills); 3 with 4 planes in shared
+// memory 991.
+constexpr int WG_CTAS = 2;
+constexpr int WG_AHEAD = 2;
 
 struct WgItem {
     int b, x, y, z0, z1;
@@ -742,28 +746,38 @@ __global__ void __launch_bounds__(WG_THREADS, WG_CTAS)
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
         const WgItem q = wg_item(item, runs, run, columns, So);
         const uint16_t *hp = h2 + (q.b * s3 + q.x + dx + (int64_t)S * (q.y + dy) + s2 * q.z0) * 16;
-        const float *gp = gc + q.b * (o2 * So) + q.x + (int64_t)So * q.y;
-        float g1 = 0.f, g2 = 0.f; // gc one and two planes below
-        Raw16 next = load_raw(hp);
-        float gn = q.ok ? __ldg(gp + q.z0 * o2) : 0.f;
-        for (int z = q.z0; z < q.z1 + 2; ++z) {
-            const Raw16 cur = next;
-            const float g0 = gn;
-            if (z + 1 < q.z1 + 2) {
-                hp += s2 * 16;
-                next = load_raw(hp);
-                gn = q.ok && z + 1 < q.z1 ? __ldg(gp + (z + 1) * o2) : 0.f;
-            }
-            float2 v[8];
-            unpack_raw(cur, v); // plane z of h2: dz 0 of cell z, 1 of z - 1, 2 of z - 2
+        const float *gp = gc + q.b * (o2 * So) + q.x + (int64_t)So * q.y + o2 * q.z0;
+        const int nz = q.z1 - q.z0, planes = nz + 2;
+        Raw16 hb[WG_AHEAD]; // the next planes of h2 and of gc (0 past the run and for lanes without a column)
+        float gb[WG_AHEAD];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                acc[0][i] = fma2(g0, v[i], acc[0][i]);
-                acc[1][i] = fma2(g1, v[i], acc[1][i]);
-                acc[2][i] = fma2(g2, v[i], acc[2][i]);
+        for (int k = 0; k < WG_AHEAD; ++k) {
+            if (k < planes) hb[k] = load_raw(hp + k * s2 * 16);
+            gb[k] = q.ok && k < nz ? __ldg(gp + k * o2) : 0.f;
+        }
+        hp += WG_AHEAD * s2 * 16;
+        gp += WG_AHEAD * o2;
+        float g1 = 0.f, g2 = 0.f; // gc at planes z - 1, z - 2
+        for (int z = 0; z < planes; z += WG_AHEAD) {
+#pragma unroll
+            for (int k = 0; k < WG_AHEAD; ++k) {
+                if (z + k >= planes) break;
+                float2 v[8];
+                unpack_raw(hb[k], v); // plane z of h2: dz 0 of cell z, 1 of z - 1, 2 of z - 2
+                const float g0 = gb[k];
+                if (z + k + WG_AHEAD < planes) hb[k] = load_raw(hp);
+                gb[k] = q.ok && z + k + WG_AHEAD < nz ? __ldg(gp) : 0.f;
+                hp += s2 * 16;
+                gp += o2;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    acc[0][i] = fma2(g0, v[i], acc[0][i]);
+                    acc[1][i] = fma2(g1, v[i], acc[1][i]);
+                    acc[2][i] = fma2(g2, v[i], acc[2][i]);
+                }
+                g2 = g1;
+                g1 = g0;
             }
-            g2 = g1;
-            g1 = g0;
         }
     }
     wg_add(acc, gW3 + w * 16, 16);
@@ -787,29 +801,42 @@ __global__ void __launch_bounds__(WG_THREADS, WG_CTAS)
         const WgItem q = wg_item(item, runs, run, columns, So);
         const float *xp = x + (2 * q.b + i) * s3 + q.x + dx + (int64_t)S * (q.y + dy) + s2 * q.z0;
         const uint16_t *gp = gh1 + (q.b * (o2 * So) + q.x + (int64_t)So * q.y + o2 * q.z0) * 16;
-        // x at planes z .. z + 2 (0 for lanes without a column), the next one in flight
-        float v0 = q.ok ? __ldg(xp) : 0.f, v1 = q.ok ? __ldg(xp + s2) : 0.f, vn = q.ok ? __ldg(xp + 2 * s2) : 0.f;
+        const int nz = q.z1 - q.z0;
+        // x at planes z, z + 1 (0 for lanes without a column), and the next planes of gh1 and x
+        float v0 = q.ok ? __ldg(xp) : 0.f, v1 = q.ok ? __ldg(xp + s2) : 0.f;
+        Raw16 gb[WG_AHEAD];
+        float vb[WG_AHEAD];
         xp += 2 * s2;
-        Raw16 next = load_raw(gp);
-        for (int z = q.z0; z < q.z1; ++z) {
-            const Raw16 cur = next;
-            const float v2 = vn;
-            if (z + 1 < q.z1) {
+#pragma unroll
+        for (int k = 0; k < WG_AHEAD; ++k) {
+            if (k >= nz) break;
+            gb[k] = load_raw(gp + k * o2 * 16);
+            vb[k] = q.ok ? __ldg(xp + k * s2) : 0.f;
+        }
+        gp += WG_AHEAD * o2 * 16;
+        xp += WG_AHEAD * s2;
+        for (int z = 0; z < nz; z += WG_AHEAD) {
+#pragma unroll
+            for (int k = 0; k < WG_AHEAD; ++k) {
+                if (z + k >= nz) break;
+                float2 g[8];
+                unpack_raw(gb[k], g);
+                const float v2 = vb[k];
+                if (z + k + WG_AHEAD < nz) {
+                    gb[k] = load_raw(gp);
+                    vb[k] = q.ok ? __ldg(xp) : 0.f;
+                }
                 gp += o2 * 16;
                 xp += s2;
-                next = load_raw(gp);
-                vn = q.ok ? __ldg(xp) : 0.f;
-            }
-            float2 g[8];
-            unpack_raw(cur, g);
 #pragma unroll
-            for (int o = 0; o < 8; ++o) {
-                acc[0][o] = fma2(v0, g[o], acc[0][o]);
-                acc[1][o] = fma2(v1, g[o], acc[1][o]);
-                acc[2][o] = fma2(v2, g[o], acc[2][o]);
+                for (int o = 0; o < 8; ++o) {
+                    acc[0][o] = fma2(v0, g[o], acc[0][o]);
+                    acc[1][o] = fma2(v1, g[o], acc[1][o]);
+                    acc[2][o] = fma2(v2, g[o], acc[2][o]);
+                }
+                v0 = v1;
+                v1 = v2;
             }
-            v0 = v1;
-            v1 = v2;
         }
     }
     wg_add(acc, gW1 + w * 32 + 16 * i, 32);
