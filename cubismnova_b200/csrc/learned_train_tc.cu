@@ -24,6 +24,7 @@
 // rows, one accumulator per (dx, dy), added to gW with atomics once per CTA.
 // Every wait in both kernels is bounded (an error word is set and the CTA
 // stops issuing).
+#include "cn_fastdiv.h"
 #include "cn_internal.h"
 #include "cn_tc.cuh"
 #include "cn_tma.cuh"
@@ -272,14 +273,20 @@ struct BrickGeo {
     int MT;                // 128-row M tiles covering the brick's rows
     int SROWS;             // staged rows: 128 MT + the largest tap offset (zero past the region)
     int bricks[3];         // bricks per patch along x, y, z
+    FastDiv dRX, dRXY;     // divisions by RX, RX RY
 };
 
 constexpr int BRICK_NT = 256;
-constexpr int BRICK_MAX_ROWS = 2880;    // 2 planes x 2880 x 16 B = 90 KB: two CTAs per SM
-constexpr int BRICK_MAX_MT = 16;        // 256 TMEM columns
+// A brick's copies, MMAs and epilogue follow one another, so small bricks and
+// four CTAs per SM, which overlap; B200, the batch of 32 patches of 32^3: two
+// CTAs (2880 rows, 16 tiles) 955 us, three 921, four 924; 5 patches of 13^3 184,
+// 172, 169.
+constexpr int BRICK_CTAS = 4;
+constexpr int BRICK_MAX_ROWS = 1352;    // 2 planes x 1352 x 16 B and the weights: a quarter of the SM's shared memory
+constexpr int BRICK_MAX_MT = 8;         // 128 TMEM columns
 
 template <int MODE>
-__global__ void __launch_bounds__(BRICK_NT, 2) brick_tc_kernel(const __grid_constant__ Args a,
+__global__ void __launch_bounds__(BRICK_NT, BRICK_CTAS) brick_tc_kernel(const __grid_constant__ Args a,
                                                                 const __grid_constant__ BrickGeo g)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -290,7 +297,7 @@ __global__ void __launch_bounds__(BRICK_NT, 2) brick_tc_kernel(const __grid_cons
     uint32_t *slot = reinterpret_cast<uint32_t *>(bar + 1);
     int *okf = reinterpret_cast<int *>(slot + 1);
     const int r = threadIdx.x, warp = r >> 5;
-    constexpr uint32_t TCOLS = 256;
+    constexpr uint32_t TCOLS = 16 * BRICK_MAX_MT;
 
     const int per = g.bricks[0] * g.bricks[1] * g.bricks[2];
     const int b = blockIdx.x / per;
@@ -310,22 +317,23 @@ __global__ void __launch_bounds__(BRICK_NT, 2) brick_tc_kernel(const __grid_cons
     }
     for (int i = r; i < (int)(WBYTES / 16); i += BRICK_NT)
         reinterpret_cast<uint4 *>(Wb)[i] = __ldg(reinterpret_cast<const uint4 *>(a.w) + i);
-    // ---- source region: lanes 2i, 2i+1 copy the two channel halves of a row
-    const int64_t si3 = (int64_t)a.Sin * a.Sin * a.Sin;
-    const int rrows = g.RX * g.RY * g.RZ;
-    for (int t = r; t < 2 * g.SROWS; t += BRICK_NT) {
-        const int u = t >> 1, hh = t & 1;
+    // ---- source region: lanes 2i, 2i+1 copy the two channel halves of a row,
+    // one column along z after the other
+    const int rxy = g.RX * g.RY;
+    const int64_t si2 = (int64_t)a.Sin * a.Sin;
+    for (int t = r; t < 2 * rxy; t += BRICK_NT) {
+        const int u = t >> 1, hh = t & 1, j = g.dRX.div(u), i = u - j * g.RX;
+        const int sx = ox + i + a.shift, sy = oy + j + a.shift, sz0 = oz + a.shift;
+        const bool xy = (unsigned)sx < (unsigned)a.Sin && (unsigned)sy < (unsigned)a.Sin;
+        const uint16_t *col = a.src + (((int64_t)b * a.Sin + sz0) * si2 + (int64_t)a.Sin * sy + sx) * 16 + 8 * hh;
         unsigned char *dst = A + hh * plane + u * 16;
-        bool in = false;
-        int64_t e = 0;
-        if (u < rrows) {
-            const int i = u % g.RX, j = (u / g.RX) % g.RY, k = u / (g.RX * g.RY);
-            const int sx = ox + i + a.shift, sy = oy + j + a.shift, sz = oz + k + a.shift;
-            in = (unsigned)sx < (unsigned)a.Sin && (unsigned)sy < (unsigned)a.Sin && (unsigned)sz < (unsigned)a.Sin;
-            if (in) e = (int64_t)b * si3 + sx + (int64_t)a.Sin * (sy + (int64_t)a.Sin * sz);
+        for (int k = 0; k < g.RZ; ++k) {
+            const bool in = xy && (unsigned)(sz0 + k) < (unsigned)a.Sin;
+            cp16(dst + k * rxy * 16, in ? col + k * si2 * 16 : a.src, in ? 16u : 0u);
         }
-        cp16(dst, in ? a.src + e * 16 + 8 * hh : a.src, in ? 16u : 0u);
     }
+    for (int t = r; t < 2 * (g.SROWS - rxy * g.RZ); t += BRICK_NT) // the rows past it
+        *reinterpret_cast<uint4 *>(A + (t & 1) * plane + (rxy * g.RZ + (t >> 1)) * 16) = make_uint4(0, 0, 0, 0);
     asm volatile("cp.async.wait_all;" ::: "memory");
     fence_proxy_async_smem();
     tc::fence_before_sync();
@@ -361,8 +369,8 @@ __global__ void __launch_bounds__(BRICK_NT, 2) brick_tc_kernel(const __grid_cons
             float v[16];
             tc::tmem_ld16(tbase + lanes + 16u * t, v);
             const int m = 128 * t + 32 * (warp & 3) + (r & 31);
-            const int z = m / (g.RX * g.RY), rem = m - z * (g.RX * g.RY);
-            const int y = rem / g.RX, x = rem - y * g.RX;
+            const int z = g.dRXY.div(m), rem = m - z * rxy;
+            const int y = g.dRX.div(rem), x = rem - y * g.RX;
             const int X = ox + x, Y = oy + y, Z = oz + z;
             if (x >= g.BX || y >= g.BY || z >= g.BZ || X >= a.Sout || Y >= a.Sout || Z >= a.Sout) continue;
             const int64_t L = (int64_t)b * so3 + X + (int64_t)a.Sout * (Y + (int64_t)a.Sout * Z);
@@ -434,6 +442,8 @@ static bool brick_geo(int So, BrickGeo &g)
     g.bricks[0] = (int)bx;
     g.bricks[1] = (So + g.BY - 1) / g.BY;
     g.bricks[2] = (So + g.BZ - 1) / g.BZ;
+    g.dRX = FastDiv((uint32_t)g.RX);
+    g.dRXY = FastDiv((uint32_t)(g.RX * g.RY));
     return true;
 }
 
