@@ -21,7 +21,8 @@
 //   weight grad    gW[t][ci][co] = sum_q h1[q + d][ci] gout[q][co]
 // runs on bricks too, with the cells as K (wgrad_tc_kernel): both operands
 // MN-major, A = (dz, channel) of the source region against the brick's gout
-// rows, one accumulator per (dx, dy), added to gW with atomics once per CTA.
+// rows shifted by dx, one accumulator per dy, added to gW with atomics once per
+// CTA.
 // Every wait in both kernels is bounded (an error word is set and the CTA
 // stops issuing).
 #include "cn_fastdiv.h"
@@ -39,8 +40,8 @@ namespace nntr {
 
 constexpr uint32_t WBYTES = 27 * 512;            // packed weights of one layer
 constexpr uint32_t IDESC_K = tc::idesc_bf16_f32(128, 16);
-// M = 64, both operands MN-major (bits 15 and 16)
-constexpr uint32_t IDESC_MN = tc::idesc_bf16_f32(64, 16) | (1u << 15) | (1u << 16);
+// M = 64, N = 48, both operands MN-major (bits 15 and 16)
+constexpr uint32_t IDESC_MN = tc::idesc_bf16_f32(64, 48) | (1u << 15) | (1u << 16);
 
 enum { FWD = 0, BWD = 1 };
 
@@ -73,15 +74,17 @@ __device__ __forceinline__ void cp16(void *dst, const void *src, uint32_t src_by
 // that are no cell of the brick.  MN-major, a plane of rows is 8 rows of A^T,
 // and the planes (z, half) are evenly spaced: 8 of them from plane z on are the
 // M = 64 of the three dz taps (the last 16 rows, a plane too far, are dropped),
-// and the taps (dx, dy) are start addresses dx + RX dy rows on.  9 MMAs per
-// 16 cells (K) into 9 accumulators of 16 columns, kept over all bricks of the
-// CTA.  Against a gather of every tap's rows (27 copies of 32 bytes a cell) a
-// cell is staged about 1.5 times; B200, 32 patches of 32^3: 384 -> 155 us, of
-// which the MMAs alone 122 (37 cycles each, M = 64 N = 16) and the staging alone
-// 66: two CTAs per SM, one staging while the other's MMAs run.
+// and dy is a start address RX dy rows on.  gout is staged three times, shifted
+// by dx rows: its planes (dx, half) are the N = 48.  3 MMAs per 16 cells (K) into
+// 3 accumulators of 48 columns, kept over all bricks of the CTA.  Against a
+// gather of every tap's rows (27 copies of 32 bytes a cell) a cell is staged 1.5
+// and its gradient 3 times; B200, 32 patches of 32^3: 384 -> 116 us (with dx as
+// start addresses too, 9 MMAs of N = 16 at 37 cycles each: 155, of which the MMAs
+// alone 122 and the staging alone 66).  Two CTAs per SM, one staging while the
+// other's MMAs run.
 constexpr int WGT_NT = 256;
 constexpr int WGT_SMEM = 110 * 1024; // two CTAs per SM
-constexpr uint32_t WGT_COLS = 256;   // 9 x 16, a power of two
+constexpr uint32_t WGT_COLS = 256;   // 3 x 48, a power of two
 
 struct WgGeo {
     int BX, BY, BZ;  // brick of output cells
@@ -100,7 +103,7 @@ __global__ void __launch_bounds__(WGT_NT, 2) wgrad_tc_kernel(const __grid_consta
     __shared__ int flag;
     const uint32_t aplane = (uint32_t)g.H * 16u, gplane = (uint32_t)g.KP * 16u;
     unsigned char *A = smem;                              // [BZ + 3][2][H][16 B], the last z plane never written
-    unsigned char *G = smem + 2 * (g.BZ + 3) * aplane;    // [BZ][2][KP][16 B]
+    unsigned char *G = smem + 2 * (g.BZ + 3) * aplane;    // [BZ][3 shifts][2][KP][16 B]
     const int r = threadIdx.x, warp = r >> 5;
     if (r == 0) {
         mbar_init(&bar, 1);
@@ -150,14 +153,14 @@ __global__ void __launch_bounds__(WGT_NT, 2) wgrad_tc_kernel(const __grid_consta
         }
         for (int t = r; t < 32 * ks; t += WGT_NT) {
             const int u = t >> 1, hh = t & 1, y = u / g.RX, x = u - y * g.RX;
-            const bool in = x < nx && y < ny;
-            const uint16_t *src = in ? a.gout + (((int64_t)b * So + oz) * so2 + (int64_t)(oy + y) * So + ox + x) * 16 + 8 * hh
-                                     : a.gout;
+            const int64_t e = (((int64_t)b * So + oz) * so2 + (int64_t)(oy + y) * So + ox + x) * 16 + 8 * hh;
             unsigned char *dst = G + hh * gplane + u * 16;
-            for (int z = 0; z < nz; ++z) {
-                cp16(dst + 2 * z * gplane, src, in ? 16u : 0u);
-                if (in) src += so2 * 16;
-            }
+            for (int z = 0; z < nz; ++z)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const bool in = (unsigned)(x - c) < (unsigned)nx && y < ny;
+                    cp16(dst + (6 * z + 2 * c) * gplane, in ? a.gout + e + (z * so2 - c) * 16 : a.gout, in ? 16u : 0u);
+                }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         fence_proxy_async_smem(); // generic-proxy smem writes -> visible to the tensor cores
@@ -171,11 +174,11 @@ __global__ void __launch_bounds__(WGT_NT, 2) wgrad_tc_kernel(const __grid_consta
             for (int z = 0; z < nz; ++z) {
 #pragma unroll 1
                 for (int k = 0; k < ks; ++k) {
-                    const uint64_t ak = da + (uint32_t)(2 * z * g.H + 16 * k), bk = db + (uint32_t)(2 * z * g.KP + 16 * k);
+                    const uint64_t ak = da + (uint32_t)(2 * z * g.H + 16 * k), bk = db + (uint32_t)(6 * z * g.KP + 16 * k);
                     const uint32_t acc = it + z + k > 0 ? 1u : 0u;
 #pragma unroll
-                    for (int t = 0; t < 9; ++t)
-                        tc::mma_bf16(tbase + 16u * t, ak + (uint32_t)(t % 3 + g.RX * (t / 3)), bk, IDESC_MN, acc);
+                    for (int dy = 0; dy < 3; ++dy)
+                        tc::mma_bf16(tbase + 48u * dy, ak + (uint32_t)(g.RX * dy), bk, IDESC_MN, acc);
                 }
             }
             tc::mma_commit(&bar);
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(WGT_NT, 2) wgrad_tc_kernel(const __grid_consta
 
 // Brick shape of the weight gradient for B output cubes of side So: of the
 // splits that fit the shared memory of half an SM, the least of (bricks per
-// CTA) x (a brick's MMAs at 16 cycles each, its staging at 40 bytes a cycle and
+// CTA) x (a brick's MMAs at 40 cycles each, its staging at 40 bytes a cycle and
 // 2500 cycles of latency) + 16 cycles of atomics per CTA.
 static WgGeo wgrad_geo(int B, int So, int ctas, size_t *smem)
 {
@@ -225,13 +228,13 @@ static WgGeo wgrad_geo(int B, int So, int ctas, size_t *smem)
             for (g.BY = 1; g.BY <= So; ++g.BY) {
                 g.KP = (g.RX * g.BY + 15) / 16 * 16;
                 g.H = (g.KP + 2 + 2 * g.RX + 7) / 8 * 8;
-                const int64_t bytes = 32LL * ((g.BZ + 3) * g.H + g.BZ * g.KP);
+                const int64_t bytes = 32LL * ((g.BZ + 3) * g.H + 3 * g.BZ * g.KP);
                 if (bytes > WGT_SMEM) break;
                 g.bricks[1] = (So + g.BY - 1) / g.BY;
                 g.bricks[2] = (So + g.BZ - 1) / g.BZ;
                 g.total = B * g.bricks[0] * g.bricks[1] * g.bricks[2];
                             const double cost = (double)((g.total + ctas - 1) / ctas) *
-                                        (9.0 * g.BZ * g.KP + bytes / 40.0 + 2500.0) +
+                                        (7.5 * g.BZ * g.KP + bytes / 40.0 + 2500.0) +
                                     16.0 * (g.total < ctas ? g.total : ctas);
                 if (best.total == 0 || cost < least) {
                     least = cost;
