@@ -46,10 +46,9 @@ def load_labs(u: Cartesian, stencil, out=None, comp: int = 0, block_begin: int =
     st = stencil.as_struct()
     ext = (C.c_int * 3)()
     _lib.check(_lib.lib().cn_lab_extent(u.handle, C.byref(st), ext))
-    n = u.getSize()[0] * u.getSize()[1] * u.getSize()[2]
-    count = n - block_begin if count is None else count
+    count = u.size() - block_begin if count is None else count
     shape = (count, ext[2], ext[1], ext[0])
-    tdt = {4: torch.float32, 8: torch.float64}[u.dtype.itemsize] if u.dtype.kind == "f" else torch.int32
+    tdt = torch.int32 if u.dtype.kind != "f" else torch.float64 if u.dtype.itemsize == 8 else torch.float32
     if out is None:
         out = torch.zeros(shape, dtype=tdt, device="cuda")
     elif tuple(out.shape) != shape or out.dtype != tdt or not out.is_contiguous() or not out.is_cuda:
