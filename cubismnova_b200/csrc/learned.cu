@@ -1005,6 +1005,11 @@ cn_status cn_mg_set_smoother_phases(cn_mg *m, cn_nn *nn, unsigned pre_mask, unsi
                 cn_status s = level_bufs(m, l);
                 if (s != CN_OK) return s;
             }
+        if ((int)m->coef.size() < m->nlevels) { // here, not at the first smoothing, which may be under capture
+            cn_status s = mg_ensure_coef(m, nullptr);
+            if (s != CN_OK) return s;
+            CN_CUDA_TRY(cudaDeviceSynchronize());
+        }
     }
     return CN_OK;
 }

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 namespace cn {
@@ -922,6 +923,45 @@ cn_status mg_ensure_coef(cn_mg *m, cudaStream_t st)
     return CN_OK;
 }
 
+// The two sums of a multigrid lie in pinned host memory that the kernel writes.
+// Allocating it for every multigrid took 1 ms of creating and 0.4 ms of
+// destroying a small one (0.6 ms in all without), so the process keeps 64
+// places in one page; more multigrids at a time than that allocate their own.
+namespace {
+struct SumPlaces {
+    std::mutex mu;
+    double *page = nullptr; // 64 places of 8 doubles
+    uint64_t taken = 0;
+};
+SumPlaces g_sum_places;
+} // namespace
+
+static double *take_sums()
+{
+    {
+        std::lock_guard<std::mutex> lk(g_sum_places.mu);
+        double *&page = g_sum_places.page;
+        if (!page && cudaHostAlloc(&page, 64 * 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) page = nullptr;
+        for (int i = 0; page && i < 64; ++i)
+            if (!(g_sum_places.taken >> i & 1)) {
+                g_sum_places.taken |= uint64_t(1) << i;
+                return page + 8 * i;
+            }
+    }
+    double *own = nullptr;
+    return cudaHostAlloc(&own, sizeof(double) * 2, cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess ? own : nullptr;
+}
+
+static void give_sums(double *sums)
+{
+    std::lock_guard<std::mutex> lk(g_sum_places.mu);
+    double *page = g_sum_places.page;
+    if (page && sums >= page && sums < page + 8 * 64)
+        g_sum_places.taken &= ~(uint64_t(1) << ((sums - page) / 8));
+    else
+        cudaFreeHost(sums);
+}
+
 // Allocates and fills the face means of a level (and its diagonal).
 template <typename T> static cn_status make_faces(cn_mg *m, int l, Faces<T> &F, T ih2, T **diag)
 {
@@ -1137,7 +1177,7 @@ cn_status cn_mg_create(cn_grid *k, int nu1, int nu2, double omega, int max_level
         m->nparts = std::max(k->nblocks * tile_of(k->n).count, (int)ctas_of(layer_of(k, width_of(k, 2), 1, 1)));
         if (cudaMalloc(&m->partials, sizeof(double) * 2 * m->nparts) != cudaSuccess ||
             cudaMalloc(&m->done, sizeof(unsigned)) != cudaSuccess || cudaMemset(m->done, 0, sizeof(unsigned)) != cudaSuccess ||
-            cudaHostAlloc(&m->sums, sizeof(double) * 2, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
+            (m->sums = take_sums()) == nullptr)
             s = fail(CN_ERR_OUT_OF_MEMORY, "cn_mg_create: sums");
     }
     if (s == CN_OK && cudaMalloc(&m->iters, sizeof(int)) != cudaSuccess)
@@ -1190,7 +1230,7 @@ cn_status cn_mg_destroy(cn_mg *m)
         if (a) cudaFree(a);
     if (m->partials) cudaFree(m->partials);
     if (m->done) cudaFree(m->done);
-    if (m->sums) cudaFreeHost(m->sums);
+    if (m->sums) give_sums(m->sums);
     if (m->iters) cudaFree(m->iters);
     delete m;
     return CN_OK;

@@ -206,3 +206,21 @@ def test_march_and_tail_match_tile_kernels(cn, nb, n, nu):
     for x, y in zip(a[:3], b[:3]):
         assert np.array_equal(x, y)
     assert abs(a[4] - b[4]) <= 1e-12 * b[4] and abs(a[5] - b[5]) <= 1e-12 * b[5]
+
+
+def test_more_multigrids_than_sum_places(cn):
+    """Multigrids beyond the shared page of residual sums hold their own, and
+    places come back: solves of the first and the last of 70, interleaved,
+    and of one made after half of them are gone, give the same residuals."""
+    nb, n = (2, 2, 2), (4, 4, 4)
+    k, f = _setup(cn, nb, n)
+
+    def rel(m):
+        p64 = cn.Grid.Cartesian(nb, n, end=_end(nb, n), dtype=np.float64)
+        return m.solve(f, p64, rtol=1e-30, max_cycles=2)[1]
+
+    ms = [cn.mg.Multigrid(k) for _ in range(70)]
+    want = rel(ms[0])
+    assert [rel(m) for m in (ms[69], ms[1], ms[65], ms[0])] == [want] * 4
+    del ms[10:45]
+    assert rel(cn.mg.Multigrid(k)) == want and rel(ms[-1]) == want
