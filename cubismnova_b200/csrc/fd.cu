@@ -337,9 +337,13 @@ static cn_status check_out(const cn_grid *in, const cn_grid *out, int out_comp, 
 }
 
 // Threads that fill the GPU (148 SMs, four CTAs): blocks with fewer columns in
-// all are cut into shorter runs of planes (twice as many threads measured the
-// same within 2 %).
+// all are cut into shorter runs of planes; up to twice as many threads, eight
+// CTAs, where the runs keep four planes.  B200, lap_grad of 128^3 FP64 from
+// memory 22.6 -> 20.5 us with the latter, of 256^3 129 -> 120, divergence of
+// 256^3 FP32 51.5 -> 47.5; runs of two planes lose (Laplacian of 128^3 FP32 6.4
+// -> 8.2).
 constexpr int64_t kFillThreads = 148 * 1024;
+constexpr int kLongRun = 4;
 
 template <typename T, int OP, int V> static cn_status launch_march(const cn_grid *u, FdParams<T> &p, cudaStream_t st)
 {
@@ -348,9 +352,12 @@ template <typename T, int OP, int V> static cn_status launch_march(const cn_grid
     constexpr int U = OP == kDiv && sizeof(T) == 8 ? 1 : 2;
     const int N2 = u->n[2], cols = u->n[0] / V * u->n[1]; // columns of a block
     const int64_t all = (int64_t)u->nblocks * cols;
-    int nzc = (int)std::min<int64_t>((N2 + U - 1) / U, std::max<int64_t>(1, (kFillThreads + all - 1) / all));
-    p.TZ = ((N2 + nzc - 1) / nzc + U - 1) / U * U;
-    nzc = (N2 + p.TZ - 1) / p.TZ;
+    auto run = [&](int64_t threads) { // planes of a run that make `threads` threads
+        const int nzc = (int)std::min<int64_t>((N2 + U - 1) / U, std::max<int64_t>(1, (threads + all - 1) / all));
+        return ((N2 + nzc - 1) / nzc + U - 1) / U * U;
+    };
+    p.TZ = std::min(run(kFillThreads), std::max(kLongRun, run(2 * kFillThreads)));
+    const int nzc = (N2 + p.TZ - 1) / p.TZ;
     const int per_block = cols * nzc;
     p.per_block = FastDiv((uint32_t)per_block);
     p.plane = FastDiv((uint32_t)cols);
