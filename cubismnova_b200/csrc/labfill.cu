@@ -30,6 +30,8 @@ constexpr int KLM = 8;             // cells per thread in flight in the one-pass
 constexpr int KLR = 3;             // rows in flight per thread of the row form
 constexpr int KLX = 3;             // x ghosts in flight per thread of the row form
 constexpr int kBulkBytes = 24576;  // largest bulk copy of a slab's block planes
+constexpr int kGhostBytes = 24576; // largest x ghosts beside them (whole runs)
+constexpr int kRunCtas = 4096;     // least CTAs of a launch with whole runs
 // target cells of a CTA's slab: three planes of the 38^2 lab of 32^3 blocks
 // with three ghosts.  Thinner slabs leave more of the SM's on-chip memory
 // to the L1 cache (the shared-memory carve-out follows the resident CTAs'
@@ -135,6 +137,7 @@ constexpr int kRows = 96; // rows resolved per round
 // Divisors of the row form (fixed per launch).
 struct LabDivs {
     FastDiv n0, n1; // block extents along x, y
+    FastDiv e0;     // lab extent along x
     FastDiv gx, gy; // ghosts per row along x: lo0 + hi0, along y: lo1 + hi1
     FastDiv wpl;    // rows per z-ghost plane, and rows with x ghosts per plane: n1, or E1 if tensorial
 };
@@ -235,7 +238,7 @@ __device__ __forceinline__ void lab_store1(const T *__restrict__ comp, const Lab
 // one-pass form.  It is a kernel of its own so that the general form's
 // per-class loops do not set its register count (it holds none of their
 // spill slots and runs at kRowsCtas CTAs per SM).
-template <typename T>
+template <typename T, bool RUNS>
 __global__ void __launch_bounds__(256, kRowsCtas)
     lab_fill_rows_kernel(const T *__restrict__ comp, LabGeom L, BcView bc, int block_begin, int pz, LabDivs dv,
                          int apply_bc, int bulk, int *err, T *__restrict__ out)
@@ -282,6 +285,12 @@ __global__ void __launch_bounds__(256, kRowsCtas)
         mbar_arrive_expect_tx(&bulk_bar, bytes0);
         bulk_g2s(lab_bulk, comp + bbase, bytes0, &bulk_bar);
     }
+    // With both x faces clear, the own rows of a plane and their x ghosts are
+    // one contiguous run of the lab, all of it plain copies.  RUNS: the ghosts
+    // wait in shared memory behind the planes and the run is stored in order,
+    // so that no sector is written in two parts.
+    const bool runs = RUNS && use_bulk && !(faces & 3);
+    T *xg = reinterpret_cast<T *>(lab_bulk + bulk);
     for (int j = threadIdx.x; j < nrows; j += blockDim.x)
         rows[j] = lab_row<T>(L, bc, mode, faces, block, bx, by, bz, abc, dv, j, ny, gy, false, zi0, nlo, zhi, z0, E0,
                              E1);
@@ -308,7 +317,7 @@ __global__ void __launch_bounds__(256, kRowsCtas)
                     deferred = true;
                 } else {
                     const int nbx = bx + r0 < 0 ? bx + r0 + L.nb[0] : (bx + r0 >= L.nb[0] ? bx + r0 - L.nb[0] : bx + r0);
-                    dst[k] = x + E0 * (y + E1 * z);
+                    dst[k] = runs ? -2 - (t - A) : x + E0 * (y + E1 * z);
                     idx[k] = (int64_t)(nbx + L.nb[0] * (by + L.nb[1] * bz)) * L.bstride + (q0 - r0 * n0) +
                              n0 * ((y - L.lo[1]) + n1 * (z - L.lo[2]));
                 }
@@ -326,12 +335,14 @@ __global__ void __launch_bounds__(256, kRowsCtas)
         T v[KLM];
 #pragma unroll
         for (int k = 0; k < KLM; ++k)
-            if (dst[k] >= 0) v[k] = comp[idx[k]];
+            if (RUNS ? dst[k] != -1 : dst[k] >= 0) v[k] = comp[idx[k]];
 #pragma unroll
         for (int k = 0; k < KLM; ++k)
             if (dst[k] >= 0) o[dst[k]] = v[k];
+            else if (RUNS && dst[k] != -1) xg[-2 - dst[k]] = v[k];
     }
     if (use_bulk) {
+        if (RUNS && runs) __syncthreads(); // the x ghosts
         // the block's cells from shared memory
         if (!mbar_wait_bounded_sleep(&bulk_bar, 0, 200)) {
             // record the error; a second bounded wait keeps the copy from
@@ -340,13 +351,25 @@ __global__ void __launch_bounds__(256, kRowsCtas)
             mbar_wait_bounded_sleep(&bulk_bar, 0, 200);
         } else {
             const T *sb = reinterpret_cast<const T *>(lab_bulk);
-            for (int t0 = threadIdx.x; t0 < A; t0 += KLM * blockDim.x) {
+            if (RUNS && runs) {
+                T *ob = o + E0 * (L.lo[1] + E1 * zi0);
+                const int run = n1 * E0, skip = E0 * (E1 - n1);
+#pragma unroll 4
+                for (int t = threadIdx.x; t < nin * run; t += blockDim.x) {
+                    const int r = dv.e0.div(t), zp = dv.n1.div(r), x = t - r * E0 - L.lo[0];
+                    const T *s = (unsigned)x < (unsigned)n0 ? sb + r * n0 + x
+                                                            : xg + r * gx + L.lo[0] + (x < 0 ? x : x - n0);
+                    ob[t + zp * skip] = *s;
+                }
+            } else {
+                for (int t0 = threadIdx.x; t0 < A; t0 += KLM * blockDim.x) {
 #pragma unroll
-                for (int k = 0; k < KLM; ++k) {
-                    const int t = t0 + k * blockDim.x;
-                    if (t < A) {
-                        const int r = dv.n0.div(t), zp = dv.n1.div(r);
-                        o[(t - r * n0 + L.lo[0]) + E0 * ((r - zp * n1 + L.lo[1]) + E1 * (zi0 + zp))] = sb[t];
+                    for (int k = 0; k < KLM; ++k) {
+                        const int t = t0 + k * blockDim.x;
+                        if (t < A) {
+                            const int r = dv.n0.div(t), zp = dv.n1.div(r);
+                            o[(t - r * n0 + L.lo[0]) + E0 * ((r - zp * n1 + L.lo[1]) + E1 * (zi0 + zp))] = sb[t];
+                        }
                     }
                 }
             }
@@ -587,6 +610,7 @@ static cn_status launch_fill(cn_grid *g, int comp, const cn_stencil *s, int b0, 
     LabDivs dv;
     dv.n0 = FastDiv((uint32_t)L.n[0]);
     dv.n1 = FastDiv((uint32_t)L.n[1]);
+    dv.e0 = FastDiv((uint32_t)E0);
     dv.gx = FastDiv((uint32_t)(L.lo[0] + L.hi[0]));
     dv.gy = FastDiv((uint32_t)(L.lo[1] + L.hi[1]));
     dv.wpl = FastDiv((uint32_t)(L.tensorial ? E1 : L.n[1]));
@@ -595,9 +619,23 @@ static cn_status launch_fill(cn_grid *g, int comp, const cn_stencil *s, int b0, 
     // dynamic shared memory for the bulk copy of a slab's block planes
     const int64_t bulk = (int64_t)pz * L.n[0] * L.n[1] * (int64_t)sizeof(T);
     const int nbulk = !grow && bulk <= kBulkBytes ? (int)bulk : 0;
+    const int64_t ghosts = (int64_t)pz * L.n[1] * (L.lo[0] + L.hi[0]) * (int64_t)sizeof(T);
+    // Whole runs pay where an x ghost is a good part of a row and its sectors
+    // (FP64, a sixth of the row and more) and many CTAs of some size hide the
+    // barrier between the ghosts' loads and their stores.  B200, FP64, ghosts
+    // as they come -> in runs: 4096 blocks of 32^3 with walls, three ghosts a
+    // side 597 -> 577 us, 512 of them 79 -> 77; 4096 of 16^3, two 105 -> 95,
+    // three 132 -> 130; 1728 of 24^3, three 137.6 -> 135.9; but 1728 of 32^3,
+    // two 220 -> 223; 4096 of 16^3, one 84.7 -> 88.1; 4096 of 8^3, one 19.2 ->
+    // 21.1; 512 of 16^3, three (1536 CTAs) 19.1 -> 21.1; FP32 32^3, three 204
+    // -> 230.
+    const bool bulk_planes = nbulk && (int64_t)L.n[0] * L.n[1] * (int64_t)sizeof(T) % 16 == 0;
+    const bool runs = one_pass && bulk_planes && sizeof(T) == 8 && L.n[0] >= 16 && 6 * (L.lo[0] + L.hi[0]) >= L.n[0] &&
+                      ghosts <= kGhostBytes && slabs * std::min(cnt, 65535) >= kRunCtas;
     if (!grow) {
-        static DeviceOnce once[3];
-        cn_status r = one_pass       ? smem_opt_in(once[0], lab_fill_rows_kernel<T>, (size_t)kBulkBytes)
+        static DeviceOnce once[4];
+        cn_status r = runs           ? smem_opt_in(once[3], lab_fill_rows_kernel<T, true>, (size_t)kBulkBytes + kGhostBytes)
+                      : one_pass    ? smem_opt_in(once[0], lab_fill_rows_kernel<T, false>, (size_t)kBulkBytes)
                       : L.tensorial ? smem_opt_in(once[1], lab_fill_kernel<T, true>, (size_t)kBulkBytes)
                                     : smem_opt_in(once[2], lab_fill_kernel<T, false>, (size_t)kBulkBytes);
         if (r != CN_OK) return r;
@@ -612,8 +650,9 @@ static cn_status launch_fill(cn_grid *g, int comp, const cn_stencil *s, int b0, 
                                                               FastDiv((uint32_t)E0), FastDiv((uint32_t)plane),
                                                               apply_bc, out);
         } else if (one_pass) {
-            lab_fill_rows_kernel<T><<<grid, threads, nbulk, st>>>(src, L, bc_view(g, comp), b0 + c0, pz, dv,
-                                                                  apply_bc, nbulk, g->d_err, out);
+            auto kernel = runs ? lab_fill_rows_kernel<T, true> : lab_fill_rows_kernel<T, false>;
+            kernel<<<grid, threads, nbulk + (runs ? (int)ghosts : 0), st>>>(src, L, bc_view(g, comp), b0 + c0, pz, dv,
+                                                                            apply_bc, nbulk, g->d_err, out);
         } else {
             auto kernel = L.tensorial ? lab_fill_kernel<T, true> : lab_fill_kernel<T, false>;
             kernel<<<grid, threads, nbulk, st>>>(src, L, bc_view(g, comp), b0 + c0, pz, dv, wl, apply_bc, nbulk,

@@ -217,3 +217,26 @@ def test_tensorial_row_widths_vs_oracle(cn, oracle_lib, n0, dt):
         want, wdef = O.lab_fill(comp, nb, n, lo, hi, True, bcl, b)
         LC.compare_defined(labs[b], written[b], want, wdef)
     g.close()
+
+
+@pytest.mark.parametrize("nb,n", [((16, 16, 16), (3, 4, 4)), ((16, 16, 16), (17, 4, 4)), ((16, 16, 16), (18, 4, 4)),
+                                  ((16, 16, 16), (19, 4, 4)), ((16, 8, 8), (16, 24, 24)), ((16, 16, 15), (18, 3, 5))])
+def test_lab_fill_whole_runs_vs_oracle(cn, oracle_lib, nb, n):
+    """Launches of at least 4096 CTAs, whose own rows are stored together with
+    their x ghosts where these are a sixth of a row (n0 16 to 18 here): both
+    sides of the rule, one and several slabs a block,
+    blocks with BCs on their x faces among the others; bit-exact against the
+    oracle."""
+    O = oracle_lib
+    rng = np.random.default_rng(43)
+    lo, hi = (2, 1, 1), (1, 1, 1)
+    nblocks = int(np.prod(nb))
+    comp = rng.standard_normal(nblocks * O.block_stride(n, np.float64)) * 10
+    bcl = {int(b): [(int(rng.integers(0, 3)), int(rng.integers(0, 2)), int(rng.integers(0, 4)),
+                     float(rng.choice([-1, 0.5, 2]))) for _ in range(2)] for b in rng.integers(0, nblocks, size=40)}
+    g = make_grid(cn, comp, nb, n, bcl)
+    labs, written = lab_fill_all(cn, g, lo, hi, False)
+    for b in sorted(set(bcl) | {0, nblocks - 1} | set(rng.integers(0, nblocks, size=40).tolist())):
+        want, wdef = O.lab_fill(comp, nb, n, lo, hi, False, bcl, b)
+        LC.compare_defined(labs[b], written[b], want, wdef)
+    g.close()
