@@ -456,8 +456,8 @@ static bool brick_geo(int So, BrickGeo &g)
 // Every kernel tiles its cells so that an operand unpacked from BF16, or a
 // tap's weights read from shared memory, serves several cells or taps; B200,
 // batch of 32 patches of 32^3 cells, against one cell and tap at a time:
-// l1_fwd_cl 170 -> 90 us, l3_fwd_cl 118 -> 62, l3_bwd_data_cl 113 -> 64,
-// l3_wgrad_cl 194 -> 60, l1_wgrad_cl 294 -> 152.
+// l1_fwd_cl 163 -> 83 us, l3_fwd_cl 114 -> 70, l3_bwd_data_cl 107 -> 45,
+// l3_wgrad_cl 161 -> 57, l1_wgrad_cl 280 -> 146.
 __device__ __forceinline__ float2 fma2(float a, float2 b, float2 c) { return __ffma2_rn(make_float2(a, a), b, c); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
@@ -577,50 +577,108 @@ __device__ __forceinline__ ZRun z_run(uint32_t t, uint32_t So)
 }
 __host__ __device__ inline uint32_t z_runs(int B, int So) { return (uint32_t)B * So * So * ((So + ZT - 1) / ZT); }
 
-// layer 3 forward: h2 [B][S^3][16] BF16 -> y [B][(S-2)^3] FP32.  ZT cells along
-// z per thread: per (dx, dy) the column's ZT + 2 inputs are unpacked once and a
-// tap's weights serve all cells.
-__global__ void __launch_bounds__(128) l3_fwd_cl(const uint16_t *__restrict__ h2, const float *__restrict__ W3,
-                                                  float *__restrict__ y, int B, int S)
+// The sums of the last layer's forward and of its data gradient come before
+// a BF16 rounding (of gh2, and of what follows from it), where another order of
+// summation moves a value by a whole BF16 step and the gradients by more than
+// FP32 rounding.  Both keep the order of one cell at a time: taps dx, dy, dz,
+// then channels, one chain of fused multiply-adds per result.
+
+// layer 3 forward: h2 [B][S^3][16] BF16 -> y [B][(S-2)^3] FP32.  A CTA takes qx
+// x yb threads' cells of one output plane, 4 cells of a row each, from a copy
+// of the rows around them in shared memory: a cell is unpacked once per (dy,
+// dz) for its three taps, a tap's weights serve 4 cells.  (Straight from global
+// memory the threads' 128-byte steps along x cost a cache line per lane and
+// load.)  16-byte chunks of a row lie 9 apart every 8, so that 8 lanes read from
+// distinct banks.
+constexpr int L3_NT = 128, L3_QX = 16; // threads; most quads of cells along x
+struct L3Geo {
+    int qx, yb;        // quads along x and rows of a CTA
+    int bx, by;        // CTAs along x and y of a plane
+    int pitch;         // 16-byte units of a staged row
+    FastDiv dqx, drow; // qx, chunks of a full row
+};
+static L3Geo l3_geo(int So, size_t *smem)
 {
+    L3Geo g;
+    const int quads = (So + 3) / 4;
+    g.bx = (quads + L3_QX - 1) / L3_QX;
+    g.qx = (quads + g.bx - 1) / g.bx;
+    g.yb = std::min(So, L3_NT / g.qx);
+    g.by = (So + g.yb - 1) / g.yb;
+    g.yb = (So + g.by - 1) / g.by;
+    g.pitch = 9 * g.qx + 8; // 9 qx + 4 used; the rest keeps the lanes' steps across rows
+    g.dqx = FastDiv((uint32_t)g.qx);
+    g.drow = FastDiv((uint32_t)(8 * g.qx + 4));
+    *smem = (size_t)3 * (g.yb + 2) * g.pitch * 16;
+    return g;
+}
+constexpr size_t L3_SMEM = (size_t)3 * (L3_NT / L3_QX + 2) * (9 * L3_QX + 8) * 16; // the largest: qx = L3_QX
+
+__global__ void __launch_bounds__(L3_NT, 3) l3_fwd_cl(const uint16_t *__restrict__ h2, const float *__restrict__ W3,
+                                                      float *__restrict__ y, int S, const __grid_constant__ L3Geo g)
+{
+    extern __shared__ __align__(16) uint4 rows[]; // [3 planes][yb + 2][pitch]
     __shared__ __align__(16) float sw[27 * 16];
-    for (int i = threadIdx.x; i < 27 * 16; i += blockDim.x) sw[i] = W3[i];
-    __syncthreads();
+    for (int i = threadIdx.x; i < 27 * 16; i += L3_NT) sw[i] = W3[i];
     const int So = S - 2;
-    const int64_t s2 = (int64_t)S * S, s3 = s2 * S;
-    const uint32_t total = z_runs(B, So);
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        const ZRun q = z_run(t, (uint32_t)So);
-        const uint16_t *src = h2 + (q.b * s3 + q.x + (int64_t)S * q.y + s2 * q.z) * 16;
-        float2 acc[ZT];
+    int u = blockIdx.x;
+    const int x0 = 4 * g.qx * (u % g.bx);
+    u /= g.bx;
+    const int y0 = g.yb * (u % g.by);
+    u /= g.by;
+    const int b = u / So, z = u - b * So;
+    const int nx = min(4 * g.qx + 2, S - x0), ny = min(g.yb, So - y0), sr = g.yb + 2;
+    const uint4 *src = reinterpret_cast<const uint4 *>(h2) +
+                       2 * (((int64_t)b * S + z) * S * S + (int64_t)S * y0 + x0);
+    const int chunks = 8 * g.qx + 4;
 #pragma unroll
-        for (int c = 0; c < ZT; ++c) acc[c] = make_float2(0.f, 0.f);
+    for (int pl = 0; pl < 3; ++pl) {
+        for (int t = threadIdx.x; t < (ny + 2) * chunks; t += L3_NT) {
+            const int j = g.drow.div(t), ch = t - j * chunks;
+            if (ch < 2 * nx) // past the cube's end: read by cells that are no output only
+                cp16(rows + (pl * sr + j) * g.pitch + ch + (ch >> 3), src + 2 * (int64_t)S * (j + (int64_t)S * pl) + ch, 16u);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const int j = g.dqx.div(threadIdx.x), q = threadIdx.x - j * g.qx, xx = x0 + 4 * q;
+    const bool ok = j < ny && xx < So;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int dz = 0; dz < 3; ++dz) {
+        if (dz == 0) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        if (dz == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        if (dz == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (!ok) continue;
 #pragma unroll 1
-        for (int r = 0; r < 9; ++r) {
-            const uint16_t *p = src + (r % 3 + (int64_t)S * (r / 3)) * 16;
-            float2 v[ZT + 2][8];
+        for (int dy = 0; dy < 3; ++dy) {
+            const uint4 *p = rows + (dz * sr + j + dy) * g.pitch + 9 * q;
+            float2 v[6][8];
 #pragma unroll
-            for (int k = 0; k < ZT + 2; ++k)
-                unpack16(p + (q.z + k < S ? k : 0) * s2 * 16, v[k]);
+            for (int k = 0; k < 6; ++k)
+                unpack_raw({p[2 * k + (k >= 4)], p[2 * k + 1 + (k >= 4)]}, v[k]);
 #pragma unroll
-            for (int dz = 0; dz < 3; ++dz) {
+            for (int dx = 0; dx < 3; ++dx) {
                 float2 w[8];
-                weights16(sw + (r + 9 * dz) * 16, w);
+                weights16(sw + (9 * dz + 3 * dy + dx) * 16, w);
 #pragma unroll
-                for (int c = 0; c < ZT; ++c)
+                for (int i = 0; i < 8; ++i)
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[c] = fma2(v[c + dz][i], w[i], acc[c]);
+                    for (int c = 0; c < 4; ++c)
+                        acc[c] = fmaf(v[c + dx][i].y, w[i].y, fmaf(v[c + dx][i].x, w[i].x, acc[c]));
             }
         }
-        float *dst = y + ((int64_t)q.b * So * So * So + q.x + (int64_t)So * (q.y + (int64_t)So * q.z));
-#pragma unroll
-        for (int c = 0; c < ZT; ++c)
-            if (q.z + c < So) dst[(int64_t)c * So * So] = acc[c].x + acc[c].y;
     }
+    if (!ok) return;
+    float *dst = y + (((int64_t)b * So + z) * So + y0 + j) * So + xx;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (xx + c < So) dst[c] = acc[c];
 }
 
 // layer 3 backward-data: gh2[c][ci] = (h2[c][ci] > 0) sum_e gc[c - 2 + e] W3[26 - e][ci]
-// for c in S^3 (gc on (S-2)^3, zero outside); ZT cells along z per thread
+// for c in S^3 (gc on (S-2)^3, zero outside); ZT cells along z per thread, which
+// share a tap's weights
 __global__ void __launch_bounds__(128) l3_bwd_data_cl(const float *__restrict__ gc, const float *__restrict__ W3,
                                                        const uint16_t *__restrict__ h2, uint16_t *__restrict__ gh2,
                                                        int B, int S)
@@ -638,25 +696,32 @@ __global__ void __launch_bounds__(128) l3_bwd_data_cl(const float *__restrict__ 
         for (int c = 0; c < ZT; ++c)
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc[c][i] = make_float2(0.f, 0.f);
+        const int ox = q.x - 2, oy = q.y - 2;
+        const bool okx[3] = {ox >= 0, (unsigned)(ox + 1) < (unsigned)So, ox + 2 < So};
 #pragma unroll 1
-        for (int r = 0; r < 9; ++r) {
-            const int ox = q.x - 2 + r % 3, oy = q.y - 2 + r / 3;
-            if ((unsigned)ox >= (unsigned)So || (unsigned)oy >= (unsigned)So) continue;
-            const float *p = gc + q.b * (o2 * So) + ox + (int64_t)So * oy;
-            float g[ZT + 2]; // gc at z - 2 .. z + ZT - 1
+        for (int ez = 0; ez < 3; ++ez) {
+            const int oz = q.z - 2 + ez;
+            bool okz[ZT];
 #pragma unroll
-            for (int k = 0; k < ZT + 2; ++k) {
-                const int oz = q.z - 2 + k;
-                g[k] = (unsigned)oz < (unsigned)So ? __ldg(p + oz * o2) : 0.f;
-            }
+            for (int c = 0; c < ZT; ++c) okz[c] = (unsigned)(oz + c) < (unsigned)So;
+            const float *pz = gc + q.b * (o2 * So) + ox + (int64_t)So * oy + o2 * oz, *wz = sw + (26 - 9 * ez) * 16;
+#pragma unroll 1
+            for (int ey = 0; ey < 3; ++ey, pz += So, wz -= 3 * 16) {
+                if ((unsigned)(oy + ey) >= (unsigned)So) continue;
+                float g[3][ZT];
 #pragma unroll
-            for (int ez = 0; ez < 3; ++ez) {
-                float2 w[8];
-                weights16(sw + (26 - r - 9 * ez) * 16, w);
+                for (int ex = 0; ex < 3; ++ex)
 #pragma unroll
-                for (int c = 0; c < ZT; ++c)
+                    for (int c = 0; c < ZT; ++c) g[ex][c] = okx[ex] && okz[c] ? __ldg(pz + ex + c * o2) : 0.f;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[c][i] = fma2(g[c + ez], w[i], acc[c][i]);
+                for (int ex = 0; ex < 3; ++ex) {
+                    float2 w[8];
+                    weights16(wz - ex * 16, w);
+#pragma unroll
+                    for (int c = 0; c < ZT; ++c)
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[c][i] = fma2(g[ex][c], w[i], acc[c][i]);
+                }
             }
         }
         const int64_t e = (q.b * (s2 * S) + q.x + (int64_t)S * q.y + s2 * q.z) * 16;
@@ -875,7 +940,7 @@ static unsigned wg_launch(int B, int So, int ctas, int &run)
     return (unsigned)(items < ctas ? items : ctas);
 }
 
-static DeviceOnce wgrad_once, brick_once[2];
+static DeviceOnce wgrad_once, brick_once[2], l3_once;
 
 // weight gradient: persistent CTAs, two per SM
 static cn_status launch_wgrad(Args &a, int B, int sms, cudaStream_t st)
@@ -933,7 +998,10 @@ cn_status train_forward_tc(const TrainBufs &T, const float *x, const float *W, i
     a.relu = 1;
     a.err = T.err;
     if ((s = launch_conv<FWD>(a, B, st)) != CN_OK) return s;
-    l3_fwd_cl<<<grid_of(z_runs(B, S3), 128, 148 * 64), 128, 0, st>>>(T.h2, W3, T.y, B, S2);
+    size_t smem = 0;
+    const L3Geo g = l3_geo(S3, &smem);
+    if ((s = smem_opt_in(l3_once, l3_fwd_cl, L3_SMEM)) != CN_OK) return s;
+    l3_fwd_cl<<<(unsigned)((int64_t)B * S3 * g.by * g.bx), L3_NT, smem, st>>>(T.h2, W3, T.y, S2, g);
     CN_CUDA_TRY(cudaGetLastError());
     return CN_OK;
 }

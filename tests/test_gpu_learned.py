@@ -107,6 +107,95 @@ def test_tensor_core_training_edges(cn, B, P, offset):
         assert _rel(g, w) < TOL_TC_GRAD
 
 
+def _fma32(a, b, c):
+    """float32 fused multiply-add: the product is exact in float64, the sum is
+    rounded to odd there, so that the rounding to float32 is the only one."""
+    p, c = a.astype(np.float64) * b.astype(np.float64), c.astype(np.float64)
+    s = p + c
+    v = s - p
+    err = (p - (s - v)) + (c - v)
+    even = (s.view(np.int64) & 1) == 0
+    s = np.where((err != 0) & even, np.nextafter(s, np.where(err > 0, np.inf, -np.inf)), s)
+    return s.astype(np.float32)
+
+
+def _bf16(v):
+    u = np.ascontiguousarray(v, dtype=np.float32).view(np.uint32).astype(np.uint64)
+    return (((u + 0x7FFF + ((u >> 16) & 1)) >> 16) << 16).astype(np.uint32).view(np.float32)
+
+
+@pytest.mark.parametrize("B,P,seed", [(1, 1, 0), (1, 2, 1), (2, 5, 2), (3, 8, 3), (1, 8, 4), (2, 13, 5), (1, 30, 6),
+                                      (1, 63, 7)])
+def test_last_layer_sums_in_tap_order(cn, B, P, seed):
+    """The last layer's forward and data gradient, bit for bit in the order of
+    one cell at a time: taps x fastest, then y, then z, the channels of a tap in
+    turn, one chain of fused multiply-adds per result.  Both come before BF16
+    roundings, so another order shows in the gradients.
+
+    One cell of h1 is 1 and all others are 0, so h2 is W2 (in BF16) in the 27
+    cells around it, and the gradient of W2 is gh2 there, single exact products.
+    With k = 1, ih2 = 1, omega = 0 and r = +-1 near that cell, the loss kernels'
+    float32 operations have one order and no rounding that a contraction changes;
+    the loss (sums in float64) then shows any last bit of y."""
+    import torch
+    rng = np.random.default_rng(100 + seed)
+    S, S1, R = P + 8, P + 6, P + 2
+    active = B - 1
+    ends = (2, S1 - 3)  # 27 cells of h2 around the h1 cell: [2, S1 - 3]
+    c = np.array([ends[seed % 2], int(rng.integers(2, S1 - 2)), ends[(seed // 2) % 2]])  # x, y, z
+    W1 = np.zeros((27, 2, 16), np.float32)
+    W1[13, 0, 0] = 1.0
+    W2 = np.zeros((27, 16, 16), np.float32)
+    W2[:, 0, :] = _bf16(rng.uniform(0.5, 1.5, (27, 16)).astype(np.float32))
+    W3 = rng.standard_normal((27, 16, 1)).astype(np.float32)
+    nn = cn.learned.LearnedSmoother(seed=1, omega=0.0, init_scale=0.05)
+    nn.set_training("tensor")
+    nn.set_weights(W1, W2, W3)
+    x = np.zeros((B, 2, S, S, S), np.float32)
+    x[active, 0, c[2] + 1, c[1] + 1, c[0] + 1] = 1.0
+    r = np.zeros((B, P, P, P), np.float32)
+    lo, hi = np.maximum(c - 6, 0), np.minimum(c + 2, P)
+    win = tuple(slice(lo[d], hi[d]) for d in (2, 1, 0))
+    r[active][win] = rng.choice(np.array([-1.0, 1.0], np.float32), size=r[active][win].shape)
+    t = lambda a: torch.tensor(a, device="cuda").reshape(B, -1).contiguous()
+    loss, grads = nn.loss_grad(t(x), t(np.ones((B, R, R, R), np.float32)), t(r), P, 1.0)
+
+    # the same in float32, [z][y][x] windows of the whole cubes padded by zeros
+    h2 = np.zeros((P + 4,) * 3 + (16,), np.float32)
+    taps = [(q % 3, (q // 3) % 3, q // 9) for q in range(27)]
+    for q, d in enumerate(taps):
+        h2[c[2] - d[2], c[1] - d[1], c[0] - d[0]] = W2[q, 0]
+    y = np.zeros((R, R, R), np.float32)
+    a, b = np.maximum(c - 4, 0), np.minimum(c + 1, R)
+    acc = np.zeros(tuple((b - a)[::-1]), np.float32)
+    for q, d in enumerate(taps):
+        v = h2[a[2] + d[2]:b[2] + d[2], a[1] + d[1]:b[1] + d[1], a[0] + d[0]:b[0] + d[0]]
+        for i in range(16):
+            acc = _fma32(v[..., i], W3[q, i], acc)
+    y[a[2]:b[2], a[1]:b[1], a[0]:b[0]] = acc
+    m = y[1:-1, 1:-1, 1:-1]
+    f = [(y[1:-1, 1:-1, 2:] - m) - (m - y[1:-1, 1:-1, :-2]), (y[1:-1, 2:, 1:-1] - m) - (m - y[1:-1, :-2, 1:-1]),
+         (y[2:, 1:-1, 1:-1] - m) - (m - y[:-2, 1:-1, 1:-1])]
+    e = r[active] - ((f[0] + f[1]) + f[2])
+    rr = float(np.sum(r[active].astype(np.float64) ** 2))
+    want = float(np.sum(e.astype(np.float64) ** 2)) / rr / B
+    ep = np.pad(e, 2)  # e at (z, y, x) of the cube of side R is ep[z + 1, y + 1, x + 1]
+    g = ep[1:-1, 1:-1, 1:-1] * np.float32(-6.0)
+    for o in ((0, 0, 1), (0, 0, -1), (0, 1, 0), (0, -1, 0), (1, 0, 0), (-1, 0, 0)):
+        g = g + ep[1 + o[0]:R + 1 + o[0], 1 + o[1]:R + 1 + o[1], 1 + o[2]:R + 1 + o[2]]
+    g = np.float32(-2.0 / (rr * B)) * g
+    gp = np.pad(g, 2)  # gc at c - 2 + e of h2's cell c is gp[c + e]
+    for q, d in enumerate(taps):
+        cell = c - np.array(d)
+        acc = np.zeros(16, np.float32)
+        for e_, s in enumerate(taps):
+            v = gp[cell[2] + s[2], cell[1] + s[1], cell[0] + s[0]]
+            acc = _fma32(np.full(16, v, np.float32), W3[26 - e_, :, 0], acc)
+        assert np.array_equal(grads[1][q, 0], _bf16(acc)), (q, grads[1][q, 0], _bf16(acc))
+    # the float64 sums' own rounding: at most 9^3 terms
+    assert abs(loss - want) <= 1e-12 * want, (loss, want)
+
+
 def test_tensor_core_training_step_matches_fp32(cn):
     """One Adam step from the same weights with either training path moves
     the weights the same way (BF16 gradients point where the FP32 ones do)."""
