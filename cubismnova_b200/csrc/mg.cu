@@ -1069,9 +1069,21 @@ static cn_status coarse_inverse(cn_mg *m)
 }
 
 // whether the FP64 residual of p64 takes the marching kernel
-static bool marches64(const cn_mg *m, const cn_grid *p64)
+static bool marches64(const cn_grid *p64) { return !p64->bc_count; }
+
+static bool same_blocks(const cn_grid *a, const cn_grid *b)
 {
-    return !p64->bc_count && p64->n[1] == m->p[0]->n[1] && p64->n[2] == m->p[0]->n[2];
+    return a->nblocks == b->nblocks && a->n[0] == b->n[0] && a->n[1] == b->n[1] && a->n[2] == b->n[2];
+}
+// The fields of the FP64 outer iteration: the kernels index p64 by the extents
+// of the multigrid's blocks, f and r32 (optional) by its storage.
+static cn_status check_outer(const cn_mg *m, const cn_grid *p64, const cn_grid *f, const cn_grid *r32)
+{
+    const cn_grid *g = m->p[0];
+    if (p64->dtype != CN_FLOAT64 || !same_blocks(p64, g) || f->dtype != CN_FLOAT32 || f->comp_stride != g->comp_stride ||
+        (r32 && (r32->dtype != CN_FLOAT32 || r32->comp_stride < g->comp_stride)))
+        return fail(CN_ERR_SIZE_MISMATCH, "Cartesian: Can not assign two grids of unequal size.");
+    return CN_OK;
 }
 
 // The FP64 residual of cn_mg_residual; with p0 (only where marches64), also
@@ -1080,15 +1092,14 @@ static cn_status residual(cn_mg *m, const cn_grid *p64, const cn_grid *f, cn_gri
                           cudaStream_t st)
 {
     if (!m || !p64 || !f) return fail(CN_ERR_INVALID_ARGUMENT, "NULL argument");
-    if (p64->dtype != CN_FLOAT64 || f->dtype != CN_FLOAT32 || p64->nblocks != m->p[0]->nblocks ||
-        p64->n[0] != m->p[0]->n[0] || f->comp_stride != m->p[0]->comp_stride)
-        return fail(CN_ERR_SIZE_MISMATCH, "Cartesian: Can not assign two grids of unequal size.");
-    cn_status s = sync_bc(const_cast<cn_grid *>(p64), st);
+    cn_status s = check_outer(m, p64, f, r32);
+    if (s != CN_OK) return s;
+    s = sync_bc(const_cast<cn_grid *>(p64), st);
     if (s != CN_OK) return s;
     const double *p = reinterpret_cast<const double *>(p64->d_data);
     const float *fin = reinterpret_cast<const float *>(f->d_data);
     float *out = r32 ? fptr(r32) : nullptr;
-    if (!marches64(m, p64)) {
+    if (!marches64(p64)) {
         KArgs a = kargs(m, 0);
         a.G.L.bstride = p64->block_stride;
         a.G.bc = bc_view(p64, 0);
@@ -1279,13 +1290,15 @@ cn_status cn_mg_solve(cn_mg *m, const cn_grid *f, cn_grid *p64, double rtol, int
                       int *cycles, double *relres, void *stream)
 {
     if (!m || !f || !p64) return fail(CN_ERR_INVALID_ARGUMENT, "NULL argument");
+    cn_status s = check_outer(m, p64, f, nullptr);
+    if (s != CN_OK) return s;
     cudaStream_t st = as_stream(stream);
     CN_CUDA_TRY(cudaMemsetAsync(p64->d_data, 0, (size_t)p64->comp_stride * 8, st));
     double rr = 0, ff = 0;
     // the residual also writes the cycle's first sweep where that is Jacobi's
-    const bool fused = first_fused(m, 0) && marches64(m, p64);
+    const bool fused = first_fused(m, 0) && marches64(p64);
     float *p0 = fused ? fptr(m->pt[0]) : nullptr;
-    cn_status s = residual(m, p64, f, m->f[0], p0, &rr, &ff, st);
+    s = residual(m, p64, f, m->f[0], p0, &rr, &ff, st);
     if (s != CN_OK) return s;
     const double fn = std::sqrt(ff);
     double rel = fn > 0 ? std::sqrt(rr) / fn : 0.0;
@@ -1313,8 +1326,7 @@ cn_status cn_mg_accumulate(cn_mg *m, cn_grid *p64, void *stream)
 {
     if (!m || !p64) return fail(CN_ERR_INVALID_ARGUMENT, "NULL argument");
     const cn_grid *g = m->p[0];
-    if (p64->dtype != CN_FLOAT64 || p64->nblocks != g->nblocks || p64->n[0] != g->n[0] || p64->n[1] != g->n[1] ||
-        p64->n[2] != g->n[2])
+    if (p64->dtype != CN_FLOAT64 || !same_blocks(p64, g))
         return fail(CN_ERR_SIZE_MISMATCH, "Cartesian: Can not assign two grids of unequal size.");
     const int64_t cells = (int64_t)g->n[0] * g->n[1] * g->n[2];
     axpy64_kernel<<<grid_for(cells * g->nblocks), 256, 0, as_stream(stream)>>>(

@@ -224,3 +224,27 @@ def test_more_multigrids_than_sum_places(cn):
     assert [rel(m) for m in (ms[69], ms[1], ms[65], ms[0])] == [want] * 4
     del ms[10:45]
     assert rel(cn.mg.Multigrid(k)) == want and rel(ms[-1]) == want
+
+
+@pytest.mark.parametrize("n64", [(16, 8, 8), (16, 16, 32), (16, 8, 32), (8, 16, 16)])
+def test_solution_of_other_extents_is_refused(cn, n64):
+    """The outer iteration takes p64 by the multigrid's block extents: fields
+    of as many blocks whose extents differ along any dimension (along y and z
+    only, with the storage of one component smaller, larger or the same), and
+    residual fields too small for it, are refused before any of them is written."""
+    nb, n = (2, 2, 2), (16, 16, 16)
+    k, f = _setup(cn, nb, n)
+    m = cn.mg.Multigrid(k)
+    p64 = cn.Grid.Cartesian(nb, n64, dtype=np.float64)
+    p64.tensor(0).fill_(7.0)
+    for call in (lambda: m.solve(f, p64), lambda: m.residual(p64, f)):
+        with pytest.raises(cn.CnError, match="unequal size"):
+            call()
+    assert float(p64.tensor(0).min()) == 7.0
+    good = cn.Grid.Cartesian(nb, n, dtype=np.float64)
+    small = cn.Grid.Cartesian(nb, (16, 8, 16), dtype=np.float32)
+    with pytest.raises(cn.CnError, match="unequal size"):
+        m.residual(good, f, small)
+    with pytest.raises(cn.CnError, match="unequal size"):
+        m.solve(f, f)  # an FP32 solution
+    assert m.solve(f, good, rtol=1e-8)[1] <= 1e-8
