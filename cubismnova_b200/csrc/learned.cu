@@ -384,13 +384,14 @@ struct FeatArgs {
     LabGeom L;
     BcView pbc, kbc;
     const float *p, *k, *f;
-    const float *coef; // level coefficients of the multigrid, 8 per cell
+    mg::Faces<float> F; // the level's face means and diagonal
+    const float *D;
     float ih2;
     float *x0, *x1, *rout;
     uint16_t *packed;
 };
 
-__global__ void __launch_bounds__(mg::kTileThreads, mg::kTileMinCtas) features_tile(const __grid_constant__ FeatArgs A,
+__global__ void __launch_bounds__(mg::kTileThreads, 4) features_tile(const __grid_constant__ FeatArgs A,
                                                                   const __grid_constant__ mg::Tile T)
 {
     __shared__ __align__(16) float sp[mg::kRegionMax];
@@ -414,9 +415,15 @@ __global__ void __launch_bounds__(mg::kTileThreads, mg::kTileMinCtas) features_t
         mg::tile_cell(T, c, x, y, z);
         const int64_t lc = (q.x0 + x) + (int64_t)L.n[0] * ((q.y0 + y) + (int64_t)L.n[1] * (q.z0 + z));
         const int64_t o = (int64_t)q.block * L.bstride + lc;
-        float Lp, D, pc;
-        mg::op7_coef<float, float>(sp, mg::ridx(q, x, y, z), st, A.coef + ((int64_t)q.block * bcells + lc) * mg::kCoefPerCell,
-                                   A.ih2, Lp, D, pc);
+        const int64_t t = q.block * bcells + lc;
+        const float D = __ldg(A.D + t);
+        float km[6];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            km[d] = __ldg(A.F.k[d] + t);
+            km[3 + d] = mg::upper_mean<float>(A.F, L, t, q.block, q.x0 + x, q.y0 + y, q.z0 + z, d);
+        }
+        const float Lp = mg::op7_tile<float>(sp, mg::ridx(q, x, y, z), st, km, A.ih2);
         const float fc = __ldg(A.f + o);
         const float r = fc - Lp;
         const float a = (Lp - fc) / D;
@@ -820,8 +827,6 @@ static cn_status features(cn_mg *m, int l, const float *p, const float *f, float
                           uint16_t *packed = nullptr)
 {
     cn_grid *X = m->nn_bufs[4 * l];
-    const cn_status cs = mg_ensure_coef(m, st);
-    if (cs != CN_OK) return cs;
     FeatArgs A;
     A.L = make_geom(m->p[l], &kS1);
     A.pbc = bc_view(m->p[l], 0);
@@ -829,7 +834,8 @@ static cn_status features(cn_mg *m, int l, const float *p, const float *f, float
     A.p = p;
     A.k = fptr(m->k[l]);
     A.f = f;
-    A.coef = m->coef[l];
+    A.F = m->faces[l];
+    A.D = m->diag[l];
     A.ih2 = (float)(1.0 / (m->p[l]->h[0] * m->p[l]->h[0]));
     A.x0 = reinterpret_cast<float *>(X->d_data);
     A.x1 = A.x0 + X->comp_stride;
@@ -1005,11 +1011,6 @@ cn_status cn_mg_set_smoother_phases(cn_mg *m, cn_nn *nn, unsigned pre_mask, unsi
                 cn_status s = level_bufs(m, l);
                 if (s != CN_OK) return s;
             }
-        if ((int)m->coef.size() < m->nlevels) { // here, not at the first smoothing, which may be under capture
-            cn_status s = mg_ensure_coef(m, nullptr);
-            if (s != CN_OK) return s;
-            CN_CUDA_TRY(cudaDeviceSynchronize());
-        }
     }
     return CN_OK;
 }

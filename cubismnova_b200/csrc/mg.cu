@@ -65,9 +65,8 @@ __device__ __forceinline__ T fetch(const T *comp, const LabGeom &L, const BcView
 
 struct KArgs {
     Geo G;
-    BcView kbc;
-    const float *k;
-    const float *coef; // level coefficients, 8 per cell (see op7_coef)
+    Faces<float> F;  // of the level
+    const float *D;
     float ih2;
     double ih2d;
 };
@@ -79,7 +78,7 @@ __device__ __forceinline__ int64_t dense_cell(const LabGeom &L, const TilePos &q
 }
 
 // Face means of one level from the lab of k, and with D the diagonal, with the
-// operations of op7_math in T.
+// operations of op7_faces in T.
 template <typename T>
 __global__ void __launch_bounds__(256)
     faces_kernel(const __grid_constant__ LabGeom L, const __grid_constant__ BcView kbc, const float *k, int nblocks, T ih2,
@@ -109,39 +108,11 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// mean across the upper face along d of dense cell t = (b, x, y, z)
-template <typename T>
-__device__ __forceinline__ T upper_mean(const Faces<T> &F, const LabGeom &L, int64_t t, int b, int x, int y, int z, int d)
-{
-    const int q = d == 0 ? x : (d == 1 ? y : z);
-    const int64_t st = d == 0 ? 1 : (d == 1 ? L.n[0] : (int64_t)L.n[0] * L.n[1]);
-    if (q + 1 < L.n[d]) return __ldg(F.k[d] + t + st);
-    const int64_t i = d == 0 ? y + (int64_t)L.n[1] * z : (d == 1 ? x + (int64_t)L.n[0] * z : x + (int64_t)L.n[0] * y);
-    return __ldg(F.u[d] + (int64_t)b * ((int64_t)L.n[0] * L.n[1] * L.n[2] / L.n[d]) + i);
-}
-
-// The tile kernels' coefficients (see op7_coef) from the face means.
-__global__ void __launch_bounds__(256)
-    coef_kernel(const __grid_constant__ LabGeom L, int nblocks, const __grid_constant__ Faces<float> F, const float *D,
-                float *coef)
-{
-    const int64_t total = (int64_t)nblocks * L.n[0] * L.n[1] * L.n[2];
-    for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < total; t += (int64_t)gridDim.x * 256) {
-        int b, x, y, z;
-        cell_of(t, L, b, x, y, z);
-        float *cv = coef + t * kCoefPerCell;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            cv[d] = upper_mean<float>(F, L, t, b, x, y, z, d);
-            cv[3 + d] = F.k[d][t];
-        }
-        cv[6] = D[t];
-        cv[7] = 0.0f;
-    }
-}
-
-// weighted Jacobi sweep: pout = pin + omega (L pin - f) / D
-__global__ void __launch_bounds__(kTileThreads, kTileMinCtas) jacobi_kernel(const __grid_constant__ KArgs a,
+// weighted Jacobi sweep: pout = pin + omega (L pin - f) / D.  Five CTAs per SM
+// (48 registers; a V(2,2) cycle of 256^3 cells by the tile kernels 2436 us, at
+// four and at six 2499 and 2433, of 64^3 244, 235 and 246).  A table of 8
+// coefficients per cell made the former 2310 us, for 32 bytes a cell more.
+__global__ void __launch_bounds__(kTileThreads, 5) jacobi_kernel(const __grid_constant__ KArgs a,
                                                               const __grid_constant__ Tile T, const float *pin,
                                                               const float *f, float *pout, float omega)
 {
@@ -158,47 +129,32 @@ __global__ void __launch_bounds__(kTileThreads, kTileMinCtas) jacobi_kernel(cons
     int x, y, z0, zl;
     if (!column_run(T, x, y, z0, zl)) return;
     const int st[3] = {1, q.rs, q.rs * q.ey};
-    const int64_t cells = (int64_t)L.n[0] * L.n[1] * L.n[2];
-    const int64_t oz = (int64_t)L.n[0] * L.n[1];
-    int64_t c = dense_cell(L, q, x, y, z0);
+    const int64_t cells = (int64_t)L.n[0] * L.n[1] * L.n[2], oz = (int64_t)L.n[0] * L.n[1];
+    const int64_t c = dense_cell(L, q, x, y, z0);
+    int64_t t = q.block * cells + c, o = q.block * L.bstride + c;
     int u = ridx(q, x, y, z0);
-    const float4 *cv = reinterpret_cast<const float4 *>(a.coef + ((int64_t)q.block * cells + c) * kCoefPerCell);
-    const int64_t cvz = oz * kCoefPerCell / 4;
-    int64_t o = (int64_t)q.block * L.bstride + c;
+    FaceColumn<float> fw;
+    fw.start(a.F, L, t, q.block, q.x0 + x, q.y0 + y, q.z0 + z0);
     // the next cell's loads go out before this cell's store
-    float4 ca = __ldg(cv), cb = __ldg(cv + 1);
-    float fc = __ldg(f + o);
-    for (int k = 0; k < zl; ++k, u += st[2]) {
-        float4 na = ca, nb = cb;
-        float nf = fc;
+    const int top = L.n[2] - 1 - (q.z0 + z0); // index of the block's upper plane in the run
+    float kn[6], fn = __ldg(f + o), Dn = __ldg(a.D + t);
+    fw.next(top == 0, kn);
+    for (int k = 0; k < zl; ++k, u += st[2], o += oz) {
+        const float Lp = op7_tile<float>(sp, u, st, kn, a.ih2), fc = fn, D = Dn;
         if (k + 1 < zl) {
-            na = __ldg(cv + cvz);
-            nb = __ldg(cv + cvz + 1);
-            nf = __ldg(f + o + oz);
+            t += oz;
+            fw.next(k + 1 == top, kn);
+            fn = __ldg(f + o + oz);
+            Dn = __ldg(a.D + t);
         }
-        const float cc[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
-        const float pc = sp[u];
-        float fl[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float kp = cc[d], km = cc[3 + d];
-            fl[d] = kp * (sp[u + st[d]] - pc) - km * (pc - sp[u - st[d]]);
-        }
-        const float Lp = a.ih2 * ((fl[0] + fl[1]) + fl[2]);
-        pout[o] = pc + omega * ((Lp - fc) / cb.z);
-        ca = na;
-        cb = nb;
-        fc = nf;
-        cv += cvz;
-        o += oz;
+        pout[o] = sp[u] + omega * ((Lp - fc) / D);
     }
 }
 
 // residual of the fine level restricted onto the coarse right-hand side:
 // fc = (sum of its 8 children's f - L p) / 8, children summed in the order
 // ((r0+r1)+(r2+r3))+((r4+r5)+(r6+r7)), child c = dx | dy<<1 | dz<<2.
-// Compiled for 4 CTAs per SM (64 registers): at the tile kernels' 6 it
-// spills 188 bytes per thread and the solve takes 1 % longer.
+// Compiled for 4 CTAs per SM (64 registers).
 __global__ void __launch_bounds__(kTileThreads, 4) resid_restrict_kernel(const __grid_constant__ KArgs a,
                                                                       const __grid_constant__ Tile T,
                                                                       const float *p, const float *f,
@@ -224,11 +180,12 @@ __global__ void __launch_bounds__(kTileThreads, 4) resid_restrict_kernel(const _
             int64_t c = dense_cell(L, q, x, y, z0);
             int u = ridx(q, x, y, z0);
             int ct = x + T.t[0] * (y + T.t[1] * z0);
+            FaceColumn<float> fw;
+            fw.start(a.F, L, q.block * cells + c, q.block, q.x0 + x, q.y0 + y, q.z0 + z0);
             for (int k = 0; k < zl; ++k, c += oz, u += st[2], ct += T.t[0] * T.t[1]) {
-                float Lp, D, pc;
-                op7_coef<float, float>(sp, u, st, a.coef + ((int64_t)q.block * cells + c) * kCoefPerCell, a.ih2, Lp,
-                                       D, pc);
-                sr[ct] = __ldg(f + (int64_t)q.block * L.bstride + c) - Lp;
+                float km[6];
+                fw.next(q.z0 + z0 + k + 1 == L.n[2], km);
+                sr[ct] = __ldg(f + q.block * L.bstride + c) - op7_tile<float>(sp, u, st, km, a.ih2);
             }
         }
     }
@@ -318,8 +275,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileMinCtas) prolong_kernel(con
 
 // FP64 residual of the outer iteration: r = f - L p64, r32 = (float) r,
 // per-CTA FP64 partial sums of r^2 and f^2.  The tile's p64 is staged with
-// its one-cell halo; the six FP64 face means of a cell are applied in
-// op7_coef's order.
+// its one-cell halo.
 __global__ void __launch_bounds__(kTileThreads, 4) resid64_kernel(const __grid_constant__ KArgs a,
                                                                const __grid_constant__ Tile T, const double *p64,
                                                                const float *f, float *r32, double *partials,
@@ -340,26 +296,17 @@ __global__ void __launch_bounds__(kTileThreads, 4) resid64_kernel(const __grid_c
     int x, y, z0, zl;
     if (column_run(T, x, y, z0, zl)) {
         const int st[3] = {1, q.rs, q.rs * q.ey};
-        const int gx = q.x0 + x, gy = q.y0 + y;
-        int64_t dc = dense_cell(Lk, q, x, y, z0);
+        const int64_t dc = dense_cell(Lk, q, x, y, z0);
         const int64_t cells = (int64_t)Lk.n[0] * Lk.n[1] * Lk.n[2], oz = (int64_t)Lk.n[0] * Lk.n[1];
         int64_t o = (int64_t)q.block * Lk.bstride + dc; // FP32 fields (f, r32)
         int u = ridx(q, x, y, z0);
-        for (int k = 0; k < zl; ++k, u += st[2], o += oz, dc += oz) {
-            const int64_t t = (int64_t)q.block * cells + dc;
+        FaceColumn<double> fw;
+        fw.start(F, Lk, q.block * cells + dc, q.block, q.x0 + x, q.y0 + y, q.z0 + z0);
+        for (int k = 0; k < zl; ++k, u += st[2], o += oz) {
+            double km[6];
+            fw.next(q.z0 + z0 + k + 1 == Lk.n[2], km);
             const float fcf = __ldg(f + o);
-            double km[3], kp[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                km[d] = __ldg(F.k[d] + t);
-                kp[d] = upper_mean<double>(F, Lk, t, q.block, gx, gy, q.z0 + z0 + k, d);
-            }
-            const double pc = sp[u];
-            double fd[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-                fd[d] = kp[d] * (sp[u + st[d]] - pc) - km[d] * (pc - sp[u - st[d]]);
-            const double Lp = a.ih2d * ((fd[0] + fd[1]) + fd[2]);
+            const double Lp = op7_tile<double>(sp, u, st, km, a.ih2d);
             const double fc = (double)fcf;
             const double r = fc - Lp;
             if (r32) r32[o] = (float)r;
@@ -625,9 +572,8 @@ KArgs kargs(cn_mg *m, int l)
     a.G.Lk = a.G.L;
     a.G.bc = bc_view(m->p[l], 0);
     a.G.nblocks = m->p[l]->nblocks;
-    a.kbc = bc_view(m->k[l], 0);
-    a.k = reinterpret_cast<const float *>(m->k[l]->d_data);
-    a.coef = (int)m->coef.size() > l ? m->coef[l] : nullptr;
+    a.F = m->faces[l];
+    a.D = m->diag[l];
     a.ih2d = 1.0 / (m->p[l]->h[0] * m->p[l]->h[0]);
     a.ih2 = (float)a.ih2d;
     return a;
@@ -680,19 +626,22 @@ static int width_of(const cn_grid *g, int most)
 }
 static float level_ih2(const cn_grid *g) { return (float)(1.0 / (g->h[0] * g->h[0])); }
 
-// one sweep by the marching kernel; with p64: also p64 += pout
+// one sweep by the marching kernel; with p64: also p64 += pout (levels that are
+// smoothed in a cycle have even extents, so not one cell at a time)
 template <int V> static void launch_jacobi(cn_mg *m, int l, const float *src, const float *f, float *dst, cn_grid *p64, cudaStream_t st)
 {
     const cn_grid *g = m->p[l];
     const float ih2 = level_ih2(g), om = (float)m->omega;
-    if (p64) {
-        const Layer a = layer_of(g, V, 1, 1, p64);
-        jacobi_march<V, 2, true><<<ctas_of(a), 256, 0, st>>>(a, m->faces[l], ih2, om, src, f, dst,
-                                                             reinterpret_cast<double *>(p64->d_data));
-    } else {
-        const Layer a = layer_of(g, V, 1, 1);
-        jacobi_march<V, 2, false><<<ctas_of(a), 256, 0, st>>>(a, m->faces[l], ih2, om, src, f, dst, nullptr);
+    if constexpr (V > 1) {
+        if (p64) {
+            const Layer a = layer_of(g, V, 1, 1, p64);
+            jacobi_march<V, 2, true><<<ctas_of(a), 256, 0, st>>>(a, m->faces[l], ih2, om, src, f, dst,
+                                                                 reinterpret_cast<double *>(p64->d_data));
+            return;
+        }
     }
+    const Layer a = layer_of(g, V, 1, 1);
+    jacobi_march<V, 2, false><<<ctas_of(a), 256, 0, st>>>(a, m->faces[l], ih2, om, src, f, dst, nullptr);
 }
 // (g: the grid whose BCs hold, m->p[l] as the smoothing starts; with p64, dst
 // is m->p[l] by now)
@@ -700,8 +649,6 @@ static cn_status jacobi_sweep(cn_mg *m, int l, const cn_grid *g, const float *sr
                               cudaStream_t st)
 {
     if (g->bc_count) {
-        cn_status s = mg_ensure_coef(m, st);
-        if (s != CN_OK) return s;
         const Tile T = tile_of(g->n);
         KArgs a = kargs(m, l);
         a.G.bc = bc_view(g, 0);
@@ -751,8 +698,6 @@ static cn_status restrict_residual(cn_mg *m, int l, const float *p, const float 
 {
     const cn_grid *g = m->p[l];
     if (g->bc_count) {
-        cn_status s = mg_ensure_coef(m, st);
-        if (s != CN_OK) return s;
         const Tile T = tile_of(g->n);
         resid_restrict_kernel<<<(unsigned)(g->nblocks * T.count), kTileThreads, 0, st>>>(kargs(m, l), T, p, f, make_geom(fc, &kS1),
                                                                                          fptr(fc));
@@ -907,21 +852,6 @@ static cn_status vcycle_from(cn_mg *m, int l, bool first_done, cn_grid *add, cud
 }
 
 cn_status vcycle(cn_mg *m, int l, cudaStream_t st) { return vcycle_from(m, l, false, nullptr, st); }
-
-cn_status mg_ensure_coef(cn_mg *m, cudaStream_t st)
-{
-    for (int l = (int)m->coef.size(); l < m->nlevels; ++l) {
-        const cn_grid *g = m->p[l];
-        const int64_t cells = (int64_t)g->nblocks * g->n[0] * g->n[1] * g->n[2];
-        float *c = nullptr;
-        if (cudaMalloc(&c, sizeof(float) * kCoefPerCell * cells) != cudaSuccess)
-            return fail(CN_ERR_OUT_OF_MEMORY, "multigrid: coefficients");
-        m->coef.push_back(c);
-        coef_kernel<<<grid_for(cells), 256, 0, st>>>(make_geom(g, &kS1), g->nblocks, m->faces[l], m->diag[l], c);
-        CN_CUDA_TRY(cudaGetLastError());
-    }
-    return CN_OK;
-}
 
 // The two sums of a multigrid lie in pinned host memory that the kernel writes.
 // Allocating it for every multigrid took 1 ms of creating and 0.4 ms of
@@ -1233,8 +1163,6 @@ cn_status cn_mg_destroy(cn_mg *m)
     }
     cn_grid_destroy(m->r32);
     for (void *q : m->owned) cudaFree(q);
-    for (float *c : m->coef)
-        if (c) cudaFree(c);
     if (m->coarse_inv) cudaFree(m->coarse_inv);
     for (cn_grid *g : m->nn_bufs) cn_grid_destroy(g);
     for (void *a : m->nn_act)

@@ -28,9 +28,6 @@ struct cn_mg {
     std::vector<float *> diag;          // per level: D of every cell, dense
     cn::mg::Faces<double> faces64;      // finest level, FP64
     std::vector<void *> owned;          // device allocations of the above
-    // per level: 8 FP32 per cell (k+ faces x,y,z, k- faces x,y,z, D, 0), made
-    // from the faces when a tile kernel first needs them (mg_ensure_coef)
-    std::vector<float *> coef;
     cn_grid *r32 = nullptr;             // finest FP32 residual
     double *partials = nullptr;
     unsigned *done = nullptr; // CTAs of a residual that have finished
@@ -65,8 +62,6 @@ extern const cn_stencil kS1, kS1t;
 unsigned grid_for(int64_t n);
 float *fptr(cn_grid *g);
 cn_status vcycle(cn_mg *m, int l, cudaStream_t st);
-// the tile kernels' per-cell coefficients (m->coef) of every level
-cn_status mg_ensure_coef(cn_mg *m, cudaStream_t st);
 // learned smoothing: `apps` applications of the network on level l
 extern "C" cn_status cn_mg_accumulate(cn_mg *m, cn_grid *p64, void *stream);
 extern "C" cn_status cn_mg_residual(cn_mg *m, const cn_grid *p64, const cn_grid *f, cn_grid *r32, double *rr,

@@ -5,13 +5,12 @@
 // planes and marches up it: p of planes z - 1 and z and the z face means stay
 // in registers, everything else is a cached load issued before anything waits.
 // Fields with BCs take the tile kernels of mg.cu.  Operations and their order
-// are those of op7_math, uncontracted, so results are bit for bit the same.
+// are those of the tile kernels (op7_tile), uncontracted, so results are bit for bit the same.
 //
 // The operator is stored as one harmonic mean per face: per cell the means
 // across its lower x, y, z faces, and per block those across its upper
 // boundary faces (harm is symmetric to the bit, so a face has one value from
-// either side), 12 B per cell in FP32 against 32 B for the eight per-cell
-// coefficients of the tile kernels.  Sweeps that only need the right-hand side
+// either side), 12 B per cell in FP32.  Sweeps that only need the right-hand side
 // (the first one, from a zero guess) ride on the kernel that makes it, and the
 // FP64 accumulation on the last sweep.
 //

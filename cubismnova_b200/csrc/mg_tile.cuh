@@ -7,6 +7,7 @@
 #include "cn_fastdiv.h"
 #include "cn_internal.h"
 #include "cn_tma.cuh"
+#include "mg_internal.h"
 
 namespace cn {
 namespace mg {
@@ -17,67 +18,65 @@ template <typename T> __device__ __forceinline__ T harm(T a, T b)
     return (t + t) / (a + b);
 }
 
-// L p and the diagonal D at one cell from its 13 values; TP is the solution
-// type (float in the V-cycle, double in the outer residual), k is FP32.
-template <typename TP>
-__device__ __forceinline__ void op7_math(const TP (&v)[14], TP ih2, TP &Lp, TP &D, TP &pc)
+// mean across the upper face along d of cell (x, y, z) of block b, dense index
+// t (over all blocks)
+template <typename T>
+__device__ __forceinline__ T upper_mean(const Faces<T> &F, const LabGeom &L, int64_t t, int b, int x, int y, int z, int d)
 {
-    pc = v[0];
-    const TP kc = v[1];
-    TP f[3], s[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const TP pp = v[2 + 4 * d], pm = v[3 + 4 * d];
-        const TP kp = harm<TP>(kc, v[4 + 4 * d]);
-        const TP km = harm<TP>(v[5 + 4 * d], kc);
-        f[d] = kp * (pp - pc) - km * (pc - pm);
-        s[d] = kp + km;
-    }
-    Lp = ih2 * ((f[0] + f[1]) + f[2]);
-    D = ih2 * ((s[0] + s[1]) + s[2]);
+    const int q = d == 0 ? x : (d == 1 ? y : z);
+    const int64_t n0 = L.n[0], n1 = L.n[1], n2 = L.n[2];
+    if (q + 1 < L.n[d]) return __ldg(F.k[d] + t + (d == 0 ? 1 : (d == 1 ? n0 : n0 * n1)));
+    const int64_t i = d == 0 ? y + n1 * (z + n2 * b) : (d == 1 ? x + n0 * (z + n2 * b) : x + n0 * (y + n1 * b));
+    return __ldg(F.u[d] + i);
 }
 
-// Operator coefficients of a level, precomputed once from k (they depend on
-// k only): per cell 8 contiguous values, the harmonic face means
-// kp_d = harm(k, k(+e_d)) (d = x, y, z), km_d = harm(k(-e_d), k) (neighbours
-// through the lab), the diagonal D = ih2 ((s0 + s1) + s2) with
-// s_d = kp_d + km_d, and a zero pad, so one cell's set is two (FP32) or four
-// (FP64) 16-byte loads.  Cell (block b, dense in-block index c) at
-// (b cells_per_block + c) * 8.  Evaluated with the same operations as
-// op7_math, so L p and D come out bit for bit the same.
-constexpr int kCoefPerCell = 8;
-
-template <typename TC> __device__ __forceinline__ void load_coef8(const TC *cv, TC (&c)[8])
-{
-    if constexpr (sizeof(TC) == 4) {
-        const float4 a = __ldg(reinterpret_cast<const float4 *>(cv)), b = __ldg(reinterpret_cast<const float4 *>(cv) + 1);
-        c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w;
-        c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const double2 v = __ldg(reinterpret_cast<const double2 *>(cv) + i);
-            c[2 * i] = v.x;
-            c[2 * i + 1] = v.y;
-        }
+// The face means along a column of cells going up z from cell (x, y, z) of
+// block b, dense index t.
+template <typename T> struct FaceColumn {
+    const T *lx, *ly, *lz, *ux, *uy, *top; // lower means, upper ones, those of the block's upper boundary
+    int64_t s2;
+    int sx, sy; // steps per plane of ux and uy
+    T zm;       // lower z mean
+    __device__ __forceinline__ void start(const Faces<T> &F, const LabGeom &L, int64_t t, int b, int x, int y, int z)
+    {
+        const int64_t n0 = L.n[0], n1 = L.n[1], n2 = L.n[2];
+        s2 = n0 * n1;
+        lx = F.k[0] + t;
+        ly = F.k[1] + t;
+        lz = F.k[2] + t;
+        ux = x + 1 < L.n[0] ? lx + 1 : F.u[0] + y + n1 * (z + n2 * b);
+        sx = x + 1 < L.n[0] ? (int)s2 : L.n[1];
+        uy = y + 1 < L.n[1] ? ly + n0 : F.u[1] + x + n0 * (z + n2 * b);
+        sy = y + 1 < L.n[1] ? (int)s2 : L.n[0];
+        top = F.u[2] + x + n0 * (y + n1 * b);
+        zm = __ldg(lz);
     }
-}
-
-template <typename TP, typename TC>
-__device__ __forceinline__ void op7_coef(const TP *sp, int u, const int (&st)[3], const TC *cv, TP ih2, TP &Lp,
-                                         TP &D, TP &pc)
-{
-    TC c[8];
-    load_coef8<TC>(cv, c);
-    pc = sp[u];
-    TP f[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const TP kp = (TP)c[d], km = (TP)c[3 + d];
-        f[d] = kp * (sp[u + st[d]] - pc) - km * (pc - sp[u - st[d]]);
+    // the six means of the cell (lower x, y, z, upper x, y, z), and one plane up;
+    // last: the cell is in the block's upper plane
+    __device__ __forceinline__ void next(bool last, T (&k)[6])
+    {
+        k[0] = __ldg(lx);
+        k[1] = __ldg(ly);
+        k[2] = zm;
+        k[3] = __ldg(ux);
+        k[4] = __ldg(uy);
+        k[5] = zm = __ldg(last ? top : lz + s2);
+        lx += s2;
+        ly += s2;
+        lz += s2;
+        ux += sx;
+        uy += sy;
     }
-    Lp = ih2 * ((f[0] + f[1]) + f[2]);
-    D = (TP)c[6];
+};
+// L p at entry u of the staged region (steps st to its neighbours)
+template <typename T>
+__device__ __forceinline__ T op7_tile(const T *sp, int u, const int (&st)[3], const T (&k)[6], T ih2)
+{
+    const T pc = sp[u];
+    T f[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) f[d] = k[3 + d] * (sp[u + st[d]] - pc) - k[d] * (pc - sp[u - st[d]]);
+    return ih2 * ((f[0] + f[1]) + f[2]);
 }
 
 // ---------------------------------------------------------------- tiles
@@ -322,24 +321,6 @@ __device__ __forceinline__ void stage_region(const T *comp, const LabGeom &L, co
             for (int i = lane; i < q.ex; i += 32)
                 stage_cell<T>(comp, L, bc, q, tensorial, snb, plain, q.x0 + i - 1, y, z, s + (i - 1 + q.xo) + q.rs * r);
         }
-    }
-}
-
-// the 13 operator values of tile cell (x, y, z) from the staged region
-template <typename TP>
-__device__ __forceinline__ void region7(const TP *sp, const float *sk, const TilePos &q, int x, int y, int z,
-                                        TP (&v)[14])
-{
-    const int u = ridx(q, x, y, z);
-    const int st[3] = {1, q.rs, q.rs * q.ey};
-    v[0] = sp[u];
-    v[1] = (TP)sk[u];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        v[2 + 4 * d] = sp[u + st[d]];
-        v[3 + 4 * d] = sp[u - st[d]];
-        v[4 + 4 * d] = (TP)sk[u + st[d]];
-        v[5 + 4 * d] = (TP)sk[u - st[d]];
     }
 }
 

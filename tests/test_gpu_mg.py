@@ -248,3 +248,81 @@ def test_solution_of_other_extents_is_refused(cn, n64):
     with pytest.raises(cn.CnError, match="unequal size"):
         m.solve(f, f)  # an FP32 solution
     assert m.solve(f, good, rtol=1e-8)[1] <= 1e-8
+
+
+def _base_bcs(cn, g):
+    """A Base BC (the periodic no-op) on every block: the tile kernels run."""
+    for b in range(g.size()):
+        g.field(b, 0).getBC().push_back(cn.BC.Base(0, 0))
+    g.sync_bcs()
+
+
+@pytest.mark.parametrize("nb,n,nu", [((4, 4, 4), (16, 16, 16), (2, 2)), ((2, 2, 2), (12, 12, 12), (2, 1)),
+                                     ((3, 2, 2), (8, 8, 8), (1, 2)), ((2, 2, 2), (2, 4, 8), (3, 2)),
+                                     ((2, 1, 1), (24, 8, 16), (0, 1)), ((1, 1, 1), (32, 32, 32), (1, 0))])
+def test_tile_kernels_from_the_face_means(cn, nb, n, nu):
+    """Cycles with a BC on the solution of every level, on both of the fields
+    that alternate as it where a sweep count is odd, against cycles without:
+    the tile kernels and the marching ones read the same face means and give
+    the same bits.  The first call of one multigrid is under stream capture,
+    where nothing may be left to allocate or to fill."""
+    import torch
+    k, f = _setup(cn, nb, n)
+    m, plain = (cn.mg.Multigrid(k, nu1=nu[0], nu2=nu[1], omega=0.8) for _ in range(2))
+    e = [cn.Grid.Cartesian(nb, n, end=_end(nb, n), dtype=np.float32) for _ in range(3)]
+    for l in range(m.nlevels):
+        _base_bcs(cn, m.level(l, "p"))
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    g = cn.amr.Graph.capture(lambda: m.vcycle(f, e[0], stream=s), s)
+    if sum(nu) % 2:  # now the other field of each level is its solution
+        for l in range(m.nlevels - 1):
+            _base_bcs(cn, m.level(l, "p"))
+    g.launch(s)
+    s.synchronize()
+    m.vcycle(f, e[1])
+    plain.vcycle(f, e[2])
+    torch.cuda.synchronize()
+    got = [x.blocks_view(x.download()) for x in e]
+    assert np.array_equal(got[1], got[2])
+    assert np.array_equal(got[0], got[2])
+
+
+def test_tile_kernels_on_two_streams(cn):
+    """The first sweeps of a new multigrid with BCs, on two streams that do not
+    wait for one another."""
+    import torch
+    nb, n = (4, 4, 4), (32, 32, 32)
+    k, f = _setup(cn, nb, n)
+    m, plain = cn.mg.Multigrid(k), cn.mg.Multigrid(k)
+    p, q, a, b, want = (cn.Grid.Cartesian(nb, n, dtype=np.float32) for _ in range(5))
+    cn.workloads.poisson_rhs(p, seed=9)
+    q.tensor(0).copy_(p.tensor(0))
+    plain.jacobi(p, f, want)
+    _base_bcs(cn, m.level(0, "p"))
+    torch.cuda.synchronize()
+    s, t = torch.cuda.Stream(), torch.cuda.Stream()
+    m.jacobi(p, f, a, stream=s)
+    m.jacobi(q, f, b, stream=t)
+    torch.cuda.synchronize()
+    assert torch.equal(a.tensor(0), want.tensor(0)) and torch.equal(b.tensor(0), want.tensor(0))
+
+
+@pytest.mark.parametrize("nb,n", [((2, 3, 2), (5, 7, 3)), ((3, 1, 2), (1, 9, 1)), ((2, 2, 2), (6, 3, 3)), ((1, 2, 1), (12, 3, 6))])
+@pytest.mark.parametrize("bcs", [False, True])
+def test_jacobi_of_odd_blocks_matches_oracle(cn, oracle_lib, nb, n, bcs):
+    """One sweep on blocks of odd extents, rows of one, two and four cells a
+    thread: the marching and the tile kernel against the oracle."""
+    import torch
+    k, f = _setup(cn, nb, n)
+    m = cn.mg.Multigrid(k)
+    p, out = (cn.Grid.Cartesian(nb, n, end=_end(nb, n), dtype=np.float32) for _ in range(2))
+    ph = np.zeros(p.comp_stride, dtype=np.float32)
+    p.blocks_view(ph)[:] = np.random.default_rng(5).standard_normal(p.blocks_view(ph).shape)
+    p.upload(ph)
+    if bcs:
+        _base_bcs(cn, m.level(0, "p"))
+    m.jacobi(p, f, out)
+    torch.cuda.synchronize()
+    want = oracle_lib.mg_jacobi(ph, k.download(), f.download(), nb, n, 0.8, np.float32(1.0 / p.getCellSize()[0] ** 2))
+    assert np.array_equal(p.blocks_view(out.download()), p.blocks_view(want))
