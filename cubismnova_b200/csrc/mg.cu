@@ -1282,6 +1282,9 @@ cn_status cn_mg_restrict_residual(cn_mg *m, const cn_grid *p, const cn_grid *f, 
 cn_status cn_mg_prolong(cn_mg *m, const cn_grid *ec, cn_grid *p, void *stream)
 {
     if (!m || !ec || !p) return fail(CN_ERR_INVALID_ARGUMENT, "bad argument");
+    bool fit = p->dtype == CN_FLOAT32 && ec->dtype == CN_FLOAT32 && p->nblocks == ec->nblocks;
+    for (int d = 0; d < 3; ++d) fit = fit && p->n[d] == 2 * ec->n[d]; // a thread takes pairs of fine cells along x and z
+    if (!fit) return fail(CN_ERR_SIZE_MISMATCH, "Cartesian: Can not assign two grids of unequal size.");
     cn_status s = sync_bc(const_cast<cn_grid *>(ec), as_stream(stream));
     if (s != CN_OK) return s;
     return prolong(ec, p, as_stream(stream));

@@ -326,3 +326,16 @@ def test_jacobi_of_odd_blocks_matches_oracle(cn, oracle_lib, nb, n, bcs):
     torch.cuda.synchronize()
     want = oracle_lib.mg_jacobi(ph, k.download(), f.download(), nb, n, 0.8, np.float32(1.0 / p.getCellSize()[0] ** 2))
     assert np.array_equal(p.blocks_view(out.download()), p.blocks_view(want))
+
+
+@pytest.mark.parametrize("fine,coarse", [((5, 5, 5), (2, 2, 2)), ((8, 8, 7), (4, 4, 3)), ((8, 8, 8), (4, 4, 2)),
+                                         ((8, 8, 8), (8, 8, 8)), ((8, 8, 8), (2, 2, 2))])
+def test_prolongation_of_other_extents_is_refused(cn, fine, coarse):
+    """The prolongation takes pairs of fine cells and indexes the coarse field
+    by halves: anything but a field of half the extents is refused."""
+    nb = (2, 2, 2)
+    k, _ = _setup(cn, nb, (8, 8, 8))
+    m = cn.mg.Multigrid(k)
+    p, e = (cn.Grid.Cartesian(nb, n, dtype=np.float32) for n in (fine, coarse))
+    with pytest.raises(cn.CnError, match="unequal size"):
+        m.prolong(e, p)
