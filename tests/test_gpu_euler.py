@@ -127,6 +127,23 @@ def test_max_speed_sees_every_cell(cn, dtype, nb, n):
         np.testing.assert_allclose(cn.euler.max_speed(U), want, rtol=16 * np.finfo(dtype).eps)
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("nb", [(3, 1, 1), (5, 7, 3)])
+def test_max_speed_across_blocks(cn, dtype, nb):
+    """Passes of two 8^3 blocks and a last one of one: the largest value in
+    the first and last cell of the first, a middle and the last block."""
+    U = _state(cn, nb, (8, 8, 8), dtype, bcs=False)
+    blocks = int(np.prod(nb))
+    for i, (blk, cell) in enumerate(((0, 0), (0, 511), (blocks // 2, 0), (blocks // 2, 511), (blocks - 1, 0),
+                                     (blocks - 1, 511))):
+        U.tensor(1)[blk, cell] = 10.0 + i
+        U.tensor(4)[blk, cell] = 400.0 + 100.0 * i
+        r, m0, m1, m2, E = (np.asarray(U.tensor(c)[:, :512].cpu(), dtype=np.float64) for c in range(5))
+        c = np.sqrt(GAMMA * (GAMMA - 1) * (E - 0.5 * (m0 ** 2 + m1 ** 2 + m2 ** 2) / r) / r)
+        want = [np.max(np.abs(m / r) + c) for m in (m0, m1, m2)]
+        np.testing.assert_allclose(cn.euler.max_speed(U), want, rtol=16 * np.finfo(dtype).eps)
+
+
 def test_uniform_state_full_size_is_steady(cn):
     """512^3 cells (16^3 blocks of 32^3), C2 BCs: a uniform far-field state has
     an exactly zero RHS (every face sees the same six cells)."""
