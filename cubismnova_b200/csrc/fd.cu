@@ -6,18 +6,25 @@
 // x and y neighbours are cached loads, across a face of the block at a
 // constant offset in the neighbour block.  Threads run over all columns of all
 // blocks, x fastest, so that blocks of any extent fill the warps.  Cells beside
-// faces that carry a BC or a skipped neighbour are left to a few CTAs of the
-// same launch that resolve them one by one (Absorbing and Symmetry lead to the
-// own cell at ghost width 1, Dirichlet and undefined cells to a constant):
-// together the lab of a stencil (-1,2) non-tensorial (Block/FieldLab.h:180-224).
+// faces that carry a BC or a skipped neighbour are left to other CTAs of the
+// same launch, which find what lies behind each face once (Absorbing and
+// Symmetry lead to the own cell at ghost width 1, Dirichlet and undefined cells
+// to a constant): together the lab of a stencil (-1,2) non-tensorial
+// (Block/FieldLab.h:180-224).
 //
 // Bound by DRAM at large sizes and by latency and the launch at small ones.
 // Against tiles staged in shared memory (one bulk copy per z slab, faces cell
 // by cell), B200: Laplacian + gradient FP64 128^3 22.3 -> 18.5 us, 512^3 1003
-// -> 891 us (94 % of the copy bandwidth); divergence FP64 512^3 2161 -> 695
+// -> 891 us (94 % of the copy bandwidth); divergence FP64 512^3 2161 -> 705
 // us, FP32 on 30 x 33 x 27 blocks with walls (25.7 M cells) 406 -> 81 us;
 // Laplacian FP32 512^3 793 -> 199 us.  BC code inlined into the march cost the
 // registers of a third of the warps (84 -> 107 us on the ragged case).
+//
+// Faces with BCs: a few CTAs that walked their cells one face after the other,
+// each cell with its own chain of BC loads, set the time of small grids and of
+// large faces.  FP64 Laplacian with walls, that -> now: 128^3 25 -> 15 us, 36 x
+// 36 x 200 blocks (2.1 M cells) 95 -> 15, one block of 32^3 24 -> 7; a BC on every
+// face of every 8^3 block of 128^3 179 -> 48.
 //
 // Arithmetic uses __d*_rn / __f*_rn intrinsics so nothing is contracted into
 // an FMA: results are bit-identical to the reference loops compiled without
@@ -63,9 +70,12 @@ template <typename T> struct FdParams {
     int64_t out_cstride;
     T ih[3], ih2[3];
     int TZ, block0, total;       // planes per thread, first block and threads of this launch
+    uint32_t face_share;          // share of CTAs that look at faces, / 2^32
     FastDiv per_block, plane, n0; // threads per block, N0 * N1, N0
     FastDiv nb0, nb1, f0, f1;     // blocks along x, y; N0, N1
-    int faces, faces_per_cta, face_ctas; // faces of this launch's blocks, CTAs that look at them
+    int xw;                       // cells of a row beside x faces that bc_faces takes
+    FastDiv fxw;
+    int faces, faces_per_cta, parts; // faces of this launch's blocks; see bc_faces
 };
 
 // Outputs of one cell from its six neighbours (kDiv: x neighbours of the
@@ -118,38 +128,6 @@ template <typename T, int V> __device__ __forceinline__ Pack<T, V> load(const T 
 template <typename T, int V> __device__ __forceinline__ void store(T *p, const Pack<T, V> &r)
 {
     *reinterpret_cast<Pack<T, V> *>(p) = r;
-}
-
-// A neighbour of a column's cells: cell o's neighbour is in[o + off], times
-// `value` behind a face with Absorbing or Symmetry (kind 2; off leads to the
-// own cell), or `value` itself (kind 1).
-template <typename T> struct Side {
-    int64_t off;
-    T value;
-    int kind;
-};
-
-template <typename T> __device__ __noinline__ FaceRule<T> rule_of(const LabGeom &L, const BcView &bc, int block, int d, int s)
-{
-    return face_rule<T>(L, bc, block, d, s);
-}
-
-// side s of direction d (stride st) of a cell at coordinate q
-template <typename T>
-__device__ __forceinline__ Side<T> side_of(const LabGeom &L, const BcView &bc, int block, int b, int d, int s, int q,
-                                           int64_t st)
-{
-    Side<T> r = {s ? st : -st, T(1), 0};
-    const int n = L.n[d];
-    if (s ? q + 1 < n : q > 0) return r;
-    if ((__ldg(bc.faces + block) >> (2 * d + s)) & 1) {
-        const FaceRule<T> f = rule_of<T>(L, bc, block, d, s);
-        if (f.kind != kRuleCopy) return {0, f.value, f.kind == kRuleValue ? 1 : 2};
-    }
-    const int m = L.nb[d], nbr = s ? (b + 1 < m ? b + 1 : 0) : (b > 0 ? b - 1 : m - 1);
-    const int bs = d == 0 ? 1 : (d == 1 ? L.nb[0] : L.nb[0] * L.nb[1]);
-    r.off += (int64_t)(nbr - b) * bs * L.bstride + (s ? -n : n) * st;
-    return r;
 }
 
 // One thread's run of planes from cell o, all neighbours plain cells: U planes
@@ -209,73 +187,6 @@ __device__ __forceinline__ void march(const FdParams<T> &p, int64_t o, int64_t s
     }
 }
 
-// One cell with BCs on any side.
-template <typename T, int OP>
-__device__ __forceinline__ void bc_cell(const FdParams<T> &p, int block, int b0, int b1, int b2, int x, int y, int z)
-{
-    const LabGeom &L = p.L;
-    const int64_t s1 = L.n[0], s2 = (int64_t)L.n[0] * L.n[1];
-    const int64_t o = (int64_t)block * L.bstride + x + s1 * y + s2 * z;
-    Side<T> e[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-        e[k] = side_of<T>(L, p.bc[k >> 1], block, pick3(k >> 1, b0, b1, b2), k >> 1, k & 1, pick3(k >> 1, x, y, z),
-                          k < 2 ? 1 : (k < 4 ? s1 : s2));
-    T v[6]; // lower and upper neighbour along x, y, z
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-        v[k] = __ldg(p.in[k >> 1] + o + e[k].off);
-    const T c = __ldg(p.in[0] + o);
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-        v[k] = e[k].kind == 1 ? e[k].value : (e[k].kind == 2 ? Arith<T>::mul(e[k].value, v[k]) : v[k]);
-    T l, g0, g1, g2;
-    cell_eval<T, OP>(p, c, v[1], v[0], v[3], v[2], v[5], v[4], l, g0, g1, g2);
-    if (OP == kLap || OP == kLapGrad || OP == kDiv) p.lap[o] = l;
-    if (OP == kGrad || OP == kLapGrad) {
-        p.grad[o] = g0;
-        p.grad[o + p.out_cstride] = g1;
-        p.grad[o + 2 * p.out_cstride] = g2;
-    }
-}
-
-// The cells beside block faces that carry a BC or a skipped neighbour, which
-// the marching threads leave out: a CTA looks at some of the nblocks * 6 faces
-// and walks the cells of those (x faces: the V cells of the columns there).
-// Out of line, so that its registers stay its own.
-constexpr int kFacesPerCta = 8; // at most
-template <typename T, int OP, int V> __device__ __noinline__ void bc_faces(const FdParams<T> &p)
-{
-    const LabGeom &L = p.L;
-    const int lane = threadIdx.x & 31, first = blockIdx.x * p.faces_per_cta;
-    bool set = false;
-    if (lane < p.faces_per_cta && first + lane < p.faces) {
-        const int f = (first + lane) % 6;
-        const BcView &bc = f < 2 ? p.bc[0] : (f < 4 ? p.bc[1] : p.bc[2]);
-        set = (__ldg(bc.faces + p.block0 + (first + lane) / 6) >> f) & 1;
-    }
-    for (unsigned m = __ballot_sync(0xffffffffu, set); m; m &= m - 1) {
-        const int item = first + __ffs(m) - 1, f = item % 6, d = f >> 1, block = p.block0 + item / 6;
-        const int b12 = p.nb0.div(block), b0 = block - b12 * (int)p.nb0.d, b2 = p.nb1.div(b12), b1 = b12 - b2 * (int)p.nb1.d;
-        const int n = d == 0 ? V * L.n[1] * L.n[2] : L.n[0] * pick3(d, 0, L.n[2], L.n[1]);
-        for (int i = threadIdx.x; i < n; i += 256) {
-            int x, y, z;
-            if (d == 0) {
-                const int q = i / V;
-                z = p.f1.div(q);
-                y = q - z * L.n[1];
-                x = i - q * V + (f & 1 ? L.n[0] - V : 0);
-            } else {
-                const int q = p.f0.div(i);
-                x = i - q * L.n[0];
-                y = d == 1 ? (f & 1 ? L.n[1] - 1 : 0) : q;
-                z = d == 2 ? (f & 1 ? L.n[2] - 1 : 0) : q;
-            }
-            bc_cell<T, OP>(p, block, b0, b1, b2, x, y, z);
-        }
-    }
-}
-
 // offset to a neighbour across a side without BCs: side s of direction d
 // (stride st) at coordinate q of block coordinate b
 __device__ __forceinline__ int64_t side_offset(const LabGeom &L, int b, int d, int s, int q, int64_t st)
@@ -287,14 +198,113 @@ __device__ __forceinline__ int64_t side_offset(const LabGeom &L, int b, int d, i
     return (s ? st : -st) + (int64_t)(nbr - b) * bs * L.bstride + (s ? -n : n) * st;
 }
 
-template <typename T, int OP, int V, int U>
-__global__ void __launch_bounds__(256) fd_kernel(const __grid_constant__ FdParams<T> p)
+// What lies behind a face of a block for a cell beside it: the cell at distance
+// off (kind 0), times `value` behind Absorbing or Symmetry (kind 2; they lead to
+// the own cell), or `value` itself (kind 1).
+template <typename T> struct Side {
+    int64_t off;
+    T value;
+    int kind;
+};
+
+// The cells beside block faces that carry a BC or a skipped neighbour, which
+// the marching threads leave out: `parts` CTAs look at the same few of the
+// nblocks * 6 faces and walk the cells of those one after the other, 256 parts
+// apart (x faces: the V cells of the columns there).  The BCs are a chain of
+// dependent loads, so one thread each finds what lies behind the faces of
+// these blocks, for all cells.  Out of line, so that its registers stay its own.
+constexpr int kFacesPerCta = 32;                     // at most
+constexpr int kFaceBlocks = (kFacesPerCta + 10) / 6; // blocks they belong to, at most
+template <typename T, int OP, int V> __device__ __noinline__ void bc_faces(const FdParams<T> &p, int cta)
 {
-    if ((int)blockIdx.x < p.face_ctas) {
-        bc_faces<T, OP, V>(p);
-        return;
+    const LabGeom &L = p.L;
+    const int lane = threadIdx.x & 31, group = cta / p.parts, first = group * p.faces_per_cta;
+    bool set = false;
+    if (lane < p.faces_per_cta && first + lane < p.faces) {
+        const int f = (first + lane) % 6;
+        const BcView &bc = f < 2 ? p.bc[0] : (f < 4 ? p.bc[1] : p.bc[2]);
+        set = (__ldg(bc.faces + p.block0 + (first + lane) / 6) >> f) & 1;
     }
-    const int t = ((int)blockIdx.x - p.face_ctas) * 256 + threadIdx.x;
+    unsigned m = __ballot_sync(0xffffffffu, set); // the same in all warps
+    if (!m) return;
+    __shared__ Side<T> sides[kFaceBlocks][6];
+    const int64_t s1 = L.n[0], s2 = (int64_t)L.n[0] * L.n[1];
+    const int b6 = first / 6;
+    if (threadIdx.x < 6 * kFaceBlocks && 6 * b6 + (int)threadIdx.x < p.faces) {
+        const int f = threadIdx.x % 6, d = f >> 1, block = p.block0 + b6 + threadIdx.x / 6;
+        const int b12 = p.nb0.div(block), b0 = block - b12 * (int)p.nb0.d, b2 = p.nb1.div(b12),
+                  b1 = b12 - b2 * (int)p.nb1.d;
+        const FaceRule<T> r = face_rule<T>(L, f < 2 ? p.bc[0] : (f < 4 ? p.bc[1] : p.bc[2]), block, d, f & 1);
+        Side<T> e = {0, r.value, r.kind == kRuleValue ? 1 : 2};
+        if (r.kind == kRuleCopy)
+            e = {side_offset(L, pick3(d, b0, b1, b2), d, f & 1, f & 1 ? L.n[d] - 1 : 0, d == 0 ? 1 : (d == 1 ? s1 : s2)), T(1), 0};
+        sides[threadIdx.x / 6][f] = e;
+    }
+    __syncthreads();
+    int i = (cta - group * p.parts) * 256 + threadIdx.x; // in the current face
+    while (m) {
+        const int item = first + __ffs(m) - 1, blk = item / 6, f = item - 6 * blk, d = f >> 1;
+        const int n = d == 0 ? p.xw * L.n[1] * L.n[2] : L.n[0] * pick3(d, 0, L.n[2], L.n[1]);
+        if (i >= n) {
+            i -= n;
+            m &= m - 1;
+            continue;
+        }
+        int q[3];
+        if (d == 0) {
+            const int r = p.fxw.div(i);
+            q[2] = p.f1.div(r);
+            q[1] = r - q[2] * L.n[1];
+            q[0] = i - r * p.xw + (f & 1 ? L.n[0] - p.xw : 0);
+        } else {
+            const int r = p.f0.div(i);
+            q[0] = i - r * L.n[0];
+            q[1] = d == 1 ? (f & 1 ? L.n[1] - 1 : 0) : r;
+            q[2] = d == 2 ? (f & 1 ? L.n[2] - 1 : 0) : r;
+        }
+        i += 256 * p.parts;
+        const int64_t o = (int64_t)(p.block0 + blk) * L.bstride + q[0] + s1 * q[1] + s2 * q[2];
+        const Side<T> *e = sides[blk - b6];
+        T v[6]; // lower and upper neighbour along x, y, z
+        bool at[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const int64_t st = k < 2 ? 1 : (k < 4 ? s1 : s2);
+            at[k] = k & 1 ? q[k >> 1] + 1 == L.n[k >> 1] : q[k >> 1] == 0;
+            v[k] = __ldg(p.in[k >> 1] + o + (at[k] ? e[k].off : (k & 1 ? st : -st)));
+        }
+        const T c = __ldg(p.in[0] + o);
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            if (at[k] && e[k].kind) v[k] = e[k].kind == 1 ? e[k].value : Arith<T>::mul(e[k].value, v[k]);
+        T l, g0, g1, g2;
+        cell_eval<T, OP>(p, c, v[1], v[0], v[3], v[2], v[5], v[4], l, g0, g1, g2);
+        if (OP == kLap || OP == kLapGrad || OP == kDiv) p.lap[o] = l;
+        if (OP == kGrad || OP == kLapGrad) {
+            p.grad[o] = g0;
+            p.grad[o + p.out_cstride] = g1;
+            p.grad[o + 2 * p.out_cstride] = g2;
+        }
+    }
+}
+
+// Resident CTAs per SM: three for the FP64 divergence (78 registers; of 512^3
+// cells 705 us, with the four that its 62 registers would allow 816).
+// BCS: the grid carries BCs.
+template <typename T, int OP> constexpr int min_ctas() { return OP == kDiv && sizeof(T) == 8 ? 3 : 0; }
+template <typename T, int OP, int V, int U, bool BCS>
+__global__ void __launch_bounds__(256, min_ctas<T, OP>()) fd_kernel(const __grid_constant__ FdParams<T> p)
+{
+    int cta = blockIdx.x;
+    if constexpr (BCS) {
+        const int fc = __umulhi(cta, p.face_share); // face CTAs before this one
+        if (__umulhi(cta + 1, p.face_share) != fc) {
+            bc_faces<T, OP, V>(p, fc);
+            return;
+        }
+        cta -= fc;
+    }
+    const int t = cta * 256 + threadIdx.x;
     if (t >= p.total) return;
     const LabGeom &L = p.L;
     const int bl = p.per_block.div(t), r = t - bl * (int)p.per_block.d;
@@ -302,23 +312,23 @@ __global__ void __launch_bounds__(256) fd_kernel(const __grid_constant__ FdParam
     const int y = p.n0.div(c), x = V * (c - y * (int)p.n0.d);
     const int block = p.block0 + bl;
     int z0 = zc * p.TZ, z1 = min(z0 + p.TZ, L.n[2]);
-    // faces of the block that this run touches; those with BCs are bc_faces'
-    const unsigned fx = (x == 0 ? 1u : 0u) | (x + V == L.n[0] ? 2u : 0u), fy = (y == 0 ? 4u : 0u) | (y + 1 == L.n[1] ? 8u : 0u),
-                   fz = (z0 == 0 ? 16u : 0u) | (z1 == L.n[2] ? 32u : 0u);
-    bool skip0 = false, skip1 = false;
-    if (fx && (__ldg(p.bc[0].faces + block) & fx)) return;
-    if (fy && (__ldg(p.bc[1].faces + block) & fy)) return;
-    if (fz) {
-        const unsigned f = __ldg(p.bc[2].faces + block) & fz;
-        skip0 = f & 16u;
-        skip1 = f & 32u;
+    if constexpr (BCS) {
+        // faces of the block that this run touches; those with BCs are bc_faces'
+        const unsigned fx = (x < p.xw ? 1u : 0u) | (x + V > L.n[0] - p.xw ? 2u : 0u),
+                       fy = (y == 0 ? 4u : 0u) | (y + 1 == L.n[1] ? 8u : 0u),
+                       fz = (z0 == 0 ? 16u : 0u) | (z1 == L.n[2] ? 32u : 0u);
+        if (fx && (__ldg(p.bc[0].faces + block) & fx)) return;
+        if (fy && (__ldg(p.bc[1].faces + block) & fy)) return;
+        if (fz) {
+            const unsigned f = __ldg(p.bc[2].faces + block) & fz;
+            z0 += (f & 16u) ? 1 : 0;
+            z1 -= (f & 32u) ? 1 : 0;
+        }
+        if (z0 >= z1) return;
     }
     const int b12 = p.nb0.div(block), b0 = block - b12 * (int)p.nb0.d;
     const int b2 = p.nb1.div(b12), b1 = b12 - b2 * (int)p.nb1.d;
     const int64_t s1 = L.n[0], s2 = (int64_t)L.n[0] * L.n[1];
-    z0 += skip0;
-    z1 -= skip1;
-    if (z0 >= z1) return;
     march<T, OP, V, U>(p, (int64_t)block * L.bstride + x + s1 * y + s2 * z0, s2, z1 - z0, side_offset(L, b0, 0, 0, x, 1),
                        side_offset(L, b0, 0, 1, x + V - 1, 1), side_offset(L, b1, 1, 0, y, s1),
                        side_offset(L, b1, 1, 1, y, s1), side_offset(L, b2, 2, 0, z0, s2),
@@ -366,15 +376,46 @@ template <typename T, int OP, int V> static cn_status launch_march(const cn_grid
     p.nb1 = FastDiv((uint32_t)u->nb[1]);
     p.f0 = FastDiv((uint32_t)u->n[0]);
     p.f1 = FastDiv((uint32_t)u->n[1]);
-    // one launch; beyond 2^30 threads, several over block ranges
-    const int most = (1 << 30) / per_block;
+    // Without BCs nothing is skipped either, and no CTA looks at faces.  A
+    // captured call may meet BCs that are pushed later.
+    bool bcs = u->bc_count != 0;
+    if (!bcs && st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CN_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+        bcs = cap != cudaStreamCaptureStatusNone;
+    }
+    // one launch; beyond 2^30 threads or 2^28 blocks, several over block ranges
+    const int most = std::min((1 << 30) / per_block, 1 << 28);
     for (p.block0 = 0; p.block0 < u->nblocks; p.block0 += most) {
         p.total = std::min(most, u->nblocks - p.block0) * per_block;
-        p.faces = p.total / per_block * 6;
-        // few blocks: a CTA each, so that their cells are resolved side by side
-        p.faces_per_cta = std::min(kFacesPerCta, p.faces / (148 * 2) + 1);
-        p.face_ctas = (p.faces + p.faces_per_cta - 1) / p.faces_per_cta;
-        fd_kernel<T, OP, V, U><<<(unsigned)(p.face_ctas + (p.total + 255) / 256), 256, 0, st>>>(p);
+        const int march = (p.total + 255) / 256;
+        if (!bcs) {
+            fd_kernel<T, OP, V, U, false><<<(unsigned)march, 256, 0, st>>>(p);
+        } else {
+            // A CTA takes few faces where these are large or few in all, and
+            // several CTAs share large ones as long as there are few: at most
+            // four per SM.  Face CTAs are spread over the launch, so that the
+            // cells beside x faces, parts of sectors, are written when the
+            // march writes the rest (the same blocks in order).
+            p.faces = p.total / per_block * 6;
+            // Cells beside x faces are written apart from the rest of their
+            // sector.  For several outputs that do not fit L2 (126 MB) they are
+            // taken by whole sectors: Laplacian + gradient of 512^3 FP64 cells
+            // with walls 1105 -> 900 us; the Laplacian alone 581 -> 591, and
+            // of 128^3 with the gradient 21 -> 25.
+            constexpr int sector = 32 / sizeof(T);
+            const bool wide = (OP == kGrad || OP == kLapGrad) && V > 1 && u->n[0] % sector == 0 &&
+                              (int64_t)u->nblocks * u->block_stride * (int64_t)sizeof(T) * 3 > (126 << 20);
+            p.xw = wide ? sector : V;
+            p.fxw = FastDiv((uint32_t)p.xw);
+            const int large = std::max({p.xw * u->n[1] * N2, u->n[0] * N2, u->n[0] * u->n[1]}); // cells of the largest face
+            p.faces_per_cta = std::max(1, std::min({kFacesPerCta, p.faces / (148 * 2) + 1, 8192 / large}));
+            const int groups = (p.faces + p.faces_per_cta - 1) / p.faces_per_cta;
+            p.parts = std::max(1, std::min((large + 255) / 256, 148 * 4 / groups));
+            const int faces = groups * p.parts, ctas = faces + march;
+            p.face_share = (uint32_t)((((uint64_t)faces << 32) + ctas - 1) / ctas); // exact: faces of them in all
+            fd_kernel<T, OP, V, U, true><<<(unsigned)ctas, 256, 0, st>>>(p);
+        }
         CN_CUDA_TRY(cudaGetLastError());
     }
     return CN_OK;

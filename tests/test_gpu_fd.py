@@ -268,3 +268,61 @@ def test_random_bc_vectors_vs_oracle_labs(cn, oracle_lib, dtype, nb, n):
         want.append(T(0.5) * ((dv[0] + dv[1]) + dv[2]))
         for what, (a, w) in enumerate(zip(got, want)):
             assert np.array_equal(a[b], w), f"output {what}, block {b}"
+
+
+@pytest.mark.parametrize("nb,n,share", [((2, 2, 1), (12, 10, 40), 0.6), ((1, 1, 1), (36, 36, 60), 1.0),
+                                        ((9, 8, 11), (4, 3, 5), 0.4), ((8, 8, 8), (2, 4, 3), 1.0),
+                                        ((7, 5, 6), (8, 6, 2), 0.05), ((6, 6, 6), (32, 32, 32), 0.15)])
+def test_faces_with_bcs_vs_oracle(cn, oracle_lib, nb, n, share):
+    """BCs on a share of all block faces: large faces that several CTAs walk,
+    many small ones to a CTA, CTAs without any, and outputs beyond L2, where x
+    faces are taken by whole sectors.  Then without BCs again, and with BCs
+    pushed between the capture of a call and its replay."""
+    import torch
+    O = oracle_lib
+    rng = np.random.default_rng(nb[0] + n[0])
+    nbk, stride = int(np.prod(nb)), O.block_stride(n, np.float64)
+    comp = rng.standard_normal(nbk * stride)
+    g = cn.Grid.Cartesian(nb, n)
+    g.upload(comp)
+    lap, grad = cn.Grid.Cartesian(nb, n), cn.Grid.Cartesian(nb, n, ncomp=3)
+    h = g.getCellSize()
+
+    def check(bcl):
+        wl = O.laplacian_f64(comp, nb, n, bcl, [1 / (x * x) for x in h])
+        wg = O.gradient_f64(comp, nb, n, bcl, [1 / x for x in h])
+        assert np.array_equal(lap.blocks_view(lap.download(0)), lap.blocks_view(wl))
+        for d in range(3):
+            assert np.array_equal(grad.blocks_view(grad.download(d)), grad.blocks_view(wg[d]))
+
+    kinds = {O.BC_DIRICHLET: cn.BC.Dirichlet, O.BC_ABSORBING: cn.BC.Absorbing, O.BC_SYMMETRY: cn.BC.Symmetry}
+    faces = [(b, d, s) for b in range(nbk) for d in range(3) for s in range(2) if rng.random() < share]
+    bcl = {}
+    for b, d, s in faces:
+        bcl.setdefault(b, []).append((d, s, int(rng.choice(list(kinds))), float(rng.choice([0.5, -1.0]))))
+
+    def push():
+        for b, lst in bcl.items():
+            for d, s, k, v in lst:
+                g.field(b).getBC().push_back(kinds[k](d, s) if k == O.BC_ABSORBING else kinds[k](d, s, v))
+        g.sync_bcs()
+
+    def clear():
+        for b in bcl:
+            g.field(b).getBC().clear()
+        g.sync_bcs()
+
+    push()
+    cn.ops.lap_grad(g, lap, grad)
+    torch.cuda.synchronize()
+    check(bcl)
+    clear()
+    cn.ops.lap_grad(g, lap, grad)
+    torch.cuda.synchronize()
+    check({})
+    s = torch.cuda.Stream()
+    graph = cn.amr.Graph.capture(lambda: cn.ops.lap_grad(g, lap, grad, stream=s), s)
+    push()
+    graph.launch(s)
+    s.synchronize()
+    check(bcl)
