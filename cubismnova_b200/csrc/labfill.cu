@@ -22,11 +22,13 @@
 #include "cn_tma.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace cn {
 
 constexpr int KL = 4;              // cells per thread resolved before their loads
 constexpr int KLM = 8;             // cells per thread in flight in the one-pass form
+constexpr int KLO = 8;              // own cells in flight per thread of the row form without the copy
 constexpr int KLR = 3;             // rows in flight per thread of the row form
 constexpr int KLX = 3;             // x ghosts in flight per thread of the row form
 constexpr int kBulkBytes = 24576;  // largest bulk copy of a slab's block planes
@@ -550,18 +552,38 @@ __global__ void __launch_bounds__(256, kWarpRowCtas)
             }
         }
     } else {
-        for (int x = lx; x < n0; x += 1 << wl)
-            for (int r0 = grp; r0 < own; r0 += KLR * ngrp) {
-                T v[KLR];
+        // planes too large for the copy: their rows as one run, in pairs of
+        // cells where rows hold whole pairs.  Row by row, KLR loads in flight
+        // and a part of the lanes idle at each row's end, took up to 1.4 times
+        // as long: B200, tensorial labs of 64 blocks of 96 x 96 x 40, one ghost,
+        // FP64 111 -> 91 us, FP32 71 -> 58; non-tensorial ones of 128 blocks of
+        // 100 x 100 x 30, FP64, 186 -> 143.
+        auto copy = [&](auto pair) {
+            constexpr int V = decltype(pair)::value, N = KLO / V;
+            struct alignas(sizeof(T) * V) Cells {
+                T v[V];
+            };
+            const Cells *src = reinterpret_cast<const Cells *>(src0);
+            const int cnt = own * n0 / V;
+            for (int p0 = threadIdx.x; p0 < cnt; p0 += N * blockDim.x) {
+                Cells v[N];
 #pragma unroll
-                for (int k = 0; k < KLR; ++k)
-                    if (r0 + k * ngrp < own) v[k] = src0[(r0 + k * ngrp) * n0 + x];
+                for (int k = 0; k < N; ++k)
+                    if (p0 + k * blockDim.x < cnt) v[k] = src[p0 + k * blockDim.x];
 #pragma unroll
-                for (int k = 0; k < KLR; ++k) {
-                    const int r = r0 + k * ngrp, zp = dv.n1.div(r);
-                    if (r < own) o[L.lo[0] + E0 * ((r - zp * n1 + L.lo[1]) + E1 * (zi0 + zp)) + x] = v[k];
+                for (int k = 0; k < N; ++k) {
+                    const int p = p0 + k * blockDim.x, t = V * p, r = dv.n0.div(t), zp = dv.n1.div(r);
+                    T *d = o + (t - r * n0 + L.lo[0]) + E0 * ((r - zp * n1 + L.lo[1]) + E1 * (zi0 + zp));
+                    if (p < cnt)
+#pragma unroll
+                        for (int i = 0; i < V; ++i) d[i] = v[k].v[i];
                 }
             }
+        };
+        if (n0 % 2 == 0)
+            copy(std::integral_constant<int, 2>{});
+        else
+            copy(std::integral_constant<int, 1>{});
     }
     if (deferred) { // this thread's x ghosts beyond faces with BCs or skips, one by one
         for (int t = threadIdx.x; t < B; t += blockDim.x) {

@@ -240,3 +240,26 @@ def test_lab_fill_whole_runs_vs_oracle(cn, oracle_lib, nb, n):
         want, wdef = O.lab_fill(comp, nb, n, lo, hi, False, bcl, b)
         LC.compare_defined(labs[b], written[b], want, wdef)
     g.close()
+
+
+@pytest.mark.parametrize("tens", [False, True])
+@pytest.mark.parametrize("dt,n", [(np.float64, (56, 57, 3)), (np.float64, (57, 55, 4)), (np.float64, (30, 108, 3)),
+                                  (np.float32, (62, 100, 3)), (np.float32, (79, 81, 2)), (np.int32, (63, 98, 3))])
+def test_lab_fill_large_planes_vs_oracle(cn, oracle_lib, dt, n, tens):
+    """Blocks whose planes are larger than the shared-memory copy (24 KB): the
+    own rows in pairs of cells and, of odd extents, cell by cell, of tensorial
+    labs and of others with more ghost rows than the one-pass kernel's table;
+    bit-exact against the oracle."""
+    O = oracle_lib
+    rng = np.random.default_rng(sum(n))
+    nb, lo, hi = (2, 1, 2), (1, 2, 1), (2, 1, 2)
+    size = 4 * O.block_stride(n, dt)
+    comp = (rng.integers(-1000, 1000, size=size) if dt == np.int32 else rng.standard_normal(size) * 10).astype(dt)
+    bcl = {b: [(int(rng.integers(0, 3)), int(rng.integers(0, 2)), int(rng.integers(0, 4)),
+                float(rng.choice([-1, 1, 2]))) for _ in range(3)] for b in (1, 2)}
+    g = make_grid(cn, comp, nb, n, bcl)
+    labs, written = lab_fill_all(cn, g, lo, hi, tens)
+    for b in range(4):
+        want, wdef = O.lab_fill(comp, nb, n, lo, hi, tens, bcl, b)
+        LC.compare_defined(labs[b], written[b], want, wdef)
+    g.close()
