@@ -642,18 +642,27 @@ static cn_status launch_fill(cn_grid *g, int comp, const cn_stencil *s, int b0, 
     const int64_t bulk = (int64_t)pz * L.n[0] * L.n[1] * (int64_t)sizeof(T);
     const int nbulk = !grow && bulk <= kBulkBytes ? (int)bulk : 0;
     const int64_t ghosts = (int64_t)pz * L.n[1] * (L.lo[0] + L.hi[0]) * (int64_t)sizeof(T);
-    // Whole runs pay where an x ghost is a good part of a row and its sectors
-    // (FP64, a sixth of the row and more) and many CTAs of some size hide the
-    // barrier between the ghosts' loads and their stores.  B200, FP64, ghosts
-    // as they come -> in runs: 4096 blocks of 32^3 with walls, three ghosts a
-    // side 597 -> 577 us, 512 of them 79 -> 77; 4096 of 16^3, two 105 -> 95,
-    // three 132 -> 130; 1728 of 24^3, three 137.6 -> 135.9; but 1728 of 32^3,
-    // two 220 -> 223; 4096 of 16^3, one 84.7 -> 88.1; 4096 of 8^3, one 19.2 ->
-    // 21.1; 512 of 16^3, three (1536 CTAs) 19.1 -> 21.1; FP32 32^3, three 204
-    // -> 230.
+    // Whole runs pay where x ghosts are a good part of a row (FP64, a sixth of
+    // it and more), planes and runs are whole sectors, and many CTAs of some
+    // size hide the barrier between the ghosts' loads and their stores.  B200,
+    // FP64, without BCs, ghosts as they come -> in runs: 4096 blocks of 32^3,
+    // three ghosts a side 597 -> 570 us; 4096 of 16^3, two 103 -> 90, three 131
+    // -> 125; 1728 of 24^3, two 114 -> 103, three 135 -> 130.  With walls it
+    // loses (4096 of 32^3, three 612 -> 622; 1728 of 24^3, three 147 -> 152):
+    // grids without BCs only, and not under capture, where they may be pushed
+    // later.  Without whole sectors: 8000 of 18 x 17 x 19, two 222 -> 228; with
+    // smaller ghosts: 4096 of 16^3, one 84.7 -> 88.1, 1728 of 32^3, two 220 ->
+    // 223; FP32 32^3, three 204 -> 230; with few CTAs: 512 of 16^3, three (1536)
+    // 19.1 -> 21.1.
     const bool bulk_planes = nbulk && (int64_t)L.n[0] * L.n[1] * (int64_t)sizeof(T) % 16 == 0;
-    const bool runs = one_pass && bulk_planes && sizeof(T) == 8 && L.n[0] >= 16 && 6 * (L.lo[0] + L.hi[0]) >= L.n[0] &&
-                      ghosts <= kGhostBytes && slabs * std::min(cnt, 65535) >= kRunCtas;
+    bool runs = one_pass && g->bc_count == 0 && bulk_planes && sizeof(T) == 8 && L.n[0] >= 16 &&
+                6 * (L.lo[0] + L.hi[0]) >= L.n[0] && E0 * L.n[1] % 4 == 0 && plane % 4 == 0 && ghosts <= kGhostBytes &&
+                slabs * std::min(cnt, 65535) >= kRunCtas;
+    if (runs && st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CN_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+        runs = cap == cudaStreamCaptureStatusNone;
+    }
     if (!grow) {
         static DeviceOnce once[4];
         cn_status r = runs           ? smem_opt_in(once[3], lab_fill_rows_kernel<T, true>, (size_t)kBulkBytes + kGhostBytes)

@@ -263,3 +263,47 @@ def test_lab_fill_large_planes_vs_oracle(cn, oracle_lib, dt, n, tens):
         want, wdef = O.lab_fill(comp, nb, n, lo, hi, tens, bcl, b)
         LC.compare_defined(labs[b], written[b], want, wdef)
     g.close()
+
+
+@pytest.mark.parametrize("nb,n", [((16, 16, 16), (16, 4, 4)), ((16, 16, 16), (18, 4, 3)), ((16, 16, 16), (24, 8, 5)),
+                                  ((16, 8, 8), (16, 24, 24)), ((16, 16, 16), (17, 4, 4)), ((16, 16, 16), (20, 3, 4))])
+def test_lab_fill_whole_runs_without_bcs_vs_oracle(cn, oracle_lib, nb, n):
+    """The same form in grids without BCs, which it is for: one and several
+    slabs a block, the last one short, and both sides of the rule (runs or
+    planes that are no whole sectors).  Then BCs pushed between the capture of
+    a call and its replay."""
+    import torch
+    O = oracle_lib
+    rng = np.random.default_rng(47)
+    lo, hi = (2, 1, 1), (2, 1, 1)
+    nblocks = int(np.prod(nb))
+    comp = rng.standard_normal(nblocks * O.block_stride(n, np.float64))
+    g = make_grid(cn, comp, nb, n, {})
+    some = sorted({0, nblocks - 1} | set(rng.integers(0, nblocks, size=40).tolist()))
+    st = cn.Core.Stencil((-2, -1, -1), (3, 2, 2), False)
+
+    def check(labs, bcl):
+        labs = labs.cpu().numpy()
+        for b in some:
+            want, wdef = O.lab_fill(comp, nb, n, lo, hi, False, bcl, b)
+            assert np.array_equal(labs[b][wdef], want[wdef])
+
+    out = cn.ops.load_labs(g, st)
+    torch.cuda.synchronize()
+    check(out, {})
+    push = lambda: [g.field(b).getBC().push_back(cn.BC.Dirichlet(0, 1, 0.25)) for b in some]
+    push()  # the table grows here, not after the capture
+    g.sync_bcs()
+    for b in some:
+        g.field(b).getBC().clear()
+    g.sync_bcs()
+    s = torch.cuda.Stream()
+    graph = cn.amr.Graph.capture(lambda: cn.ops.load_labs(g, st, out=out, stream=s), s)
+    push()
+    g.sync_bcs()
+    out.zero_()
+    torch.cuda.synchronize()
+    graph.launch(s)
+    s.synchronize()
+    check(out, {b: [(0, 1, O.BC_DIRICHLET, 0.25)] for b in some})
+    g.close()
