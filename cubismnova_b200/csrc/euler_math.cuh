@@ -26,6 +26,7 @@
 // Range.  The sums are formed as 4 s_k.  A jump J in the data gives 4 s ~ 13
 // J^2 and products of two squares ~ 5e3 J^8, which leaves the FP32 range
 // above J ~ 2e4 (a pressure jump of a fifth of a bar in SI units).  So in FP32
+// the sums are formed as s_k (4 s_k would leave the range at half the jump) and
 // t_k is formed from s_k * 2^-e, with e the mean of the binary exponents of
 // the largest and the middle s_k (rounded down).  Scaling by a power of two is
 // exact and cancels in every ratio below.  With it the dominant product
@@ -48,16 +49,14 @@ namespace euler {
 constexpr float kUnscaledMax = 1000.0f;
 
 template <typename T> struct K {
-    static constexpr T c133 = T(13.0 / 3.0);
-    static constexpr T eps4 = T(4e-6);
+    static constexpr T c133 = T(13.0 / 3.0), c1312 = T(13.0 / 12.0);
+    static constexpr T eps4 = T(4e-6), eps = T(1e-6);
     static constexpr T third = T(1.0 / 3.0);
     static constexpr T half = T(0.5);
 };
 
 __device__ __forceinline__ double dfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float dfma(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double dsqrt(double a) { return sqrt(a); }
-__device__ __forceinline__ float dsqrt(float a) { return sqrtf(a); }
 __device__ __forceinline__ double dabs(double a) { return fabs(a); }
 __device__ __forceinline__ float dabs(float a) { return fabsf(a); }
 __device__ __forceinline__ double dmax(double a, double b) { return fmax(a, b); }
@@ -95,7 +94,7 @@ __device__ __forceinline__ float rsqrt_pos(float x) { return rsqrtf(x); }
 // and the middle of the three (E_max + E_mid = E0 + E1 + E2 - E_min).  The
 // exponents come from the bit patterns (integer instructions only).  A NaN
 // or infinite s gives NaN states, and so do two sums above 2^127 (~1.7e38,
-// jumps ~5e18: the factor leaves the normal range there).
+// jumps ~1e19: the factor leaves the normal range there).
 __device__ __forceinline__ float weno5_scale(float s0, float s1, float s2)
 {
     const int e0 = __float_as_int(s0) >> 23, e1 = __float_as_int(s1) >> 23, e2 = __float_as_int(s2) >> 23;
@@ -162,7 +161,7 @@ __device__ __forceinline__ float2 range_scale(float2 s0, float2 s1, float2 s2)
 // the smoothness sums are
 //   4 s0 = 13/3 a0^2 + (a0 + 2 d12)^2 + 4 eps,   4 s1 = 13/3 a1^2 + (d12 + d23)^2 + 4 eps,
 //   4 s2 = 13/3 a2^2 + (a2 - 2 d23)^2 + 4 eps
-// (the factor 4 cancels in the weights), so the term q = 13/3 a^2 + 4 eps of
+// (the factor 4 cancels in the weights, the rescaled FP32 form goes without it), so the term q = 13/3 a^2 + 4 eps of
 // a second difference serves the three cells around it.  The candidates
 // differ from the middle one by third differences only,
 //   6 q0 - 6 q1 = -2 b01,  6 q2 - 6 q1 = -b12,  b01 = a1 - a0, b12 = a2 - a1,
@@ -188,16 +187,23 @@ __device__ __forceinline__ void weno5_run(const V (&u)[8], V (&wl)[3], V (&wr)[3
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
         a[k] = vsub(d[k + 1], d[k]);
-        q[k] = vfma(vmul(vset<V>(C::c133), a[k]), a[k], vset<V>(C::eps4));
+        q[k] = vfma(vmul(vset<V>(SCALED ? C::c1312 : C::c133), a[k]), a[k], vset<V>(SCALED ? C::eps : C::eps4));
     }
 #pragma unroll
     for (int k = 0; k < 5; ++k)
         b[k] = vsub(a[k + 1], a[k]);
 #pragma unroll
     for (int j = 0; j < 4; ++j) { // cell u[j + 2]
-        const V h0 = vfma(vset<V>(T(2)), d[j + 1], a[j]);
-        const V h1 = vadd(d[j + 1], d[j + 2]);
-        const V h2 = vfma(vset<V>(T(-2)), d[j + 2], a[j + 2]);
+        V h0, h1, h2;
+        if constexpr (SCALED) { // half of the others, to the bit
+            h0 = vfma(vset<V>(C::half), a[j], d[j + 1]);
+            h1 = vmul(vset<V>(C::half), vadd(d[j + 1], d[j + 2]));
+            h2 = vfma(vset<V>(-C::half), a[j + 2], d[j + 2]);
+        } else {
+            h0 = vfma(vset<V>(T(2)), d[j + 1], a[j]);
+            h1 = vadd(d[j + 1], d[j + 2]);
+            h2 = vfma(vset<V>(T(-2)), d[j + 2], a[j + 2]);
+        }
         V s0 = vfma(h0, h0, q[j]), s1 = vfma(h1, h1, q[j + 1]), s2 = vfma(h2, h2, q[j + 2]);
         if constexpr (SCALED) { // FP32: exact power-of-two rescaling
             const V sc = range_scale(s0, s1, s2);

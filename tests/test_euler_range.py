@@ -121,3 +121,35 @@ def test_device_rk3_step_si_units_matches_oracle(cn, oracle_lib, dtype):
     got = np.stack([U.download(c) for c in range(5)])
     assert_close(_cells(got, N, dtype), _cells(want, N, dtype),
                  TOL_F64 if dtype == np.float64 else TOL_F32_STATE, f"SI rk3 step {np.dtype(dtype).name}")
+
+
+def wave_state(P, dtype):
+    """Pressure waves of 5 cells, 0.6 P to 1.4 P, at uniform density and small
+    velocities: all three smoothness sums of a stencil are of the size of the
+    jumps' squares (a jump beside constant data, where one of them is the 1e-6
+    of the weights, ends the FP32 range at ~1e16)."""
+    z, y, x = np.meshgrid(*[np.arange(NB[d] * N[d]) for d in (2, 1, 0)], indexing="ij")
+    p = P * (1.0 + 0.4 * np.sin(2 * np.pi * (x + y + z) / 5))
+    rho = np.full(p.shape, 1.2)
+    vel = [0.01 * np.sqrt(GAMMA * P) * np.sin(2 * np.pi * (x + 2 * y + 3 * z + d) / 7) for d in range(3)]
+    E = p / (GAMMA - 1) + 0.5 * rho * (vel[0] ** 2 + vel[1] ** 2 + vel[2] ** 2)
+    stride = O.block_stride(N, np.dtype(dtype))
+    return np.stack([_to_blocks(q.astype(dtype), NB, N, stride) for q in (rho, *(rho * v for v in vel), E)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("P", [1e15, 9e18, 1.2e19])
+def test_device_fp32_rhs_up_to_the_sums_own_range(cn, oracle_lib, P):
+    """The FP32 smoothness sums are formed as in the oracle, so that the largest
+    of them (0.71 P^2 here) leaves the range where the oracle's does and not at
+    half the jumps: four times the sum does at P = 1.1e19."""
+    import torch
+    host = wave_state(P, np.float32)
+    U = _device_state(cn, host, np.float32)
+    R = cn.euler.like(U)
+    cn.euler.rhs(U, R)
+    torch.cuda.synchronize()
+    want = _cells(oracle_lib.euler_stage(host, None, NB, N, None, 0, 0.0, GAMMA, U.getCellSize()), N, np.float32)
+    got = _cells(np.stack([R.download(c) for c in range(5)]), N, np.float32)
+    assert np.isfinite(want).all() and np.isfinite(got).all()
+    assert_close(got, want, TOL_F32_RHS, f"wave rhs P={P:g} FP32")
