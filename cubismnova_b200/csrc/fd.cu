@@ -449,10 +449,23 @@ static cn_status launch_fd(cn_grid *u, int comp, cn_grid *o1, int c1, cn_grid *o
     const int N0 = u->n[0], N1 = u->n[1];
     if (plane_bytes(N0, N1, sizeof(T), OP == kDiv ? 3 : 1) > kMaxPlaneBytes)
         return fail(CN_ERR_UNSUPPORTED, "block too large for the fused stencil tile");
+    // An output on top of an input would be written while it is read: the march
+    // then reads a copy of the inputs.
+    const int nin = OP == kDiv ? 3 : 1;
+    auto on_input = [&](const cn_grid *o, int c, int n) { return o == u && c < comp + nin && comp < c + n; };
+    T *copy = nullptr;
+    if (on_input(o1, c1, 1) || on_input(o2, c2, 3)) {
+        const size_t bytes = (size_t)nin * u->comp_stride * sizeof(T);
+        CN_CUDA_TRY(cudaMallocAsync(&copy, bytes, st));
+        CN_CUDA_TRY(cudaMemcpyAsync(copy, p.in[0], bytes, cudaMemcpyDeviceToDevice, st));
+        for (int c = 0; c < 3; ++c) p.in[c] = copy + (OP == kDiv ? c * u->comp_stride : 0);
+    }
     // cells per thread along x: 16 bytes where rows are multiples of them
-    if (sizeof(T) == 4 && N0 % 4 == 0) return launch_march<T, OP, 16 / sizeof(T)>(u, p, st);
-    if (N0 % 2 == 0) return launch_march<T, OP, 2>(u, p, st);
-    return launch_march<T, OP, 1>(u, p, st);
+    if (sizeof(T) == 4 && N0 % 4 == 0) stt = launch_march<T, OP, 16 / sizeof(T)>(u, p, st);
+    else if (N0 % 2 == 0) stt = launch_march<T, OP, 2>(u, p, st);
+    else stt = launch_march<T, OP, 1>(u, p, st);
+    if (copy) CN_CUDA_TRY(cudaFreeAsync(copy, st));
+    return stt;
 }
 
 template <int OP>

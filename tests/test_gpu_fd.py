@@ -326,3 +326,38 @@ def test_faces_with_bcs_vs_oracle(cn, oracle_lib, nb, n, share):
     graph.launch(s)
     s.synchronize()
     check(bcl)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("nb,n", [((1, 1, 1), (8, 8, 8)), ((1, 1, 1), (12, 10, 9)), ((2, 1, 3), (7, 6, 5))])
+def test_outputs_on_top_of_inputs(cn, dtype, nb, n):
+    """Operators written onto components they read give what they give into
+    another grid."""
+    import torch
+    rng = np.random.default_rng(12)
+    g, lap, grad = (cn.Grid.Cartesian(nb, n, ncomp=k, dtype=dtype) for k in (4, 1, 3))
+    data = [rng.standard_normal(g.comp_stride).astype(dtype) for _ in range(4)]
+    cells = lambda grid, c: grid.blocks_view(grid.download(c))
+
+    def fresh():
+        for c in range(4):
+            g.upload(data[c], c)
+
+    fresh()
+    cn.ops.lap_grad(g, lap, grad, comp=1)
+    torch.cuda.synchronize()
+    want_l, want_g = cells(lap, 0), [cells(grad, d) for d in range(3)]
+    cn.ops.laplacian(g, g, comp=1, out_comp=1)
+    torch.cuda.synchronize()
+    assert np.array_equal(cells(g, 1), want_l)
+    fresh()
+    cn.ops.gradient(g, g, comp=1, out_comp=0)
+    torch.cuda.synchronize()
+    assert all(np.array_equal(cells(g, d), want_g[d]) for d in range(3))
+    fresh()
+    cn.ops.divergence(g, lap, comp=1)
+    torch.cuda.synchronize()
+    want_d = cells(lap, 0)
+    cn.ops.divergence(g, g, comp=1, out_comp=3)
+    torch.cuda.synchronize()
+    assert np.array_equal(cells(g, 3), want_d)
