@@ -69,7 +69,7 @@ struct cn_grid {
     // BC vectors [comp][block]
     std::vector<std::vector<std::vector<cn::HostBC>>> bcs;
     bool bc_dirty;
-    int64_t bc_count = 0; // BCs in all vectors
+    int64_t bc_count = 0, bc_count_x = 0; // BCs in all vectors, of those along x
     // device BC tables, component c at c*(nblocks+1) / c*nblocks
     int32_t *d_bc_off;
     cn::DevBC *d_bc_ent;

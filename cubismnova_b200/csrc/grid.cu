@@ -511,6 +511,7 @@ cn_status cn_bc_push(cn_grid *g, int comp, int block, int dir, int side, cn_bc_k
     }
     v.push_back(HostBC{dir, side, (int)kind, value});
     ++g->bc_count;
+    g->bc_count_x += dir == 0;
     g->bc_dirty = true;
     return CN_OK;
 }
@@ -536,14 +537,11 @@ cn_status cn_bc_clear(cn_grid *g, int comp, int block)
     if (!g || comp < 0 || comp >= g->ncomp || block < -1 || block >= g->nblocks) {
         return fail(CN_ERR_INVALID_ARGUMENT, "cn_bc_clear: bad grid, component or block");
     }
-    if (block < 0) {
-        for (auto &v : g->bcs[comp]) {
-            g->bc_count -= (int64_t)v.size();
-            v.clear();
-        }
-    } else {
-        g->bc_count -= (int64_t)g->bcs[comp][block].size();
-        g->bcs[comp][block].clear();
+    for (int b = block < 0 ? 0 : block; b < (block < 0 ? g->nblocks : block + 1); ++b) {
+        auto &v = g->bcs[comp][b];
+        g->bc_count -= (int64_t)v.size();
+        for (const HostBC &bc : v) g->bc_count_x -= bc.dir == 0;
+        v.clear();
     }
     g->bc_dirty = true;
     return CN_OK;

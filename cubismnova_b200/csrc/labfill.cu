@@ -645,19 +645,21 @@ static cn_status launch_fill(cn_grid *g, int comp, const cn_stencil *s, int b0, 
     // Whole runs pay where x ghosts are a good part of a row (FP64, a sixth of
     // it and more), planes and runs are whole sectors, and many CTAs of some
     // size hide the barrier between the ghosts' loads and their stores.  B200,
-    // FP64, without BCs, ghosts as they come -> in runs: 4096 blocks of 32^3,
+    // FP64, ghosts as they come -> in runs, without BCs: 4096 blocks of 32^3,
     // three ghosts a side 597 -> 570 us; 4096 of 16^3, two 103 -> 90, three 131
-    // -> 125; 1728 of 24^3, two 114 -> 103, three 135 -> 130.  With walls it
-    // loses (4096 of 32^3, three 612 -> 622; 1728 of 24^3, three 147 -> 152):
-    // grids without BCs only, and not under capture, where they may be pushed
-    // later.  Without whole sectors: 8000 of 18 x 17 x 19, two 222 -> 228; with
-    // smaller ghosts: 4096 of 16^3, one 84.7 -> 88.1, 1728 of 32^3, two 220 ->
-    // 223; FP32 32^3, three 204 -> 230; with few CTAs: 512 of 16^3, three (1536)
-    // 19.1 -> 21.1.
+    // -> 125; 1728 of 24^3, two 114 -> 103, three 135 -> 130.  Walls along y and z
+    // (their ghosts take a second pass): 601 -> 579, 106 -> 96, 133 -> 131, 115 ->
+    // 107, 139 -> 136, but 512 of 32^3, three 81 -> 84: twice as many CTAs there.
+    // With walls along x, whose blocks store as they come, it loses (4096 of
+    // 32^3, three 612 -> 622; 1728 of 24^3, three 147 -> 152), without whole
+    // sectors too (8000 of 18 x 17 x 19, two 222 -> 228), with smaller ghosts
+    // (4096 of 16^3, one 84.7 -> 88.1; 1728 of 32^3, two 220 -> 223), in FP32
+    // (32^3, three 204 -> 230) and with few CTAs (512 of 16^3, three, 1536 CTAs
+    // 19.1 -> 21.1).  Not under capture: BCs may be pushed later.
     const bool bulk_planes = nbulk && (int64_t)L.n[0] * L.n[1] * (int64_t)sizeof(T) % 16 == 0;
-    bool runs = one_pass && g->bc_count == 0 && bulk_planes && sizeof(T) == 8 && L.n[0] >= 16 &&
+    bool runs = one_pass && g->bc_count_x == 0 && bulk_planes && sizeof(T) == 8 && L.n[0] >= 16 &&
                 6 * (L.lo[0] + L.hi[0]) >= L.n[0] && E0 * L.n[1] % 4 == 0 && plane % 4 == 0 && ghosts <= kGhostBytes &&
-                slabs * std::min(cnt, 65535) >= kRunCtas;
+                slabs * std::min(cnt, 65535) >= (g->bc_count ? 2 * kRunCtas : kRunCtas);
     if (runs && st) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         CN_CUDA_TRY(cudaStreamIsCapturing(st, &cap));

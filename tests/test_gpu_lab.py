@@ -266,12 +266,13 @@ def test_lab_fill_large_planes_vs_oracle(cn, oracle_lib, dt, n, tens):
 
 
 @pytest.mark.parametrize("nb,n", [((16, 16, 16), (16, 4, 4)), ((16, 16, 16), (18, 4, 3)), ((16, 16, 16), (24, 8, 5)),
-                                  ((16, 8, 8), (16, 24, 24)), ((16, 16, 16), (17, 4, 4)), ((16, 16, 16), (20, 3, 4))])
+                                  ((16, 8, 8), (16, 24, 24)), ((16, 16, 16), (17, 4, 4)), ((16, 16, 16), (20, 3, 4)),
+                                  ((32, 16, 16), (16, 4, 4))])
 def test_lab_fill_whole_runs_without_bcs_vs_oracle(cn, oracle_lib, nb, n):
-    """The same form in grids without BCs, which it is for: one and several
+    """The same form in grids without BCs along x, which it is for: one and several
     slabs a block, the last one short, and both sides of the rule (runs or
-    planes that are no whole sectors).  Then BCs pushed between the capture of
-    a call and its replay."""
+    planes that are no whole sectors); without BCs and with some along y and z.
+    Then BCs along x pushed between the capture of a call and its replay."""
     import torch
     O = oracle_lib
     rng = np.random.default_rng(47)
@@ -291,6 +292,16 @@ def test_lab_fill_whole_runs_without_bcs_vs_oracle(cn, oracle_lib, nb, n):
     out = cn.ops.load_labs(g, st)
     torch.cuda.synchronize()
     check(out, {})
+    walls = {b: [(1, 0, O.BC_ABSORBING, 0.0), (2, 1, O.BC_SYMMETRY, -1.0)] for b in some}
+    for b in some:
+        g.field(b).getBC().push_back(cn.BC.Absorbing(1, 0))
+        g.field(b).getBC().push_back(cn.BC.Symmetry(2, 1, -1.0))
+    out.zero_()
+    cn.ops.load_labs(g, st, out=out)
+    torch.cuda.synchronize()
+    check(out, walls)
+    for b in some:
+        g.field(b).getBC().clear()
     push = lambda: [g.field(b).getBC().push_back(cn.BC.Dirichlet(0, 1, 0.25)) for b in some]
     push()  # the table grows here, not after the capture
     g.sync_bcs()
