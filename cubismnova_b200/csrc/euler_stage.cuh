@@ -1,9 +1,10 @@
 // euler_stage.cuh -- the fused lab + WENO5-JS + Rusanov + flux-divergence +
 // SSP-RK3 stage computation of one 8x8x8 tile, shared by the uniform-grid
 // kernel (euler.cu) and the AMR block kernel (amr.cu).  Where the tile comes
-// from and how halo cells outside the tile's block are resolved is a policy
-// (`Src`): the uniform grid uses the Cartesian lab resolution of FieldLab,
-// the AMR layout its own interface ghost fill.
+// from and how its halo cells arrive differs: a uniform grid's tile (CartSrc)
+// takes them as TMA boxes, and by a rule per face where the face carries a BC or
+// a skipped neighbour (what FieldLab's lab holds there); an AMR block's by
+// asynchronous copies and its own interface ghost fill (the policy `Src`).
 #pragma once
 
 #include "cn_fastdiv.h"
@@ -91,8 +92,8 @@ struct TileMaps {
     CUtensorMap core, hx, hy, hz;
 };
 
-// Uniform Cartesian grid: tiles in block order, halo cells through the
-// FieldLab lab resolution (cn::lab_value) with each component's BC vector.
+// Uniform Cartesian grid: tiles in block order; which sides of a tile are boxes
+// of one block's cells, from each component's BC tables.
 struct CartSrc {
     LabGeom L;
     BcView bc[5];
@@ -119,10 +120,10 @@ struct CartSrc {
     }
     // By the lanes of one warp: bit 2 d + s of the result is set when side
     // (d, s) of the tile lies outside its block and is not a plain copy of the
-    // neighbour block's cells in all five components (what cn::lab_value
-    // gives: no component's block carries a BC or skip flag (mode byte 0), or
-    // the face carries no BC other than Base and no skip flag in any
-    // component, BcView::faces).
+    // neighbour block's cells in all five components, as in a lab: no
+    // component's block carries a BC or skip flag (mode byte 0), or the face
+    // carries no BC other than Base and no skip flag in any component
+    // (BcView::faces).
     template <typename T> __device__ __forceinline__ unsigned slow_sides(const TileInfo<T> &t) const
     {
         const int lane = threadIdx.x & 31, c = lane < 5 ? lane : 0;

@@ -50,8 +50,10 @@ template <> struct Arith<float> {
     static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 };
 
-// Largest block the operators take: a plane of it with the planes and rows
-// around it, each array padded to 4 elements, within 100 KB.
+// Largest block plane the operators take, a limit of the interface that the
+// kernel does not need: a plane with the planes and rows around it, each array
+// padded to 4 elements, within 100 KB (square planes up to 36 cells for the
+// FP64 divergence, 64 for an FP64 Laplacian).
 constexpr size_t kMaxPlaneBytes = 100 * 1024 - 128;
 static size_t plane_bytes(int n0, int n1, size_t es, int nc)
 {

@@ -13,10 +13,9 @@
 // form of labs without edges and corners, lab_fill_kernel walks row by row
 // (tensorial labs, and labs with more ghost rows than the former's table);
 // node and face grids (lab_fill_grow_kernel) take per-cell resolution.  Stores
-// are coalesced along the lab's rows.  The stencil kernels fuse the same
-// resolution into their shared-memory staging; this kernel gives the
-// reference's FieldLab contents for user stencils and the bit-exact comparison
-// with it.
+// are coalesced along the lab's rows.  The stencil kernels read what their labs
+// would hold without making them; these kernels give the reference's FieldLab
+// contents for user stencils and the bit-exact comparison with it.
 #include "cn_fastdiv.h"
 #include "cn_internal.h"
 #include "cn_tma.cuh"
@@ -28,7 +27,7 @@ namespace cn {
 
 constexpr int KL = 4;              // cells per thread resolved before their loads
 constexpr int KLM = 8;             // cells per thread in flight in the one-pass form
-constexpr int KLO = 8;              // own cells in flight per thread of the row form without the copy
+constexpr int KLO = 8;             // own cells in flight per thread of the row form without the copy
 constexpr int KLR = 3;             // rows in flight per thread of the row form
 constexpr int KLX = 3;             // x ghosts in flight per thread of the row form
 constexpr int kBulkBytes = 24576;  // largest bulk copy of a slab's block planes
@@ -126,7 +125,7 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// a row of class 2 or 3: the source of its first cell and its first cell's
+// a y- or z-ghost row: the source of its first cell and its first cell's
 // offset in the lab
 template <typename T> struct alignas(16) RowSrc {
     int64_t idx; // of the first cell in the component
@@ -145,7 +144,7 @@ struct LabDivs {
 };
 
 // lab coordinates of x ghost u of the inside rows
-__device__ __forceinline__ void class1_cell(const LabDivs &dv, int u, int gx, int n0, int n1, int lo0, int lo1, int zi0,
+__device__ __forceinline__ void x_ghost_cell(const LabDivs &dv, int u, int gx, int n0, int n1, int lo0, int lo1, int zi0,
                                             int &x, int &y, int &z)
 {
     const int r = dv.gx.div(u), zp = dv.n1.div(r);
@@ -235,11 +234,9 @@ __device__ __forceinline__ void lab_store1(const T *__restrict__ comp, const Lab
     o[dst] = x;
 }
 
-// Cell grids with non-tensorial labs whose ghost rows (classes 2 and 3
-// below) fit in shared memory (kRows per slab), the common case: the
-// one-pass form.  It is a kernel of its own so that the general form's
-// per-class loops do not set its register count (it holds none of their
-// spill slots and runs at kRowsCtas CTAs per SM).
+// Cell grids with non-tensorial labs whose y- and z-ghost rows fit in shared
+// memory (kRows per slab), the common case: the one-pass form, at kRowsCtas
+// CTAs per SM.
 template <typename T, bool RUNS>
 __global__ void __launch_bounds__(256, kRowsCtas)
     lab_fill_rows_kernel(const T *__restrict__ comp, LabGeom L, BcView bc, int block_begin, int pz, LabDivs dv,
@@ -269,7 +266,7 @@ __global__ void __launch_bounds__(256, kRowsCtas)
     __shared__ RowSrc<T> rows[kRows];
     // One pass over all three kinds of plain copies, KLM loads in flight
     // per thread: the block's own cells, the x ghosts behind clear faces
-    // and the rows (classes 2, 3) whose source is a plain cell run.  The
+    // and the ghost rows whose source is a plain cell run.  The
     // rows are resolved first; cells that need BC chains or skips are
     // left to a second pass.
     const int A = nin * n1 * n0, B = nin * n1 * gx, tot = A + B + nrows * n0;
@@ -313,7 +310,7 @@ __global__ void __launch_bounds__(256, kRowsCtas)
                 idx[k] = bbase + t;
             } else if (t < A + B) {
                 int x, y, z;
-                class1_cell(dv, t - A, gx, n0, n1, L.lo[0], L.lo[1], zi0, x, y, z);
+                x_ghost_cell(dv, t - A, gx, n0, n1, L.lo[0], L.lo[1], zi0, x, y, z);
                 const int q0 = x - L.lo[0], r0 = q0 < 0 ? -1 : 1;
                 if (faces & (r0 < 0 ? 1 : 2)) {
                     deferred = true;
@@ -385,7 +382,7 @@ __global__ void __launch_bounds__(256, kRowsCtas)
             int dst[1] = {-1};
             if (t < A + B) {
                 int x, y, z;
-                class1_cell(dv, t - A, gx, n0, n1, L.lo[0], L.lo[1], zi0, x, y, z);
+                x_ghost_cell(dv, t - A, gx, n0, n1, L.lo[0], L.lo[1], zi0, x, y, z);
                 if (!(faces & (x < L.lo[0] ? 1 : 2))) continue;
                 lab_resolve<T, false>(L, bc, mode, block, bx, by, bz, x - L.lo[0], y - L.lo[1], z - L.lo[2], abc,
                                       src[0]);

@@ -233,7 +233,7 @@ static WgGeo wgrad_geo(int B, int So, int ctas, size_t *smem)
                 g.bricks[1] = (So + g.BY - 1) / g.BY;
                 g.bricks[2] = (So + g.BZ - 1) / g.BZ;
                 g.total = B * g.bricks[0] * g.bricks[1] * g.bricks[2];
-                            const double cost = (double)((g.total + ctas - 1) / ctas) *
+                const double cost = (double)((g.total + ctas - 1) / ctas) *
                                         (7.5 * g.BZ * g.KP + bytes / 40.0 + 2500.0) +
                                     16.0 * (g.total < ctas ? g.total : ctas);
                 if (best.total == 0 || cost < least) {
@@ -589,7 +589,8 @@ __host__ __device__ inline uint32_t z_runs(int B, int So) { return (uint32_t)B *
 // dz) for its three taps, a tap's weights serve 4 cells.  (Straight from global
 // memory the threads' 128-byte steps along x cost a cache line per lane and
 // load.)  16-byte chunks of a row lie 9 apart every 8, so that 8 lanes read from
-// distinct banks.
+// distinct banks.  The planes arrive one after the other (all at once: 73 us
+// instead of 70).
 constexpr int L3_NT = 128, L3_QX = 16; // threads; most quads of cells along x
 struct L3Geo {
     int qx, yb;        // quads along x and rows of a CTA

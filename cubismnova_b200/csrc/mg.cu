@@ -13,9 +13,11 @@
 // ... -> 1^3), so fine block b maps onto coarse block b.  V-cycle fields are
 // FP32; the outer defect correction keeps the fine solution, its residual and
 // the residual norm in FP64, because an FP32 solution cannot be represented
-// accurately enough for a 1e-8 relative residual.  Neighbour values come from
-// the same lab resolution as every other stencil (periodic block wrap, and the
-// grid's BCs if any); halo cells inside a block are plain cached loads.
+// accurately enough for a 1e-8 relative residual.  Fields without BCs, which the
+// levels' own are, take the marching kernels of mg_march.cuh: periodic
+// neighbours at constant offsets.  Fields with BCs (the FP64 solution's grid, or
+// BCs pushed onto a level's grid) take the tile kernels below, which stage a
+// tile with its halo through the lab.
 #include "cn_internal.h"
 #include "mg_march.cuh"
 #include "mg_tile.cuh"

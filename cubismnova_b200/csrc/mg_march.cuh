@@ -5,7 +5,8 @@
 // planes and marches up it: p of planes z - 1 and z and the z face means stay
 // in registers, everything else is a cached load issued before anything waits.
 // Fields with BCs take the tile kernels of mg.cu.  Operations and their order
-// are those of the tile kernels (op7_tile), uncontracted, so results are bit for bit the same.
+// are those of the tile kernels (op7_tile), uncontracted, so results are bit
+// for bit the same.
 //
 // The operator is stored as one harmonic mean per face: per cell the means
 // across its lower x, y, z faces, and per block those across its upper

@@ -1,7 +1,8 @@
 // mg_tile.cuh -- tiles of a block for the level operators of the multigrid
-// solver and the learned smoother's features: tile geometry, asynchronous
-// staging of a tile plus its one-cell halo into shared memory, and the
-// variable-coefficient 7-point operator evaluated from the staged region.
+// solver on fields with BCs and for the learned smoother's features: tile
+// geometry, asynchronous staging of a tile plus its one-cell halo into shared
+// memory, and the variable-coefficient 7-point operator evaluated from the
+// staged region and the level's face means.
 #pragma once
 
 #include "cn_fastdiv.h"
@@ -83,7 +84,7 @@ __device__ __forceinline__ T op7_tile(const T *sp, int u, const int (&st)[3], co
 // The level operators work on tiles of one block: up to 32 x 8 x 4 cells
 // (extents: the largest divisors of the block's cells within those caps,
 // even when the block's extent is even, so fine tiles hold whole coarse
-// cells).  A CTA stages its tile plus a one-cell halo of p and k into shared
+// cells).  A CTA stages its tile plus a one-cell halo of p into shared
 // memory (halo cells outside the block through cn::lab_fetch: periodic
 // neighbour or the BC chain), then every thread evaluates its cells from
 // shared memory with the same operation order as the per-cell form.
