@@ -220,7 +220,7 @@ class C1:
     # dram__bytes_write.sum, mean of 3 launches) of this workload: the field
     # (16.8 MB) is read from DRAM, the 67 MB of results mostly stay dirty in the
     # 126 MB L2 and are written back during the flush that follows
-    traffic_per_cell_step = 11.12
+    traffic_per_cell_step = 11.55
     traffic_source = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of fd_kernel on this workload, "
                       "mean of 3 launches; results stay dirty in L2 and are written back during the flush")
 
@@ -328,7 +328,7 @@ class Euler:
     # DRAM bytes per cell per step of the three stage launches from one ncu
     # capture on 8x8x4 blocks of 32^3 (8.4 M cells, inputs 5x larger than L2),
     # scaled to the workload's cells: traffic grows with the cells processed
-    traffic_per_cell_step = 327.80
+    traffic_per_cell_step = 329.25
     traffic_source = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 3 stage_kernel launches "
                       "of one step on 8x8x4 blocks of 32^3, per cell, scaled by the workload's cells")
     sample_nb = (4, 4, 4)  # CPU sample grid: 64 blocks of the same block size
@@ -520,7 +520,7 @@ class C4(Euler):
     bytes_per_cell_step = (80 + 120 + 120) // 2
     # capture on 8x8x4 blocks (168 MB of state, comparable to L2, so slightly
     # under the full-size figure)
-    traffic_per_cell_step = 156.84
+    traffic_per_cell_step = 156.81
 
 
 class C3:
@@ -540,9 +540,9 @@ class C3:
     stages = 3
     launches_per_step = 3
     bytes_per_cell_step = 320
-    traffic_per_cell_step = 394.0
+    traffic_per_cell_step = 387.8
     traffic_source = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 3 stage_kernel launches of one "
-                      "step on this layout (5302 MB per step), per cell and scaled to a launch")
+                      "step on this layout (5219 MB per step), per cell and scaled to a launch")
     nb, n = ("amr", "amr")
 
     def __init__(self):
@@ -690,7 +690,7 @@ class C5:
     # Jacobi damping: 6/7 minimises the largest amplification of the
     # high-frequency error modes for the 7-point operator in 3-D (standard
     # local Fourier analysis of damped Jacobi); measured on this problem: 15
-    # V(2,2) cycles, 23.4 ms, against 16 cycles, 25.0 ms at omega 0.8
+    # V(2,2) cycles, 10.3 ms, against 16 cycles, 11.0 ms at omega 0.8
     omega = 6.0 / 7.0
     nu = (2, 2)  # pre- and post-smoothing sweeps (bench.py --mg-nu, --mg-omega)
     name = "c5"
@@ -725,17 +725,22 @@ class C5:
         self.updates_per_step = self.cells
         self.cycles, self.relres = self.mg.solve(self.f, self.p64, self.rtol, max_cycles=100)
         torch.cuda.synchronize()
-        # kernels per solve: initial residual (2), per cycle 6 per non-coarsest
-        # level + coarsest CG + accumulate + residual (2)
         L = self.mg.nlevels
-        self.gpu_launches_per_step = 2 + self.cycles * (6 * (L - 1) + 4)
-        # compulsory HBM bytes per fine cell (FP32 4 B, FP64 8 B): a V(2,2)
-        # level pass moves 81 B per level cell (Jacobi from zero 12, Jacobi 16
-        # x 3, residual restriction 12.5, prolongation 8.5), the coarsest CG
-        # 12 B, accumulate + FP64 residual 40 B per fine cell; 28 B once
         ncl = [self.cells // 8 ** l for l in range(L)]
-        per_cycle = 81 * sum(ncl[:-1]) + 12 * ncl[-1] + 40 * ncl[0]
-        self.bytes_per_cell_step = (28 * self.cells + self.cycles * per_cycle) / self.cells
+        # kernels per solve: the initial residual; per cycle, on each level of
+        # more than 4096 cells, nu1 - 1 pre-sweeps (the first one rides on the
+        # kernel that makes the right-hand side), restriction, prolongation and
+        # nu2 post-sweeps, one launch for the smaller levels, and the residual
+        per_level = max(self.nu[0] - 1, 0) + 2 + self.nu[1]
+        self.gpu_launches_per_step = 1 + self.cycles * (per_level * sum(c > 4096 for c in ncl) + 2)
+        # compulsory HBM bytes per cell (FP32 4 B, FP64 8 B; p, k, f of a cell
+        # read once by a pass and its result written): a V(2,2) level pass moves
+        # 69.5 B per level cell (three sweeps 16 each, restriction 13 with the
+        # coarse right-hand side and first sweep, prolongation 8.5), the coarsest
+        # solve 12 B, per fine cell the FP64 residual with the next cycle's first
+        # sweep 24 B and the accumulation 16 B; 32 B once
+        per_cycle = 69.5 * sum(ncl[:-1]) + 12 * ncl[-1] + 40 * ncl[0]
+        self.bytes_per_cell_step = (32 * self.cells + self.cycles * per_cycle) / self.cells
         self.learned = self._learned() if self.with_learned else None
         self.desc = self.desc + f"; {L} levels, {self.cycles} cycles (relres {self.relres:.2e})"
         self.h_f = self.h_p = None
@@ -879,12 +884,12 @@ class LAB:
     # of the written lab cells, (32^3 + 6 x 3 x 32^2) / 32^3 x 8 B = 12.5 B;
     # ghost cells read from neighbours are re-reads and not counted
     bytes_per_cell_step = 5 * (8 + 8 * (32 ** 3 + 6 * 3 * 32 ** 2) / 32 ** 3)
-    # DRAM bytes per cell of one ncu capture of a launch on 8x8x8 blocks of
-    # 32^3 (147.6 MB read + 163.6 MB written for 16.8 M cells, mean of 3
-    # launches), times the 5 launches of a step; traffic grows with the
-    # blocks processed
-    traffic_per_cell_step = 92.7
-    traffic_source = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of lab_fill_rows_kernel on 8x8x8 blocks "
+    # DRAM bytes per cell of one ncu capture of a launch on 16x8x8 blocks of
+    # 32^3 (328.6 MB read + 380.7 MB written for 33.6 M cells, mean of 3
+    # launches; fewer than 631 blocks take another form of the kernel), times
+    # the 5 launches of a step; traffic grows with the blocks processed
+    traffic_per_cell_step = 105.7
+    traffic_source = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of lab_fill_rows_kernel on 16x8x8 blocks "
                       "of 32^3 (mean of 3 launches), per cell, times the 5 launches of a step")
     cpu_nb = (8, 8, 4)
 
